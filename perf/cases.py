@@ -305,8 +305,8 @@ def work(case):
         total = 3 * e * n + 3 * e * edges
         if kind == "hop":      # the relabel reads seeds, rows and columns and writes rows, columns and the frontier
             total += e * n + 4 * e * edges + e * (n + 0.5 * edges)
-        else:                  # every weight of a row decides; rows met along edges are longer than the mean
-            total += 4 * n * 20 * case["deg"]
+        else:                  # every weight of a row decides; rows met along edges are 11 to 15 times the mean
+            total += 4 * n * 13 * case["deg"]
         return {"bytes": total, "flops": 0}
     return {"bytes": _block_bytes(case) * (BATCHES if kind == "pipeline" else 1), "flops": 0}
 
