@@ -31,10 +31,10 @@
 //     insertion; keys are compared in the log domain, log(u)/w, which orders
 //     exactly like u^(1/w) but does not underflow for small weights.  Rows
 //     are read in 512-edge windows (16 loads in flight per lane) and rows longer
-//     than 4096 edges are shared by the eight warps of the CTA and merged.
+//     than that are shared by the eight warps of the CTA and merged.
 //   * weighted sampling with replacement builds no cumulative array in global
-//     memory: the row is streamed twice through a warp scan and each draw is
-//     resolved by a ballot in the 32-edge window it falls into.
+//     memory: the row is summed once in windows of 512 edges, and each draw is
+//     resolved by ballots in the stretch, the window and the 32 edges it falls into.
 //   * counts, offsets and the total come from ONE plan kernel: every CTA scans
 //     its 256 seeds and the CTA that finishes last (an atomic ticket, nobody
 //     waits) scans the per-tile sums; the total goes to a caller-supplied
@@ -356,32 +356,77 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
 }
 
 // ---------------------------------------------------------------------------
-// weighted sampling: one warp per seed; rows longer than HUB_DEG edges are then
+// weighted sampling: one warp per seed; rows longer than LONG_ROW edges are then
 // taken on by all eight warps of the CTA together
 // ---------------------------------------------------------------------------
+// a weight of a row that straddles storage regions (at most one row per boundary); out of line, because its
+// address arithmetic, inlined at every load, made the sampling kernel 300 KB of code
+__device__ __noinline__ float straddling_weight(const dgs_chunk_desc* probs, int64_t e) {
+  return load_at<float>(*probs, 2, e);
+}
+
 struct RowWeights {
   const dgs_chunk_desc& probs;
   const float* direct;  // non-null when the whole row lies in one storage region
   int64_t rb;
   __device__ __forceinline__ float operator()(int64_t e) const {
-    return direct != nullptr ? direct[e] : load_at<float>(probs, 2, rb + e);
+    return direct != nullptr ? direct[e] : straddling_weight(&probs, rb + e);
+  }
+  // COUNT weights at base + 32 j + lane, all loads in flight together; 0 past the row's end
+  template <int COUNT>
+  __device__ __forceinline__ void load(float (&v)[COUNT], int64_t base, int64_t deg, int l) const {
+    if (direct != nullptr) {
+      const float* p = direct + base + l;
+      const int left = deg - base - l < 32 * COUNT ? static_cast<int>(deg - base - l) : 32 * COUNT;  // <= 0: none
+#pragma unroll
+      for (int j = 0; j < COUNT; ++j) v[j] = j * 32 < left ? p[j * 32] : 0.f;
+    } else {
+#pragma unroll
+      for (int j = 0; j < COUNT; ++j) v[j] = base + j * 32 + l < deg ? straddling_weight(&probs, rb + base + j * 32 + l) : 0.f;
+    }
   }
 };
+__device__ __forceinline__ RowWeights row_weights(const dgs_chunk_desc& probs, int64_t rb, int64_t deg) {
+  int64_t run;
+  const char* wp = resolve(probs, 2, rb, &run);
+  return RowWeights{probs, run >= deg ? reinterpret_cast<const float*>(wp) : nullptr, rb};
+}
 
-constexpr int64_t HUB_DEG = 4096;   // rows above this are scanned by the whole CTA
-constexpr int ARES_QUADS = 4;       // Philox blocks per lane and 512-edge window
+constexpr int64_t HUB_DEG = 4096;  // with replacement: rows above this are left to the whole CTA
+constexpr int WEIGHTED_WARPS = SAMPLE_BLOCK / 32;
+
+// Sorts 32 (key, position) pairs, one per lane, by (key descending, position ascending).  Out of line: called from
+// three places, 15 exchange steps each.
+__device__ __noinline__ float2 sort32(float key, float position) {
+  const int l = threadIdx.x & 31;
+  uint32_t pos = __float_as_uint(position);
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+    for (int d = size >> 1; d > 0; d >>= 1) {
+      const float ok = __shfl_xor_sync(FULL_MASK, key, d);
+      const uint32_t op = __shfl_xor_sync(FULL_MASK, pos, d);
+      const bool mine_first = key > ok || (key == ok && pos < op);
+      const bool want_first = ((l & d) == 0) == ((l & size) == 0);
+      if (mine_first != want_first) {
+        key = ok;
+        pos = op;
+      }
+    }
+  }
+  return make_float2(key, __uint_as_float(pos));
+}
 
 // The running top-k of one warp: lane j holds the j-th largest key and its
-// position in the row; `thresh` is the key held by lane k-1 (the entry bar).
+// place in the warp's share of the row; `thresh` is the key held by lane k-1 (the entry bar).
+template <typename P>
 struct TopK {
   float key;
-  int64_t pos;
+  P pos;
   float thresh;
-  __device__ __forceinline__ void insert(float nk, int64_t np, int l, int k) {
-    // warp-uniform call with nk > thresh; the keys >= nk form a prefix of the lanes
-    const int p = __popc(__ballot_sync(FULL_MASK, key >= nk));  // p <= k-1
+  __device__ __forceinline__ void shift_in(float nk, P np, int p, int l, int k) {
     const float up_key = __shfl_up_sync(FULL_MASK, key, 1);
-    const int64_t up_pos = __shfl_up_sync(FULL_MASK, pos, 1);
+    const P up_pos = __shfl_up_sync(FULL_MASK, pos, 1);
     if (l > p) {
       key = up_key;
       pos = up_pos;
@@ -391,64 +436,223 @@ struct TopK {
     }
     thresh = __shfl_sync(FULL_MASK, key, k - 1);
   }
+  __device__ __forceinline__ void insert(float nk, P np, int l, int k) {
+    // warp-uniform call with nk > thresh; the keys >= nk form a prefix of the lanes
+    shift_in(nk, np, __popc(__ballot_sync(FULL_MASK, key >= nk)), l, k);  // p <= k-1
+  }
+  // one key per lane: the order that 32 single insertions give
+  __device__ __forceinline__ void fill(float nk, uint32_t np, int k) {
+    const float2 sorted = sort32(nk, __uint_as_float(np));
+    key = sorted.x;
+    pos = __float_as_uint(sorted.y);
+    thresh = __shfl_sync(FULL_MASK, key, k - 1);
+  }
 };
+using ShareList = TopK<uint32_t>;  // places within a share: 512 per window
 
-// A-Res over one window of 512 edges starting at `base`: key = log(u)/w, which
-// orders like u^(1/w).  The 16 weights a lane needs are loaded together (2 KB in
-// flight per warp); the uniforms come from one Philox block per four edges,
-// addressed by (seed position, edge index) so that the result does not depend on
-// which warp scans the window.
-__device__ __forceinline__ void ares_window(TopK& top, const RowWeights& W, int64_t base, int64_t deg,
-                                            uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k) {
-  const float NEG_INF = __int_as_float(0xff800000);
+// Floats in an order-preserving integer form (for atomicMax in shared memory); its own inverse.
+__device__ __forceinline__ int ordered_float(float f) {
+  const int i = __float_as_int(f);
+  return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ float float_of_ordered(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+
+__device__ __forceinline__ float ares_key(uint32_t word, float w) {
   const float FLOOR_ZERO_W = -3.402823466e+38f;  // weight <= 0: behind every positive weight
   const float FLOOR_POS_W = -3.0e+38f;           // clamp for positive weights
-  float wv[4 * ARES_QUADS];
-#pragma unroll
-  for (int j = 0; j < 4 * ARES_QUADS; ++j) {
-    const int64_t e = base + j * 32 + l;
-    wv[j] = (e < deg) ? W(e) : 0.f;
-  }
-#pragma unroll
-  for (int q = 0; q < ARES_QUADS; ++q) {
-    if (base + q * 128 >= deg) break;  // warp-uniform
-    const uint64_t ctr = static_cast<uint64_t>((base >> 2) + q * 32) + static_cast<uint64_t>(l);
-    const Philox4 r = philox4x32_10(key ^ (static_cast<uint64_t>(TAG_ARES) << 32), i_lo, i_hi,
-                                    static_cast<uint32_t>(ctr), static_cast<uint32_t>(ctr >> 32));
-    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t e0 = base + (q * 4 + j) * 32;  // first edge of this group of 32
-      const float w = wv[q * 4 + j];
-      float ck = NEG_INF;
-      if (e0 + l < deg)
-        ck = (w > 0.f) ? fmaxf(__fdividef(__logf(unit_float(rw[j])), w), FLOOR_POS_W) : FLOOR_ZERO_W;
-      unsigned cand = __ballot_sync(FULL_MASK, ck > top.thresh);
-      while (cand) {
-        const int src = __ffs(cand) - 1;
-        cand &= cand - 1;
-        const float nk = __shfl_sync(FULL_MASK, ck, src);
-        if (nk > top.thresh) top.insert(nk, e0 + src, l, k);  // the bar may have risen since the ballot
-      }
+  float ck = fmaxf(__fdividef(__logf(unit_float(word)), w), FLOOR_POS_W);
+  asm volatile("" : "+f"(ck));  // computed by every lane: a branch around it costs more than the few it would spare
+  return (w > 0.f) ? ck : FLOOR_ZERO_W;
+}
+
+// The next key below: "at or above x" as "above key_below(x)".
+__device__ __forceinline__ float key_below(float x) {
+  return x == __int_as_float(0xff800000) ? x : float_of_ordered(ordered_float(x) - 1);
+}
+
+__device__ __forceinline__ Philox4 ares_words(uint64_t key, uint32_t i_lo, uint32_t i_hi, int64_t e0, int l) {
+  // one Philox block per four edges, addressed by (seed position, edge index): the result does not depend on
+  // which warp scans the window
+  const uint64_t ctr = static_cast<uint64_t>(e0 >> 2) + static_cast<uint64_t>(l);
+  return philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(ctr), static_cast<uint32_t>(ctr >> 32));
+}
+
+// `entry`: only keys above it are of interest (the list's own bar or a higher one the caller knows of)
+__device__ __forceinline__ void insert_above(ShareList& top, float& entry, float ck, uint32_t place, int l, int k) {
+  unsigned cand = __ballot_sync(FULL_MASK, ck > entry);
+  while (cand) {
+    const int src = __ffs(cand) - 1;
+    cand &= cand - 1;
+    const float nk = __shfl_sync(FULL_MASK, ck, src);
+    if (nk > entry) {  // the bar may have risen since the ballot
+      top.insert(nk, place + src, l, k);
+      entry = fmaxf(entry, top.thresh);
     }
   }
 }
 
-// One warp's share of a row: windows base0, base0 + stride, ...
+constexpr int ARES_EDGES = 512;  // edges per window
+constexpr int ARES_ITEMS = ARES_EDGES / 32;
+
+// The first 512 edges of a row.  Every lane computes its 16 keys; the k-th largest of the 32 lane maxima is a bar that at
+// least k keys reach and, for k well below 32, few more than k (expected -32 ln(1 - k/32) of them: 12 at k = 10, 22
+// at k = 16), so those are packed into one per lane and sorted at once -- 15 exchange steps, where inserting one
+// after the other is a chain of ~28 insertions of ~150 cycles each for k = 10.  With more than 32 at the bar (large
+// k, ties) they are inserted one by one after all.
+__device__ __forceinline__ void ares_first_window(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key,
+                                                  uint32_t i_lo, uint32_t i_hi, int l, int k, float* pack_key,
+                                                  uint16_t* pack_at) {
+  const float NEG_INF = __int_as_float(0xff800000);
+  float ck[ARES_ITEMS];
+  W.load(ck, 0, deg, l);
+  float best = NEG_INF;
+  const int left = deg < ARES_EDGES ? static_cast<int>(deg) - l : ARES_EDGES;
+#pragma unroll
+  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
+    if (q * 128 < deg) {  // warp-uniform
+      const Philox4 r = ares_words(key, i_lo, i_hi, q * 128, l);
+      const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+      for (int j = 4 * q; j < 4 * q + 4; ++j) {
+        ck[j] = j * 32 < left ? ares_key(rw[j - 4 * q], ck[j]) : NEG_INF;
+        best = fmaxf(best, ck[j]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 4 * q; j < 4 * q + 4; ++j) ck[j] = NEG_INF;
+    }
+  }
+  if (deg <= 32) {
+    top.fill(ck[0], static_cast<uint32_t>(l), k);
+    return;
+  }
+  ShareList maxima;
+  maxima.fill(best, static_cast<uint32_t>(l), k);
+  const float bar = maxima.thresh;
+  int have = 0;
+#pragma unroll
+  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
+    if (q * 128 >= deg) break;  // warp-uniform
+#pragma unroll
+    for (int j = 4 * q; j < 4 * q + 4; ++j) {
+      const bool in = ck[j] >= bar && ck[j] > NEG_INF;
+      const unsigned m = __ballot_sync(FULL_MASK, in);
+      const int at = have + __popc(m & ((1u << l) - 1u));
+      if (in && at < 32) {
+        pack_key[at] = ck[j];
+        pack_at[at] = static_cast<uint16_t>(j * 32 + l);
+      }
+      have += __popc(m);
+    }
+  }
+  __syncwarp();
+  if (have <= 32) {
+    top.fill(l < have ? pack_key[l] : NEG_INF, l < have ? pack_at[l] : ARES_EDGES + l, k);
+  } else {
+    top.fill(ck[0], static_cast<uint32_t>(l), k);
+    float above = fmaxf(top.thresh, key_below(bar));
+#pragma unroll 1
+    for (int j = 1; j < ARES_ITEMS; ++j) {
+      float c = ck[0];
+#pragma unroll
+      for (int x = 1; x < ARES_ITEMS; ++x) c = x == j ? ck[x] : c;
+      insert_above(top, above, c, j * 32, l, k);
+    }
+  }
+  __syncwarp();
+}
+
+// A further window of a list.  Of a row's n edges only about k (1 + ln(n/k)) ever enter the list, so the logarithm
+// and the division are spent only on edges that a bound lets through: log(u) <= u - 1, so an edge whose
+// u - 1 <= bar * w cannot beat the bar.  The test below is that inequality with the slack that the errors of __logf
+// (2^-21.4 absolute on [0.5, 2]), __fdividef (2 ulp) and of the 23 random bits it looks at need, so every edge that
+// the exact key lets in passes, and the exact key decides.  One vote per 128 edges.  A bar above -1e-30 is taken as
+// -1e-30 (weights so large that __fdividef gives 0 then always pass); products that are no number (0 * inf: a list
+// that is not full and a weight <= 0) pass too.
+__device__ __forceinline__ void ares_next_window(ShareList& top, float& entry, const RowWeights& W, int64_t base,
+                                                 uint32_t place, int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k) {
+  const float NEG_INF = __int_as_float(0xff800000);
+  constexpr float PASS = 2.0f - 0x1p-18f;
+  float wv[ARES_ITEMS];
+  W.load(wv, base, deg, l);
+#pragma unroll
+  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
+    const int64_t e0 = base + q * 128;
+    if (e0 >= deg) break;  // warp-uniform
+    const Philox4 r = ares_words(key, i_lo, i_hi, e0, l);
+    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+    const float bar = fminf(entry * 1.00001f, -1e-30f);
+    bool pass[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float v = __uint_as_float((rw[j] >> 9) | 0x3f800000u);
+      pass[j] = !(v <= fmaf(bar, fmaxf(wv[q * 4 + j], 0.f), PASS));
+    }
+    if (!__any_sync(FULL_MASK, pass[0] || pass[1] || pass[2] || pass[3])) continue;
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      const bool p = j == 0 ? pass[0] : j == 1 ? pass[1] : j == 2 ? pass[2] : pass[3];
+      if (!__any_sync(FULL_MASK, p)) continue;
+      const uint32_t word = j == 0 ? rw[0] : j == 1 ? rw[1] : j == 2 ? rw[2] : rw[3];
+      const float w = j == 0 ? wv[q * 4] : j == 1 ? wv[q * 4 + 1] : j == 2 ? wv[q * 4 + 2] : wv[q * 4 + 3];
+      insert_above(top, entry, p && e0 + j * 32 + l < deg ? ares_key(word, w) : NEG_INF, place + q * 128 + j * 32, l, k);
+    }
+  }
+}
+
 // (The exponential-jump form of the sampler -- keys only for the edges that enter, a
 // streamed prefix sum for the rest -- was built and measured here: with fan-outs of
 // 10-32 and rows of 10^3-10^4 edges an entry costs ~250 instructions at a rate of k/n
 // per edge, and the kernel ran 1.6-2.3x slower than with per-edge keys, so it is not used.)
-__device__ __forceinline__ void ares_scan(TopK& top, const RowWeights& W, int64_t base0, int64_t stride,
-                                          int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k) {
-  for (int64_t base = base0; base < deg; base += stride) ares_window(top, W, base, deg, key, i_lo, i_hi, l, k);
+
+// How a row is dealt out: share r of (at most) eight takes windows r, r + 8, ...  Within a share places ascend, and
+// shares are joined in order, so equal keys (zero weights, equal weights) keep one fixed order: by position up to
+// eight windows, by share and then position above.
+__device__ __forceinline__ int row_shares(int64_t deg) {
+  const int64_t windows = (deg + ARES_EDGES - 1) / ARES_EDGES;
+  return windows < WEIGHTED_WARPS ? static_cast<int>(windows) : WEIGHTED_WARPS;
+}
+// position in the row of a place (512 per window) in share r
+__device__ __forceinline__ int64_t position_of(int r, uint32_t place) {
+  return static_cast<int64_t>(place & ~(ARES_EDGES - 1u)) * WEIGHTED_WARPS + r * ARES_EDGES + (place & (ARES_EDGES - 1u));
 }
 
+// What is left of one share of a row after the row's window 0, into shared memory.  `bar` (shared by the row's shares,
+// ordered form) is the best k-th key any of them holds: whatever is below it cannot be among the row's top k.
+__device__ __forceinline__ void ares_share(const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi,
+                                           int r, int l, int k, int* bar, float* list_key, uint32_t* list_place) {
+  const float NEG_INF = __int_as_float(0xff800000);
+  // share 0 goes on from the list of window 0; the others start empty, with the row's bar to beat
+  ShareList top{r == 0 ? list_key[l] : NEG_INF, r == 0 ? list_place[l] : 0u, NEG_INF};
+  top.thresh = __shfl_sync(FULL_MASK, top.key, k - 1);
+  float entry = top.thresh;
+  for (uint32_t place = r == 0 ? ARES_EDGES : 0;; place += ARES_EDGES) {
+    const int64_t base = position_of(r, place);
+    if (base >= deg) break;
+    const int mine = ordered_float(top.thresh);
+    const int best = __shfl_sync(FULL_MASK, *static_cast<volatile int*>(bar), 0);  // one value for the warp
+    if (mine > best) {
+      if (l == 0) atomicMax(bar, mine);
+    } else {
+      entry = fmaxf(entry, key_below(float_of_ordered(best)));  // a key equal to it may still win by its place
+    }
+    ares_next_window(top, entry, W, base, place, deg, key, i_lo, i_hi, l, k);
+  }
+  list_key[l] = top.key;
+  list_place[l] = top.pos;
+}
+
+// A-Res without replacement.  Bound by issue slots (150 warp instructions per 32 edges) and the latency of the list
+// operations, not by the bytes of the weights.  Eight seeds per CTA of eight warps: each warp takes the first 512
+// edges of its own row, which gives the row a bar to beat; what is left of the CTA's longer rows is dealt out to its
+// warps in shares, and one warp per row joins them.  11 000 rows, 9.1 M weights, fan-out 10: 89 us, against 188 us
+// when a warp kept its row up to 4096 edges and inserted every key by itself.  (Four CTAs per SM at 64 registers
+// measured the same as three at 72.)
 template <typename IdT>
-__global__ void __launch_bounds__(SAMPLE_BLOCK)
+__global__ void __launch_bounds__(SAMPLE_BLOCK, 3)
 sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
                        const __grid_constant__ dgs_chunk_desc probs, const IdT* __restrict__ seeds,
-                       const Count nc, const int64_t k, const bool replace,
+                       const Count nc, const int64_t k,
                        const int64_t* __restrict__ plan_rb, const int64_t* __restrict__ plan_deg,
                        const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                        const RngKey rng, IdT* coo_row, IdT* coo_col,
@@ -456,128 +660,308 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
                        const bool row_is_position, int32_t* __restrict__ status) {
   const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
   pdl_enter();
+  const uint64_t key = key_of(rng) ^ (static_cast<uint64_t>(TAG_ARES) << 32);
+  const int64_t n = count_of(nc);
+  const int l = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int kk = static_cast<int>(k);
+  const float NEG_INF = __int_as_float(0xff800000);
+  __shared__ int s_shares[WEIGHTED_WARPS];  // of each warp's seed; 0: nothing to sample
+  __shared__ int s_bar[WEIGHTED_WARPS];
+  __shared__ int64_t s_rb[WEIGHTED_WARPS], s_deg[WEIGHTED_WARPS];
+  __shared__ float s_key[WEIGHTED_WARPS][WEIGHTED_WARPS][32];       // [row][share][rank]
+  __shared__ uint32_t s_place[WEIGHTED_WARPS][WEIGHTED_WARPS][32];
+  __shared__ float s_pack_key[WEIGHTED_WARPS][32];
+  __shared__ uint16_t s_pack_at[WEIGHTED_WARPS][32];
+
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * WEIGHTED_WARPS;
+  SeedPlan sp{0, 0, 0};
+  int64_t seed = 0, pick = -1;  // lane l emits the edge at `pick` as the seed's l-th
+  int my_shares = 0;
+  if (i0 + warp < n) {
+    sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
+    seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
+    if (sp.deg <= k) {
+      if (l < sp.deg) pick = l;
+    } else if (sp.rb + sp.deg > probs.total || sp.deg >> 35 != 0) {  // places within a share fit 32 bits below 2^35
+      if (l == 0) raise_status(status, DGS_ERR_RANGE);
+    } else {
+      my_shares = row_shares(sp.deg);
+      const uint64_t i = static_cast<uint64_t>(i0 + warp);
+      ShareList top{NEG_INF, 0, NEG_INF};
+      ares_first_window(top, row_weights(probs, sp.rb, sp.deg), sp.deg, key, static_cast<uint32_t>(i),
+                        static_cast<uint32_t>(i >> 32), l, kk, s_pack_key[warp], s_pack_at[warp]);
+      s_key[warp][0][l] = top.key;
+      s_place[warp][0][l] = top.pos;
+      if (l == 0) s_bar[warp] = ordered_float(top.thresh);
+    }
+  }
+  if (l == 0) {
+    s_shares[warp] = my_shares;
+    s_rb[warp] = sp.rb;
+    s_deg[warp] = sp.deg;
+  }
+  __syncthreads();
+  int task = 0;
+#pragma unroll 1
+  for (int row = 0; row < WEIGHTED_WARPS; ++row) {
+    if (s_shares[row] == 0) continue;
+    const int64_t deg = s_deg[row];
+    const int from = deg > ARES_EDGES * WEIGHTED_WARPS ? 0 : 1;  // share 0 of up to eight windows is done
+    const int shares = s_shares[row] - from;
+    const int r = from + ((warp - task) & (WEIGHTED_WARPS - 1));  // this warp's share of the row, if it has so many
+    task += shares;
+    if (r >= shares + from) continue;
+    const uint64_t i = static_cast<uint64_t>(i0 + row);
+    ares_share(row_weights(probs, s_rb[row], deg), deg, key, static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), r,
+               l, kk, &s_bar[row], s_key[row][r], s_place[row][r]);
+  }
+  __syncthreads();
+  if (my_shares > 0) {
+    TopK<int64_t> top{s_key[warp][0][l], position_of(0, s_place[warp][0][l]), NEG_INF};
+    top.thresh = __shfl_sync(FULL_MASK, top.key, kk - 1);
+#pragma unroll 1
+    for (int r = 1; r < my_shares; ++r)
+      for (int t = 0; t < kk; ++t) {
+        const float nk = s_key[warp][r][t];  // same address for all lanes: broadcast
+        if (!(nk > top.thresh)) break;       // every list is sorted: the rest of this one is behind the bar too
+        top.insert(nk, position_of(r, s_place[warp][r][t]), l, kk);
+      }
+    if (l < k) pick = top.pos;
+  }
+  if (pick >= 0) emit(sp.o, l, seed, sp.rb, pick);
+}
+
+// ---- proportional draws with replacement --------------------------------------
+// A row is kept as the sums of stretches of 2^m * 32 edges, at most 128 of them, in shared memory: groups of 32 for
+// rows of up to 4096 edges.  The sums of a 512-edge window (16 loads per lane in flight) are folded across the warp
+// with 16 shuffles in all, where a scan of every 32 edges takes 80, and their prefixes are formed once per row; each
+// lane then looks its own draw up by bisection and walks the 32 edges that it falls into.
+struct CtaSeeds {  // what phase 1 read about the CTA's seeds
+  int64_t rb[WEIGHTED_WARPS], deg[WEIGHTED_WARPS], o[WEIGHTED_WARPS], seed[WEIGHTED_WARPS];
+};
+
+constexpr int MAX_GROUPS = 128;
+constexpr int WINDOW_ITEMS = 16;
+
+// 16 sums of 32 edges from `base`, sum j in lanes 2j and 2j + 1
+__device__ __forceinline__ float group_sums(const RowWeights& W, int64_t base, int64_t deg, int l) {
+  float v[WINDOW_ITEMS];
+  W.load(v, base, deg, l);
+#pragma unroll
+  for (int j = 0; j < WINDOW_ITEMS; ++j) v[j] = fmaxf(v[j], 0.f);
+#pragma unroll
+  for (int half = 8, d = 16; half >= 1; half >>= 1, d >>= 1) {
+    const bool upper = (l & d) != 0;
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      const float give = upper ? v[j] : v[j + half];
+      v[j] = (upper ? v[j + half] : v[j]) + __shfl_xor_sync(FULL_MASK, give, d);
+    }
+  }
+  return v[0] + __shfl_xor_sync(FULL_MASK, v[0], 1);
+}
+
+__device__ __forceinline__ float warp_inclusive_sum(float s, int l) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const float t = __shfl_up_sync(FULL_MASK, s, d);
+    if (l >= d) s += t;
+  }
+  return s;
+}
+
+// The edge of the 32 from `base` that r (a distance into their sum) falls on: the first with a weight whose prefix
+// is above r, the last with a weight where rounding leaves none.  -1: no edge of them has a weight, or r is not
+// below their sum and !stop_here (r is then what is left behind them).
+__device__ __forceinline__ int64_t edge_of_32(const RowWeights& W, int64_t base, int64_t deg, float* r, bool stop_here,
+                                              int l) {
+  const int64_t e = base + l;
+  const float w = (e < deg) ? fmaxf(W(e), 0.f) : 0.f;
+  const float s = warp_inclusive_sum(w, l);
+  const unsigned some = __ballot_sync(FULL_MASK, w > 0.f);
+  const unsigned hit = __ballot_sync(FULL_MASK, w > 0.f && s > *r);
+  if (hit) return base + __ffs(hit) - 1;
+  if (stop_here) return some ? base + 31 - __clz(static_cast<int>(some)) : -1;
+  *r -= __shfl_sync(FULL_MASK, s, 31);
+  return -1;
+}
+
+struct RowGroups {
+  float sum[MAX_GROUPS];   // of each group
+  float incl[MAX_GROUPS];  // inclusive prefix
+};
+
+// groups g0, g0 + step, ... of the row (in units of one window when shift == 0)
+__device__ __forceinline__ void sum_groups(const RowWeights& W, int64_t deg, int shift, int first, int step, int l,
+                                           float* sum) {
+  if (shift == 0) {
+    for (int64_t w = first; w * 512 < deg; w += step) {
+      const float s = group_sums(W, w * 512, deg, l);
+      if ((l & 1) == 0 && w * 512 + (l >> 1) * 32 < deg) sum[w * 16 + (l >> 1)] = s;
+    }
+  } else {
+    const int64_t len = static_cast<int64_t>(32) << shift;
+    for (int64_t g = first; g * len < deg; g += step) {
+      const int64_t end = (g + 1) * len < deg ? (g + 1) * len : deg;
+      float acc = 0.f;
+      for (int64_t b = g * len; b < end; b += 512) acc += group_sums(W, b, end, l);
+      // lanes 2j and 2j + 1 hold the same sum: fold over j
+#pragma unroll
+      for (int d = 2; d < 32; d <<= 1) acc += __shfl_xor_sync(FULL_MASK, acc, d);
+      if (l == 0) sum[g] = acc;
+    }
+  }
+}
+
+__device__ __forceinline__ int group_shift(int64_t deg) {
+  int shift = 0;
+  while ((static_cast<int64_t>(32 * MAX_GROUPS) << shift) < deg) ++shift;
+  return shift;
+}
+
+// prefixes of the row's group sums; returns the row's total.  sum[] past the last group is 0.
+__device__ __forceinline__ float prefix_groups(RowGroups& g, int l) {
+  float4 v = reinterpret_cast<const float4*>(g.sum)[l];
+  v.y += v.x;
+  v.z += v.y;
+  v.w += v.z;
+  const float before = warp_inclusive_sum(v.w, l) - v.w;
+  const float up = __shfl_up_sync(FULL_MASK, before + v.w, 1);
+  const float base = l == 0 ? 0.f : up;  // the neighbour's last prefix, so that prefixes never step back
+  reinterpret_cast<float4*>(g.incl)[l] = make_float4(base + v.x, base + v.y, base + v.z, base + v.w);
+  return __shfl_sync(FULL_MASK, base + v.w, 31);
+}
+
+// This lane's draw (0 <= draw < total): the group it falls into, and what is left of it there.
+__device__ __forceinline__ int group_of(const RowGroups& g, float draw, float* rest) {
+  int lo = 0, hi = MAX_GROUPS - 1;  // first group whose inclusive prefix is above the draw
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (g.incl[mid] > draw) hi = mid;
+    else lo = mid + 1;
+  }
+  while (lo < MAX_GROUPS - 1 && !(g.sum[lo] > 0.f)) ++lo;  // rounding can lift a group that adds nothing
+  while (lo > 0 && !(g.sum[lo] > 0.f)) --lo;
+  *rest = lo > 0 ? draw - g.incl[lo - 1] : draw;
+  return lo;
+}
+
+// Bound by the latency of dependent loads and shuffles, not by bytes.  One warp per row of up to HUB_DEG edges;
+// longer rows are summed by all warps of the CTA.  4 096 rows, 1.4 M weights, fan-out 10: 13 us, against 68 us when a
+// warp scanned every 32 edges of its row twice.
+template <typename IdT>
+__global__ void __launch_bounds__(SAMPLE_BLOCK)
+sample_weighted_replace_kernel(const __grid_constant__ dgs_chunk_desc indices,
+                               const __grid_constant__ dgs_chunk_desc probs, const IdT* __restrict__ seeds,
+                               const Count nc, const int64_t k,
+                               const int64_t* __restrict__ plan_rb, const int64_t* __restrict__ plan_deg,
+                               const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
+                               const RngKey rng, IdT* coo_row, IdT* coo_col,
+                               const int64_t out_capacity, int64_t* __restrict__ picked_pos,
+                               const bool row_is_position, int32_t* __restrict__ status) {
+  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
+  pdl_enter();
   const uint64_t key = key_of(rng);
   const int64_t n = count_of(nc);
   const int l = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  constexpr int WARPS = SAMPLE_BLOCK / 32;
-  const float NEG_INF = __int_as_float(0xff800000);
-  __shared__ int s_hub[WARPS];  // warps whose seed is left to the whole CTA
-  __shared__ int s_nhub;
-  __shared__ float s_mkey[WARPS][32];
-  __shared__ int64_t s_mpos[WARPS][32];
-  if (threadIdx.x == 0) s_nhub = 0;
+  __shared__ __align__(16) RowGroups s_row[WEIGHTED_WARPS];
+  __shared__ int s_long[WEIGHTED_WARPS];
+  __shared__ int s_nlong;
+  __shared__ CtaSeeds s_seed;
+  if (threadIdx.x == 0) s_nlong = 0;
+  for (int x = l; x < MAX_GROUPS; x += 32) s_row[warp].sum[x] = 0.f;
   __syncthreads();
+
+  // draws t0 .. t0 + 31 of a row, one per lane; the calling warp resolves them all
+  auto draws = [&](const RowGroups& g, float total, const RowWeights& W, int64_t deg, int64_t i, int64_t seed,
+                   int64_t rb, int64_t o, int64_t t0) {
+    const int64_t t = t0 + l;
+    const uint32_t i_lo = static_cast<uint32_t>(i), i_hi = static_cast<uint32_t>(static_cast<uint64_t>(i) >> 32);
+    const Philox4 r = philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(t), TAG_WREPL);
+    const float draw = unit_float(r.x) * total;
+    const int shift = group_shift(deg);
+    int64_t pos = deg - 1;  // a draw not below the final sum maps to the last edge
+    float rest = 0.f;
+    int group = -1;
+    if (t < k && draw < total) group = group_of(g, draw, &rest);
+    if (shift == 0) {
+      // 32 edges, just read: every lane walks those of its own draw (a scan by the whole warp per draw takes ~60
+      // instructions a draw; this takes ~160 for all 32)
+      if (group >= 0) {
+        const int lo = group * 32, end = lo + 32 < deg ? lo + 32 : static_cast<int>(deg);
+        float s = 0.f;
+        int last = -1, at = -1;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+          const int e = lo + j;
+          const float w = e < end ? W(e) : 0.f;
+          if (w > 0.f) {
+            s += w;
+            last = e;
+            if (at < 0 && s > rest) at = e;
+          }
+        }
+        if (last >= 0) pos = at >= 0 ? at : last;  // a rounding short of the group's sum: its last edge with a weight
+      }
+    } else {
+      for (unsigned m = __ballot_sync(FULL_MASK, group >= 0); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        float left = __shfl_sync(FULL_MASK, rest, src);
+        const int64_t lo = static_cast<int64_t>(__shfl_sync(FULL_MASK, group, src)) * (static_cast<int64_t>(32) << shift);
+        const int64_t end = lo + (static_cast<int64_t>(32) << shift) < deg ? lo + (static_cast<int64_t>(32) << shift) : deg;
+        int64_t at = -1;
+        for (int64_t b = lo; b < end && at < 0; b += 32) at = edge_of_32(W, b, deg, &left, false, l);
+        // a rounding short of the group's sum: its last edge with a weight
+        for (int64_t b = (end - 1 - lo) / 32 * 32 + lo; b >= lo && at < 0; b -= 32) at = edge_of_32(W, b, deg, &left, true, l);
+        if (l == src && at >= 0) pos = at;
+      }
+    }
+    if (t < k) emit(o, t, seed, rb, pos);
+  };
 
   // ---- phase 1: one seed per warp ----
-  do {
-    const int64_t slot = static_cast<int64_t>(blockIdx.x) * WARPS + warp;
-    if (slot >= n) break;  // warp-uniform
-    const int64_t i = slot;
-    const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i, true);
-    const int64_t deg = sp.deg, rb = sp.rb, o = sp.o;
-    const int64_t seed = row_is_position ? i : static_cast<int64_t>(seeds[i]);
-    const uint32_t i_lo = static_cast<uint32_t>(i), i_hi = static_cast<uint32_t>(static_cast<uint64_t>(i) >> 32);
-    if (deg <= 0) break;
-
-    if (!replace && deg <= k) {
-      for (int64_t t = l; t < deg; t += 32) emit(o, t, seed, rb, t);
-      break;
-    }
-    if (rb + deg > probs.total) {
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * WEIGHTED_WARPS;
+  if (i0 + warp < n) {
+    const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
+    const int64_t seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
+    if (sp.deg > 0 && sp.rb + sp.deg > probs.total) {
       if (l == 0) raise_status(status, DGS_ERR_RANGE);
-      break;
-    }
-    if (!replace && deg > HUB_DEG) {
-      if (l == 0) s_hub[atomicAdd(&s_nhub, 1)] = warp;
-      break;
-    }
-    int64_t run;
-    const char* wp = resolve(probs, 2, rb, &run);
-    const RowWeights W{probs, run >= deg ? reinterpret_cast<const float*>(wp) : nullptr, rb};
-
-    if (!replace) {
-      TopK top{NEG_INF, -1, NEG_INF};
-      ares_scan(top, W, 0, 128 * ARES_QUADS, deg, key, i_lo, i_hi, l, static_cast<int>(k));
-      if (l < k) emit(o, l, seed, rb, top.pos);
-    } else {
-      // ---- proportional draws: stream the row twice through a warp scan ----
-      float total = 0.f;
-      for (int64_t base = 0; base < deg; base += 32) {
-        const int64_t e = base + l;
-        float w = (e < deg) ? fmaxf(W(e), 0.f) : 0.f;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const float t = __shfl_up_sync(FULL_MASK, w, d);
-          if (l >= d) w += t;
-        }
-        total = __shfl_sync(FULL_MASK, total + w, 31);
+    } else if (sp.deg > HUB_DEG) {
+      if (l == 0) {
+        s_long[atomicAdd(&s_nlong, 1)] = warp;
+        s_seed.rb[warp] = sp.rb;
+        s_seed.deg[warp] = sp.deg;
+        s_seed.o[warp] = sp.o;
+        s_seed.seed[warp] = seed;
       }
-      for (int64_t t0 = 0; t0 < k; t0 += 32) {
-        const int64_t t = t0 + l;
-        const bool mine = t < k;
-        const Philox4 r = philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(t), TAG_WREPL);
-        const float draw = unit_float(r.x) * total;
-        bool done = !mine;
-        int64_t pos = deg - 1;  // a draw not below the final sum maps to the last edge
-        float carry = 0.f;
-        for (int64_t base = 0; base < deg; base += 32) {
-          const int64_t e = base + l;
-          float w = (e < deg) ? fmaxf(W(e), 0.f) : 0.f;
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const float x = __shfl_up_sync(FULL_MASK, w, d);
-            if (l >= d) w += x;
-          }
-          const float cdf = carry + w;  // inclusive prefix up to edge e
-          const float window_end = __shfl_sync(FULL_MASK, cdf, 31);
-          unsigned hit = __ballot_sync(FULL_MASK, !done && draw < window_end);
-          while (hit) {
-            const int src = __ffs(hit) - 1;
-            hit &= hit - 1;
-            const float d0 = __shfl_sync(FULL_MASK, draw, src);
-            const unsigned above = __ballot_sync(FULL_MASK, cdf > d0);  // non-empty: lane 31 is above
-            if (l == src) {
-              int64_t q = base + (__ffs(above) - 1);
-              pos = q < deg ? q : deg - 1;
-              done = true;
-            }
-          }
-          carry = window_end;
-          if (__all_sync(FULL_MASK, done)) break;
-        }
-        if (mine) emit(o, t, seed, rb, pos);
-      }
+    } else if (sp.deg > 0) {
+      const RowWeights W = row_weights(probs, sp.rb, sp.deg);
+      sum_groups(W, sp.deg, 0, 0, 1, l, s_row[warp].sum);
+      __syncwarp();
+      const float total = prefix_groups(s_row[warp], l);
+      __syncwarp();
+      for (int64_t t0 = 0; t0 < k; t0 += 32) draws(s_row[warp], total, W, sp.deg, i0 + warp, seed, sp.rb, sp.o, t0);
     }
-  } while (false);
+  }
 
-  // ---- phase 2: hub rows, all warps of the CTA on one row at a time ----
+  // ---- phase 2: rows above HUB_DEG ----
   __syncthreads();
-  const int nhub = s_nhub;
-  for (int h = 0; h < nhub; ++h) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * WARPS + s_hub[h];
-    const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i, true);
-    const int64_t deg = sp.deg, rb = sp.rb, o = sp.o;
-    const uint32_t i_lo = static_cast<uint32_t>(i), i_hi = static_cast<uint32_t>(static_cast<uint64_t>(i) >> 32);
-    int64_t run;
-    const char* wp = resolve(probs, 2, rb, &run);
-    const RowWeights W{probs, run >= deg ? reinterpret_cast<const float*>(wp) : nullptr, rb};
-    TopK top{NEG_INF, -1, NEG_INF};
-    ares_scan(top, W, static_cast<int64_t>(warp) * 128 * ARES_QUADS, 128 * ARES_QUADS * WARPS, deg, key, i_lo,
-              i_hi, l, static_cast<int>(k));
-    s_mkey[warp][l] = top.key;
-    s_mpos[warp][l] = top.pos;
-    __syncthreads();
-    if (warp == 0) {  // merge the other warps' lists into this one; every list is sorted, so stop at the bar
-      for (int ww = 1; ww < WARPS; ++ww)
-        for (int t = 0; t < k; ++t) {
-          const float nk = s_mkey[ww][t];  // same address for all lanes: broadcast
-          if (!(nk > top.thresh)) break;
-          top.insert(nk, s_mpos[ww][t], l, static_cast<int>(k));
-        }
-      if (l < k) emit(o, l, row_is_position ? i : static_cast<int64_t>(seeds[i]), rb, top.pos);
-    }
-    __syncthreads();
+  const int nlong = s_nlong;
+  for (int h = 0; h < nlong; ++h) {
+    RowGroups& g = s_row[s_long[h]];  // the seed's own: phase 1 left it at 0
+    const int64_t deg = s_seed.deg[s_long[h]];
+    sum_groups(row_weights(probs, s_seed.rb[s_long[h]], deg), deg, group_shift(deg), warp, WEIGHTED_WARPS, l, g.sum);
+  }
+  __syncthreads();
+  if (warp < nlong) {
+    const int src = s_long[warp];
+    const float total = prefix_groups(s_row[src], l);
+    __syncwarp();
+    const RowWeights W = row_weights(probs, s_seed.rb[src], s_seed.deg[src]);
+    for (int64_t t0 = 0; t0 < k; t0 += 32)
+      draws(s_row[src], total, W, s_seed.deg[src], i0 + src, s_seed.seed[src], s_seed.rb[src], s_seed.o[src], t0);
   }
 }
 
@@ -625,9 +1009,10 @@ int weighted_typed(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, c
                    int64_t k, bool replace, const PlanView& pv, RngKey key,
                    void* coo_row, void* coo_col, int64_t cap, int64_t* pos, bool rowpos, int32_t* status,
                    cudaStream_t s) {
-  const unsigned grid = static_cast<unsigned>((n.bound + SAMPLE_BLOCK / 32 - 1) / (SAMPLE_BLOCK / 32));
-  DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, sample_weighted_kernel<IdT>, grid, SAMPLE_BLOCK, s, indices, probs,
-                              static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, pv.local_off,
+  const unsigned grid = static_cast<unsigned>((n.bound + WEIGHTED_WARPS - 1) / WEIGHTED_WARPS);
+  auto kernel = replace ? sample_weighted_replace_kernel<IdT> : sample_weighted_kernel<IdT>;
+  DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, kernel, grid, SAMPLE_BLOCK, s, indices, probs,
+                              static_cast<const IdT*>(seeds), n, k, pv.row_begin, pv.deg, pv.local_off,
                               pv.tile_off, key, static_cast<IdT*>(coo_row), static_cast<IdT*>(coo_col), cap,
                               pos, rowpos, status));
   return DGS_OK;

@@ -1,0 +1,105 @@
+"""Weighted sampling at the sizes where its paths meet: rows around 32, 128, 512 edges (one list, windows), 4096
+(eight windows; one warp per row with replacement) and above, against the draws recomputed on the host."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import Words, plain_desc, sample
+
+pytestmark = pytest.mark.gpu
+
+DEGREES = [1, 5, 31, 32, 33, 127, 128, 129, 511, 512, 513, 1023, 1025, 4095, 4096, 4097, 8193, 40001]
+
+
+@pytest.fixture
+def words():
+    return Words()
+
+
+def mix64(z):
+    m = (1 << 64) - 1
+    z = (z + 0x9E3779B97F4A7C15) & m
+    z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & m
+    z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & m
+    return z ^ (z >> 31)
+
+
+def philox(key, c0, c1, c2, c3):
+    """Philox4x32-10 on arrays of counters: four uint32 arrays."""
+    c = [np.broadcast_to(np.asarray(x, dtype=np.uint64), np.shape(c2)).copy() for x in (c0, c1, c2, c3)]
+    k0, k1, low = key & 0xFFFFFFFF, key >> 32, np.uint64(0xFFFFFFFF)
+    for _ in range(10):
+        p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        c = [(p1 >> np.uint64(32)) ^ c[1] ^ np.uint64(k0), p1 & low, (p0 >> np.uint64(32)) ^ c[3] ^ np.uint64(k1), p0 & low]
+        k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
+    return c
+
+
+def unit(word):
+    return ((word >> np.uint64(8)).astype(np.float64) + 1.0) / 16777216.0
+
+
+def graph(weights_of):
+    """One row per degree, twice over, neighbours numbered; seeds in an order that mixes long and short rows."""
+    deg = np.array(DEGREES + DEGREES[::-1], dtype=np.int64)
+    indptr = np.concatenate([[0], np.cumsum(deg)])
+    w = np.concatenate([weights_of(d, i) for i, d in enumerate(deg)]).astype(np.float32)
+    order = np.random.default_rng(3).permutation(deg.size)
+    t = [torch.from_numpy(x).cuda() for x in (indptr, np.arange(indptr[-1], dtype=np.int64), w, order.astype(np.int64))]
+    return deg, w, indptr, order, t
+
+
+@pytest.mark.parametrize("k", [1, 10, 17, 32])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_without_replacement_follows_the_keys(words, k, zeros):
+    # weights are 1 (or 0), so a key's order is that of its uniform; __logf is off by 2^-21.4 at most, so two keys can
+    # change places only when their uniforms are closer than 2 * 2^-21.4 (7.2e-7 in the logarithm, hence in u <= 1)
+    rng = np.random.default_rng(1)
+    deg, w, indptr, order, (ip, ix, wt, seeds) = graph(
+        lambda d, i: (rng.random(d) < 0.02 if zeros else np.ones(d)))
+    key = mix64(7) ^ mix64(5 ^ 0xA5A5A5A55A5A5A5A) ^ (0x41524553 << 32)
+    row, col, pos = sample(plain_desc(ip), plain_desc(ix), seeds, k, False, words, probs_desc=plain_desc(wt), rng=(7, 5))
+    assert words.take_status() == 0
+    at = 0
+    for i, s in enumerate(order):
+        d = int(deg[s])
+        m = min(d, k)
+        got, at = pos[at:at + m], at + m
+        assert np.all(row[at - m:at] == s) and np.all(col[at - m:at] == indptr[s] + got)
+        if d <= k:
+            assert np.array_equal(got, np.arange(d))
+            continue
+        assert np.unique(got).size == k
+        e = np.arange(d)
+        block = philox(key, i & 0xFFFFFFFF, 0, (e // 128) * 32 + e % 32, np.zeros(d))
+        u = unit(np.choose(e % 128 // 32, block))
+        ws = w[indptr[s]:indptr[s + 1]]
+        positive = int((ws > 0).sum())
+        n_pos = min(k, positive)
+        assert np.all(ws[got[:n_pos]] > 0) and not np.any(ws[got[n_pos:]] > 0)
+        best = np.sort(u[ws > 0])[::-1][:n_pos]
+        assert np.all(u[got[:n_pos]] >= best - 8e-7)
+        if n_pos < k:  # the rest are zero weights, in scan order (above eight windows: by window modulo eight first)
+            zero = e[ws == 0]
+            place = zero if d <= 4096 else np.lexsort((zero, zero // 512 % 8))
+            assert np.array_equal(got[n_pos:], (zero if d <= 4096 else zero[place])[:k - n_pos])
+
+
+@pytest.mark.parametrize("k", [1, 10, 33, 70])
+def test_with_replacement_follows_the_prefix_sums(words, k):
+    # whole-number weights: every sum of them is exact in fp32, so the edge of a draw is known exactly
+    rng = np.random.default_rng(2)
+    deg, w, indptr, order, (ip, ix, wt, seeds) = graph(
+        lambda d, i: np.where(rng.random(d) < 0.6, 0, rng.integers(1, 8, d)) if i % 3 else np.zeros(d) if i % 5 == 0
+        else rng.integers(0, 3, d))
+    key = mix64(7) ^ mix64(5 ^ 0xA5A5A5A55A5A5A5A)
+    row, col, pos = sample(plain_desc(ip), plain_desc(ix), seeds, k, True, words, probs_desc=plain_desc(wt), rng=(7, 5))
+    assert words.take_status() == 0
+    pos = pos.reshape(-1, k)
+    for i, s in enumerate(order):
+        d = int(deg[s])
+        cdf = np.cumsum(w[indptr[s]:indptr[s + 1]].astype(np.float64))
+        u = unit(philox(key, i & 0xFFFFFFFF, 0, np.arange(k), np.full(k, 0x57524550))[0]).astype(np.float32)
+        draw = u * np.float32(cdf[-1])
+        want = np.minimum(np.searchsorted(cdf, draw.astype(np.float64), side="right"), d - 1)
+        assert np.array_equal(pos[i], want), (i, d)
