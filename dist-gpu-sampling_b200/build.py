@@ -35,6 +35,7 @@ HEADERS = [
     "kernels/tile_scan.cuh",
     "kernels/launchers.h",
     "kernels/relabel_device.cuh",
+    "kernels/sample_device.cuh",
     "host/comm.h",
     "../../include/dgs_b200.h",
 ]

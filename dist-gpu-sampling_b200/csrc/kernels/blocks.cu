@@ -14,13 +14,15 @@
 // than the graph has), and the actual sizes go to a caller-supplied (pinned)
 // array that the host reads once, after everything is queued.
 //
-// Per hop: plan -> sample -> insert -> count -> number; the plan launch also
-// carries, as extra CTAs, two jobs that depend on nothing it does: clearing the
-// table this hop will fill and relabelling the COO of the hop before (whose
-// numbering is complete by then).  The last hop's COO is relabelled by a launch
-// of its own.  From the second hop on the seed list is a relabel's unique list,
-// so a seed's relabelled id is its position and the sampler writes that directly;
-// only the first hop (whose seeds the caller may repeat) looks its rows up.
+// Per hop: sample -> insert -> number.  The number launch of a hop also makes the
+// plan of the next one (its unique list is the next seed list); only the first
+// hop has a plan launch.  The sample launch carries, as extra CTAs, two jobs that
+// depend on nothing it does: clearing the table this hop will fill and relabelling
+// the COO of the hop before (whose numbering is complete by then).  The last hop's
+// COO is relabelled by a launch of its own.  From the second hop on the seed list
+// is a relabel's unique list, so a seed's relabelled id is its position and the
+// sampler writes that directly; only the first hop (whose seeds the caller may
+// repeat) looks its rows up.
 #include <cstdlib>
 #include <new>
 
@@ -37,8 +39,7 @@ inline size_t ws_align(size_t x) { return (x + WS_ALIGN - 1) / WS_ALIGN * WS_ALI
 struct InitWords {
   int64_t* n0;
   int64_t n0_value;
-  int n_tickets;
-  unsigned int* tickets[2 * DGS_MAX_HOPS];
+  unsigned int* ticket;  // of the first hop's plan
   // a recorded sequence takes its random stream from memory: (seed, offset) at rng_src, read by this
   // kernel on every replay and folded into one Philox key per hop for the sampling kernels behind it
   const uint64_t* rng_src;
@@ -48,8 +49,10 @@ struct InitWords {
 
 __global__ void blocks_init_kernel(const InitWords w) {
   pdl_enter();
-  if (threadIdx.x == 0) *w.n0 = w.n0_value;
-  if (threadIdx.x < w.n_tickets) *w.tickets[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) {
+    *w.n0 = w.n0_value;
+    *w.ticket = 0u;
+  }
   if (w.rng_src != nullptr && threadIdx.x < w.n_keys) {
     const volatile uint64_t* src = w.rng_src;  // host-written words: no cached copy
     w.keys[threadIdx.x] = fold_rng_key(src[0], src[1] + static_cast<uint64_t>(threadIdx.x));
@@ -177,32 +180,28 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
   void* table[DGS_MAX_HOPS];
   static_assert(sizeof(int64_t) * (1 + DGS_MAX_HOPS) <= WS_ALIGN, "the control words hold n0 and one key per hop");
   uint64_t* keys_dev = reinterpret_cast<uint64_t*>(n0_dev + 1);
-  InitWords init{n0_dev, n0, 0, {}, rng_words, keys_dev, n_hops};
   for (int h = 0; h < n_hops; ++h) {
     const int64_t key_bound = hops[h].seed_bound * (1 + hops[h].fanout);
     plan[h] = p;
     p += ws_align(dgs_sample_plan_bytes(hops[h].seed_bound));
     table[h] = p;
     p += ws_align(dgs_relabel_table_bytes(key_bound));
-    init.tickets[init.n_tickets++] = sample_plan_ticket(plan[h], hops[h].seed_bound);
-    init.tickets[init.n_tickets++] = unique_ticket(table[h], key_bound);
   }
+  const InitWords init{n0_dev, n0, sample_plan_ticket(plan[0], n0), rng_words, keys_dev, n_hops};
   DGS_CUDA_TRY(launch_chained(SITE_INIT, blocks_init_kernel, 1u, 32u, s, init));
 
-  // one-word table slots when every node id fits 32 bits (relabel_device.cuh); DGS_RELABEL_WIDE=1 keeps the
-  // two-word slots for comparison
-  static const bool force_wide = [] {
-    const char* e = std::getenv("DGS_RELABEL_WIDE");
-    return e != nullptr && e[0] == '1';
-  }();
-  const bool compact = !force_wide && (!ids64 || indptr->total - 1 < COMPACT_KEY_LIMIT);
+  // a graph with fewer nodes than 2^32 - 1 has no ids beyond
+  const long long max_key = !ids64 || indptr->total - 1 < COMPACT_KEY_LIMIT ? COMPACT_KEY_LIMIT - 1 : INT64_MAX;
 
   // ---- queue every hop; no size is read back in between ----
   const void* hop_seeds = seeds;
   const int64_t* n_dev = n0_dev;
-  LookupJob pending{};  // relabelling of the previous hop's COO, carried by the next plan launch
+  LookupJob pending{};  // relabelling of the previous hop's COO, carried by the next sample launch
   SizesReport report{};
   report.dst = sizes;
+  rc = launch_sample_plan(*indptr, seeds, ids64 != 0, Count{n0, n0_dev, nullptr}, hops[0].fanout, replace != 0, plan[0],
+                          nullptr, false, status, s);
+  if (rc != DGS_OK) return rc;
   for (int h = 0; h < n_hops; ++h) {
     const dgs_hop& hp = hops[h];
     const int64_t k = hp.fanout;
@@ -210,30 +209,29 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
     const int64_t key_bound = hp.seed_bound + edge_bound;
     const Count n{hp.seed_bound, n_dev, nullptr};
     // the table is dimensioned before the neighbours are drawn: seeds * (1 + fanout) keys at most
-    const TableSize size{n, 1 + k, compact};
-    rc = launch_sample_plan(*indptr, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], nullptr, false,
-                            make_clear_job(table[h], key_bound, size), pending, status, s);
-    if (rc != DGS_OK) return rc;
+    const TableSize size{n, 1 + k, max_key};
+    const SideJobs jobs{make_clear_job(table[h], key_bound, size), pending, 0u};
     const int64_t* nnz_dev = sample_plan_total(plan[h], hp.seed_bound);
     const RngKey key = rng_words != nullptr
                            ? RngKey{0, keys_dev + h}
                            : host_key(sample_rng_key(rng_seed, rng_offset + static_cast<uint64_t>(h)));
-    const bool row_is_position = h > 0;
+    const bool later = h > 0;  // the plan came with the numbering of these seeds, which are unique
     rc = probs != nullptr
-             ? launch_sample_weighted(*indices, *probs, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h],
-                                      key, hp.coo_row, hp.coo_col, edge_bound, nullptr, row_is_position, status, s)
-             : launch_sample_uniform(*indices, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], key,
-                                     hp.coo_row, hp.coo_col, edge_bound, nullptr, row_is_position, status, s);
+             ? launch_sample_weighted(*indices, *probs, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], later,
+                                      key, hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, status, s)
+             : launch_sample_uniform(*indices, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], later, key,
+                                     hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, status, s);
     if (rc != DGS_OK) return rc;
     const Count nnz{edge_bound, nnz_dev, nullptr};
     report.src[2 * h] = nnz_dev;
     report.src[2 * h + 1] = unique_total(table[h], key_bound);
-    if (h == n_hops - 1) report.n = 2 * n_hops;  // the last hop's count kernel sends all sizes to the host at once
+    NextPlan next{};
+    if (h + 1 < n_hops) next = make_next_plan(*indptr, hops[h + 1].seed_bound, hops[h + 1].fanout, replace != 0, plan[h + 1]);
+    else report.n = 2 * n_hops;  // the last hop's numbering sends all sizes to the host at once
     rc = launch_unique_pair(ids64 != 0, hop_seeds, n, hp.coo_col, nnz, key_bound, size, table[h], hp.frontier,
-                            hp.frontier_bound, nullptr, report, status, s);
+                            hp.frontier_bound, nullptr, report, next, status, s);
     if (rc != DGS_OK) return rc;
-    pending = make_lookup_job(table[h], key_bound, size, row_is_position ? nullptr : hp.coo_row, hp.coo_col, nnz,
-                              hp.coo_row, hp.coo_col);
+    pending = make_lookup_job(table[h], key_bound, size, later ? nullptr : hp.coo_row, hp.coo_col, nnz, n);
     hop_seeds = hp.frontier;
     n_dev = unique_total(table[h], key_bound);
   }
@@ -253,7 +251,7 @@ extern "C" int dgs_sample_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_d
 }
 
 // ---- the sequence recorded once and replayed ------------------------------------
-// Queuing a batch is ~18 kernel launches with the same parameters every time as long as the buffers, the
+// Queuing a batch is a dozen kernel launches with the same parameters every time as long as the buffers, the
 // bounds (the number of seeds) and the tables stay the same; only the random stream differs.  A recording
 // holds those launches as one executable graph (stream capture keeps the programmatic edges between the
 // kernels), and a replay is a single launch call.

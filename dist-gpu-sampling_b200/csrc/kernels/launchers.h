@@ -11,25 +11,39 @@ namespace dgs {
 // receives the number of sampled edges; the same number stays in the plan at
 // sample_plan_total().  The plan's ticket word must be zero at launch: it is
 // cleared here when zero_ticket is set and resets itself after every use.
-// clear / lookup (either may have ctas == 0): independent jobs run by extra CTAs of
-// the plan launch -- clearing the table this hop will fill, relabelling the COO of
-// the hop before it.
 int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, Count n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, const ClearJob& clear,
-                       const LookupJob& lookup, int32_t* status, cudaStream_t s);
+                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, int32_t* status, cudaStream_t s);
+// The plan of a hop whose seeds are being numbered (launch_unique_pair writes it): offsets are those in the whole
+// output, so sampling takes whole_offsets = true.  n_edges == nullptr: no plan wanted.
+struct NextPlan {
+  dgs_chunk_desc indptr;
+  int64_t k;
+  bool replace;
+  int64_t *row_begin, *deg, *off;
+  int64_t* n_edges;
+};
+NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k, bool replace, void* plan);
 int64_t* sample_plan_total(void* plan, int64_t n_bound);
 unsigned int* sample_plan_ticket(void* plan, int64_t n_bound);
+
+// Independent jobs run by extra CTAs of a sampling launch (either may have ctas == 0).
+struct SideJobs {
+  ClearJob clear;
+  LookupJob lookup;
+  unsigned main_ctas;  // set by the launcher
+};
 
 // row_is_position: write the seed's position in the seed list to coo_row instead
 // of the seed id (valid as a relabelled id when the seed list has no duplicates).
 int launch_sample_uniform(const dgs_chunk_desc& indices, const void* seeds, bool ids64, Count n, int64_t k,
-                          bool replace, void* plan, RngKey key, void* coo_row,
+                          bool replace, void* plan, bool whole_offsets, RngKey key, void* coo_row,
                           void* coo_col, int64_t out_capacity, int64_t* picked_pos, bool row_is_position,
-                          int32_t* status, cudaStream_t s);
+                          const SideJobs& jobs, int32_t* status, cudaStream_t s);
 int launch_sample_weighted(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds,
-                           bool ids64, Count n, int64_t k, bool replace, void* plan,
+                           bool ids64, Count n, int64_t k, bool replace, void* plan, bool whole_offsets,
                            RngKey key, void* coo_row, void* coo_col, int64_t out_capacity,
-                           int64_t* picked_pos, bool row_is_position, int32_t* status, cudaStream_t s);
+                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, int32_t* status,
+                           cudaStream_t s);
 uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset);
 
 // ---- relabel.cu ----------------------------------------------------------------
@@ -37,20 +51,19 @@ uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset);
 // says how much of it is in use (cleared, probed); every kernel of one table gets
 // the same TableSize.
 ClearJob make_clear_job(void* table, int64_t key_bound, const TableSize& size);
-LookupJob make_lookup_job(const void* table, int64_t key_bound, const TableSize& size, const void* a, const void* b,
-                          Count n, void* out_a, void* out_b);
-int launch_clear(const ClearJob& job, cudaStream_t s);            // as a launch of its own
-int launch_lookup(const LookupJob& job, bool ids64, cudaStream_t s);
+LookupJob make_lookup_job(void* table, int64_t key_bound, const TableSize& size, void* row, void* col, Count n,
+                          Count n_seeds);
+int launch_lookup(const LookupJob& job, bool ids64, cudaStream_t s);  // as a launch of its own
 
 // First-occurrence unique of the logical concatenation a[0:na) ++ b[0:nb) whose
 // lengths are device words, into a table that has been cleared.  unique_out holds
 // unique_capacity ids; a larger result raises DGS_ERR_RANGE in the status word and
-// is cut off.  The table's ticket word must be zero at launch (it resets itself).  `report`
-// (n may be 0) is carried out by the kernel that knows the number of distinct keys.
+// is cut off.  `report` (n may be 0) is carried out by the kernel that knows the number of distinct keys; `plan` is
+// filled for the distinct keys as the next hop's seeds.
 int launch_unique_pair(bool ids64, const void* a, Count na, const void* b, Count nb, int64_t key_bound,
                        const TableSize& size, void* table, void* unique_out, int64_t unique_capacity,
-                       int64_t* n_unique_out, const SizesReport& report, int32_t* status, cudaStream_t s);
+                       int64_t* n_unique_out, const SizesReport& report, const NextPlan& plan, int32_t* status,
+                       cudaStream_t s);
 int64_t* unique_total(void* table, int64_t key_bound);
-unsigned int* unique_ticket(void* table, int64_t key_bound);
 
 }  // namespace dgs

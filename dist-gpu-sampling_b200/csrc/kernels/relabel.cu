@@ -12,54 +12,49 @@
 // (:28,123), so the result does not depend on hash layout or thread timing.
 //
 // Different (the design):
-//   * one 16-byte slot {key, value} per entry (a probe touches one sector, not
-//     three arrays), mixed 64-bit hash, linear probing, load factor <= 50 %.
+//   * one 8-byte slot per entry, mixed hash, linear probing, load factor <= 50 %.
 //   * inputs are read through a segment list instead of being concatenated.
 //   * the insert pass remembers each input's slot, so later passes index the
 //     table directly instead of probing again.
-//   * numbering is count-per-tile (the last CTA to finish scans the tile sums,
-//     no extra launch) -> write; the label is
-//     stored into the slot's value with the top bit set, which can never be
-//     mistaken for an input index by a concurrent reader, so no third table.
+//   * first occurrences are counted and numbered in ONE pass (a look-back over
+//     the tiles' sums); the label is stored into the slot with the top bit set,
+//     which can never be mistaken for an input index by a concurrent reader, so
+//     no third table.  In the multi-hop sequence the same pass reads the row
+//     bounds of the nodes it numbers and places their outputs: the next hop's plan.
 //   * the number of distinct keys goes to a caller-supplied (pinned) word.
 #include "common.cuh"
 #include "launchers.h"
 #include "relabel_device.cuh"
-#include "philox.cuh"
+#include "sample_device.cuh"
 #include "tile_scan.cuh"
+
+#include <type_traits>
 
 namespace dgs {
 namespace {
 
-constexpr int RL_ITEMS = 4;
-constexpr int RL_TILE = RL_BLOCK * RL_ITEMS;
-
-struct TableView {
-  Slot* slots;         // [cap]
-  uint32_t* slot_of;   // [n]  slot of every input
-  int64_t* tile_off;   // [ntiles]
-  int64_t* total;      // [1]
-  unsigned int* ticket;  // [1]
-  uint64_t cap;
-  int64_t ntiles;
-};
-
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
-inline TableView table_view(void* mem, int64_t n) {
-  TableView t;
-  t.cap = slots_for(n);
+// words | ticket, tile words, wide keys (within 8 bytes per slot: slots >= 2n) | slot_of | total
+inline TableParts table_view(void* mem, int64_t n) {
+  TableParts t;
+  const uint64_t cap = slots_for(n);
   t.ntiles = (n + RL_TILE - 1) / RL_TILE;
   char* p = static_cast<char*>(mem);
-  t.slots = reinterpret_cast<Slot*>(p);
-  p += t.cap * sizeof(Slot);
+  t.words = reinterpret_cast<unsigned long long*>(p);
+  char* q = p + cap * sizeof(unsigned long long);
+  t.ticket = reinterpret_cast<unsigned int*>(q);
+  t.tiles = reinterpret_cast<unsigned long long*>(q + 16);
+  t.tiles2 = t.tiles + t.ntiles;
+  t.wide_keys = reinterpret_cast<long long*>(t.tiles2 + t.ntiles);
+  p += 2 * cap * sizeof(unsigned long long);
   t.slot_of = reinterpret_cast<uint32_t*>(p);
   p += align_up(static_cast<size_t>(n) * sizeof(uint32_t), 16);
-  t.tile_off = reinterpret_cast<int64_t*>(p);
-  t.total = t.tile_off + t.ntiles;
-  t.ticket = reinterpret_cast<unsigned int*>(t.total + 1);
+  t.total = reinterpret_cast<int64_t*>(p) + t.ntiles;
   return t;
 }
+// the ticket and the tile words, in units of 16 bytes
+inline int64_t ticket_units(const TableParts& t) { return 1 + t.ntiles; }
 
 // ---- where the keys come from ---------------------------------------------------
 // A host-known segment list (the per-operator entry points) ...
@@ -88,166 +83,159 @@ struct PairKeys {
   }
 };
 
-// pass 0 of the sequence with device-side counts, when it does not ride on another
-// launch: clear only the slots the table will use (the per-operator path clears
-// with a memset instead)
-__global__ void __launch_bounds__(RL_BLOCK) relabel_clear_kernel(const ClearJob job) {
-  pdl_enter();
-  run_clear_cta(job, blockIdx.x);
-}
-
 // pass 1: insert every key, keep the smallest input index per key
 template <typename IdT, typename Keys>
 __global__ void __launch_bounds__(RL_BLOCK)
-relabel_insert_kernel(const __grid_constant__ Keys keys, const TableSize size, Slot* slots,
+relabel_insert_kernel(const __grid_constant__ Keys keys, const TableSize size, unsigned long long* words,
                       uint32_t* __restrict__ slot_of, int32_t* __restrict__ status) {
   pdl_enter();
   const int64_t n = keys.size();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * RL_BLOCK + threadIdx.x;
   if (i >= n) return;
-  const uint64_t mask = table_slots(size) - 1;
   const long long key = static_cast<long long>(keys.template load<IdT>(i));
-  if (key < 0 || (size.compact && key >= COMPACT_KEY_LIMIT)) {
+  if (key < 0 || key > size.max_key) {
     raise_status(status, DGS_ERR_RANGE);
     slot_of[i] = NO_SLOT;
     return;
   }
+  const uint32_t mask32 = static_cast<uint32_t>(table_slots(size) - 1), key32 = static_cast<uint32_t>(key);
+  const uint32_t flag = is_wide(key) ? WIDE_BIT32 : 0u;
+  const unsigned long long mine =
+      (static_cast<unsigned long long>(key32) << 32) | static_cast<unsigned long long>(flag | static_cast<uint32_t>(i));
   uint32_t found = NO_SLOT;
-  if (size.compact) {
-    unsigned long long* words = reinterpret_cast<unsigned long long*>(slots);
-    const uint32_t mask32 = static_cast<uint32_t>(mask), key32 = static_cast<uint32_t>(key);
-    const unsigned long long mine = (static_cast<unsigned long long>(key32) << 32) | static_cast<unsigned long long>(i);
-    uint32_t h = hash_key32(key32) & mask32;
-    for (uint32_t probes = 0; probes <= mask32; ++probes) {
-      unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&words[h]);
-      if (cur == EMPTY_COMPACT) {
-        cur = atomicCAS(&words[h], EMPTY_COMPACT, mine);
-        if (cur == EMPTY_COMPACT) {  // claimed, and the first index is in place: nothing else to do
-          found = h;
-          break;
-        }
-      }
-      if (static_cast<uint32_t>(cur >> 32) == key32) {
+  uint32_t h = home_slot(key, mask32);
+  for (uint32_t probes = 0; probes <= mask32; ++probes) {
+    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&words[h]);
+    if (cur == EMPTY_WORD) {
+      cur = atomicCAS(&words[h], EMPTY_WORD, mine);
+      if (cur == EMPTY_WORD) {  // claimed, and the first index is in place: nothing else to do
         found = h;
-        // same high half, so the minimum of the words is the minimum of the indices; a stale read can only
-        // cause a redundant atomic (indices only ever decrease)
-        if (static_cast<uint32_t>(cur) > static_cast<uint32_t>(i)) atomicMin(&words[h], mine);
         break;
       }
-      h = (h + 1) & mask32;
     }
-    slot_of[i] = found;
-    if (found == NO_SLOT) raise_status(status, DGS_ERR_TABLE_FULL);
-    return;
-  }
-  uint64_t h = hash_key(key) & mask;
-  for (uint64_t probes = 0; probes <= mask; ++probes) {
-    long long cur = *reinterpret_cast<volatile long long*>(&slots[h].key);
-    if (cur == EMPTY_KEY)
-      cur = static_cast<long long>(atomicCAS(reinterpret_cast<unsigned long long*>(&slots[h].key),
-                                             static_cast<unsigned long long>(EMPTY_KEY),
-                                             static_cast<unsigned long long>(key)));
-    if (cur == EMPTY_KEY || cur == key) {
-      found = static_cast<uint32_t>(h);
+    const uint32_t low = static_cast<uint32_t>(cur);
+    if (static_cast<uint32_t>(cur >> 32) == key32 && (low & WIDE_BIT32) == flag &&
+        (flag == 0u || static_cast<long long>(keys.template load<IdT>(low & VALUE_MASK32)) == key)) {
+      found = h;
+      // same high half and flag, so the minimum of the words is the minimum of the indices; a stale read can only
+      // cause a redundant atomic (indices only ever decrease)
+      if (cur > mine) atomicMin(&words[h], mine);
       break;
     }
-    h = (h + 1) & mask;
+    h = (h + 1) & mask32;
   }
   slot_of[i] = found;
-  if (found == NO_SLOT) {
-    raise_status(status, DGS_ERR_TABLE_FULL);
-    return;
-  }
-  // values only ever decrease, so a stale read can only cause a redundant atomic
-  if (*reinterpret_cast<volatile unsigned long long*>(&slots[found].val) > static_cast<unsigned long long>(i))
-    atomicMin(&slots[found].val, static_cast<unsigned long long>(i));
+  if (found == NO_SLOT) raise_status(status, DGS_ERR_TABLE_FULL);
 }
 
-// pass 2: input i is a first occurrence iff the stored minimum equals i;
-// the last CTA to finish turns the per-tile counts into offsets and publishes
-// the number of distinct keys
+// pass 2: input i is a first occurrence iff the stored minimum equals i.  A tile counts its first occurrences, learns
+// from the tiles before it where its labels begin, emits the keys and stores the labels in the slots; the last tile
+// publishes the number of distinct keys.
+// With a plan (n_edges != nullptr; the multi-hop sequence), the tile then reads the row bounds of the nodes it has
+// numbered -- they are the next hop's seeds -- and a second look-back places their outputs, so that the next hop needs
+// no plan launch.
+// Bound by dependent L2 round trips (slot, word, look-back, row bounds, second look-back), a tile's worth of keys per
+// CTA so that a mini-batch's tiles are all in flight together.  Counting, numbering and planning in launches of their
+// own (three per hop) a batch of 1 024 seeds and 826 k edges took 153 us of sampling sequence, this way 135 us; 880 k
+// keys by themselves 26 us for count + number, now 21.
+template <typename IdT, typename Keys, bool PLAN>
 __global__ void __launch_bounds__(RL_BLOCK)
-relabel_count_kernel(const Count nc, const Slot* __restrict__ slots, const bool compact,
-                     const uint32_t* __restrict__ slot_of, int64_t* tile_sums, unsigned int* ticket,
-                     int64_t* total_dev, int64_t* n_unique_out, const SizesReport report) {
-  __shared__ int s_cnt;
-  __shared__ int64_t s_scan[RL_BLOCK / 32 + 1];
+relabel_number_kernel(const __grid_constant__ Keys keys, const TableParts t, IdT* __restrict__ unique_out,
+                      const int64_t unique_capacity, int64_t* n_unique_out, const SizesReport report,
+                      const __grid_constant__ NextPlan plan, int32_t* __restrict__ status) {
+  __shared__ int64_t smem[RL_BLOCK / 32 + 1];
+  __shared__ TileScanShared<RL_BLOCK> s_tiles;
+  __shared__ unsigned int s_tile;
   pdl_enter();
-  if (threadIdx.x == 0) s_cnt = 0;
+  if (threadIdx.x == 0) s_tile = atomicAdd(t.ticket, 1u) + 1u;
   __syncthreads();
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * RL_TILE + threadIdx.x * RL_ITEMS;
-  // slot_of has room for nc.bound entries: read it while the live count is still on its way
-  uint32_t sl[RL_ITEMS];
-#pragma unroll
-  for (int u = 0; u < RL_ITEMS; ++u) sl[u] = base + u < nc.bound ? slot_of[base + u] : NO_SLOT;
-  const int64_t n = count_of(nc);
-  int c = 0;
-#pragma unroll
-  for (int u = 0; u < RL_ITEMS; ++u) {
-    const int64_t i = base + u;
-    if (i < n && sl[u] != NO_SLOT) {
-      const bool first =
-          compact ? reinterpret_cast<const uint2*>(slots)[sl[u]].x == static_cast<uint32_t>(i)  // low half of the word
-                  : slots[sl[u]].val == static_cast<unsigned long long>(i);
-      if (first) ++c;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(FULL_MASK, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_cnt, c);
-  __syncthreads();
-  const bool last = publish_and_scan_tiles<RL_BLOCK>(static_cast<int64_t>(s_cnt), tile_sums, ticket, total_dev,
-                                                     n_unique_out, s_scan);
-  if (last && threadIdx.x == 0 && report.n > 0) {  // same thread that wrote *total_dev just above
-    for (int k = 0; k < report.n; ++k) report.dst[k] = *report.src[k];
-    __threadfence_system();
-  }
-}
-
-// pass 3: number the first occurrences, emit them, store the label in the slot
-template <typename IdT, typename Keys>
-__global__ void __launch_bounds__(RL_BLOCK)
-relabel_number_kernel(const __grid_constant__ Keys keys, Slot* slots, const bool compact,
-                      const uint32_t* __restrict__ slot_of,
-                      const int64_t* __restrict__ tile_off, IdT* __restrict__ unique_out,
-                      const int64_t unique_capacity, int32_t* __restrict__ status) {
-  __shared__ int smem[RL_BLOCK / 32 + 1];
-  pdl_enter();
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * RL_TILE + threadIdx.x * RL_ITEMS;
-  bool first[RL_ITEMS];
-  uint32_t slot[RL_ITEMS];
+  const int64_t tile = s_tile;
+  const int64_t base = tile * RL_TILE + threadIdx.x * RL_ITEMS;
   const int64_t room = keys.bound();
-#pragma unroll
-  for (int u = 0; u < RL_ITEMS; ++u) slot[u] = base + u < room ? slot_of[base + u] : NO_SLOT;  // ahead of the count
+  uint32_t slot[RL_ITEMS] = {NO_SLOT, NO_SLOT, NO_SLOT, NO_SLOT};
+  if (base < room) {  // ahead of the count; the array is padded to 16 bytes
+    const uint4 v = *reinterpret_cast<const uint4*>(t.slot_of + base);
+    slot[0] = v.x;
+    slot[1] = v.y;
+    slot[2] = v.z;
+    slot[3] = v.w;
+  }
   const int64_t n = keys.size();
+  if (tile > 0 && tile * RL_TILE >= n) return;  // past the live keys
+  const bool last_tile = (tile + 1) * RL_TILE >= n;
+  bool first[RL_ITEMS];
   int c = 0;
 #pragma unroll
   for (int u = 0; u < RL_ITEMS; ++u) {
     const int64_t i = base + u;
-    first[u] = false;
-    if (i >= n) slot[u] = NO_SLOT;
-    if (i < n) {
-      // a slot already relabelled by another CTA carries LABEL_BIT and cannot equal i
-      if (slot[u] != NO_SLOT)
-        first[u] = compact ? *reinterpret_cast<const volatile uint32_t*>(reinterpret_cast<const uint2*>(slots) + slot[u]) ==
-                                 static_cast<uint32_t>(i)
-                           : *reinterpret_cast<const volatile unsigned long long*>(&slots[slot[u]].val) ==
-                                 static_cast<unsigned long long>(i);
-      c += first[u] ? 1 : 0;
+    // a slot already relabelled by another CTA carries LABEL_BIT32 and cannot equal i
+    first[u] = i < n && slot[u] != NO_SLOT &&
+               (*reinterpret_cast<const volatile uint32_t*>(reinterpret_cast<const uint2*>(t.words) + slot[u]) &
+                ~WIDE_BIT32) == static_cast<uint32_t>(i);
+    c += first[u] ? 1 : 0;
+  }
+  int64_t total;
+  const int64_t ex = block_exclusive_scan<int64_t, RL_BLOCK>(c, smem, &total);
+  const int64_t before = sum_of_tiles_before<RL_BLOCK>(tile, total, t.tiles, s_tiles, status);
+  if (last_tile && threadIdx.x == 0) {
+    *t.total = before + total;
+    if (n_unique_out != nullptr) {
+      *n_unique_out = before + total;
+      __threadfence_system();
+    }
+    if (report.n > 0) {  // the same thread that wrote *t.total just above
+      for (int k = 0; k < report.n; ++k) report.dst[k] = *report.src[k];
+      __threadfence_system();
     }
   }
-  int total;
-  const int ex = block_exclusive_scan<int, RL_BLOCK>(c, smem, &total);
-  int64_t label = tile_off[blockIdx.x] + ex;
+  int64_t label = before + ex;
+  int64_t id[RL_ITEMS];
 #pragma unroll
   for (int u = 0; u < RL_ITEMS; ++u) {
+    id[u] = -1;
     if (first[u]) {
-      if (label < unique_capacity) unique_out[label] = keys.template load<IdT>(base + u);
-      else raise_status(status, DGS_ERR_RANGE);
-      if (compact) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint2*>(slots) + slot[u]) = LABEL_BIT32 | static_cast<uint32_t>(label);
-      else slots[slot[u]].val = LABEL_BIT | static_cast<unsigned long long>(label);
+      const IdT key = keys.template load<IdT>(base + u);
+      if (label < unique_capacity) {
+        unique_out[label] = key;
+        id[u] = static_cast<int64_t>(key);
+      } else {
+        raise_status(status, DGS_ERR_RANGE);
+      }
+      uint32_t flag = 0u;
+      if (is_wide(static_cast<long long>(key))) {
+        flag = WIDE_BIT32;
+        t.wide_keys[label] = static_cast<long long>(key);
+      }
+      reinterpret_cast<uint2*>(t.words)[slot[u]].x = LABEL_BIT32 | flag | static_cast<uint32_t>(label);
       ++label;
     }
+  }
+  if (!PLAN) return;
+  label = before + ex;
+  int64_t rb[RL_ITEMS], deg[RL_ITEMS], cnt = 0;
+  bool good[RL_ITEMS];
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    good[u] = id[u] >= 0 && id[u] + 1 < plan.indptr.total;
+    if (id[u] >= 0 && !good[u]) raise_status(status, DGS_ERR_RANGE);
+  }
+  row_bounds<IdT, RL_ITEMS>(plan.indptr, id, good, rb, deg, status);
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) cnt += pick_count(deg[u], plan.k, plan.replace);
+  int64_t tile_edges;
+  int64_t at = block_exclusive_scan<int64_t, RL_BLOCK>(cnt, smem, &tile_edges);
+  at += sum_of_tiles_before<RL_BLOCK>(tile, tile_edges, t.tiles2, s_tiles, status);
+  if (last_tile && threadIdx.x == RL_BLOCK - 1) *plan.n_edges = at + cnt;
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    if (!first[u]) continue;
+    if (id[u] >= 0) {  // the list has room for it
+      plan.row_begin[label] = rb[u];
+      plan.deg[label] = deg[u];
+      plan.off[label] = at;
+    }
+    at += pick_count(deg[u], plan.k, plan.replace);
+    ++label;
   }
 }
 
@@ -255,12 +243,12 @@ relabel_number_kernel(const __grid_constant__ Keys keys, Slot* slots, const bool
 template <typename IdT>
 __global__ void __launch_bounds__(RL_BLOCK)
 relabel_lookup_kernel(const __grid_constant__ dgs_segments in, const int64_t n,
-                      const Slot* __restrict__ slots, const uint64_t mask, const bool compact,
-                      IdT* __restrict__ out) {
+                      const unsigned long long* __restrict__ words, const long long* __restrict__ wide_keys,
+                      const uint64_t mask, IdT* __restrict__ out) {
   pdl_enter();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * RL_BLOCK + threadIdx.x;
   if (i >= n) return;
-  out[i] = static_cast<IdT>(probe_label(slots, mask, static_cast<long long>(seg_load<IdT>(in, i)), compact));
+  out[i] = static_cast<IdT>(probe_label(words, wide_keys, mask, static_cast<long long>(seg_load<IdT>(in, i))));
 }
 
 // lookup of the sequence with device-side counts, when it does not ride on another launch
@@ -287,58 +275,59 @@ int check_segments(const dgs_segments* s, const char* who) {
 
 __global__ void zero_word_kernel(int64_t* w) { *w = 0; }
 
-// insert -> count -> number over a cleared table; n_bound sizes the grids
+// insert -> number over a cleared table; the bounds size the grids
 template <typename IdT, typename Keys>
-int run_unique(const Keys& keys, Count n_keys, const TableSize& size, const TableView& t, void* unique_out,
-               int64_t unique_capacity, int64_t* n_unique, const SizesReport& report, int32_t* status,
-               cudaStream_t s) {
-  const unsigned per_key_grid = static_cast<unsigned>((n_keys.bound + RL_BLOCK - 1) / RL_BLOCK);
-  DGS_CUDA_TRY(launch_chained(SITE_INSERT, relabel_insert_kernel<IdT, Keys>, per_key_grid, RL_BLOCK, s, keys, size, t.slots,
+int run_unique(const Keys& keys, int64_t n_bound, const TableSize& size, const TableParts& t, void* unique_out,
+               int64_t unique_capacity, int64_t* n_unique, const SizesReport& report, const NextPlan& plan,
+               int32_t* status, cudaStream_t s) {
+  const unsigned per_key_grid = static_cast<unsigned>((n_bound + RL_BLOCK - 1) / RL_BLOCK);
+  DGS_CUDA_TRY(launch_chained(SITE_INSERT, relabel_insert_kernel<IdT, Keys>, per_key_grid, RL_BLOCK, s, keys, size, t.words,
                               t.slot_of, status));
-  DGS_CUDA_TRY(launch_chained(SITE_COUNT, relabel_count_kernel, static_cast<unsigned>(t.ntiles), RL_BLOCK, s, n_keys, t.slots,
-                              size.compact, t.slot_of, t.tile_off, t.ticket, t.total, n_unique, report));
-  DGS_CUDA_TRY(launch_chained(SITE_NUMBER, relabel_number_kernel<IdT, Keys>, static_cast<unsigned>(t.ntiles), RL_BLOCK, s, keys,
-                              t.slots, size.compact, t.slot_of, t.tile_off, static_cast<IdT*>(unique_out), unique_capacity,
-                              status));
+  if constexpr (std::is_same<Keys, PairKeys>::value) {
+    if (plan.n_edges != nullptr) {
+      DGS_CUDA_TRY(launch_chained(SITE_NUMBER, relabel_number_kernel<IdT, Keys, true>, static_cast<unsigned>(t.ntiles),
+                                  RL_BLOCK, s, keys, t, static_cast<IdT*>(unique_out), unique_capacity, n_unique, report,
+                                  plan, status));
+      return DGS_OK;
+    }
+  }
+  DGS_CUDA_TRY(launch_chained(SITE_NUMBER, relabel_number_kernel<IdT, Keys, false>, static_cast<unsigned>(t.ntiles), RL_BLOCK,
+                              s, keys, t, static_cast<IdT*>(unique_out), unique_capacity, n_unique, report, plan, status));
   return DGS_OK;
 }
 
 }  // namespace
 
 int64_t* unique_total(void* table, int64_t key_bound) { return table_view(table, key_bound).total; }
-unsigned int* unique_ticket(void* table, int64_t key_bound) { return table_view(table, key_bound).ticket; }
 
 ClearJob make_clear_job(void* table, int64_t key_bound, const TableSize& size) {
-  const TableView t = table_view(table, key_bound);
-  return ClearJob{t.slots, size, static_cast<unsigned>((t.cap + CLEAR_SLOTS_PER_CTA - 1) / CLEAR_SLOTS_PER_CTA)};
+  const TableParts t = table_view(table, key_bound);
+  const int64_t units = static_cast<int64_t>(slots_for(key_bound) / 2) + ticket_units(t);
+  return ClearJob{t.words, t.ticket, ticket_units(t), size,
+                  static_cast<unsigned>((units + CLEAR_UNITS_PER_CTA - 1) / CLEAR_UNITS_PER_CTA)};
 }
 
-LookupJob make_lookup_job(const void* table, int64_t key_bound, const TableSize& size, const void* a, const void* b,
-                          Count n, void* out_a, void* out_b) {
-  const TableView t = table_view(const_cast<void*>(table), key_bound);
-  return LookupJob{a, b, out_a, out_b, n, t.slots, size, static_cast<unsigned>((n.bound + RL_BLOCK - 1) / RL_BLOCK)};
-}
-
-int launch_clear(const ClearJob& job, cudaStream_t s) {
-  if (job.ctas == 0) return DGS_OK;
-  DGS_CUDA_TRY(launch_chained(SITE_CLEAR, relabel_clear_kernel, job.ctas, RL_BLOCK, s, job));
-  return DGS_OK;
+LookupJob make_lookup_job(void* table, int64_t key_bound, const TableSize& size, void* row, void* col, Count n,
+                          Count n_seeds) {
+  const TableParts t = table_view(table, key_bound);
+  return LookupJob{row, col, n, n_seeds, t.words, t.slot_of, t.wide_keys, size,
+                   static_cast<unsigned>((n.bound + RL_BLOCK - 1) / RL_BLOCK)};
 }
 
 int launch_unique_pair(bool ids64, const void* a, Count na, const void* b, Count nb, int64_t key_bound,
                        const TableSize& size, void* table, void* unique_out, int64_t unique_capacity,
-                       int64_t* n_unique_out, const SizesReport& report, int32_t* status, cudaStream_t s) {
+                       int64_t* n_unique_out, const SizesReport& report, const NextPlan& plan, int32_t* status,
+                       cudaStream_t s) {
   DGS_REQUIRE(key_bound > 0 && key_bound < (1ll << 30) && na.bound + nb.bound <= key_bound, DGS_ERR_UNSUPPORTED,
               "relabel: %lld keys", (long long)key_bound);
   DGS_REQUIRE(na.dev != nullptr && nb.dev != nullptr && na.dev2 == nullptr && nb.dev2 == nullptr, DGS_ERR_INVALID,
               "relabel: the pair form takes one device word per length");
-  const TableView t = table_view(table, key_bound);
-  const Count n_keys{key_bound, na.dev, nb.dev};
+  const TableParts t = table_view(table, key_bound);
   const PairKeys keys{a, b, na, nb};
-  return ids64 ? run_unique<int64_t, PairKeys>(keys, n_keys, size, t, unique_out, unique_capacity, n_unique_out,
-                                               report, status, s)
-               : run_unique<int32_t, PairKeys>(keys, n_keys, size, t, unique_out, unique_capacity, n_unique_out,
-                                               report, status, s);
+  return ids64 ? run_unique<int64_t, PairKeys>(keys, key_bound, size, t, unique_out, unique_capacity, n_unique_out,
+                                               report, plan, status, s)
+               : run_unique<int32_t, PairKeys>(keys, key_bound, size, t, unique_out, unique_capacity, n_unique_out,
+                                               report, plan, status, s);
 }
 
 int launch_lookup(const LookupJob& job, bool ids64, cudaStream_t s) {
@@ -354,7 +343,7 @@ extern "C" size_t dgs_relabel_table_bytes(int64_t n) {
   using namespace dgs;
   if (n < 0) n = 0;
   const int64_t ntiles = (n + RL_TILE - 1) / RL_TILE;
-  return slots_for(n) * sizeof(Slot) + align_up(static_cast<size_t>(n) * sizeof(uint32_t), 16) +
+  return 2 * slots_for(n) * sizeof(unsigned long long) + align_up(static_cast<size_t>(n) * sizeof(uint32_t), 16) +
          static_cast<size_t>(ntiles + 2) * sizeof(int64_t);
 }
 
@@ -372,9 +361,10 @@ extern "C" int dgs_unique_first_occurrence(const dgs_segments* keys, int32_t ids
   DGS_REQUIRE((reinterpret_cast<uintptr_t>(table) & 15) == 0, DGS_ERR_INVALID,
               "dgs_unique_first_occurrence: table must be 16-byte aligned");
   DGS_REQUIRE(n < (1ll << 30), DGS_ERR_UNSUPPORTED, "dgs_unique_first_occurrence: %lld keys", (long long)n);
-  const TableView t = table_view(table, n);
+  const TableParts t = table_view(table, n);
+  // slots, ticket and tile words lie one behind the other
+  DGS_CUDA_TRY(cudaMemsetAsync(table, 0xFF, slots_for(n) * sizeof(unsigned long long) + ticket_units(t) * 16, s));
   if (n == 0) {
-    DGS_CUDA_TRY(cudaMemsetAsync(t.slots, 0xFF, t.cap * sizeof(Slot), s));
     if (n_unique != nullptr) {
       zero_word_kernel<<<1, 1, 0, s>>>(n_unique);
       DGS_LAUNCH_CHECK();
@@ -382,15 +372,10 @@ extern "C" int dgs_unique_first_occurrence(const dgs_segments* keys, int32_t ids
     return DGS_OK;
   }
   DGS_REQUIRE(unique_out != nullptr, DGS_ERR_INVALID, "dgs_unique_first_occurrence: null output");
-  DGS_CUDA_TRY(cudaMemsetAsync(t.slots, 0xFF, t.cap * sizeof(Slot), s));
-  DGS_CUDA_TRY(cudaMemsetAsync(t.ticket, 0, sizeof(unsigned int), s));
   const SegKeys sk{*keys, n};
-  // 32-bit ids always fit the one-word slots; for 64-bit ids this entry point knows nothing about the id space
-  const TableSize size{exact_count(n), 1, ids64 == 0};
-  return ids64 ? run_unique<int64_t, SegKeys>(sk, exact_count(n), size, t, unique_out, n, n_unique, SizesReport{},
-                                              status, s)
-               : run_unique<int32_t, SegKeys>(sk, exact_count(n), size, t, unique_out, n, n_unique, SizesReport{},
-                                              status, s);
+  const TableSize size{exact_count(n), 1, INT64_MAX};
+  return ids64 ? run_unique<int64_t, SegKeys>(sk, n, size, t, unique_out, n, n_unique, SizesReport{}, NextPlan{}, status, s)
+               : run_unique<int32_t, SegKeys>(sk, n, size, t, unique_out, n, n_unique, SizesReport{}, NextPlan{}, status, s);
 }
 
 extern "C" int dgs_relabel_lookup(const void* table, size_t table_bytes, int64_t n_keys_built,
@@ -405,14 +390,15 @@ extern "C" int dgs_relabel_lookup(const void* table, size_t table_bytes, int64_t
               DGS_ERR_INVALID, "dgs_relabel_lookup: bad table");
   DGS_REQUIRE(out != nullptr, DGS_ERR_INVALID, "dgs_relabel_lookup: null output");
   DGS_REQUIRE((n + RL_BLOCK - 1) / RL_BLOCK <= 0x7fffffffLL, DGS_ERR_UNSUPPORTED, "dgs_relabel_lookup: too many ids");
-  const TableView t = table_view(const_cast<void*>(table), n_keys_built);
+  const TableParts t = table_view(const_cast<void*>(table), n_keys_built);
+  const uint64_t mask = slots_for(n_keys_built) - 1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const unsigned grid = static_cast<unsigned>((n + RL_BLOCK - 1) / RL_BLOCK);
   if (ids64)
-    DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, relabel_lookup_kernel<int64_t>, grid, RL_BLOCK, s, *in, n, t.slots, t.cap - 1,
-                                false, static_cast<int64_t*>(out)));
-  else  // the table of dgs_unique_first_occurrence for 32-bit ids has one-word slots
-    DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, relabel_lookup_kernel<int32_t>, grid, RL_BLOCK, s, *in, n, t.slots, t.cap - 1,
-                                true, static_cast<int32_t*>(out)));
+    DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, relabel_lookup_kernel<int64_t>, grid, RL_BLOCK, s, *in, n, t.words, t.wide_keys,
+                                mask, static_cast<int64_t*>(out)));
+  else
+    DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, relabel_lookup_kernel<int32_t>, grid, RL_BLOCK, s, *in, n, t.words, t.wide_keys,
+                                mask, static_cast<int32_t*>(out)));
   return DGS_OK;
 }

@@ -8,26 +8,24 @@
 namespace dgs {
 
 constexpr int RL_BLOCK = 256;
-constexpr unsigned long long LABEL_BIT = 0x8000000000000000ull;
-constexpr long long EMPTY_KEY = -1;  // cleared slot: key = -1, value = 2^64-1
+constexpr int RL_ITEMS = 4;
+constexpr int RL_TILE = RL_BLOCK * RL_ITEMS;
 constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
-constexpr int CLEAR_SLOTS_PER_CTA = RL_BLOCK * 4;
+constexpr int CLEAR_UNITS_PER_CTA = RL_BLOCK * 4;  // of 16 bytes
 
-struct __align__(16) Slot {
-  long long key;
-  unsigned long long val;
-};
-
-// Compact tables: when every key is below 2^32 - 1 (32-bit ids, or 64-bit ids of a graph with fewer nodes
-// than that) a slot is ONE 64-bit word, key in the high half and the minimum input index (later the label)
-// in the low half.  Claiming a slot and setting its first index is then a single compare-and-swap, a
-// repeated key costs one load and at most one atomicMin, and every later pass reads 8 bytes per key instead
-// of 16; the table (and the clearing of it) is half the size.  Input indices and labels stay below 2^30
-// (the key count is limited to that), so bit 31 of the low half marks a label.  The same memory holds
-// either form: a table laid out for `cap` 16-byte slots uses its first half as `cap` compact slots.
-constexpr unsigned long long EMPTY_COMPACT = ~0ull;
+// A slot is ONE 64-bit word: the low 32 bits of the key in the high half, the minimum input index (later the label)
+// in the low half.  Claiming a slot and setting its first index is a single compare-and-swap, a repeated key costs
+// one load and at most one atomicMin, and every later pass reads 8 bytes per key.  Input indices and labels stay
+// below 2^30 (the key count is limited to that): bit 31 of the low half marks a label, bit 30 a key of 2^32 or more.
+// Two keys below 2^32 are equal when their words agree in the high half and in bit 30; such wide keys are compared in
+// full as well, with the input the index names or, once numbered, with the key kept beside the label (wide_keys).
+// (64-bit ids used to have 16-byte {key, index} slots: 880 k keys took 27 + 18 + 25 + 27 us for insert, count,
+// number and lookup where the one-word form of the multi-hop sequence took 21 + 16 + 26 + 22.)
+constexpr unsigned long long EMPTY_WORD = ~0ull;
 constexpr uint32_t LABEL_BIT32 = 0x80000000u;
-constexpr long long COMPACT_KEY_LIMIT = 0xFFFFFFFFll;  // keys must be below this
+constexpr uint32_t WIDE_BIT32 = 0x40000000u;
+constexpr uint32_t VALUE_MASK32 = 0x3FFFFFFFu;
+constexpr long long COMPACT_KEY_LIMIT = 0xFFFFFFFFll;  // ids of a graph with fewer nodes than this
 
 // slots in use for a table built for n keys: the power of two >= max(2n, 64)
 __host__ __device__ __forceinline__ uint64_t slots_for(int64_t n) {
@@ -48,7 +46,19 @@ __host__ __device__ __forceinline__ uint64_t slots_for(int64_t n) {
 struct TableSize {
   Count n;
   int64_t mult;
-  bool compact;  // one-word slots (see above)
+  long long max_key;  // keys above are out of range
+};
+
+// The device arrays of one table.
+struct TableParts {
+  unsigned long long* words;    // [cap]
+  unsigned int* ticket;         // [4]       all ones when cleared: the first draw is 0
+  unsigned long long* tiles;    // [ntiles]  running count of distinct keys, see tile_scan.cuh
+  unsigned long long* tiles2;   // [ntiles]  the same of the edges that the distinct keys will be given
+  long long* wide_keys;         // [n]       by label: keys of 2^32 and more (64-bit ids only)
+  uint32_t* slot_of;            // [n]       slot of every input
+  int64_t* total;               // [1]
+  int64_t ntiles;
 };
 
 // Sizes that only the host needs (how much of each output is valid): device words copied to a
@@ -81,74 +91,75 @@ __device__ __forceinline__ uint32_t hash_key32(uint32_t k) {
   return k ^ (k >> 16);
 }
 
-__device__ __forceinline__ long long probe_label(const Slot* __restrict__ slots, uint64_t mask, long long key,
-                                                 bool compact) {
+__device__ __forceinline__ bool is_wide(long long key) { return (static_cast<unsigned long long>(key) >> 32) != 0; }
+__device__ __forceinline__ uint32_t home_slot(long long key, uint32_t mask32) {
+  return (is_wide(key) ? static_cast<uint32_t>(hash_key(key)) : hash_key32(static_cast<uint32_t>(key))) & mask32;
+}
+
+__device__ __forceinline__ long long probe_label(const unsigned long long* words, const long long* wide_keys,
+                                                 uint64_t mask, long long key) {
   if (key < 0) return -1;
-  if (compact) {
-    if (key >= COMPACT_KEY_LIMIT) return -1;
-    const unsigned long long* __restrict__ words = reinterpret_cast<const unsigned long long*>(slots);
-    const uint32_t mask32 = static_cast<uint32_t>(mask), key32 = static_cast<uint32_t>(key);
-    uint32_t h = hash_key32(key32) & mask32;
-    for (uint32_t probes = 0; probes <= mask32; ++probes) {
-      const uint2 w = reinterpret_cast<const uint2*>(words)[h];  // one 8-byte load: x = index / label, y = key
-      if (w.y == key32) return static_cast<long long>(w.x & ~LABEL_BIT32);
-      if ((w.x & w.y) == 0xFFFFFFFFu) break;                     // empty slot
-      h = (h + 1) & mask32;
+  const uint32_t mask32 = static_cast<uint32_t>(mask), key32 = static_cast<uint32_t>(key);
+  const uint32_t flag = is_wide(key) ? WIDE_BIT32 : 0u;
+  uint32_t h = home_slot(key, mask32);
+  for (uint32_t probes = 0; probes <= mask32; ++probes) {
+    const uint2 w = reinterpret_cast<const uint2*>(words)[h];  // one 8-byte load: x = index / label, y = key
+    if ((w.x & w.y) == 0xFFFFFFFFu) break;                     // empty slot
+    if (w.y == key32 && (w.x & WIDE_BIT32) == flag) {
+      const uint32_t label = w.x & VALUE_MASK32;
+      if (flag == 0u || wide_keys[label] == key) return static_cast<long long>(label);
     }
-    return -1;
-  }
-  uint64_t h = hash_key(key) & mask;
-  for (uint64_t probes = 0; probes <= mask; ++probes) {
-    const Slot s = slots[h];  // one 16-byte load
-    if (s.key == key) return static_cast<long long>(s.val & ~LABEL_BIT);
-    if (s.key == EMPTY_KEY) break;
-    h = (h + 1) & mask;
+    h = (h + 1) & mask32;
   }
   return -1;
 }
 
 // ---- jobs that can ride on another kernel's launch -----------------------------
-// Clear the slots a table will use.  Runs before anything touches the table.
+// Clear the slots a table will use, its ticket and its tile words.  Runs before anything touches the table.
 struct ClearJob {
-  Slot* slots;
+  unsigned long long* words;
+  unsigned int* ticket;   // ticket and tile words are one run of 16-byte units
+  int64_t ticket_units;
   TableSize size;
-  unsigned ctas;  // CLEAR_SLOTS_PER_CTA slots each; 0: no job
+  unsigned ctas;  // CLEAR_UNITS_PER_CTA units each; 0: no job
 };
 __device__ __forceinline__ void run_clear_cta(const ClearJob& j, unsigned cta) {
-  // in 16-byte units: compact slots are half as wide
-  const uint64_t cap = j.size.compact ? table_slots(j.size) / 2 : table_slots(j.size);
-  const uint64_t i = static_cast<uint64_t>(cta) * CLEAR_SLOTS_PER_CTA + threadIdx.x;
+  const int64_t slots = static_cast<int64_t>(table_slots(j.size) / 2);  // two to a unit
+  const int64_t i = static_cast<int64_t>(cta) * CLEAR_UNITS_PER_CTA + threadIdx.x;
   const ulonglong2 empty = make_ulonglong2(~0ull, ~0ull);
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const uint64_t at = i + static_cast<uint64_t>(u) * RL_BLOCK;
-    if (at < cap) *reinterpret_cast<ulonglong2*>(&j.slots[at]) = empty;
+    const int64_t at = i + static_cast<int64_t>(u) * RL_BLOCK;
+    if (at < slots) reinterpret_cast<ulonglong2*>(j.words)[at] = empty;
+    else if (at - slots < j.ticket_units) reinterpret_cast<ulonglong2*>(j.ticket)[at - slots] = empty;
   }
 }
 
-// Relabel a finished hop's COO: out_a[i] = label(a[i]) (skipped when a is null),
-// out_b[i] = label(b[i]), i < n; in place is fine.  Needs that hop's numbering.
+// Relabel a finished hop's COO in place: row[i] = label(row[i]) (skipped when row is null), and col[i] = the label
+// in the slot that input n_seeds + i was inserted at, i < n.  Needs that hop's numbering.
 struct LookupJob {
-  const void* a;
-  const void* b;
-  void* out_a;
-  void* out_b;
-  Count n;
-  const Slot* slots;
+  void* row;
+  void* col;
+  Count n, n_seeds;
+  const unsigned long long* words;
+  const uint32_t* slot_of;
+  const long long* wide_keys;
   TableSize size;
   unsigned ctas;  // RL_BLOCK ids each; 0: no job
 };
 template <typename IdT>
 __device__ __forceinline__ void run_lookup_cta(const LookupJob& j, unsigned cta) {
   const int64_t i = static_cast<int64_t>(cta) * RL_BLOCK + threadIdx.x;
-  // the ids are read while the live count and the table size are still on their way (room for n.bound ids)
-  const bool in_bound = i < j.n.bound;
-  const long long ka = (in_bound && j.a != nullptr) ? static_cast<long long>(static_cast<const IdT*>(j.a)[i]) : -1;
-  const long long kb = in_bound ? static_cast<long long>(static_cast<const IdT*>(j.b)[i]) : -1;
+  // what does not depend on the live counts is read while they are on their way (room for n.bound ids)
+  const long long kr = (i < j.n.bound && j.row != nullptr) ? static_cast<long long>(static_cast<const IdT*>(j.row)[i]) : -1;
+  const int64_t n_seeds = count_of(j.n_seeds);
   if (i >= count_of(j.n)) return;
-  const uint64_t mask = table_slots(j.size) - 1;
-  if (j.a != nullptr) static_cast<IdT*>(j.out_a)[i] = static_cast<IdT>(probe_label(j.slots, mask, ka, j.size.compact));
-  static_cast<IdT*>(j.out_b)[i] = static_cast<IdT>(probe_label(j.slots, mask, kb, j.size.compact));
+  const uint32_t slot = j.slot_of[n_seeds + i];
+  if (j.row != nullptr)
+    static_cast<IdT*>(j.row)[i] = static_cast<IdT>(probe_label(j.words, j.wide_keys, table_slots(j.size) - 1, kr));
+  static_cast<IdT*>(j.col)[i] =
+      slot == NO_SLOT ? static_cast<IdT>(-1)
+                      : static_cast<IdT>(reinterpret_cast<const uint2*>(j.words)[slot].x & VALUE_MASK32);
 }
 
 #endif  // __CUDACC__

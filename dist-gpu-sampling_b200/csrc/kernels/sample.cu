@@ -46,6 +46,7 @@
 #include "common.cuh"
 #include "launchers.h"
 #include "philox.cuh"
+#include "sample_device.cuh"
 #include "tile_scan.cuh"
 
 namespace dgs {
@@ -54,9 +55,6 @@ namespace {
 constexpr int SAMPLE_TILE = 256;   // seeds per CTA
 constexpr int SAMPLE_BLOCK = 256;  // threads per CTA
 
-constexpr uint32_t TAG_UNIFORM = 0x554E4931u;
-constexpr uint32_t TAG_REPLACE = 0x5245504Cu;
-constexpr uint32_t TAG_FLOYD = 0x464C4F59u;
 constexpr uint32_t TAG_ARES = 0x41524553u;
 constexpr uint32_t TAG_WREPL = 0x57524550u;
 
@@ -82,10 +80,6 @@ inline PlanView plan_view(void* plan, int64_t n) {
   return v;
 }
 
-__device__ __forceinline__ int64_t pick_count(int64_t deg, int64_t k, bool replace) {
-  return replace ? (deg > 0 ? k : 0) : (deg < k ? deg : k);
-}
-
 // ---------------------------------------------------------------------------
 // plan: row range per seed + per-tile output counts
 // ---------------------------------------------------------------------------
@@ -95,17 +89,9 @@ sample_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __r
                    const Count nc, const int64_t k, const bool replace,
                    int64_t* __restrict__ row_begin, int64_t* __restrict__ deg_out,
                    int64_t* __restrict__ local_off, int64_t* tile_sums, int64_t* total_out,
-                   unsigned int* ticket, int64_t* nnz_out, const unsigned int plan_tiles,
-                   const ClearJob clear, const LookupJob lookup, int32_t* __restrict__ status) {
+                   unsigned int* ticket, int64_t* nnz_out, int32_t* __restrict__ status) {
   __shared__ int64_t smem[SAMPLE_BLOCK / 32 + 1];
-  constexpr int sh = sizeof(IdT) == 8 ? 3 : 2;
   pdl_enter();
-  if (blockIdx.x >= plan_tiles) {  // CTAs beyond the plan's tiles carry the independent jobs
-    const unsigned int extra = blockIdx.x - plan_tiles;
-    if (extra < clear.ctas) run_clear_cta(clear, extra);
-    else run_lookup_cta<IdT>(lookup, extra - clear.ctas);
-    return;
-  }
   const int64_t i = static_cast<int64_t>(blockIdx.x) * SAMPLE_TILE + threadIdx.x;
   // the seed is read before the live count arrives (the list has room for nc.bound entries), so that
   // the two round trips overlap; an entry past the count is never used
@@ -114,79 +100,34 @@ sample_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __r
   const int64_t s = static_cast<int64_t>(seed_raw);
   const bool good = i < n && s >= 0 && s + 1 < indptr.total;
   if (i < n && !good) raise_status(status, DGS_ERR_RANGE);
-  // indptr[s] and indptr[s + 1] are fetched by TWO NEIGHBOURING LANES in one load instruction, half a warp's
-  // seeds at a time: the two addresses (almost always) lie in the same 128-byte line, so the pair costs one
-  // memory request instead of the two that two loads of one thread cost.  Inside one GPU that is noise; when
-  // the row of indptr lives on a peer, requests are what the link can deliver only so many of per second.
-  const int lane = threadIdx.x & 31;
-  int64_t pair[2] = {0, 0};  // this lane's (row begin, row end) after the two half-warp passes
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int owner = half * 16 + (lane >> 1);  // the lane whose seed this lane fetches an element for
-    const int64_t so = __shfl_sync(FULL_MASK, s, owner);
-    const bool ok = __shfl_sync(FULL_MASK, good ? 1 : 0, owner) != 0;
-    const int64_t v = ok ? static_cast<int64_t>(load_at<IdT>(indptr, sh, so + (lane & 1))) : 0;
-    const int64_t lo = __shfl_sync(FULL_MASK, v, 2 * (lane & 15));
-    const int64_t hi = __shfl_sync(FULL_MASK, v, 2 * (lane & 15) + 1);
-    if ((lane >> 4) == half) {
-      pair[0] = lo;
-      pair[1] = hi;
-    }
-  }
+  const int64_t seed[1] = {s};
+  const bool ok[1] = {good};
+  int64_t rb[1], deg[1];
+  row_bounds<IdT, 1>(indptr, seed, ok, rb, deg, status);
   int64_t cnt = 0;
   if (i < n) {
-    int64_t rb = 0, deg = 0;
-    if (good) {
-      rb = pair[0];
-      deg = pair[1] - rb;
-      if (deg < 0 || rb < 0) {
-        raise_status(status, DGS_ERR_RANGE);
-        deg = 0;
-        rb = 0;
-      }
-    }
-    row_begin[i] = rb;
-    deg_out[i] = deg;
-    cnt = pick_count(deg, k, replace);
+    row_begin[i] = rb[0];
+    deg_out[i] = deg[0];
+    cnt = pick_count(deg[0], k, replace);
   }
   int64_t total;
   const int64_t ex = block_exclusive_scan<int64_t, SAMPLE_BLOCK>(cnt, smem, &total);
   if (i < n) local_off[i] = ex;
 
   // publish the tile sum; the CTA that draws the last ticket scans all of them
-  publish_and_scan_tiles<SAMPLE_BLOCK>(total, tile_sums, ticket, total_out, nnz_out, smem, plan_tiles);
+  publish_and_scan_tiles<SAMPLE_BLOCK>(total, tile_sums, ticket, total_out, nnz_out, smem);
 }
 
-// ---------------------------------------------------------------------------
-// shared pieces of the sampling kernels
-// ---------------------------------------------------------------------------
+// CTAs of a sampling launch beyond the main ones carry two jobs of the multi-hop sequence that depend on nothing the
+// launch does: clearing the table this hop will fill, relabelling the COO of the hop before.
 template <typename IdT>
-struct Emit {
-  const dgs_chunk_desc& indices;
-  IdT* coo_row;
-  IdT* coo_col;
-  int64_t* picked_pos;
-  int64_t out_capacity;
-  int32_t* status;
-
-  // t-th output of a seed whose outputs start at o; `pos` = position in its row
-  __device__ __forceinline__ void operator()(int64_t o, int64_t t, int64_t seed, int64_t rb,
-                                             int64_t pos) const {
-    constexpr int sh = sizeof(IdT) == 8 ? 3 : 2;
-    const int64_t at = o + t;
-    if (at >= out_capacity) {
-      raise_status(status, DGS_ERR_RANGE);
-      return;
-    }
-    const int64_t e = rb + pos;
-    IdT c = static_cast<IdT>(-1);
-    if (e >= 0 && e < indices.total) c = load_at<IdT>(indices, sh, e);
-    else raise_status(status, DGS_ERR_RANGE);
-    coo_row[at] = static_cast<IdT>(seed);
-    coo_col[at] = c;
-    if (picked_pos != nullptr) picked_pos[at] = pos;
-  }
-};
+__device__ __forceinline__ bool run_side_job(const SideJobs& jobs) {
+  if (blockIdx.x < jobs.main_ctas) return false;
+  const unsigned int extra = blockIdx.x - jobs.main_ctas;
+  if (extra < jobs.clear.ctas) run_clear_cta(jobs.clear, extra);
+  else run_lookup_cta<IdT>(jobs.lookup, extra - jobs.clear.ctas);
+  return true;
+}
 
 // What a group / warp needs to know about its seed.
 struct SeedPlan {
@@ -200,7 +141,7 @@ __device__ __forceinline__ SeedPlan seed_plan(const int64_t* __restrict__ plan_r
   if (valid) {
     p.rb = plan_rb[i];
     p.deg = plan_deg[i];
-    p.o = tile_off[i / SAMPLE_TILE] + local_off[i];
+    p.o = (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0) + local_off[i];
   }
   return p;
 }
@@ -216,143 +157,27 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
                       const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                       const RngKey rng, IdT* coo_row, IdT* coo_col,
                       const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                      const bool row_is_position, int32_t* __restrict__ status) {
+                      const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                      int32_t* __restrict__ status) {
   const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
   pdl_enter();
+  if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng);
   constexpr int GROUPS = SAMPLE_BLOCK / G;  // seeds per CTA
-  constexpr int TAKEN_WORDS = 4096;         // 16 KB of position bitmaps per CTA, split between its groups
-  __shared__ uint32_t s_taken[TAKEN_WORDS];
-  const int lane = threadIdx.x & 31;
-  const int l = threadIdx.x % G;        // lane inside the group
-  const int group = threadIdx.x / G;    // group inside the CTA
-  const int gw = lane / G;              // group inside the warp
-  const unsigned gmask = (G == 32) ? FULL_MASK : (((1u << G) - 1u) << (gw * G));
-  const bool fast = !replace && k <= G;  // uniform over the grid
-
-  {  // one seed per group; all 32 lanes of a warp walk through the same code
-    const int64_t slot = static_cast<int64_t>(blockIdx.x) * GROUPS + group;
-    // everything that only needs the slot is read before the live count arrives (all arrays have room for
-    // nc.bound entries); what belongs to a slot past the count is dropped below
-    const bool in_bound = slot < nc.bound;
-    const int64_t i = slot;  // the seed this group serves
-    const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i, in_bound);
-    const int64_t seed_raw = !in_bound ? 0 : (row_is_position ? i : static_cast<int64_t>(seeds[i]));
-    const bool valid = slot < count_of(nc);
-    const int64_t deg = valid ? sp.deg : 0, rb = valid ? sp.rb : 0, o = valid ? sp.o : 0;
-    const int64_t seed = valid ? seed_raw : 0;
-    const uint32_t i_lo = static_cast<uint32_t>(i), i_hi = static_cast<uint32_t>(static_cast<uint64_t>(i) >> 32);
-
-    if (replace) {
-      if (valid && deg > 0)
-        for (int64_t t = l; t < k; t += G) {
-          const Philox4 r = philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(t), TAG_REPLACE);
-          emit(o, t, seed, rb, static_cast<int64_t>(bounded(r, static_cast<uint64_t>(deg))));
-        }
-      return;
-    }
-
-    if (fast) {
-      // -- distinct positions by parallel rejection (all 32 lanes take part) --
-      // Every lane of a group draws a position and marks it in the group's bitmap
-      // in shared memory; a lane that finds its bit already set draws again.  Only
-      // equality of positions matters, so every k-subset is equally likely.
-      constexpr int WORDS = TAKEN_WORDS / GROUPS;         // bitmap words per group
-      constexpr int64_t MAP_DEG = static_cast<int64_t>(WORDS) * 32;
-      uint32_t* taken = s_taken + group * WORDS;
-      const bool sampled = valid && deg > k;
-      const bool complement = sampled && 2 * k > deg;  // draw the deg-k positions to leave out
-      const int64_t m = sampled ? (complement ? deg - k : k) : 0;
-      const bool active = l < m;
-      const bool in_map = deg <= MAP_DEG;              // longer rows compare candidates across the warp
-      if (sampled && in_map)
-        for (int wd = l; wd < static_cast<int>((deg + 31) >> 5); wd += G) taken[wd] = 0u;
-      __syncwarp();
-      bool need = active;
-      int64_t c = 0;
-      const bool small_row = deg <= 0xFFFFFFFFll;  // every real graph; longer rows take the general path
-      const uint32_t deg32 = static_cast<uint32_t>(deg);
-      Philox4 rnd{0u, 0u, 0u, 0u};
-      for (uint32_t round = 0; __any_sync(FULL_MASK, need); ++round) {
-        // one Philox block per lane feeds four rounds of (re)draws
-        if ((round & 3u) == 0u && active && round < 64)
-          rnd = philox4x32_10(key, i_lo, i_hi, ((round >> 2) << 8) | static_cast<uint32_t>(l), TAG_UNIFORM);
-        bool usable = true;  // false: this attempt hit Lemire's rejection zone, draw again next round
-        if (need) {
-          if (round >= 64) {  // never reached in practice: step to a neighbour, keeps the loop bounded
-            c = (c + 1 == deg) ? 0 : c + 1;
-          } else if (small_row) {
-            const uint32_t word = (round & 2u) ? ((round & 1u) ? rnd.w : rnd.z) : ((round & 1u) ? rnd.y : rnd.x);
-            uint32_t pick;
-            usable = bounded_try(word, deg32, &pick);
-            c = pick;
-          } else {
-            const Philox4 r = philox4x32_10(key, i_lo, i_hi, (round << 8) | static_cast<uint32_t>(l), TAG_UNIFORM ^ 1u);
-            c = static_cast<int64_t>(bounded(r, static_cast<uint64_t>(deg)));
-          }
-          if (in_map && usable) {
-            const uint32_t bit = 1u << (static_cast<uint32_t>(c) & 31u);
-            need = (atomicOr(&taken[c >> 5], bit) & bit) != 0u;
-          }
-        }
-        if (__any_sync(FULL_MASK, active && !in_map)) {
-          // lanes holding the same position inside one group see each other; the lowest keeps it
-          const bool mine = active && !in_map;
-          const unsigned long long tag =
-              (mine && usable) ? (static_cast<unsigned long long>(c) | (static_cast<unsigned long long>(gw) << 58))
-                               : (0x8000000000000000ull | static_cast<unsigned long long>(lane));
-          const unsigned same = __match_any_sync(FULL_MASK, tag);
-          if (mine) need = !usable || (__ffs(same) - 1 != lane);
-        }
-        if (round >= 64 + 1024) {
-          if (need) raise_status(status, DGS_ERR_TABLE_FULL);
-          break;
-        }
-      }
-      __syncwarp();
-      if (complement) {
-        // the row has at most 2k-1 <= 63 positions, so its bitmap is one or two words:
-        // every lane ranks its own two positions (a = l and b = l + G cover the row)
-        // among the kept ones
-        const unsigned long long out_mask =
-            static_cast<unsigned long long>(taken[0]) |
-            (deg > 32 ? static_cast<unsigned long long>(taken[1]) << 32 : 0ull);
-        const unsigned long long row_mask = (1ull << deg) - 1ull;  // deg <= 63
-        const unsigned long long kept = ~out_mask & row_mask;
-        const int a = l, b = l + G;
-        if ((kept >> a) & 1ull) emit(o, __popcll(kept & ((1ull << a) - 1ull)), seed, rb, a);
-        if (b < 64 && ((kept >> b) & 1ull)) emit(o, __popcll(kept & ((1ull << b) - 1ull)), seed, rb, b);
-      }
-      if (sampled && !complement) {
-        if (active) emit(o, l, seed, rb, c);
-      } else if (valid && !sampled) {
-        if (l < deg) emit(o, l, seed, rb, l);  // whole row, CSC order (deg <= k <= G)
-      }
-      return;
-    }
-
-    // -- general k (> G is only possible with G == 32: the group is the warp) --
-    if (!valid) return;
-    if (deg <= k) {
-      for (int64_t t = l; t < deg; t += G) emit(o, t, seed, rb, t);
-    } else if (o + k > out_capacity) {
-      if (l == 0) raise_status(status, DGS_ERR_RANGE);
-    } else {
-      // Floyd's subset algorithm; the chosen positions are parked in coo_col
-      volatile IdT* slots = coo_col + o;
-      int64_t have = 0;
-      for (int64_t j = deg - k; j < deg; ++j, ++have) {
-        const Philox4 r = philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(have), TAG_FLOYD);
-        const int64_t t = static_cast<int64_t>(bounded(r, static_cast<uint64_t>(j + 1)));
-        bool found = false;
-        for (int64_t q = l; q < have; q += G) found |= (static_cast<int64_t>(slots[q]) == t);
-        found = __any_sync(gmask, found);
-        if (l == 0) slots[have] = static_cast<IdT>(found ? j : t);
-        __syncwarp(gmask);
-      }
-      for (int64_t q = l; q < k; q += G) emit(o, q, seed, rb, static_cast<int64_t>(slots[q]));
-    }
-  }
+  __shared__ uint32_t s_taken[SAMPLE_BLOCK * TAKEN_WORDS_PER_LANE];
+  const int group = threadIdx.x / G;  // group inside the CTA
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * GROUPS + group;  // the seed this group serves
+  // everything that only needs the slot is read before the live count arrives (all arrays have room for
+  // nc.bound entries); what belongs to a slot past the count is dropped below
+  const bool in_bound = i < nc.bound;
+  const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i, in_bound);
+  const int64_t seed_raw = !in_bound ? 0 : (row_is_position ? i : static_cast<int64_t>(seeds[i]));
+  const bool valid = i < count_of(nc);
+  const int64_t o = valid ? sp.o : 0;
+  if (!sample_uniform_row(key, i, valid ? sp.deg : 0, k, replace, G, s_taken + group * (G * TAKEN_WORDS_PER_LANE),
+                          coo_col + o, o + k <= out_capacity, status,
+                          [&](int64_t t, int64_t pos) { emit(o, t, seed_raw, sp.rb, pos); }))
+    raise_status(status, DGS_ERR_RANGE);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,9 +482,11 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
                        const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                        const RngKey rng, IdT* coo_row, IdT* coo_col,
                        const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                       const bool row_is_position, int32_t* __restrict__ status) {
+                       const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                       int32_t* __restrict__ status) {
   const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
   pdl_enter();
+  if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng) ^ (static_cast<uint64_t>(TAG_ARES) << 32);
   const int64_t n = count_of(nc);
   const int l = threadIdx.x & 31;
@@ -859,9 +686,11 @@ sample_weighted_replace_kernel(const __grid_constant__ dgs_chunk_desc indices,
                                const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                                const RngKey rng, IdT* coo_row, IdT* coo_col,
                                const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                               const bool row_is_position, int32_t* __restrict__ status) {
+                               const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                               int32_t* __restrict__ status) {
   const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
   pdl_enter();
+  if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng);
   const int64_t n = count_of(nc);
   const int l = threadIdx.x & 31;
@@ -977,25 +806,26 @@ int check_sample_args(const char* who, const void* seeds, int64_t n, int64_t k, 
 
 template <typename IdT>
 int plan_typed(const dgs_chunk_desc& indptr, const void* seeds, Count n, int64_t k, bool replace,
-               const PlanView& pv, int64_t* nnz, const ClearJob& clear, const LookupJob& lookup, int32_t* status,
-               cudaStream_t s) {
-  const unsigned tiles = static_cast<unsigned>(pv.ntiles);
-  DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_plan_kernel<IdT>, tiles + clear.ctas + lookup.ctas, SAMPLE_BLOCK, s, indptr,
+               const PlanView& pv, int64_t* nnz, int32_t* status, cudaStream_t s) {
+  DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_plan_kernel<IdT>, static_cast<unsigned>(pv.ntiles), SAMPLE_BLOCK, s, indptr,
                               static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, pv.local_off,
-                              pv.tile_off, pv.total, pv.ticket, nnz, tiles, clear, lookup, status));
+                              pv.tile_off, pv.total, pv.ticket, nnz, status));
   return DGS_OK;
 }
 
 template <typename IdT>
 int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int64_t k, bool replace,
                   const PlanView& pv, RngKey key, void* coo_row, void* coo_col,
-                  int64_t cap, int64_t* pos, bool rowpos, int32_t* status, cudaStream_t s) {
-#define DGS_LAUNCH_U(G)                                                                                      \
-  DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, sample_uniform_kernel<IdT, G>,                                                 \
-                              static_cast<unsigned>((n.bound + SAMPLE_BLOCK / G - 1) / (SAMPLE_BLOCK / G)),  \
-                              SAMPLE_BLOCK, s, indices, static_cast<const IdT*>(seeds), n, k, replace,       \
-                              pv.row_begin, pv.deg, pv.local_off, pv.tile_off, key,                          \
-                              static_cast<IdT*>(coo_row), static_cast<IdT*>(coo_col), cap, pos, rowpos, status))
+                  int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, int32_t* status, cudaStream_t s) {
+#define DGS_LAUNCH_U(G)                                                                                       \
+  do {                                                                                                        \
+    jobs.main_ctas = static_cast<unsigned>((n.bound + SAMPLE_BLOCK / G - 1) / (SAMPLE_BLOCK / G));            \
+    DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, sample_uniform_kernel<IdT, G>,                                   \
+                                jobs.main_ctas + jobs.clear.ctas + jobs.lookup.ctas, SAMPLE_BLOCK, s,         \
+                                indices, static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, \
+                                pv.local_off, pv.tile_off, key, static_cast<IdT*>(coo_row),                   \
+                                static_cast<IdT*>(coo_col), cap, pos, rowpos, jobs, status));                 \
+  } while (0)
   if (k <= 4) DGS_LAUNCH_U(4);
   else if (k <= 8) DGS_LAUNCH_U(8);
   else if (k <= 16) DGS_LAUNCH_U(16);
@@ -1007,14 +837,14 @@ int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int
 template <typename IdT>
 int weighted_typed(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds, Count n,
                    int64_t k, bool replace, const PlanView& pv, RngKey key,
-                   void* coo_row, void* coo_col, int64_t cap, int64_t* pos, bool rowpos, int32_t* status,
+                   void* coo_row, void* coo_col, int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, int32_t* status,
                    cudaStream_t s) {
-  const unsigned grid = static_cast<unsigned>((n.bound + WEIGHTED_WARPS - 1) / WEIGHTED_WARPS);
+  jobs.main_ctas = static_cast<unsigned>((n.bound + WEIGHTED_WARPS - 1) / WEIGHTED_WARPS);
   auto kernel = replace ? sample_weighted_replace_kernel<IdT> : sample_weighted_kernel<IdT>;
-  DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, kernel, grid, SAMPLE_BLOCK, s, indices, probs,
-                              static_cast<const IdT*>(seeds), n, k, pv.row_begin, pv.deg, pv.local_off,
+  DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, kernel, jobs.main_ctas + jobs.clear.ctas + jobs.lookup.ctas, SAMPLE_BLOCK, s,
+                              indices, probs, static_cast<const IdT*>(seeds), n, k, pv.row_begin, pv.deg, pv.local_off,
                               pv.tile_off, key, static_cast<IdT*>(coo_row), static_cast<IdT*>(coo_col), cap,
-                              pos, rowpos, status));
+                              pos, rowpos, jobs, status));
   return DGS_OK;
 }
 
@@ -1028,35 +858,42 @@ uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset) {
 }
 
 int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, Count n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, const ClearJob& clear,
-                       const LookupJob& lookup, int32_t* status, cudaStream_t s) {
-  static_assert(SAMPLE_BLOCK == RL_BLOCK, "the jobs riding on the plan launch assume its CTA size");
+                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, int32_t* status, cudaStream_t s) {
   const PlanView pv = plan_view(plan, n.bound);
   if (zero_ticket) DGS_CUDA_TRY(cudaMemsetAsync(pv.ticket, 0, sizeof(unsigned int), s));
-  return ids64 ? plan_typed<int64_t>(indptr, seeds, n, k, replace, pv, nnz_out, clear, lookup, status, s)
-               : plan_typed<int32_t>(indptr, seeds, n, k, replace, pv, nnz_out, clear, lookup, status, s);
+  return ids64 ? plan_typed<int64_t>(indptr, seeds, n, k, replace, pv, nnz_out, status, s)
+               : plan_typed<int32_t>(indptr, seeds, n, k, replace, pv, nnz_out, status, s);
+}
+
+NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k, bool replace, void* plan) {
+  const PlanView pv = plan_view(plan, n_bound);
+  return NextPlan{indptr, k, replace, pv.row_begin, pv.deg, pv.local_off, pv.total};
 }
 
 int launch_sample_uniform(const dgs_chunk_desc& indices, const void* seeds, bool ids64, Count n, int64_t k,
-                          bool replace, void* plan, RngKey key, void* coo_row,
+                          bool replace, void* plan, bool whole_offsets, RngKey key, void* coo_row,
                           void* coo_col, int64_t out_capacity, int64_t* picked_pos, bool row_is_position,
-                          int32_t* status, cudaStream_t s) {
-  const PlanView pv = plan_view(plan, n.bound);
+                          const SideJobs& jobs, int32_t* status, cudaStream_t s) {
+  static_assert(SAMPLE_BLOCK == RL_BLOCK, "the jobs riding on the sampling launch assume its CTA size");
+  PlanView pv = plan_view(plan, n.bound);
+  if (whole_offsets) pv.tile_off = nullptr;
   return ids64 ? uniform_typed<int64_t>(indices, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                        out_capacity, picked_pos, row_is_position, status, s)
+                                        out_capacity, picked_pos, row_is_position, jobs, status, s)
                : uniform_typed<int32_t>(indices, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                        out_capacity, picked_pos, row_is_position, status, s);
+                                        out_capacity, picked_pos, row_is_position, jobs, status, s);
 }
 
 int launch_sample_weighted(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds,
-                           bool ids64, Count n, int64_t k, bool replace, void* plan,
+                           bool ids64, Count n, int64_t k, bool replace, void* plan, bool whole_offsets,
                            RngKey key, void* coo_row, void* coo_col, int64_t out_capacity,
-                           int64_t* picked_pos, bool row_is_position, int32_t* status, cudaStream_t s) {
-  const PlanView pv = plan_view(plan, n.bound);
+                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, int32_t* status,
+                           cudaStream_t s) {
+  PlanView pv = plan_view(plan, n.bound);
+  if (whole_offsets) pv.tile_off = nullptr;
   return ids64 ? weighted_typed<int64_t>(indices, probs, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                         out_capacity, picked_pos, row_is_position, status, s)
+                                         out_capacity, picked_pos, row_is_position, jobs, status, s)
                : weighted_typed<int32_t>(indices, probs, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                         out_capacity, picked_pos, row_is_position, status, s);
+                                         out_capacity, picked_pos, row_is_position, jobs, status, s);
 }
 
 }  // namespace dgs
@@ -1085,8 +922,7 @@ extern "C" int dgs_sample_plan(const dgs_chunk_desc* indptr, const void* seeds, 
     }
     return DGS_OK;
   }
-  return launch_sample_plan(*indptr, seeds, ids64 != 0, exact_count(n), k, replace != 0, plan, nnz, true, ClearJob{},
-                            LookupJob{}, status, s);
+  return launch_sample_plan(*indptr, seeds, ids64 != 0, exact_count(n), k, replace != 0, plan, nnz, true, status, s);
 }
 
 extern "C" int dgs_sample_uniform(const dgs_chunk_desc* indices, const void* seeds, int32_t ids64,
@@ -1112,8 +948,8 @@ extern "C" int dgs_sample_uniform(const dgs_chunk_desc* indices, const void* see
   DGS_REQUIRE(out_capacity == 0 || (coo_row != nullptr && coo_col != nullptr), DGS_ERR_INVALID,
               "dgs_sample_uniform: null output");
   rc = launch_sample_uniform(*indices, seeds, ids64 != 0, exact_count(n), k, replace != 0, const_cast<void*>(plan),
-                             host_key(sample_rng_key(rng_seed, rng_offset)), coo_row, coo_col, out_capacity,
-                             picked_pos, false, status, s);
+                             false, host_key(sample_rng_key(rng_seed, rng_offset)), coo_row, coo_col, out_capacity,
+                             picked_pos, false, SideJobs{}, status, s);
   if (rc != DGS_OK) return rc;
   if (nnz != nullptr) {
     copy_total_kernel<<<1, 1, 0, s>>>(sample_plan_total(const_cast<void*>(plan), n), nnz);
@@ -1152,8 +988,8 @@ extern "C" int dgs_sample_weighted(const dgs_chunk_desc* indices, const dgs_chun
   DGS_REQUIRE(out_capacity == 0 || (coo_row != nullptr && coo_col != nullptr), DGS_ERR_INVALID,
               "dgs_sample_weighted: null output");
   rc = launch_sample_weighted(*indices, *probs, seeds, ids64 != 0, exact_count(n), k, replace != 0,
-                              const_cast<void*>(plan), host_key(sample_rng_key(rng_seed, rng_offset)), coo_row,
-                              coo_col, out_capacity, picked_pos, false, status, s);
+                              const_cast<void*>(plan), false, host_key(sample_rng_key(rng_seed, rng_offset)), coo_row,
+                              coo_col, out_capacity, picked_pos, false, SideJobs{}, status, s);
   if (rc != DGS_OK) return rc;
   if (nnz != nullptr) {
     copy_total_kernel<<<1, 1, 0, s>>>(sample_plan_total(const_cast<void*>(plan), n), nnz);
