@@ -110,6 +110,18 @@ struct ChunkRows {
     if (run < D || !vector_copy_ok<VEC, REALIGN>(src, run << sh, D << sh)) return DGS_ROW_SLOW;
     return src;
   }
+  // a row whose covering 16-byte blocks lie inside its region (which starts on a 16-byte boundary)
+  __device__ __forceinline__ const char* locate_covered(int64_t row, uint32_t row_bytes, int32_t* status) const {
+    if (row < 0 || row >= n_rows_total) {
+      raise_status(status, DGS_ERR_RANGE);
+      return DGS_ROW_ZERO;
+    }
+    int64_t run;
+    const char* src = resolve(d, sh, row * D, &run);
+    const uint32_t mis = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src) & 15u);
+    const int64_t need = static_cast<int64_t>((mis + row_bytes + 15u) & ~15u) - mis;
+    return (run << sh) >= need ? src : DGS_ROW_SLOW;
+  }
   __device__ __forceinline__ const char* element(int64_t i, int64_t j) const {
     int64_t run;
     return resolve(d, sh, static_cast<int64_t>(idx[i]) * D + j, &run);
@@ -600,6 +612,208 @@ int launch_gather_bulk(const Src& rows, Count nc, int64_t D, int sh, void* out, 
   return DGS_OK;
 }
 
+// ---- rows off the 16-byte grid, repacked in shared memory -----------------------------
+// A row of an odd number of words starts anywhere, on the output side as well, so the register form moves
+// it in pieces of 4 bytes both ways and has a quarter of its usual bytes in flight (49 % of the HBM rate).  Here every row comes in
+// with one bulk copy of the aligned 16-byte blocks that cover it, and leaves repacked: a warp reads the words of its
+// group of rows from shared memory and writes the output, which is contiguous, in 16-byte vectors.  Pipeline, waits and
+// rare rows as in the bulk form.  Needs 4-byte elements at least, regions that start on 16-byte boundaries, and a
+// region's last row is copied element by element where the covering blocks would reach past its end.
+constexpr int REPACK_WARPS = 8;
+constexpr int REPACK_STAGES = 3;
+
+template <typename Src>
+__global__ void __launch_bounds__(REPACK_WARPS * 32)
+gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_bound, const int64_t* __restrict__ n_dev,
+                          const int64_t D, const int sh, const uint32_t row_bytes, const uint32_t slot_bytes,
+                          const uint32_t group, const uint32_t div_magic, char* __restrict__ out,
+                          int32_t* __restrict__ status) {
+  extern __shared__ __align__(128) unsigned char repack_smem[];
+  const uint64_t policy = l2_evict_first_policy();
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int n_warps = blockDim.x >> 5;
+  const uint32_t stage_bytes = group * slot_bytes;
+  unsigned char* my_stages = repack_smem + static_cast<size_t>(warp) * REPACK_STAGES * stage_bytes;
+  unsigned char* tail = repack_smem + static_cast<size_t>(n_warps) * REPACK_STAGES * stage_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tail) + warp * REPACK_STAGES;
+  // where each row of a buffer begins, in bytes from the buffer's start
+  uint32_t* begins = reinterpret_cast<uint32_t*>(tail + sizeof(uint64_t) * REPACK_STAGES * n_warps) + warp * REPACK_STAGES * 32;
+  if (lane == 0) {
+#pragma unroll
+    for (int s = 0; s < REPACK_STAGES; ++s) mbar_init(smem_addr(bars + s), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  pdl_enter();
+
+  int64_t n = n_bound;
+  if (n_dev != nullptr) {
+    const int64_t live = *n_dev;
+    n = live < n_bound ? (live < 0 ? 0 : live) : n_bound;
+  }
+  const int64_t n_groups = (n + group - 1) / group;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * n_warps;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * n_warps + warp;
+  const uint32_t nw = row_bytes / 4;  // words per row
+
+  auto fetch_id = [&](int64_t g) -> int64_t {
+    const int64_t i = g * group + lane;
+    return (g < n_groups && lane < static_cast<int>(group) && i < n) ? rows.row_id(i) : 0;
+  };
+  auto issue = [&](int64_t g, int st, int64_t row) {
+    const int64_t i = g * group + lane;
+    const bool valid = lane < static_cast<int>(group) && i < n;
+    const char* src = valid ? rows.locate_covered(row, row_bytes, status) : nullptr;
+    const bool whole = valid && reinterpret_cast<uintptr_t>(src) > 1;
+    const uint32_t bar = smem_addr(bars + st);
+    unsigned char* slot = my_stages + static_cast<size_t>(st) * stage_bytes + static_cast<size_t>(lane) * slot_bytes;
+    const uint32_t mis = whole ? static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src) & 15u) : 0u;
+    const uint32_t bytes = whole ? (mis + row_bytes + 15u) & ~15u : 0u;
+    uint32_t expect = bytes;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) expect += __shfl_xor_sync(FULL_MASK, expect, o);
+    begins[st * 32 + lane] = lane * slot_bytes + mis;
+    if (lane == 0) mbar_expect_tx(bar, expect);  // also the one arrival the barrier waits for
+    __syncwarp();
+    if (whole) {
+      bulk_load(smem_addr(slot), src - mis, bytes, bar, policy, true);
+    } else if (valid) {
+      // rare: zero row (bad id), a row that straddles two storage regions or ends one, element by element
+      for (int64_t j = 0; j < D; ++j) {
+        const char* p = src == DGS_ROW_ZERO ? nullptr : rows.element(i, j);
+        unsigned char* q = slot + (j << sh);
+        if (sh == 3) *reinterpret_cast<uint64_t*>(q) = p == nullptr ? 0ull : *reinterpret_cast<const uint64_t*>(p);
+        else *reinterpret_cast<uint32_t*>(q) = p == nullptr ? 0u : *reinterpret_cast<const uint32_t*>(p);
+      }
+    }
+  };
+
+  int64_t g_issue = first;
+#pragma unroll
+  for (int s = 0; s < REPACK_STAGES - 1; ++s) {
+    if (g_issue < n_groups) issue(g_issue, s, fetch_id(g_issue));
+    g_issue += stride;
+  }
+  int64_t next_row = fetch_id(g_issue);
+  uint32_t phase_bits = 0;
+  int st = 0, st_issue = REPACK_STAGES - 1;
+  bool alive = true;
+  for (int64_t g = first; g < n_groups && alive; g += stride) {
+    // the buffer that is loaded next was emptied one iteration ago
+    const int64_t row_now = next_row;
+    next_row = fetch_id(g_issue + stride);
+    if (g_issue < n_groups) issue(g_issue, st_issue, row_now);
+    if (!mbar_wait_bounded(smem_addr(bars + st), (phase_bits >> st) & 1u)) {
+      raise_status(status, DGS_ERR_CUDA);
+      alive = false;
+    }
+    alive = __all_sync(FULL_MASK, alive);
+    if (!alive) break;
+    __syncwarp();  // rows that lanes wrote into the buffer themselves
+    phase_bits ^= 1u << st;
+    const int64_t row0 = g * group;
+    const uint32_t here = n - row0 < static_cast<int64_t>(group) ? static_cast<uint32_t>(n - row0) : group;
+    const unsigned char* stage = my_stages + static_cast<size_t>(st) * stage_bytes;
+    const uint32_t* begin = begins + st * 32;
+    const uint32_t words = here * nw;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(out + row0 * row_bytes);  // groups are multiples of 16 bytes
+#pragma unroll 4
+    for (uint32_t w = 4 * lane; w + 4 <= words; w += 128) {
+      uint32_t r = __umulhi(w, div_magic);  // w / nw, exact while w * nw < 2^32
+      uint32_t j = w - r * nw;
+      const unsigned char* at = stage + begin[r] + 4 * j;
+      uint32_t v[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        v[x] = *reinterpret_cast<const uint32_t*>(at);
+        at += 4;
+        if (++j == nw && x < 3) {
+          j = 0;
+          at = stage + begin[++r];
+        }
+      }
+      *reinterpret_cast<uint4*>(dst + w) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    const uint32_t w = (words & ~3u) + lane;  // the last group may end off the grid
+    if (w < words) {
+      const uint32_t r = __umulhi(w, div_magic);
+      dst[w] = *reinterpret_cast<const uint32_t*>(stage + begin[r] + 4 * (w - r * nw));
+    }
+    __syncwarp();
+    g_issue += stride;
+    st = st + 1 == REPACK_STAGES ? 0 : st + 1;
+    st_issue = st_issue + 1 == REPACK_STAGES ? 0 : st_issue + 1;
+  }
+  if (!alive) {
+    // give the copies still in flight a bounded chance to land before the buffers go away
+    for (int s = 0; s < REPACK_STAGES; ++s) mbar_wait_bounded(smem_addr(bars + s), (phase_bits >> s) & 1u);
+  }
+}
+
+inline uint32_t gcd_u32(uint32_t a, uint32_t b) { return b == 0 ? a : gcd_u32(b, a % b); }
+
+template <typename Src>
+int launch_gather_repack(const Src& rows, Count nc, int64_t D, int sh, void* out, int32_t* status, int warps,
+                         cudaStream_t stream) {
+  const uint32_t row_bytes = static_cast<uint32_t>(D << sh);
+  const uint32_t slot_bytes = (row_bytes + 12u + 15u) & ~15u;
+  const uint32_t unit = 16u / gcd_u32(16u, row_bytes);  // rows that make a multiple of 16 bytes
+  uint32_t group = 8192u / slot_bytes / unit * unit;
+  if (group > 32u) group = 32u;
+  const uint32_t nw = row_bytes / 4;
+  const uint32_t magic = static_cast<uint32_t>(((1ull << 32) + nw - 1) / nw);
+  const size_t smem = static_cast<size_t>(warps) * REPACK_STAGES * (group * slot_bytes + sizeof(uint64_t) + 32 * sizeof(uint32_t));
+  // per device and safe to reach from several host threads: the SM count, and whether this instantiation has
+  // been allowed its dynamic shared memory there (the attribute belongs to the device's copy of the kernel)
+  constexpr int kMaxDevices = 64;
+  constexpr int kMaxSmem = 208 * 1024;
+  static std::atomic<int> sm_count[kMaxDevices] = {};
+  DGS_REQUIRE(group >= 1 && smem <= kMaxSmem, DGS_ERR_UNSUPPORTED, "gather: %zu bytes of shared memory per CTA", smem);
+  int dev = 0;
+  DGS_CUDA_TRY(cudaGetDevice(&dev));
+  DGS_REQUIRE(dev >= 0 && dev < kMaxDevices, DGS_ERR_UNSUPPORTED, "gather: device ordinal %d", dev);
+  auto kernel = gather_rows_repack_kernel<Src>;
+  int sms = sm_count[dev].load(std::memory_order_acquire);
+  if (sms == 0) {
+    DGS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    DGS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    sm_count[dev].store(sms, std::memory_order_release);
+  }
+  const int64_t groups = (nc.bound + group - 1) / group;
+  int64_t grid = (groups + warps - 1) / warps;
+  if (grid > static_cast<int64_t>(sms)) grid = static_cast<int64_t>(sms);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  cfg.blockDim = dim3(warps * 32, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained_launches_enabled(SITE_GATHER) ? 1 : 0;
+  DGS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, rows, nc.bound, nc.dev, D, sh, row_bytes, slot_bytes, group, magic,
+                                  static_cast<char*>(out), status));
+  return DGS_OK;
+}
+
+// Rows that the register form would move in 4-byte pieces, from regions on 16-byte boundaries.  Measured with 333 k
+// rows (register form -> this one): 132 bytes 30.0 -> 29.4 us, 300 bytes 63.3 -> 46.9, 596 bytes 121.8 -> 82.0,
+// 1204 bytes 246.9 -> 138.5 (5.8 TB/s); 76 bytes 17.4 -> 22.3, since the copy engine takes ~40 cycles a row whatever
+// its size.  Rows of 8-byte pieces stay with the register form (200 bytes 33.3 -> 35.9, 600 bytes 79.1 -> 81.4).
+// DGS_GATHER_REPACK=0 switches it off.
+inline bool repack_rows_qualify(const dgs_chunk_desc& d, int vec, int64_t row_bytes, const void* out) {
+  static const bool off = [] {
+    const char* e = std::getenv("DGS_GATHER_REPACK");
+    return e != nullptr && e[0] == '0';
+  }();
+  if (off || vec != 4 || row_bytes < 160 || row_bytes > 2000 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
+  for (int p = 0; p < d.num_parts && p * d.each < d.threshold; ++p)
+    if ((reinterpret_cast<uintptr_t>(d.dev[p]) & 15) != 0) return false;
+  return d.threshold >= d.total || (reinterpret_cast<uintptr_t>(d.host) & 15) == 0;
+}
+
 inline bool bulk_rows_qualify(int vec, bool realign, int64_t row_bytes) {
   return vec == 16 && !realign && (row_bytes % 16) == 0 && row_bytes >= 256 && row_bytes <= 8192;
 }
@@ -634,6 +848,8 @@ int run_gather(int vec, bool realign, const dgs_chunk_desc& d, const void* idx, 
   const int env = bulk_env();
   if ((env == 1 || (env < 0 && prefer_bulk)) && bulk_rows_qualify(vec, realign, D << sh))
     return launch_gather_bulk(rows, n, D, sh, out, status, stream);
+  if (repack_rows_qualify(d, vec, D << sh, out))  // behind a sampling sequence with room left beside it
+    return launch_gather_repack(rows, n, D, sh, out, status, prefer_bulk ? REPACK_WARPS / 2 : REPACK_WARPS, stream);
   return dispatch_vec(vec, realign, rows, n, D, sh, out, status, stream);
 }
 

@@ -1,0 +1,53 @@
+"""Rows of an odd number of words, which are repacked in shared memory: widths at the ends of the form's range, regions
+whose last row cannot be covered by whole 16-byte blocks, rows that straddle regions, bad ids, counts off the group."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def words():
+    from gpu_util import Words
+    return Words()
+
+
+@pytest.mark.parametrize("D", [39, 41, 75, 127, 255, 257, 499, 501])
+@pytest.mark.parametrize("cap_rows,extra,world", [(10 ** 9, 0, 1), (100, 0, 3), (100, 5, 4), (0, 0, 1)])
+@pytest.mark.parametrize("n", [1, 3, 97, 2500])
+def test_odd_word_rows(words, D, cap_rows, extra, world, n):
+    from gpu_util import EmulatedChunks, gather
+    rng = np.random.default_rng(D + n)
+    rows = 701
+    table = rng.integers(0, 2 ** 32, (rows, D), dtype=np.uint32).view(np.float32)
+    em = EmulatedChunks(table, D, (min(cap_rows, 10 ** 6) * D + extra) * 4, world)
+    idx = np.array(list(rng.integers(0, rows, n)) + [rows - 1, 99, 100, 199, 299][: n - 1], dtype=np.int64)
+    out = gather(em.desc, torch.from_numpy(idx).cuda(), D, torch.float32, words)
+    assert words.take_status() == 0
+    assert out.cpu().numpy().tobytes() == table[idx].tobytes()
+
+
+def test_bad_ids_and_live_count(pkg, words):
+    from gpu_util import gather, plain_desc, vp
+    D, rows, n = 75, 300, 1000
+    table = torch.randn(rows, D, device="cuda")
+    idx = torch.randint(0, rows, (n,), device="cuda", dtype=torch.int32)
+    idx[5], idx[77], idx[n - 1] = -1, rows, 1 << 30
+    out = gather(plain_desc(table), idx, D, torch.float32, words)
+    assert words.take_status() != 0
+    good = (idx >= 0) & (idx < rows)
+    assert torch.equal(out[good], table[idx[good].long()]) and not out[~good].any()
+    # a row count on the device: rows past it stay as they are
+    abi = pkg.load_abi()
+    idx = idx.clamp(0, rows - 1)
+    for live in (0, 1, 2, 3, 501, n, n + 50):
+        count = torch.tensor([live], device="cuda")
+        out = torch.full((n, D), -7.0, device="cuda")
+        d = plain_desc(table)
+        pkg.check(abi.dgs_gather_rows_counted(ctypes.byref(d), vp(idx), 0, n, vp(count), D, vp(out), vp(words.status), None))
+        assert words.take_status() == 0
+        m = min(live, n)
+        assert torch.equal(out[:m], table[idx[:m].long()]) and torch.all(out[m:] == -7.0)
