@@ -231,12 +231,13 @@ def sample_blocks(seeds, fanouts, indptr, indices, probs=None, replace=False, fu
     ops = torch.ops.dgs_ops
     chunked = not isinstance(indptr, torch.Tensor)
     if fused:
-        if probs is not None:
-            fn = ops._CAPI_sample_blocks_with_probs_with_chunk_tensor if chunked else ops._CAPI_sample_blocks_with_probs
-            frontier, rows, cols, shape = fn(seeds, indptr, indices, probs, list(fanouts), replace)
+        if chunked:
+            frontier, rows, cols, shape = indptr._CAPI_sample_blocks(seeds, indices, probs, list(fanouts), replace)
+        elif probs is not None:
+            frontier, rows, cols, shape = ops._CAPI_sample_blocks_with_probs(seeds, indptr, indices, probs,
+                                                                             list(fanouts), replace)
         else:
-            fn = ops._CAPI_sample_blocks_with_chunk_tensor if chunked else ops._CAPI_sample_blocks
-            frontier, rows, cols, shape = fn(seeds, indptr, indices, list(fanouts), replace)
+            frontier, rows, cols, shape = ops._CAPI_sample_blocks(seeds, indptr, indices, list(fanouts), replace)
         blocks = [(rows[i], cols[i], shape[2 * i], shape[2 * i + 1]) for i in range(len(rows))]
         return frontier, blocks, sum(r.numel() for r in rows)
     blocks, n_edges = [], 0

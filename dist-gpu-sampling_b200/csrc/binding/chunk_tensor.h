@@ -3,6 +3,7 @@
 // src/pybind.cc:11-22) as a thin holder of a dgs_store from the C ABI.
 #pragma once
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
@@ -46,9 +47,18 @@ inline size_t dtype_size(torch::ScalarType t) {
   }
 }
 
-inline torch::Tensor byte_scratch(size_t bytes, const torch::Device& dev) {
-  return torch::empty({static_cast<int64_t>(bytes)}, torch::TensorOptions().dtype(torch::kUInt8).device(dev));
+// An uninitialised tensor straight from the caching allocator: the operators allocate up to nine tensors a call, and
+// the way through the dispatcher costs more than the allocation.
+inline torch::Tensor device_empty(at::IntArrayRef sizes, torch::ScalarType dtype, const torch::Device& dev) {
+  return at::detail::empty_cuda(sizes, dtype, dev, c10::nullopt);
 }
+
+inline torch::Tensor byte_scratch(size_t bytes, const torch::Device& dev) {
+  return device_empty({static_cast<int64_t>(bytes)}, torch::kUInt8, dev);
+}
+
+// Cuts a 1-D tensor that this library has just allocated to its first n elements, in place (a view costs 1.5 us).
+inline void cut_to(torch::Tensor& t, int64_t n) { t.unsafeGetTensorImpl()->set_sizes_contiguous({n}); }
 
 class ChunkTensor : public torch::CustomClassHolder {
  public:
@@ -91,8 +101,7 @@ class ChunkTensor : public torch::CustomClassHolder {
     const Lease lease(op, index.device().index(), current_stream());
     index = index.contiguous();
     const int64_t n = index.numel();
-    torch::Tensor out =
-        torch::empty({n, elem_stride_}, torch::TensorOptions().dtype(dtype_).device(index.device()));
+    torch::Tensor out = device_empty({n, elem_stride_}, dtype_, index.device());
     DGS_CHECK_RC(dgs_gather_rows(&desc_, location_class, index.data_ptr(), ids64, n, elem_stride_, out.data_ptr(),
                                  lease.status(), current_stream()));
     lease.finish();
@@ -118,8 +127,7 @@ class ChunkTensor : public torch::CustomClassHolder {
     const Lease lease("_CAPI_index_counted", index.device().index(), current_stream());
     index = index.contiguous();
     const int64_t n = index.numel();
-    torch::Tensor out =
-        torch::empty({n, elem_stride_}, torch::TensorOptions().dtype(dtype_).device(index.device()));
+    torch::Tensor out = device_empty({n, elem_stride_}, dtype_, index.device());
     DGS_CHECK_RC(dgs_gather_rows_counted(&desc_, index.data_ptr(), ids64, n, count.data_ptr<int64_t>(), elem_stride_,
                                          out.data_ptr(), lease.status(), current_stream()));
     lease.finish();

@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <mutex>
 #include <vector>
 
@@ -56,7 +57,7 @@ class WordPool {
     cudaEvent_t done = nullptr; // recorded when the lease ends: later kernels of the call may still write
     const char* op = "";        // operator that holds / last held the slot
     bool busy = false;          // leased right now
-    bool fenced = false;        // `done` has been recorded at least once
+    unsigned long long stream_id = 0;  // of the stream `done` was last recorded on (never reused by the driver)
   };
 
   // one pool per device; created on first use with that device current
@@ -82,20 +83,10 @@ class WordPool {
                     ") after that call had returned; noticed on entering ", op);
       }
     }
-    // slots are reused in the order they were released, so the first candidate has normally left the GPU
-    Slot* pick = nullptr;
-    const size_t n = slots_.size();
-    for (size_t i = 0; i < n && pick == nullptr; ++i) {
-      Slot* s = slots_[(cursor_ + i) % n];
-      if (s->busy) continue;
-      if (s->fenced && cudaEventQuery(s->done) != cudaSuccess) {
-        cudaGetLastError();  // cudaErrorNotReady is no error
-        continue;
-      }
-      pick = s;
-      cursor_ = (cursor_ + i + 1) % n;
-    }
-    if (pick == nullptr) pick = grow();
+    if (free_.empty()) collect();
+    if (free_.empty()) grow();
+    Slot* pick = free_.back();
+    free_.pop_back();
     pick->busy = true;
     pick->op = op;
     return pick;
@@ -105,20 +96,43 @@ class WordPool {
   // only after they have run.
   void release(Slot* s, cudaStream_t stream) {
     std::lock_guard<std::mutex> lock(mu_);
-    if (cudaEventRecord(s->done, stream) == cudaSuccess) s->fenced = true;
-    else cudaGetLastError();
     s->busy = false;
+    s->stream_id = 0;
+    if (cudaEventRecord(s->done, stream) == cudaSuccess) {
+      if (cudaStreamGetId(stream, &s->stream_id) != cudaSuccess) s->stream_id = 0;
+    }
+    (void)cudaGetLastError();
+    released_.push_back(s);
   }
 
  private:
-  Slot* grow() {
+  // Released slots whose calls have left the GPU become free.  Work of one stream finishes in order, so one query in
+  // the middle of the list answers for all slots before it that were released on the same stream: a query per call
+  // is 1.3 us of an operator that takes 9.
+  void collect() {
+    if (released_.empty()) return;
+    size_t probe = released_.size() / 2;
+    if (cudaEventQuery(released_[probe]->done) != cudaSuccess) probe = 0;
+    const unsigned long long id = released_[probe]->stream_id;
+    const bool passed = probe > 0 || cudaEventQuery(released_[0]->done) == cudaSuccess;
+    (void)cudaGetLastError();  // cudaErrorNotReady is no error
+    if (!passed) return;
+    std::deque<Slot*> still;
+    for (size_t i = 0; i < released_.size(); ++i) {
+      Slot* s = released_[i];
+      if (i == probe || (i < probe && id != 0 && s->stream_id == id)) free_.push_back(s);
+      else still.push_back(s);
+    }
+    released_.swap(still);
+  }
+
+  void grow() {
     constexpr int kBatch = 32;
     constexpr size_t kStride = 256;  // bytes per slot: 24 sizes + status, padded
     void* p = nullptr;
     TORCH_CHECK(cudaHostAlloc(&p, kBatch * kStride, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess,
                 "dgs: cannot allocate pinned size / status words");
     std::memset(p, 0, kBatch * kStride);
-    Slot* first = nullptr;
     for (int i = 0; i < kBatch; ++i) {
       Slot* s = new Slot();
       char* base = static_cast<char*>(p) + i * kStride;
@@ -127,14 +141,14 @@ class WordPool {
       TORCH_CHECK(cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming) == cudaSuccess,
                   "dgs: cannot create an event");
       slots_.push_back(s);
-      if (first == nullptr) first = s;
+      free_.push_back(s);
     }
-    return first;
   }
 
   std::mutex mu_;
   std::vector<Slot*> slots_;
-  size_t cursor_ = 0;
+  std::vector<Slot*> free_;       // nothing of theirs is on the GPU
+  std::deque<Slot*> released_;    // in order of release; may still be written
 };
 
 // RAII lease of one slot for the duration of an operator call.

@@ -72,7 +72,7 @@ std::tuple<torch::Tensor, torch::Tensor> sample_impl(torch::Tensor seeds, const 
   c10::cuda::CUDAGuard guard(seeds.device());
   seeds = seeds.contiguous().view({-1});
   const int64_t n = seeds.numel();
-  auto opt = seeds.options();
+  auto ids = [&](int64_t count) { return device_empty({count}, seeds.scalar_type(), seeds.device()); };
   cudaStream_t stream = current_stream();
   const Lease w("_CAPI_sample_neighbors*", seeds.device().index(), stream);
   const auto rng = next_rng();
@@ -99,8 +99,8 @@ std::tuple<torch::Tensor, torch::Tensor> sample_impl(torch::Tensor seeds, const 
     // everything is enqueued first; the host then only waits for the plan
     // kernel's total, not for the sampling kernel behind it
     const int64_t cap = n * k;
-    row = torch::empty({cap}, opt);
-    col = torch::empty({cap}, opt);
+    row = ids(cap);
+    col = ids(cap);
     w.sizes()[0] = kPending;
     DGS_CHECK_RC(dgs_sample_plan(&indptr, seeds.data_ptr(), ids64, n, k, replace, plan.data_ptr(), w.sizes(),
                                  w.status(), stream));
@@ -109,15 +109,17 @@ std::tuple<torch::Tensor, torch::Tensor> sample_impl(torch::Tensor seeds, const 
     if (strict_status()) sync_stream();
     w.check();
     TORCH_CHECK(nnz >= 0 && nnz <= cap, "dgs: sampler returned an impossible size");
-    return std::make_tuple(row.narrow(0, 0, nnz), col.narrow(0, 0, nnz));
+    cut_to(row, nnz);
+    cut_to(col, nnz);
+    return std::make_tuple(row, col);
   }
   DGS_CHECK_RC(dgs_sample_plan(&indptr, seeds.data_ptr(), ids64, n, k, replace, plan.data_ptr(), w.sizes(),
                                w.status(), stream));
   sync_stream();
   nnz = w.sizes()[0];
   w.check();
-  row = torch::empty({nnz}, opt);
-  col = torch::empty({nnz}, opt);
+  row = ids(nnz);
+  col = ids(nnz);
   run(row, col, nnz, nullptr);
   w.finish();
   return std::make_tuple(row, col);
@@ -222,8 +224,8 @@ std::tuple<torch::Tensor, std::vector<torch::Tensor>> TensorRelabelCUDA(
 
   const size_t tb = dgs_relabel_table_bytes(n_keys);
   torch::Tensor table = byte_scratch(tb, first.device());
-  torch::Tensor uniq = torch::empty({n_keys}, first.options());
-  torch::Tensor out = torch::empty({n_req}, first.options());
+  torch::Tensor uniq = device_empty({n_keys}, first.scalar_type(), first.device());
+  torch::Tensor out = device_empty({n_req}, first.scalar_type(), first.device());
   // the count kernel reports the number of distinct keys; the numbering and
   // lookup kernels behind it are still in flight when this returns
   w.sizes()[0] = kPending;
@@ -234,7 +236,8 @@ std::tuple<torch::Tensor, std::vector<torch::Tensor>> TensorRelabelCUDA(
   if (strict_status()) sync_stream();
   w.check();
   TORCH_CHECK(nu >= 0 && nu <= n_keys, "dgs: relabel returned an impossible size");
-  return std::make_tuple(uniq.narrow(0, 0, nu), out.split_with_sizes(split_sizes, 0));
+  cut_to(uniq, nu);
+  return std::make_tuple(uniq, out.split_with_sizes(split_sizes, 0));
 }
 
 // ===========================================================================
@@ -300,7 +303,7 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
   };
   if (!sequence) return hop_by_hop();
 
-  auto opt = seeds.options();
+  auto ids = [&](int64_t count) { return device_empty({count}, seeds.scalar_type(), seeds.device()); };
   cudaStream_t stream = current_stream();
   const Lease w("_CAPI_sample_blocks*", seeds.device().index(), stream);
   const auto rng = next_rng(static_cast<uint64_t>(H));
@@ -308,9 +311,9 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
   std::vector<torch::Tensor> fr(H);
   for (int h = 0; h < H; ++h) {
     const int64_t cap = hops[h].seed_bound * hops[h].fanout;
-    rows[H - 1 - h] = torch::empty({cap}, opt);
-    cols[H - 1 - h] = torch::empty({cap}, opt);
-    fr[h] = torch::empty({hops[h].frontier_bound}, opt);
+    rows[H - 1 - h] = ids(cap);
+    cols[H - 1 - h] = ids(cap);
+    fr[h] = ids(hops[h].frontier_bound);
     hops[h].coo_row = rows[H - 1 - h].data_ptr();
     hops[h].coo_col = cols[H - 1 - h].data_ptr();
     hops[h].frontier = fr[h].data_ptr();
@@ -342,15 +345,16 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
   for (int h = 0; h < H; ++h) {
     const int64_t nnz = w.sizes()[2 * h], nu = w.sizes()[2 * h + 1];
     const int at = H - 1 - h;
-    rows[at] = rows[at].narrow(0, 0, nnz);
-    cols[at] = cols[at].narrow(0, 0, nnz);
+    cut_to(rows[at], nnz);
+    cut_to(cols[at], nnz);
     shape[2 * at] = std::min(nu, hops[h].frontier_bound);
     shape[2 * at + 1] = n_dst;
     n_dst = shape[2 * at];
   }
   if (strict_status()) sync_stream();
   w.check();
-  frontier = fr[H - 1].narrow(0, 0, n_dst);
+  frontier = fr[H - 1];
+  cut_to(frontier, n_dst);
   return std::make_tuple(frontier, rows, cols, shape);
 }
 
@@ -398,6 +402,17 @@ BlocksResult SampleBlocksProbWithChunkTensorCUDA(torch::Tensor seeds, c10::intru
                      fanouts, replace);
 }
 
+namespace {
+BlocksResult SampleBlocksMethod(const c10::intrusive_ptr<ChunkTensor>& indptr, torch::Tensor seeds,
+                                c10::intrusive_ptr<ChunkTensor> indices,
+                                c10::optional<c10::intrusive_ptr<ChunkTensor>> probs, std::vector<int64_t> fanouts,
+                                bool replace) {
+  return probs.has_value() && probs.value().defined()
+             ? SampleBlocksProbWithChunkTensorCUDA(seeds, indptr, indices, probs.value(), std::move(fanouts), replace)
+             : SampleBlocksWithChunkTensorCUDA(seeds, indptr, indices, std::move(fanouts), replace);
+}
+}  // namespace
+
 // ===========================================================================
 // PaGraph-style cache
 // ===========================================================================
@@ -438,7 +453,7 @@ torch::Tensor fetch_impl(torch::Tensor cpu_data, const dgs_chunk_desc& gpu, torc
   c10::cuda::CUDAGuard guard(nid.device());
   nid = nid.contiguous();
   const int64_t n = nid.numel(), D = cpu_data.size(1);
-  torch::Tensor out = torch::empty({n, D}, torch::TensorOptions().dtype(gpu_dtype).device(nid.device()));
+  torch::Tensor out = device_empty({n, D}, gpu_dtype, nid.device());
   const Lease w("_CAPI_fetch_data*", nid.device().index(), current_stream());
   DGS_CHECK_RC(dgs_cache_fetch(cpu_data.data_ptr(), cpu_data.size(0), &gpu, nid.data_ptr(), ids64, n, D,
                                hk.data_ptr(), hv.data_ptr(), hk.numel(), out.data_ptr(), w.status(),
@@ -495,7 +510,10 @@ TORCH_LIBRARY(dgs_classes, m) {
       .def("_CAPI_host_index", &ChunkTensor::HostIndex)
       .def("_CAPI_load_from_tensor", &ChunkTensor::LoadFromTensor)
       // addition (no counterpart in src/pybind.cc): the gather with its row count on the device
-      .def("_CAPI_index_counted", &ChunkTensor::IndexCounted);
+      .def("_CAPI_index_counted", &ChunkTensor::IndexCounted)
+      // addition: the one-sequence sampling operators as methods of indptr.  torch.ops looks through every argument in
+      // Python when an operator takes a custom class (20 us a call); a method call does not.
+      .def("_CAPI_sample_blocks", &SampleBlocksMethod);
   // addition (no counterpart in src/pybind.cc): mini-batches in flight, see pipeline.h
   m.class_<BlockPipeline>("BlockPipeline")
       .def(torch::init<c10::intrusive_ptr<ChunkTensor>, c10::intrusive_ptr<ChunkTensor>,
