@@ -36,29 +36,6 @@ namespace {
 constexpr size_t WS_ALIGN = 256;
 inline size_t ws_align(size_t x) { return (x + WS_ALIGN - 1) / WS_ALIGN * WS_ALIGN; }
 
-struct InitWords {
-  int64_t* n0;
-  int64_t n0_value;
-  unsigned int* ticket;  // of the first hop's plan
-  // a recorded sequence takes its random stream from memory: (seed, offset) at rng_src, read by this
-  // kernel on every replay and folded into one Philox key per hop for the sampling kernels behind it
-  const uint64_t* rng_src;
-  uint64_t* keys;
-  int n_keys;
-};
-
-__global__ void blocks_init_kernel(const InitWords w) {
-  pdl_enter();
-  if (threadIdx.x == 0) {
-    *w.n0 = w.n0_value;
-    *w.ticket = 0u;
-  }
-  if (w.rng_src != nullptr && threadIdx.x < w.n_keys) {
-    const volatile uint64_t* src = w.rng_src;  // host-written words: no cached copy
-    w.keys[threadIdx.x] = fold_rng_key(src[0], src[1] + static_cast<uint64_t>(threadIdx.x));
-  }
-}
-
 __global__ void zero_sizes_kernel(int64_t* sizes, int n) {
   if (threadIdx.x < n) sizes[threadIdx.x] = 0;
 }
@@ -187,8 +164,6 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
     table[h] = p;
     p += ws_align(dgs_relabel_table_bytes(key_bound));
   }
-  const InitWords init{n0_dev, n0, sample_plan_ticket(plan[0], n0), rng_words, keys_dev, n_hops};
-  DGS_CUDA_TRY(launch_chained(SITE_INIT, blocks_init_kernel, 1u, 32u, s, init));
 
   // a graph with fewer nodes than 2^32 - 1 has no ids beyond
   const long long max_key = !ids64 || indptr->total - 1 < COMPACT_KEY_LIMIT ? COMPACT_KEY_LIMIT - 1 : INT64_MAX;
@@ -199,8 +174,8 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
   LookupJob pending{};  // relabelling of the previous hop's COO, carried by the next sample launch
   SizesReport report{};
   report.dst = sizes;
-  rc = launch_sample_plan(*indptr, seeds, ids64 != 0, Count{n0, n0_dev, nullptr}, hops[0].fanout, replace != 0, plan[0],
-                          nullptr, false, status, s);
+  const InitWords init{n0_dev, n0, rng_words, keys_dev, n_hops};
+  rc = launch_sample_plan(*indptr, seeds, ids64 != 0, n0, hops[0].fanout, replace != 0, plan[0], nullptr, init, status, s);
   if (rc != DGS_OK) return rc;
   for (int h = 0; h < n_hops; ++h) {
     const dgs_hop& hp = hops[h];

@@ -7,12 +7,21 @@
 namespace dgs {
 
 // ---- sample.cu ---------------------------------------------------------------
-// `plan` is laid out for n.bound seeds.  nnz_out (optional, normally pinned)
+// `plan` is laid out for n seeds.  nnz_out (optional, normally pinned)
 // receives the number of sampled edges; the same number stays in the plan at
-// sample_plan_total().  The plan's ticket word must be zero at launch: it is
-// cleared here when zero_ticket is set and resets itself after every use.
-int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, Count n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, int32_t* status, cudaStream_t s);
+// sample_plan_total().
+// init: words to set before anything behind it runs (n0 == nullptr, rng_src == nullptr: none).
+struct InitWords {
+  int64_t* n0;
+  int64_t n0_value;
+  // a recorded sequence takes its random stream from memory: (seed, offset) at rng_src, read on every replay and
+  // folded into one Philox key per hop for the sampling kernels
+  const uint64_t* rng_src;
+  uint64_t* keys;
+  int n_keys;
+};
+int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, int64_t n, int64_t k,
+                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, int32_t* status, cudaStream_t s);
 // The plan of a hop whose seeds are being numbered (launch_unique_pair writes it): offsets are those in the whole
 // output, so sampling takes whole_offsets = true.  n_edges == nullptr: no plan wanted.
 struct NextPlan {
@@ -24,7 +33,6 @@ struct NextPlan {
 };
 NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k, bool replace, void* plan);
 int64_t* sample_plan_total(void* plan, int64_t n_bound);
-unsigned int* sample_plan_ticket(void* plan, int64_t n_bound);
 
 // Independent jobs run by extra CTAs of a sampling launch (either may have ctas == 0).
 struct SideJobs {

@@ -80,6 +80,20 @@ inline PlanView plan_view(void* plan, int64_t n) {
   return v;
 }
 
+// The words a multi-hop sequence wants set before anything else runs (by 32 threads at least).
+__device__ __forceinline__ void run_init(const InitWords& w) {
+  if (threadIdx.x == 0 && w.n0 != nullptr) *w.n0 = w.n0_value;
+  if (w.rng_src != nullptr && threadIdx.x < w.n_keys) {
+    const volatile uint64_t* src = w.rng_src;  // host-written words: no cached copy
+    w.keys[threadIdx.x] = fold_rng_key(src[0], src[1] + static_cast<uint64_t>(threadIdx.x));
+  }
+}
+__global__ void init_kernel(const InitWords w, unsigned int* ticket) {
+  pdl_enter();
+  if (threadIdx.x == 0) *ticket = 0u;
+  run_init(w);
+}
+
 // ---------------------------------------------------------------------------
 // plan: row range per seed + per-tile output counts
 // ---------------------------------------------------------------------------
@@ -116,6 +130,59 @@ sample_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __r
 
   // publish the tile sum; the CTA that draws the last ticket scans all of them
   publish_and_scan_tiles<SAMPLE_BLOCK>(total, tile_sums, ticket, total_out, nnz_out, smem);
+}
+
+// The plan of up to SMALL_PLAN seeds by one CTA: no ticket, hence nothing that has to be cleared before it, and in the
+// multi-hop sequence it sets the words that a launch of its own sets otherwise.  Bound by latency (seed, row bounds,
+// scan); four seeds per thread with their loads in flight together.
+constexpr int SMALL_PLAN_BLOCK = 1024;
+constexpr int SMALL_PLAN_ITEMS = 4;
+constexpr int SMALL_PLAN = SMALL_PLAN_BLOCK * SMALL_PLAN_ITEMS;
+
+template <typename IdT>
+__global__ void __launch_bounds__(SMALL_PLAN_BLOCK)
+sample_small_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __restrict__ seeds, const int n,
+                         const int64_t k, const bool replace, const PlanView plan, int64_t* nnz_out,
+                         const __grid_constant__ InitWords init, int32_t* __restrict__ status) {
+  __shared__ int64_t smem[SMALL_PLAN_BLOCK / 32 + 1];
+  pdl_enter();
+  run_init(init);
+  int64_t s[SMALL_PLAN_ITEMS], rb[SMALL_PLAN_ITEMS], deg[SMALL_PLAN_ITEMS];
+  bool good[SMALL_PLAN_ITEMS];
+#pragma unroll
+  for (int u = 0; u < SMALL_PLAN_ITEMS; ++u) {
+    const int i = u * SMALL_PLAN_BLOCK + threadIdx.x;
+    s[u] = i < n ? static_cast<int64_t>(seeds[i]) : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < SMALL_PLAN_ITEMS; ++u) {
+    good[u] = s[u] >= 0 && s[u] + 1 < indptr.total;
+    if (u * SMALL_PLAN_BLOCK + static_cast<int>(threadIdx.x) < n && !good[u]) raise_status(status, DGS_ERR_RANGE);
+  }
+  row_bounds<IdT, SMALL_PLAN_ITEMS>(indptr, s, good, rb, deg, status);
+  int64_t carry = 0;
+#pragma unroll
+  for (int u = 0; u < SMALL_PLAN_ITEMS; ++u) {
+    if (u * SMALL_PLAN_BLOCK >= n) break;  // uniform
+    const int i = u * SMALL_PLAN_BLOCK + threadIdx.x;
+    int64_t total;
+    const int64_t ex = block_exclusive_scan<int64_t, SMALL_PLAN_BLOCK>(i < n ? pick_count(deg[u], k, replace) : 0, smem, &total);
+    if (i < n) {
+      plan.row_begin[i] = rb[u];
+      plan.deg[i] = deg[u];
+      plan.local_off[i] = carry + ex;
+    }
+    carry += total;
+  }
+  // offsets are those in the whole output, whichever way the sampling launch adds them up
+  if (static_cast<int64_t>(threadIdx.x) < plan.ntiles) plan.tile_off[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    *plan.total = carry;
+    if (nnz_out != nullptr) {
+      *nnz_out = carry;
+      __threadfence_system();
+    }
+  }
 }
 
 // CTAs of a sampling launch beyond the main ones carry two jobs of the multi-hop sequence that depend on nothing the
@@ -922,7 +989,13 @@ int check_sample_args(const char* who, const void* seeds, int64_t n, int64_t k, 
 
 template <typename IdT>
 int plan_typed(const dgs_chunk_desc& indptr, const void* seeds, Count n, int64_t k, bool replace,
-               const PlanView& pv, int64_t* nnz, int32_t* status, cudaStream_t s) {
+               const PlanView& pv, int64_t* nnz, const InitWords& init, int32_t* status, cudaStream_t s) {
+  if (n.bound <= SMALL_PLAN) {
+    DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_small_plan_kernel<IdT>, 1u, SMALL_PLAN_BLOCK, s, indptr,
+                                static_cast<const IdT*>(seeds), static_cast<int>(n.bound), k, replace, pv, nnz, init, status));
+    return DGS_OK;
+  }
+  DGS_CUDA_TRY(launch_chained(SITE_INIT, init_kernel, 1u, 32u, s, init, pv.ticket));
   DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_plan_kernel<IdT>, static_cast<unsigned>(pv.ntiles), SAMPLE_BLOCK, s, indptr,
                               static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, pv.local_off,
                               pv.tile_off, pv.total, pv.ticket, nnz, status));
@@ -988,18 +1061,17 @@ int weighted_typed(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, c
 }  // namespace
 
 int64_t* sample_plan_total(void* plan, int64_t n_bound) { return plan_view(plan, n_bound).total; }
-unsigned int* sample_plan_ticket(void* plan, int64_t n_bound) { return plan_view(plan, n_bound).ticket; }
 
 uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset) {
   return fold_rng_key(rng_seed, rng_offset);
 }
 
-int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, Count n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, bool zero_ticket, int32_t* status, cudaStream_t s) {
-  const PlanView pv = plan_view(plan, n.bound);
-  if (zero_ticket) DGS_CUDA_TRY(cudaMemsetAsync(pv.ticket, 0, sizeof(unsigned int), s));
-  return ids64 ? plan_typed<int64_t>(indptr, seeds, n, k, replace, pv, nnz_out, status, s)
-               : plan_typed<int32_t>(indptr, seeds, n, k, replace, pv, nnz_out, status, s);
+int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, int64_t n, int64_t k,
+                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, int32_t* status, cudaStream_t s) {
+  const PlanView pv = plan_view(plan, n);
+  const Count nc = exact_count(n);
+  return ids64 ? plan_typed<int64_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, status, s)
+               : plan_typed<int32_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, status, s);
 }
 
 NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k, bool replace, void* plan) {
@@ -1059,7 +1131,7 @@ extern "C" int dgs_sample_plan(const dgs_chunk_desc* indptr, const void* seeds, 
     }
     return DGS_OK;
   }
-  return launch_sample_plan(*indptr, seeds, ids64 != 0, exact_count(n), k, replace != 0, plan, nnz, true, status, s);
+  return launch_sample_plan(*indptr, seeds, ids64 != 0, n, k, replace != 0, plan, nnz, InitWords{}, status, s);
 }
 
 extern "C" int dgs_sample_uniform(const dgs_chunk_desc* indices, const void* seeds, int32_t ids64,
