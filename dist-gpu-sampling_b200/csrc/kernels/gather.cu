@@ -617,17 +617,17 @@ int launch_gather_bulk(const Src& rows, Count nc, int64_t D, int sh, void* out, 
 // it in pieces of 4 bytes both ways and has a quarter of its usual bytes in flight (49 % of the HBM rate).  Here every row comes in
 // with one bulk copy of the aligned 16-byte blocks that cover it, and leaves repacked: a warp reads the words of its
 // group of rows from shared memory and writes the output, which is contiguous, in 16-byte vectors.  Pipeline, waits and
-// rare rows as in the bulk form.  Needs 4-byte elements at least, regions that start on 16-byte boundaries, and a
-// region's last row is copied element by element where the covering blocks would reach past its end.
+// rare rows as in the bulk form.  Elements are words: 1- and 2-byte elements stay with the register form, and rows of
+// 8-byte ones are never moved in 4-byte pieces.  Regions start on 16-byte boundaries, and a region's last row is copied
+// element by element where the covering blocks would reach past its end.
 constexpr int REPACK_WARPS = 8;
 constexpr int REPACK_STAGES = 3;
 
 template <typename Src>
 __global__ void __launch_bounds__(REPACK_WARPS * 32)
 gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_bound, const int64_t* __restrict__ n_dev,
-                          const int64_t D, const int sh, const uint32_t row_bytes, const uint32_t slot_bytes,
-                          const uint32_t group, const uint32_t div_magic, char* __restrict__ out,
-                          int32_t* __restrict__ status) {
+                          const uint32_t row_bytes, const uint32_t slot_bytes, const uint32_t group,
+                          const uint32_t div_magic, char* __restrict__ out, int32_t* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char repack_smem[];
   const uint64_t policy = l2_evict_first_policy();
   const int lane = threadIdx.x & 31;
@@ -655,7 +655,7 @@ gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_boun
   const int64_t n_groups = (n + group - 1) / group;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * n_warps;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * n_warps + warp;
-  const uint32_t nw = row_bytes / 4;  // words per row
+  const uint32_t nw = row_bytes / 4;  // words per row, and its elements
 
   auto fetch_id = [&](int64_t g) -> int64_t {
     const int64_t i = g * group + lane;
@@ -680,12 +680,9 @@ gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_boun
       bulk_load(smem_addr(slot), src - mis, bytes, bar, policy, true);
     } else if (valid) {
       // rare: zero row (bad id), a row that straddles two storage regions or ends one, element by element
-      for (int64_t j = 0; j < D; ++j) {
-        const char* p = src == DGS_ROW_ZERO ? nullptr : rows.element(i, j);
-        unsigned char* q = slot + (j << sh);
-        if (sh == 3) *reinterpret_cast<uint64_t*>(q) = p == nullptr ? 0ull : *reinterpret_cast<const uint64_t*>(p);
-        else *reinterpret_cast<uint32_t*>(q) = p == nullptr ? 0u : *reinterpret_cast<const uint32_t*>(p);
-      }
+      uint32_t* q = reinterpret_cast<uint32_t*>(slot);
+      for (uint32_t j = 0; j < nw; ++j)
+        q[j] = src == DGS_ROW_ZERO ? 0u : *reinterpret_cast<const uint32_t*>(rows.element(i, j));
     }
   };
 
@@ -754,9 +751,8 @@ gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_boun
 inline uint32_t gcd_u32(uint32_t a, uint32_t b) { return b == 0 ? a : gcd_u32(b, a % b); }
 
 template <typename Src>
-int launch_gather_repack(const Src& rows, Count nc, int64_t D, int sh, void* out, int32_t* status, int warps,
+int launch_gather_repack(const Src& rows, Count nc, uint32_t row_bytes, void* out, int32_t* status, int warps,
                          cudaStream_t stream) {
-  const uint32_t row_bytes = static_cast<uint32_t>(D << sh);
   const uint32_t slot_bytes = (row_bytes + 12u + 15u) & ~15u;
   const uint32_t unit = 16u / gcd_u32(16u, row_bytes);  // rows that make a multiple of 16 bytes
   uint32_t group = 8192u / slot_bytes / unit * unit;
@@ -793,14 +789,14 @@ int launch_gather_repack(const Src& rows, Count nc, int64_t D, int sh, void* out
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chained_launches_enabled(SITE_GATHER) ? 1 : 0;
-  DGS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, rows, nc.bound, nc.dev, D, sh, row_bytes, slot_bytes, group, magic,
+  DGS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, rows, nc.bound, nc.dev, row_bytes, slot_bytes, group, magic,
                                   static_cast<char*>(out), status));
   return DGS_OK;
 }
 
-// Rows that the register form would move in 4-byte pieces, from regions on 16-byte boundaries.  Measured with 333 k
-// rows (register form -> this one): 132 bytes 30.0 -> 29.4 us, 300 bytes 63.3 -> 46.9, 596 bytes 121.8 -> 82.0,
-// 1204 bytes 246.9 -> 138.5 (5.8 TB/s); 76 bytes 17.4 -> 22.3, since the copy engine takes ~40 cycles a row whatever
+// Rows of 4-byte elements that the register form would move in 4-byte pieces, from regions on 16-byte boundaries.
+// Measured with 333 k rows (register form -> this one): 132 bytes 30.0 -> 29.4 us, 300 bytes 63.3 -> 46.9, 596 bytes
+// 121.8 -> 82.0, 1204 bytes 246.9 -> 138.5 (5.8 TB/s); 76 bytes 17.4 -> 22.3, since the copy engine takes ~40 cycles a row whatever
 // its size.  Rows of 8-byte pieces stay with the register form (200 bytes 33.3 -> 35.9, 600 bytes 79.1 -> 81.4).
 // DGS_GATHER_REPACK=0 switches it off.
 inline bool repack_rows_qualify(const dgs_chunk_desc& d, int vec, int64_t row_bytes, const void* out) {
@@ -808,7 +804,8 @@ inline bool repack_rows_qualify(const dgs_chunk_desc& d, int vec, int64_t row_by
     const char* e = std::getenv("DGS_GATHER_REPACK");
     return e != nullptr && e[0] == '0';
   }();
-  if (off || vec != 4 || row_bytes < 160 || row_bytes > 2000 || (reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
+  if (off || d.esz != 4 || vec != 4 || row_bytes < 160 || row_bytes > 2000) return false;
+  if ((reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
   for (int p = 0; p < d.num_parts && p * d.each < d.threshold; ++p)
     if ((reinterpret_cast<uintptr_t>(d.dev[p]) & 15) != 0) return false;
   return d.threshold >= d.total || (reinterpret_cast<uintptr_t>(d.host) & 15) == 0;
@@ -849,7 +846,8 @@ int run_gather(int vec, bool realign, const dgs_chunk_desc& d, const void* idx, 
   if ((env == 1 || (env < 0 && prefer_bulk)) && bulk_rows_qualify(vec, realign, D << sh))
     return launch_gather_bulk(rows, n, D, sh, out, status, stream);
   if (repack_rows_qualify(d, vec, D << sh, out))  // behind a sampling sequence with room left beside it
-    return launch_gather_repack(rows, n, D, sh, out, status, prefer_bulk ? REPACK_WARPS / 2 : REPACK_WARPS, stream);
+    return launch_gather_repack(rows, n, static_cast<uint32_t>(D << sh), out, status,
+                                prefer_bulk ? REPACK_WARPS / 2 : REPACK_WARPS, stream);
   return dispatch_vec(vec, realign, rows, n, D, sh, out, status, stream);
 }
 
