@@ -737,6 +737,8 @@ gather_rows_repack_kernel(const __grid_constant__ Src rows, const int64_t n_boun
       const uint32_t r = __umulhi(w, div_magic);
       dst[w] = *reinterpret_cast<const uint32_t*>(stage + begin[r] + 4 * (w - r * nw));
     }
+    // this buffer's ordinary reads, and what lanes wrote into it themselves, before the bulk copy that fills it again
+    fence_async_smem();
     __syncwarp();
     g_issue += stride;
     st = st + 1 == REPACK_STAGES ? 0 : st + 1;

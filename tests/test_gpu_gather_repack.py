@@ -51,3 +51,24 @@ def test_bad_ids_and_live_count(pkg, words):
         assert words.take_status() == 0
         m = min(live, n)
         assert torch.equal(out[:m], table[idx[:m].long()]) and torch.all(out[m:] == -7.0)
+
+
+@pytest.mark.parametrize("D", [41, 75, 499])
+def test_buffers_filled_both_ways_in_turn(words, D):
+    # every warp goes through its buffers many times, with rows copied whole, zeroed and copied by words in all of them:
+    # a buffer that a lane wrote by ordinary stores is filled by a bulk copy next, and the other way round
+    from gpu_util import EmulatedChunks, gather
+    rng = np.random.default_rng(D)
+    rows, n = 4000, 400_000
+    table = rng.integers(0, 2 ** 32, (rows, D), dtype=np.uint32).view(np.float32)
+    em = EmulatedChunks(table, D, (500 * D + 7) * 4, 8)
+    ends = np.array([p * em.each // D for p in range(1, 8)])
+    idx = rng.integers(0, rows, n)
+    kind = rng.integers(0, 4, n)
+    idx[kind == 1] = -1 - idx[kind == 1]
+    idx[kind == 2] = rng.choice(ends, int((kind == 2).sum()))
+    out = gather(em.desc, torch.from_numpy(idx).cuda(), D, torch.float32, words).cpu().numpy()
+    assert words.take_status() == 6  # DGS_ERR_RANGE
+    want = table[np.maximum(idx, 0)]
+    want[idx < 0] = 0
+    assert out.tobytes() == want.tobytes()
