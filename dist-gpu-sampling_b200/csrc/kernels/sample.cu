@@ -271,7 +271,9 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
   const bool in_bound = i < nc.bound;              // ahead of the live count: the arrays have room for nc.bound
   const int64_t rb = in_bound ? plan_rb[i] : 0;
   const int64_t deg_plan = in_bound ? plan_deg[i] : 0;
-  const uint32_t o = in_bound ? static_cast<uint32_t>(local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0)) : 0u;
+  const int64_t o_plan = in_bound ? local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0) : 0;
+  // outputs at or past the capacity are left out, so an offset of 2^32 and more need not be held
+  const uint32_t o = o_plan < out_capacity ? static_cast<uint32_t>(o_plan) : out_capacity;
   const IdT seed = row_is_position ? static_cast<IdT>(i) : in_bound ? seeds[i] : IdT(0);
   const bool live = i < count_of(nc);
   const uint32_t deg = !live ? 0u : deg_plan > 0xFFFFFFFFll ? 0xFFFFFFFFu : static_cast<uint32_t>(deg_plan);

@@ -49,3 +49,32 @@ def test_lean_and_general_draw_the_same(idt, k):
     # and the general one is what it is with positions asked for
     row, col, _ = sample(d, chunks.desc, seeds, k, False, words, rng=(5, 9))
     assert np.array_equal(row, lean[0][:lean[2]]) and np.array_equal(col, lean[1][:lean[2]])
+
+
+@pytest.mark.parametrize("k", [3, 8, 15, 32])
+def test_offsets_past_the_capacity_are_left_out(k):
+    # a plan whose later seeds have their outputs at 2^32 and beyond, as with more than 2^32 edges in all
+    import ctypes
+    from gpu_util import pkg, vp
+    words, abi, n, cap = Words(), pkg.load_abi(), 700, 100 * k
+    rng = np.random.default_rng(k)
+    deg = rng.integers(1, 90, 200)
+    indptr = np.concatenate([[0], np.cumsum(deg)])
+    indices = rng.integers(0, 200, indptr[-1])
+    seeds = torch.from_numpy(rng.integers(0, 200, n)).cuda()
+    ip, ix = torch.from_numpy(indptr).cuda(), torch.from_numpy(indices).cuda()
+    chunks = EmulatedChunks(indices, 1, (indices.size // 3 + 1) * 8, 3)
+    plan = torch.empty(abi.dgs_sample_plan_bytes(n), dtype=torch.uint8, device="cuda")
+    d = plain_desc(ip)
+    pkg.check(abi.dgs_sample_plan(ctypes.byref(d), vp(seeds), 1, n, k, 0, vp(plan), None, vp(words.status), None))
+    local_off = plan.view(torch.int64)[2 * n:3 * n]
+    local_off[300:] += (1 << 32) - 300
+    got = []
+    for desc in (plain_desc(ix), chunks.desc):
+        row = torch.full((cap,), -7, device="cuda")
+        col = row.clone()
+        pkg.check(abi.dgs_sample_uniform(ctypes.byref(desc), vp(seeds), 1, n, k, 0, vp(plan), 5, 9, vp(row), vp(col), cap, None,
+                                         None, vp(words.status), None))
+        assert words.take_status() == 6  # DGS_ERR_RANGE
+        got.append((row.cpu().numpy(), col.cpu().numpy()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
