@@ -1029,7 +1029,7 @@ int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int
   } while (0)
   // one storage region, and everything that is counted fits 32 bits: rows (they lie in indices), outputs, seeds
   const bool lean = !replace && k <= 32 && pos == nullptr && indices.num_parts == 1 && indices.threshold == indices.total &&
-                    indices.total <= 0xFFFFFFFFll && cap < (1ll << 31) && n.bound < (1ll << 31);
+                    indices.total <= 0xFFFFFFFFll && cap >= 0 && cap < (1ll << 31) && n.bound < (1ll << 31);
   if (lean) {
     if (k <= 4) DGS_LAUNCH_LEAN(4);
     else if (k <= 8) DGS_LAUNCH_LEAN(8);

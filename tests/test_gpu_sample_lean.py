@@ -78,3 +78,21 @@ def test_offsets_past_the_capacity_are_left_out(k):
         assert words.take_status() == 6  # DGS_ERR_RANGE
         got.append((row.cpu().numpy(), col.cpu().numpy()))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+def test_no_capacity_at_all():
+    # a capacity of 0 or below: nothing is written, the status says so
+    import ctypes
+    from gpu_util import pkg, vp
+    words, abi, n, k = Words(), pkg.load_abi(), 50, 5
+    ip, ix = torch.arange(0, 101 * 9, 9, device="cuda"), torch.arange(900, device="cuda")
+    seeds = torch.arange(n, device="cuda")
+    plan = torch.empty(abi.dgs_sample_plan_bytes(n), dtype=torch.uint8, device="cuda")
+    d, dx = plain_desc(ip), plain_desc(ix)
+    pkg.check(abi.dgs_sample_plan(ctypes.byref(d), vp(seeds), 1, n, k, 0, vp(plan), None, vp(words.status), None))
+    for cap in (0, -1, -(1 << 40)):
+        row = torch.full((n * k,), -7, device="cuda")
+        col = row.clone()
+        pkg.check(abi.dgs_sample_uniform(ctypes.byref(dx), vp(seeds), 1, n, k, 0, vp(plan), 5, 9, vp(row), vp(col), cap, None,
+                                         None, vp(words.status), None))
+        assert words.take_status() == 6 and torch.all(row == -7) and torch.all(col == -7)  # DGS_ERR_RANGE
