@@ -467,17 +467,19 @@ __device__ __forceinline__ int ordered_float(float f) {
 }
 __device__ __forceinline__ float float_of_ordered(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
+constexpr float FLOOR_ZERO_W = -3.402823466e+38f;  // key of a weight <= 0: behind every positive weight
+constexpr float FLOOR_POS_W = -3.0e+38f;           // clamp for positive weights
+
 __device__ __forceinline__ float ares_key(uint32_t word, float w) {
-  const float FLOOR_ZERO_W = -3.402823466e+38f;  // weight <= 0: behind every positive weight
-  const float FLOOR_POS_W = -3.0e+38f;           // clamp for positive weights
   float ck = fmaxf(__fdividef(__logf(unit_float(word)), w), FLOOR_POS_W);
   asm volatile("" : "+f"(ck));  // computed by every lane: a branch around it costs more than the few it would spare
   return (w > 0.f) ? ck : FLOOR_ZERO_W;
 }
 
-// The next key below: "at or above x" as "above key_below(x)".
+// The next key below: "at or above x" as "above key_below(x)".  Both zeros are one key (log(1) / w is +0, the key of an
+// infinite weight -0).
 __device__ __forceinline__ float key_below(float x) {
-  return x == __int_as_float(0xff800000) ? x : float_of_ordered(ordered_float(x) - 1);
+  return x == __int_as_float(0xff800000) ? x : float_of_ordered((x == 0.f ? -1 : ordered_float(x)) - 1);
 }
 
 __device__ __forceinline__ Philox4 ares_words(uint64_t key, uint32_t i_lo, uint32_t i_hi, int64_t e0, int l) {
@@ -577,8 +579,9 @@ __device__ __forceinline__ void ares_first_window(ShareList& top, const RowWeigh
 // u - 1 <= bar * w cannot beat the bar.  The test below is that inequality with the slack that the errors of __logf
 // (2^-21.4 absolute on [0.5, 2]), __fdividef (2 ulp) and of the 23 random bits it looks at need, so every edge that
 // the exact key lets in passes, and the exact key decides.  One vote per 128 edges.  A bar above -1e-30 is taken as
-// -1e-30 (weights so large that __fdividef gives 0 then always pass); products that are no number (0 * inf: a list
-// that is not full and a weight <= 0) pass too.
+// -1e-30 (weights so large that __fdividef gives 0 then always pass); at or below the clamp of positive weights the
+// inequality says nothing about keys that were clamped, and every edge passes; so do products that are no number
+// (0 * inf: a weight <= 0 then).
 __device__ __forceinline__ void ares_next_window(ShareList& top, float& entry, const RowWeights& W, int64_t base,
                                                  uint32_t place, int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k) {
   const float NEG_INF = __int_as_float(0xff800000);
@@ -591,7 +594,7 @@ __device__ __forceinline__ void ares_next_window(ShareList& top, float& entry, c
     if (e0 >= deg) break;  // warp-uniform
     const Philox4 r = ares_words(key, i_lo, i_hi, e0, l);
     const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-    const float bar = fminf(entry * 1.00001f, -1e-30f);
+    const float bar = entry <= FLOOR_POS_W ? NEG_INF : fminf(entry * 1.00001f, -1e-30f);
     bool pass[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -103,3 +103,30 @@ def test_with_replacement_follows_the_prefix_sums(words, k):
         draw = u * np.float32(cdf[-1])
         want = np.minimum(np.searchsorted(cdf, draw.astype(np.float64), side="right"), d - 1)
         assert np.array_equal(pos[i], want), (i, d)
+
+
+def one_row(words, w, k, offset=5, replace=False):
+    """Positions picked from a single row with weights w, twice."""
+    n = w.size
+    ip, ix = torch.tensor([0, n], device="cuda"), torch.arange(n, device="cuda")
+    wt, seeds = torch.from_numpy(w).cuda(), torch.zeros(1, dtype=torch.int64, device="cuda")
+    got = [sample(plain_desc(ip), plain_desc(ix), seeds, k, replace, words, probs_desc=plain_desc(wt), rng=(7, offset))[2]
+           for _ in range(2)]
+    assert words.take_status() == 0 and np.array_equal(got[0], got[1])
+    return got[0]
+
+
+def test_ties_at_a_shared_bar(words):
+    # equal keys are taken by share (window modulo eight) and then by place, whichever share found the bar first:
+    # here window 2 fills a list early, and window 41 of an earlier share has the same keys
+    w = np.zeros(48 * 512, dtype=np.float32)
+    w[2 * 512:3 * 512] = w[41 * 512:42 * 512] = 1e-45  # the smallest positive weight: every key is the clamp
+    assert np.array_equal(one_row(words, w, 10), 41 * 512 + np.arange(10))
+    # a uniform of exactly 1 gives the key +0, infinite weights -0
+    w[:] = 0
+    w[1862] = 1.0  # its uniform at (7, 123) is 1
+    w[41 * 512:42 * 512] = np.inf
+    word = philox(mix64(7) ^ mix64(123 ^ 0xA5A5A5A55A5A5A5A) ^ (0x41524553 << 32), 0, 0, np.array([1862 // 128 * 32 + 1862 % 32]),
+                  np.zeros(1))[1862 % 128 // 32]
+    assert unit(word)[0] == 1.0
+    assert np.array_equal(one_row(words, w, 1, offset=123), [41 * 512])
