@@ -4,6 +4,7 @@
 #pragma once
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
@@ -48,8 +49,13 @@ inline size_t dtype_size(torch::ScalarType t) {
 }
 
 // An uninitialised tensor straight from the caching allocator: the operators allocate up to nine tensors a call, and
-// the way through the dispatcher costs more than the allocation.
+// the way through the dispatcher costs more than the allocation.  It is taken where somebody looks at it: a dispatch
+// mode, or the fill of uninitialised memory that goes with deterministic algorithms.
 inline torch::Tensor device_empty(at::IntArrayRef sizes, torch::ScalarType dtype, const torch::Device& dev) {
+  const at::Context& context = at::globalContext();
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+      (context.deterministicAlgorithms() && context.deterministicFillUninitializedMemory()))
+    return torch::empty(sizes, torch::TensorOptions().dtype(dtype).device(dev));
   return at::detail::empty_cuda(sizes, dtype, dev, c10::nullopt);
 }
 
