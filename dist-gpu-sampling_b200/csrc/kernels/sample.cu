@@ -841,11 +841,18 @@ __device__ __forceinline__ float prefix_groups(RowGroups& g, int l) {
   v.y += v.x;
   v.z += v.y;
   v.w += v.z;
-  const float before = warp_inclusive_sum(v.w, l) - v.w;
-  const float up = __shfl_up_sync(FULL_MASK, before + v.w, 1);
-  const float base = l == 0 ? 0.f : up;  // the neighbour's last prefix, so that prefixes never step back
-  reinterpret_cast<float4*>(g.incl)[l] = make_float4(base + v.x, base + v.y, base + v.z, base + v.w);
-  return __shfl_sync(FULL_MASK, base + v.w, 31);
+  // the sums of a scan are rounded each in its own way: the largest so far, so that prefixes never step back
+  float last = warp_inclusive_sum(v.w, l);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const float t = __shfl_up_sync(FULL_MASK, last, d);
+    if (l >= d) last = fmaxf(last, t);
+  }
+  const float up = __shfl_up_sync(FULL_MASK, last, 1);
+  const float base = l == 0 ? 0.f : up;
+  reinterpret_cast<float4*>(g.incl)[l] =
+      make_float4(fminf(base + v.x, last), fminf(base + v.y, last), fminf(base + v.z, last), last);
+  return __shfl_sync(FULL_MASK, last, 31);
 }
 
 // This lane's draw (0 <= draw < total): the group it falls into, and what is left of it there.

@@ -130,3 +130,27 @@ def test_ties_at_a_shared_bar(words):
                   np.zeros(1))[1862 % 128 // 32]
     assert unit(word)[0] == 1.0
     assert np.array_equal(one_row(words, w, 1, offset=123), [41 * 512])
+
+
+@pytest.mark.parametrize("k", [10, 70])
+@pytest.mark.parametrize("spread", [0, 3, 12])
+def test_with_replacement_fractional_weights(words, k, spread):
+    # an edge lies within the rounding of its draw: sums of a row go through at most 64 roundings (32 edges walked, 5
+    # folds of a group or 16 windows of a long one, 10 of the prefixes), each of 2^-24 of the row's total at most
+    rng = np.random.default_rng(k + spread)
+    deg, w, indptr, order, (ip, ix, wt, seeds) = graph(
+        lambda d, i: rng.random(d) * 10.0 ** rng.uniform(-spread, spread, d) * (rng.random(d) < (0.5 if i % 2 else 1)))
+    key = mix64(7) ^ mix64(5 ^ 0xA5A5A5A55A5A5A5A)
+    row, col, pos = sample(plain_desc(ip), plain_desc(ix), seeds, k, True, words, probs_desc=plain_desc(wt), rng=(7, 5))
+    assert words.take_status() == 0
+    pos = pos.reshape(-1, k)
+    for i, s in enumerate(order):
+        ws = w[indptr[s]:indptr[s + 1]].astype(np.float64)
+        cdf = np.concatenate([[0], np.cumsum(ws)])
+        if cdf[-1] == 0:
+            continue
+        draw = unit(philox(key, i & 0xFFFFFFFF, 0, np.arange(k), np.full(k, 0x57524550))[0]) * cdf[-1]
+        tol = 64 * 2.0 ** -24 * cdf[-1]
+        inside = draw < cdf[-1] - tol  # a draw that rounds up to the total is the last edge's, whatever its weight
+        assert np.all(cdf[pos[i]] <= draw + tol) and np.all(draw <= cdf[pos[i] + 1] + tol), (i, ws.size)
+        assert np.all(ws[pos[i]][inside] > 0)
