@@ -226,8 +226,8 @@ std::tuple<torch::Tensor, std::vector<torch::Tensor>> TensorRelabelCUDA(
   torch::Tensor table = byte_scratch(tb, first.device());
   torch::Tensor uniq = device_empty({n_keys}, first.scalar_type(), first.device());
   torch::Tensor out = device_empty({n_req}, first.scalar_type(), first.device());
-  // the count kernel reports the number of distinct keys; the numbering and
-  // lookup kernels behind it are still in flight when this returns
+  // the numbering kernel reports the number of distinct keys while it still writes labels; it and the
+  // lookup kernel behind it are still in flight when this returns
   w.sizes()[0] = kPending;
   DGS_CHECK_RC(dgs_unique_first_occurrence(&keys, ids64, table.data_ptr(), tb, uniq.data_ptr(), w.sizes(),
                                            w.status(), stream));

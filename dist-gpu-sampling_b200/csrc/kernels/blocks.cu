@@ -182,7 +182,7 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
     const int64_t k = hp.fanout;
     const int64_t edge_bound = hp.seed_bound * k;
     const int64_t key_bound = hp.seed_bound + edge_bound;
-    const Count n{hp.seed_bound, n_dev, nullptr};
+    const Count n{hp.seed_bound, n_dev};
     // the table is dimensioned before the neighbours are drawn: seeds * (1 + fanout) keys at most
     const TableSize size{n, 1 + k, max_key};
     const SideJobs jobs{make_clear_job(table[h], key_bound, size), pending, 0u};
@@ -197,7 +197,7 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
              : launch_sample_uniform(*indices, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], later, key,
                                      hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, status, s);
     if (rc != DGS_OK) return rc;
-    const Count nnz{edge_bound, nnz_dev, nullptr};
+    const Count nnz{edge_bound, nnz_dev};
     report.src[2 * h] = nnz_dev;
     report.src[2 * h + 1] = unique_total(table[h], key_bound);
     NextPlan next{};

@@ -45,16 +45,15 @@ static inline int esz_log2(int32_t esz) {
 }
 
 // A number of items that the host knows exactly (dev == nullptr: it is `bound`)
-// or only as an upper bound, the exact value being the sum of one or two device
-// words written by an earlier kernel on the same stream.  Launch grids are sized
-// by `bound`; kernels work on count_of().  This is what lets a whole multi-hop
-// sample -> relabel sequence be queued without the host reading a size back.
+// or only as an upper bound, the exact value being a device word written by an
+// earlier kernel on the same stream.  Launch grids are sized by `bound`; kernels
+// work on count_of().  This is what lets a whole multi-hop sample -> relabel
+// sequence be queued without the host reading a size back.
 struct Count {
   int64_t bound;
   const int64_t* dev;
-  const int64_t* dev2;
 };
-static inline Count exact_count(int64_t n) { return Count{n, nullptr, nullptr}; }
+static inline Count exact_count(int64_t n) { return Count{n, nullptr}; }
 
 // The Philox key of one sampling launch: a value the host computed, or (dev != nullptr) a device word an
 // earlier kernel of the same stream wrote -- what a recorded launch sequence needs, whose parameters are
@@ -82,8 +81,7 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // which launch this is; DGS_NO_PDL=1 turns the attribute off everywhere, DGS_PDL_OFF_MASK=<hex> per site
-enum LaunchSite { SITE_INIT = 0, SITE_PLAN, SITE_SAMPLE, SITE_INSERT, SITE_COUNT, SITE_NUMBER, SITE_LOOKUP,
-                  SITE_GATHER, SITE_CLEAR };
+enum LaunchSite { SITE_INIT = 0, SITE_PLAN, SITE_SAMPLE, SITE_INSERT, SITE_NUMBER = 5, SITE_LOOKUP, SITE_GATHER };
 bool chained_launches_enabled(int site);  // host/error.cc
 
 template <typename... KArgs, typename... Args>
@@ -104,8 +102,7 @@ inline cudaError_t launch_chained(int site, void (*kernel)(KArgs...), unsigned g
 
 __device__ __forceinline__ int64_t count_of(const Count& c) {
   if (c.dev == nullptr) return c.bound;
-  int64_t v = *c.dev;
-  if (c.dev2 != nullptr) v += *c.dev2;
+  const int64_t v = *c.dev;
   return v < c.bound ? (v < 0 ? 0 : v) : c.bound;
 }
 

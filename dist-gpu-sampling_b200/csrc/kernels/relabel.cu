@@ -320,8 +320,7 @@ int launch_unique_pair(bool ids64, const void* a, Count na, const void* b, Count
                        cudaStream_t s) {
   DGS_REQUIRE(key_bound > 0 && key_bound < (1ll << 30) && na.bound + nb.bound <= key_bound, DGS_ERR_UNSUPPORTED,
               "relabel: %lld keys", (long long)key_bound);
-  DGS_REQUIRE(na.dev != nullptr && nb.dev != nullptr && na.dev2 == nullptr && nb.dev2 == nullptr, DGS_ERR_INVALID,
-              "relabel: the pair form takes one device word per length");
+  DGS_REQUIRE(na.dev != nullptr && nb.dev != nullptr, DGS_ERR_INVALID, "relabel: the pair form takes a device word per length");
   const TableParts t = table_view(table, key_bound);
   const PairKeys keys{a, b, na, nb};
   return ids64 ? run_unique<int64_t, PairKeys>(keys, key_bound, size, t, unique_out, unique_capacity, n_unique_out,

@@ -27,19 +27,21 @@
 //   * bounded integers use Lemire's multiply-shift with rejection instead of
 //     `rand % n`.
 //   * weighted sampling without replacement keeps the top-k keys in a sorted
-//     per-warp register list (lane i = i-th largest) with ballot-gated
-//     insertion; keys are compared in the log domain, log(u)/w, which orders
-//     exactly like u^(1/w) but does not underflow for small weights.  Rows
-//     are read in 512-edge windows (16 loads in flight per lane) and rows longer
-//     than that are shared by the eight warps of the CTA and merged.
+//     per-warp register list (lane i = i-th largest); keys are compared in the
+//     log domain, log(u)/w, which orders exactly like u^(1/w) but does not
+//     underflow for small weights.  The first 512 edges of a row give one warp
+//     a list and a bar; the 512-edge windows behind them (16 loads in flight
+//     per lane) are dealt out to the eight warps of the CTA, which spend a
+//     logarithm only on edges that may beat the bar, and the lists are joined.
 //   * weighted sampling with replacement builds no cumulative array in global
-//     memory: the row is summed once in windows of 512 edges, and each draw is
-//     resolved by ballots in the stretch, the window and the 32 edges it falls into.
-//   * counts, offsets and the total come from ONE plan kernel: every CTA scans
-//     its 256 seeds and the CTA that finishes last (an atomic ticket, nobody
-//     waits) scans the per-tile sums; the total goes to a caller-supplied
-//     (pinned) word, so the host learns the output size while the sampling
-//     kernel is still running.
+//     memory: the row is summed once into at most 128 groups, and every lane
+//     finds its own draw's group by bisection and walks the edges in it.
+//   * counts, offsets and the total come from a plan: one CTA for up to 4 096
+//     seeds; above, every CTA scans its 256 seeds and the one that finishes last
+//     (an atomic ticket, nobody waits) scans the per-tile sums; from the second
+//     hop of a multi-hop sequence on, the kernel that numbers the seeds.  The
+//     total goes to a caller-supplied (pinned) word, so the host learns the
+//     output size while the sampling kernel is still running.
 //   * the sampling kernels give every seed its own group / warp and never loop
 //     over seeds, so even a 1 024-seed hop fills the machine with independent
 //     short chains instead of a few long ones.
@@ -366,8 +368,8 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
 }
 
 // ---------------------------------------------------------------------------
-// weighted sampling: one warp per seed; rows longer than LONG_ROW edges are then
-// taken on by all eight warps of the CTA together
+// weighted sampling: one warp per seed for the first 512 edges of its row; what is
+// left of longer rows is dealt out to the eight warps of the CTA
 // ---------------------------------------------------------------------------
 // a weight of a row that straddles storage regions (at most one row per boundary); out of line, because its
 // address arithmetic, inlined at every load, made the sampling kernel 300 KB of code

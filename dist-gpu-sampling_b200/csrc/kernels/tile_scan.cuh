@@ -49,29 +49,25 @@ tile_scan_kernel(int64_t* __restrict__ sums, const int64_t ntiles, int64_t* __re
 // this after computing its tile sum.  The CTA that draws the last ticket (an
 // atomic counter that must be zero at launch; nobody waits on anybody) scans
 // all tile sums in place and publishes the total.  `smem` needs BLOCK/32 + 1
-// entries; must be called by all threads of the CTA.  Returns true in that last CTA.
-// The tiles are CTAs 0 .. ntiles-1 of the launch (the launch may hold further CTAs
-// with other work, which do not call this).
+// entries; must be called by all threads of the CTA.  The tiles are the CTAs of the launch.
 template <int BLOCK>
-__device__ __forceinline__ bool publish_and_scan_tiles(int64_t my_tile_sum, int64_t* tile_sums,
+__device__ __forceinline__ void publish_and_scan_tiles(int64_t my_tile_sum, int64_t* tile_sums,
                                                        unsigned int* ticket, int64_t* total_dev,
-                                                       int64_t* total_out, int64_t* smem,
-                                                       unsigned int n_tiles = 0) {
+                                                       int64_t* total_out, int64_t* smem) {
   __shared__ bool s_last;
-  if (n_tiles == 0) n_tiles = gridDim.x;
   if (threadIdx.x == 0) {
     tile_sums[blockIdx.x] = my_tile_sum;
     __threadfence();
-    s_last = atomicAdd(ticket, 1u) == n_tiles - 1;
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!s_last) return false;
+  if (!s_last) return;
   __threadfence();
   // Every thread takes a contiguous run of `per` tiles: all loads of the CTA are issued together (one round
   // trip to L2 whatever the number of tiles, instead of one per BLOCK tiles), one block scan over the threads'
   // sums gives each run its offset, and a second walk over the run (now in L1/L2) writes the prefixes.  This
   // CTA works alone at the end of its kernel, so every microsecond here is latency of the whole sequence.
-  const int64_t ntiles = n_tiles;
+  const int64_t ntiles = gridDim.x;
   const int64_t per = (ntiles + BLOCK - 1) / BLOCK;
   const int64_t lo = static_cast<int64_t>(threadIdx.x) * per;
   const int64_t hi = lo + per < ntiles ? lo + per : ntiles;
@@ -92,7 +88,6 @@ __device__ __forceinline__ bool publish_and_scan_tiles(int64_t my_tile_sum, int6
       __threadfence_system();
     }
   }
-  return true;  // this CTA was the last one: the totals are final
 }
 
 // ---- offsets in one pass -------------------------------------------------------
