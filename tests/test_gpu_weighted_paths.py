@@ -154,3 +154,62 @@ def test_with_replacement_fractional_weights(words, k, spread):
         inside = draw < cdf[-1] - tol  # a draw that rounds up to the total is the last edge's, whatever its weight
         assert np.all(cdf[pos[i]] <= draw + tol) and np.all(draw <= cdf[pos[i] + 1] + tol), (i, ws.size)
         assert np.all(ws[pos[i]][inside] > 0)
+
+
+@pytest.mark.parametrize("k", [1, 10, 32])
+@pytest.mark.parametrize("low,high", [(-30, 30), (-3, 3), (20, 30), (-30, -20)])
+def test_without_replacement_spread_weights(words, k, low, high):
+    # the picks are the k largest of log(u) / w but for what the fp32 key may be off by: __logf 2^-21.4 absolute on
+    # [0.5, 2] and 3 ulp elsewhere, __fdividef 2 ulp, the subtraction-free rest nothing
+    rng = np.random.default_rng(k)
+    deg, w, indptr, order, (ip, ix, wt, seeds) = graph(lambda d, i: 10.0 ** rng.uniform(low, high, d))
+    key = mix64(7) ^ mix64(5 ^ 0xA5A5A5A55A5A5A5A) ^ (0x41524553 << 32)
+    row, col, pos = sample(plain_desc(ip), plain_desc(ix), seeds, k, False, words, probs_desc=plain_desc(wt), rng=(7, 5))
+    assert words.take_status() == 0
+    at = 0
+    for i, s in enumerate(order):
+        d = int(deg[s])
+        m = min(d, k)
+        got, at = pos[at:at + m], at + m
+        if d <= k:
+            assert np.array_equal(got, np.arange(d))
+            continue
+        assert np.unique(got).size == k
+        e = np.arange(d)
+        log_u = np.log(unit(np.choose(e % 128 // 32, philox(key, i & 0xFFFFFFFF, 0, (e // 128) * 32 + e % 32, np.zeros(d)))))
+        ws = w[indptr[s]:indptr[s + 1]].astype(np.float64)
+        keys = log_u / ws
+        off = 2.0 ** -21.4 * np.maximum(1, -log_u) / ws + 2.0 ** -22 * -keys
+        out = np.ones(d, bool)
+        out[got] = False
+        assert (keys + off)[got].min() >= (keys - off)[out].max()
+        ranks = keys[got]  # and they come in the order of their keys
+        assert np.all(ranks[:-1] + off[got][:-1] >= ranks[1:] - off[got][1:])
+
+
+def test_without_replacement_weights_that_are_no_number(words):
+    # infinite weights come first (their keys tie: by place), then the positive ones by key, then the rest in scan order;
+    # a weight that is no number counts as none, as negative ones do
+    for n in (100, 512, 3000):
+        w = np.zeros(n, dtype=np.float32)
+        w[5::7] = np.nan
+        w[6::7] = -1.0
+        w[[40, 77, n - 3]] = np.inf
+        w[[11, 60, 90]] = [0.5, 2.0, 1e-3]
+        got = one_row(words, w, 10)
+        assert np.array_equal(got[:3], [40, 77, n - 3]) and set(got[3:6]) == {11, 60, 90}
+        rest = np.flatnonzero(~(w > 0))
+        assert np.array_equal(got[6:], rest[:4])
+    w = np.full(9000, np.nan, dtype=np.float32)  # above eight windows: by window modulo eight, then by place
+    w[[8 * 512 + 3, 100]] = np.inf
+    assert np.array_equal(one_row(words, w, 5), [100, 8 * 512 + 3, 0, 1, 2])
+
+
+def test_with_replacement_weights_that_are_no_number(words):
+    w = np.ones(5000, dtype=np.float32)
+    w[::2] = np.nan
+    w[1::4] = -np.inf
+    assert np.all(one_row(words, w, 200, replace=True) % 4 == 3)
+    w[100] = np.inf  # no draw is below an infinite sum: the last edge
+    assert np.all(one_row(words, w, 20, replace=True) == 4999)
+    assert np.all(one_row(words, w[:300], 20, replace=True) == 299)
