@@ -755,19 +755,11 @@ inline uint32_t gcd_u32(uint32_t a, uint32_t b) { return b == 0 ? a : gcd_u32(b,
 template <typename Src>
 int launch_gather_repack(const Src& rows, Count nc, uint32_t row_bytes, void* out, int32_t* status, int warps,
                          cudaStream_t stream) {
-  const uint32_t slot_bytes = (row_bytes + 12u + 15u) & ~15u;
-  const uint32_t unit = 16u / gcd_u32(16u, row_bytes);  // rows that make a multiple of 16 bytes
-  uint32_t group = 8192u / slot_bytes / unit * unit;
-  if (group > 32u) group = 32u;
-  const uint32_t nw = row_bytes / 4;
-  const uint32_t magic = static_cast<uint32_t>(((1ull << 32) + nw - 1) / nw);
-  const size_t smem = static_cast<size_t>(warps) * REPACK_STAGES * (group * slot_bytes + sizeof(uint64_t) + 32 * sizeof(uint32_t));
   // per device and safe to reach from several host threads: the SM count, and whether this instantiation has
   // been allowed its dynamic shared memory there (the attribute belongs to the device's copy of the kernel)
   constexpr int kMaxDevices = 64;
   constexpr int kMaxSmem = 208 * 1024;
   static std::atomic<int> sm_count[kMaxDevices] = {};
-  DGS_REQUIRE(group >= 1 && smem <= kMaxSmem, DGS_ERR_UNSUPPORTED, "gather: %zu bytes of shared memory per CTA", smem);
   int dev = 0;
   DGS_CUDA_TRY(cudaGetDevice(&dev));
   DGS_REQUIRE(dev >= 0 && dev < kMaxDevices, DGS_ERR_UNSUPPORTED, "gather: device ordinal %d", dev);
@@ -778,6 +770,21 @@ int launch_gather_repack(const Src& rows, Count nc, uint32_t row_bytes, void* ou
     DGS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     sm_count[dev].store(sms, std::memory_order_release);
   }
+  const uint32_t slot_bytes = (row_bytes + 12u + 15u) & ~15u;
+  const uint32_t unit = 16u / gcd_u32(16u, row_bytes);  // rows that make a multiple of 16 bytes
+  uint32_t group = 8192u / slot_bytes / unit * unit;
+  if (group > 32u) group = 32u;
+  DGS_REQUIRE(group >= 1, DGS_ERR_UNSUPPORTED, "gather: rows of %u bytes in the repacked form", row_bytes);
+  // rows are dealt out in rounds of one group per warp: as many rounds as groups of this size need, all equally full.
+  // With whole groups 1 000 rows of 300 bytes took 4.9 us on 6 SMs, in groups of four 2.9; 32 000 rows 8.6 us, now 6.9
+  const int64_t lanes = static_cast<int64_t>(sms) * warps;
+  const int64_t rounds = (nc.bound + lanes * group - 1) / (lanes * group);
+  const int64_t even = (nc.bound + lanes * rounds - 1) / (lanes * rounds);
+  group = static_cast<uint32_t>((even + unit - 1) / unit) * unit;
+  const uint32_t nw = row_bytes / 4;
+  const uint32_t magic = static_cast<uint32_t>(((1ull << 32) + nw - 1) / nw);
+  const size_t smem = static_cast<size_t>(warps) * REPACK_STAGES * (group * slot_bytes + sizeof(uint64_t) + 32 * sizeof(uint32_t));
+  DGS_REQUIRE(smem <= kMaxSmem, DGS_ERR_UNSUPPORTED, "gather: %zu bytes of shared memory per CTA", smem);
   const int64_t groups = (nc.bound + group - 1) / group;
   int64_t grid = (groups + warps - 1) / warps;
   if (grid > static_cast<int64_t>(sms)) grid = static_cast<int64_t>(sms);
@@ -797,16 +804,24 @@ int launch_gather_repack(const Src& rows, Count nc, uint32_t row_bytes, void* ou
 }
 
 // Rows of 4-byte elements that the register form would move in 4-byte pieces, from regions on 16-byte boundaries.
-// Measured with 333 k rows (register form -> this one): 132 bytes 30.0 -> 29.4 us, 300 bytes 63.3 -> 46.9, 596 bytes
-// 121.8 -> 82.0, 1204 bytes 246.9 -> 138.5 (5.8 TB/s); 76 bytes 17.4 -> 22.3, since the copy engine takes ~40 cycles a row whatever
-// its size.  Rows of 8-byte pieces stay with the register form (200 bytes 33.3 -> 35.9, 600 bytes 79.1 -> 81.4).
+// Measured with 333 k rows (register form -> this one): 132 bytes 30.0 -> 29.4 us, 164 bytes 34.3 -> 29.8, 300 bytes
+// 62.5 -> 45.8, 596 bytes 121 -> 80, 1204 bytes 246 -> 137 (5.9 TB/s); 76 bytes 17.4 -> 22.3, since an SM takes
+// ~10 ns a row however short it is.  Rows of 8-byte pieces stay with the register form (200 bytes 33.3 -> 35.9).
+// Few rows: a warp's first rows arrive later than a register load does, the longer the row the more.  300 bytes: 4 rows
+// 1.9 -> 2.2 us, 16 rows 2.3 -> 2.3, 1 000 rows 3.3 -> 2.9; 700 bytes level up to 3 000 rows; 900 bytes: 1 000 rows
+// 3.2 -> 3.6, 2 500 rows 3.5 -> 3.8, 3 000 rows 4.4 -> 3.9; 1996 bytes: 1 000 rows 3.5 -> 4.8, 2 000 rows 5.0 -> 5.1.
 // DGS_GATHER_REPACK=0 switches it off.
-inline bool repack_rows_qualify(const dgs_chunk_desc& d, int vec, int64_t row_bytes, const void* out) {
+constexpr int64_t REPACK_MIN_ROWS = 16;
+constexpr int64_t REPACK_WIDE_BYTES = 720;
+constexpr int64_t REPACK_MIN_WIDE_ROWS = 2500;
+
+inline bool repack_rows_qualify(const dgs_chunk_desc& d, int vec, int64_t row_bytes, int64_t n, const void* out) {
   static const bool off = [] {
     const char* e = std::getenv("DGS_GATHER_REPACK");
     return e != nullptr && e[0] == '0';
   }();
   if (off || d.esz != 4 || vec != 4 || row_bytes < 160 || row_bytes > 2000) return false;
+  if (n < (row_bytes > REPACK_WIDE_BYTES ? REPACK_MIN_WIDE_ROWS : REPACK_MIN_ROWS)) return false;
   if ((reinterpret_cast<uintptr_t>(out) & 15) != 0) return false;
   for (int p = 0; p < d.num_parts && p * d.each < d.threshold; ++p)
     if ((reinterpret_cast<uintptr_t>(d.dev[p]) & 15) != 0) return false;
@@ -847,7 +862,7 @@ int run_gather(int vec, bool realign, const dgs_chunk_desc& d, const void* idx, 
   const int env = bulk_env();
   if ((env == 1 || (env < 0 && prefer_bulk)) && bulk_rows_qualify(vec, realign, D << sh))
     return launch_gather_bulk(rows, n, D, sh, out, status, stream);
-  if (repack_rows_qualify(d, vec, D << sh, out))  // behind a sampling sequence with room left beside it
+  if (repack_rows_qualify(d, vec, D << sh, n.bound, out))  // behind a sampling sequence with room left beside it
     return launch_gather_repack(rows, n, static_cast<uint32_t>(D << sh), out, status,
                                 prefer_bulk ? REPACK_WARPS / 2 : REPACK_WARPS, stream);
   return dispatch_vec(vec, realign, rows, n, D, sh, out, status, stream);

@@ -72,3 +72,15 @@ def test_buffers_filled_both_ways_in_turn(words, D):
     want = table[np.maximum(idx, 0)]
     want[idx < 0] = 0
     assert out.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("D,n", [(D, n) for D, group in ((41, 32), (75, 24), (149, 12), (179, 8), (181, 8), (301, 4), (499, 4))
+                                 for n in [1, 15, 16, 17, 2499, 2500, 2501] +
+                                 [148 * 8 * group * r + x for r in (1, 2) for x in (-1, 0, 1)] + [148 * 4 * group + 1]])
+def test_number_of_rows(words, D, n):
+    # where the form begins (16 rows, 2 500 of more than 720 bytes) and around whole rounds of groups over 148 SMs
+    from gpu_util import gather, plain_desc
+    table = torch.randn(5000, D, device="cuda")
+    idx = torch.randint(0, 5000, (n,), device="cuda")
+    out = gather(plain_desc(table), idx, D, torch.float32, words)
+    assert words.take_status() == 0 and torch.equal(out, table[idx])
