@@ -36,7 +36,7 @@
 //   * weighted sampling with replacement builds no cumulative array in global
 //     memory: the row is summed once into at most 128 groups, and every lane
 //     finds its own draw's group by bisection and walks the edges in it.
-//   * counts, offsets and the total come from a plan: one CTA for up to 4 096
+//   * counts, offsets and the total come from a plan: one CTA for up to 2 048
 //     seeds; above, every CTA scans its 256 seeds and the one that finishes last
 //     (an atomic ticket, nobody waits) scans the per-tile sums; from the second
 //     hop of a multi-hop sequence on, the kernel that numbers the seeds.  The
@@ -136,9 +136,13 @@ sample_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __r
 
 // The plan of up to SMALL_PLAN seeds by one CTA: no ticket, hence nothing that has to be cleared before it, and in the
 // multi-hop sequence it sets the words that a launch of its own sets otherwise.  Bound by latency (seed, row bounds,
-// scan); four seeds per thread with their loads in flight together.
+// scan); two seeds per thread with their loads in flight together.
+// The line, against a CTA per 256 seeds behind a clearing launch (us; indptr of 2.4 M nodes on the GPU, then of 20 M in
+// host memory): 64 seeds 2.8 against 3.9 and 3.6 against 5.5, 1 024 seeds 3.7 against 4.2 and 7.2 against 9.3, 2 048
+// seeds 4.9 against 5.0 and 11.0 against 11.6, 3 072 seeds 6.1 against 5.0 and 14.7 against 14.6, 4 096 seeds 7.5
+// against 5.0 and 18.6 against 18.3.
 constexpr int SMALL_PLAN_BLOCK = 1024;
-constexpr int SMALL_PLAN_ITEMS = 4;
+constexpr int SMALL_PLAN_ITEMS = 2;
 constexpr int SMALL_PLAN = SMALL_PLAN_BLOCK * SMALL_PLAN_ITEMS;
 
 template <typename IdT>

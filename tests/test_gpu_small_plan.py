@@ -47,3 +47,10 @@ def test_plan_offsets(n, replace, idt):
     assert np.array_equal(row_begin, rb) and np.array_equal(degree, d)
     assert np.array_equal(local + tile[np.arange(n) // 256], np.cumsum(cnt) - cnt)
     assert int(words.sizes[0]) == cnt.sum() == got[3 * n + tiles]
+
+
+@pytest.mark.parametrize("idt", [np.int64, np.int32])
+@pytest.mark.parametrize("replace", [0, 1])
+@pytest.mark.parametrize("n", [2047, 2049])
+def test_plan_offsets_at_the_line(n, replace, idt):
+    test_plan_offsets(n, replace, idt)
