@@ -277,9 +277,7 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
   const bool in_bound = i < nc.bound;              // ahead of the live count: the arrays have room for nc.bound
   const int64_t rb = in_bound ? plan_rb[i] : 0;
   const int64_t deg_plan = in_bound ? plan_deg[i] : 0;
-  const int64_t o_plan = in_bound ? local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0) : 0;
-  // outputs at or past the capacity are left out, so an offset of 2^32 and more need not be held
-  const uint32_t o = o_plan < out_capacity ? static_cast<uint32_t>(o_plan) : out_capacity;
+  const uint32_t o = in_bound ? static_cast<uint32_t>(local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0)) : 0u;
   const IdT seed = row_is_position ? static_cast<IdT>(i) : in_bound ? seeds[i] : IdT(0);
   const bool live = i < count_of(nc);
   const uint32_t deg = !live ? 0u : deg_plan > 0xFFFFFFFFll ? 0xFFFFFFFFu : static_cast<uint32_t>(deg_plan);
@@ -1043,9 +1041,11 @@ int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int
                                 pv.deg, pv.local_off, pv.tile_off, key, static_cast<IdT*>(coo_row),           \
                                 static_cast<IdT*>(coo_col), static_cast<uint32_t>(cap), rowpos, jobs, status)); \
   } while (0)
-  // one storage region, and everything that is counted fits 32 bits: rows (they lie in indices), outputs, seeds
+  // one storage region, and everything that is counted fits 32 bits: rows (they lie in indices), seeds, and the offsets of
+  // all outputs that a plan may hold, also of those past the capacity
   const bool lean = !replace && k <= 32 && pos == nullptr && indices.num_parts == 1 && indices.threshold == indices.total &&
-                    indices.total <= 0xFFFFFFFFll && cap >= 0 && cap < (1ll << 31) && n.bound < (1ll << 31);
+                    indices.total <= 0xFFFFFFFFll && cap >= 0 && cap < (1ll << 31) && n.bound < (1ll << 31) &&
+                    n.bound * k < (1ll << 32) - 64;
   if (lean) {
     if (k <= 4) DGS_LAUNCH_LEAN(4);
     else if (k <= 8) DGS_LAUNCH_LEAN(8);
