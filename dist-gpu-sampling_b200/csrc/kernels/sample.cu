@@ -279,7 +279,7 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
   const int64_t deg_plan = in_bound ? plan_deg[i] : 0;
   const uint32_t o = in_bound ? static_cast<uint32_t>(local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0)) : 0u;
   const IdT seed = row_is_position ? static_cast<IdT>(i) : in_bound ? seeds[i] : IdT(0);
-  const bool live = i < count_of(nc);
+  const bool live = in_bound && (nc.dev == nullptr || i < *nc.dev);
   const uint32_t deg = !live ? 0u : deg_plan > 0xFFFFFFFFll ? 0xFFFFFFFFu : static_cast<uint32_t>(deg_plan);
   if (live && deg_plan > 0xFFFFFFFFll) raise_status(status, DGS_ERR_RANGE);  // longer than `indices`: broken row bounds
 
