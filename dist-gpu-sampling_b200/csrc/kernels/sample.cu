@@ -138,9 +138,9 @@ sample_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __r
 // multi-hop sequence it sets the words that a launch of its own sets otherwise.  Bound by latency (seed, row bounds,
 // scan); two seeds per thread with their loads in flight together.
 // The line, against a CTA per 256 seeds behind a clearing launch (us; indptr of 2.4 M nodes on the GPU, then of 20 M in
-// host memory): 64 seeds 2.8 against 3.9 and 3.6 against 5.5, 1 024 seeds 3.7 against 4.2 and 7.2 against 9.3, 2 048
-// seeds 4.9 against 5.0 and 11.0 against 11.6, 3 072 seeds 6.1 against 5.0 and 14.7 against 14.6, 4 096 seeds 7.5
-// against 5.0 and 18.6 against 18.3.
+// host memory): 64 seeds 2.1 against 3.9 and 3.3 against 5.5, 1 024 seeds 3.0 against 4.2 and 6.7 against 9.3, 2 048
+// seeds 4.4 against 5.0 and 10.6 against 11.6.  With four seeds per thread: 3 072 seeds 6.1 against 5.0 and 14.7 against
+// 14.6, 4 096 seeds 7.5 against 5.0 and 18.6 against 18.3.
 constexpr int SMALL_PLAN_BLOCK = 1024;
 constexpr int SMALL_PLAN_ITEMS = 2;
 constexpr int SMALL_PLAN = SMALL_PLAN_BLOCK * SMALL_PLAN_ITEMS;
@@ -255,8 +255,9 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
 
 // The same for the common launch: without replacement, k <= G, `indices` in one piece on this GPU and rows and outputs
 // that 32-bit arithmetic can hold (see uniform_typed).  Same random numbers, same picks.
-// Bound by issue slots: 525 warp instructions per two seeds in the general kernel, most of them address arithmetic of
-// chunked tensors, 64-bit positions and the branches around both.  60 000 seeds, fan-out 15: 26 -> 18 us.
+// Bound by issue slots: 449 warp instructions per two seeds at 32 registers (76 % of the warps), where the general kernel
+// has 544 at 40 (57 %): the address arithmetic of chunked tensors, 64-bit positions and the branches around both.
+// 60 000 seeds, fan-out 15: 26 -> 17.7 us.
 template <typename IdT, int G>
 __global__ void __launch_bounds__(SAMPLE_BLOCK)
 sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edges, const IdT* __restrict__ seeds,
@@ -659,7 +660,7 @@ __device__ __forceinline__ void ares_share(const RowWeights& W, int64_t deg, uin
   list_place[l] = top.pos;
 }
 
-// A-Res without replacement.  Bound by issue slots (150 warp instructions per 32 edges) and the latency of the list
+// A-Res without replacement.  Bound by issue slots (164 warp instructions per 32 edges of rows of 380) and the latency of the list
 // operations, not by the bytes of the weights.  Eight seeds per CTA of eight warps: each warp takes the first 512
 // edges of its own row, which gives the row a bar to beat; what is left of the CTA's longer rows is dealt out to its
 // warps in shares, and one warp per row joins them.  11 000 rows, 9.1 M weights, fan-out 10: 89 us, against 188 us
