@@ -72,11 +72,17 @@ WORKLOADS = {
 }
 
 # kernels of this library launched per operator call (memsets and copies are not kernels)
-LAUNCHES_SAMPLE = 2      # plan (+ tile scan in its last CTA), sample
-LAUNCHES_RELABEL = 4     # insert, count (+ tile scan in its last CTA), number, lookup
+LAUNCHES_RELABEL = 3     # insert, number (+ look-back), lookup
 LAUNCHES_GATHER = 1
-LAUNCHES_HOP_FUSED = 5   # plan (+ table clear + previous hop's lookup), sample, insert, count, number
-LAUNCHES_STEP_FUSED = 2  # init words, last hop's lookup
+LAUNCHES_HOP_FUSED = 3   # sample (+ table clear + previous hop's lookup), insert, number (+ the next hop's plan)
+LAUNCHES_LAST_LOOKUP = 1
+
+
+def launches_plan(seeds):
+    """One CTA up to 2 048 seeds; above, a clearing launch and a CTA per 256 seeds."""
+    return 1 if seeds <= 2048 else 2
+
+
 PRIME_STEPS = 8          # untimed one-at-a-time steps that populate torch's caching allocator
 API_NAMES = {
     "pipeline": "BlockPipeline: %d batches in flight, each = one queued sample_blocks sequence + device-counted gather",
@@ -913,9 +919,12 @@ def main_ours(args):
             return {"api": label, "value": rate(r, name), "unit": "edges/s", "ms_per_step": r[name]["ms"] / steps}
         main = args.api
         others = [entry(red, n, args.steps) for n in ("pipeline", "blocks", "per-hop") if n != main]
-        launches_step = {"pipeline": LAUNCHES_STEP_FUSED + H * LAUNCHES_HOP_FUSED + LAUNCHES_GATHER,
-                         "blocks": LAUNCHES_STEP_FUSED + H * LAUNCHES_HOP_FUSED + LAUNCHES_GATHER,
-                         "per-hop": H * (LAUNCHES_SAMPLE + LAUNCHES_RELABEL) + LAUNCHES_GATHER}[main]
+        fused = launches_plan(args.batch) + H * LAUNCHES_HOP_FUSED + LAUNCHES_LAST_LOOKUP + LAUNCHES_GATHER
+        per_hop, seeds_bound = LAUNCHES_GATHER, args.batch
+        for k in reversed(fanouts):  # operator by operator; the later hops' seeds by their bound
+            per_hop += launches_plan(seeds_bound) + 1 + LAUNCHES_RELABEL
+            seeds_bound *= 1 + k
+        launches_step = {"pipeline": fused, "blocks": fused, "per-hop": per_hop}[main]
         bl = red["blocks"]
         line = {
             "library": "dist-gpu-sampling_b200/lib/libdgs.so",
