@@ -123,6 +123,13 @@ ABI_SIGNATURES = {
                                                 _VP, ctypes.POINTER(_VP)]),
     "dgs_sample_blocks_replay": (ctypes.c_int, [_VP, _VP]),
     "dgs_sample_blocks_recording_free": (None, [_VP]),
+    "dgs_sample_blocks_dense_wins": (_I32, [_HP, _I32, _I64]),
+    "dgs_sample_blocks_dense_workspace_bytes": (_SZ, [_HP, _I32, _I64]),
+    "dgs_sample_blocks_dense": (ctypes.c_int, [_DP, _DP, _DP, _VP, _I32, _HP, _I32, _I32, _I64, _U64, _U64, _VP, _SZ, _VP,
+                                               _VP, _VP]),
+    "dgs_sample_blocks_dense_frontier_count": (_VP, [_HP, _I32, _I64, _VP]),
+    "dgs_sample_blocks_dense_record": (ctypes.c_int, [_DP, _DP, _DP, _VP, _I32, _HP, _I32, _I32, _I64, _VP, _VP, _SZ, _VP,
+                                                      _VP, _VP, ctypes.POINTER(_VP)]),
     "dgs_cache_table_slots": (_I64, [_I64]),
     "dgs_cache_build": (ctypes.c_int, [_VP, _VP, _I32, _I64, _VP, _VP, _I64, _VP, _VP]),
     "dgs_cache_fetch": (ctypes.c_int, [_VP, _I64, _DP, _VP, _I32, _I64, _I64, _VP, _VP, _I64, _VP, _VP, _VP]),

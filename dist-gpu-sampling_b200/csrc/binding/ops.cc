@@ -307,7 +307,11 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
   cudaStream_t stream = current_stream();
   const Lease w("_CAPI_sample_blocks*", seeds.device().index(), stream);
   const auto rng = next_rng(static_cast<uint64_t>(H));
-  torch::Tensor ws = byte_scratch(ws_bytes, seeds.device());
+  // one word per id of indptr's node space where that is the faster form (bytes bounded like the hash tables above)
+  const int64_t id_space = indptr.total - 1;
+  size_t dense_bytes = 0;
+  if (dgs_sample_blocks_dense_wins(hops, H, id_space)) dense_bytes = dgs_sample_blocks_dense_workspace_bytes(hops, H, id_space);
+  torch::Tensor ws = byte_scratch(dense_bytes > 0 ? dense_bytes : ws_bytes, seeds.device());
   std::vector<torch::Tensor> fr(H);
   for (int h = 0; h < H; ++h) {
     const int64_t cap = hops[h].seed_bound * hops[h].fanout;
@@ -319,17 +323,35 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
     hops[h].frontier = fr[h].data_ptr();
     w.sizes()[2 * h] = w.sizes()[2 * h + 1] = kPending;
   }
-  DGS_CHECK_RC(dgs_sample_blocks(&indptr, &indices, probs, seeds.data_ptr(), ids64, hops, H, replace, rng.first,
-                                 rng.second, ws.data_ptr(), ws_bytes, w.sizes(), w.status(), stream));
   // the one read-back: the last size lands while that hop's numbering and lookup still run
   int64_t n_dst = n;
   bool outgrown = false;
-  for (int h = 0; h < H; ++h) {
-    const int64_t nnz = wait_size(w.sizes() + 2 * h, stream, "sample_blocks");
-    const int64_t nu = wait_size(w.sizes() + 2 * h + 1, stream, "sample_blocks");
-    TORCH_CHECK(nnz >= 0 && nnz <= hops[h].seed_bound * hops[h].fanout && nu >= 0,
-                "dgs: sample_blocks returned an impossible size");
-    outgrown = outgrown || nu > hops[h].frontier_bound;
+  auto read_sizes = [&] {
+    for (int h = 0; h < H; ++h) {
+      const int64_t nnz = wait_size(w.sizes() + 2 * h, stream, "sample_blocks");
+      const int64_t nu = wait_size(w.sizes() + 2 * h + 1, stream, "sample_blocks");
+      TORCH_CHECK(nnz >= 0 && nnz <= hops[h].seed_bound * hops[h].fanout && nu >= 0,
+                  "dgs: sample_blocks returned an impossible size");
+      outgrown = outgrown || nu > hops[h].frontier_bound;
+    }
+  };
+  if (dense_bytes > 0) {
+    DGS_CHECK_RC(dgs_sample_blocks_dense(&indptr, &indices, probs, seeds.data_ptr(), ids64, hops, H, replace, id_space,
+                                         rng.first, rng.second, ws.data_ptr(), dense_bytes, w.sizes(), w.status(), stream));
+    read_sizes();
+    if (*static_cast<volatile int32_t*>(w.status()) == DGS_ERR_ID_SPACE) {
+      // column ids beyond indptr's nodes (a bipartite CSC): the same batch again through the form that takes any id
+      sync_stream();
+      *w.status() = 0;
+      for (int h = 0; h < 2 * H; ++h) w.sizes()[h] = kPending;
+      dense_bytes = 0;
+      ws = byte_scratch(ws_bytes, seeds.device());
+    }
+  }
+  if (dense_bytes == 0) {
+    DGS_CHECK_RC(dgs_sample_blocks(&indptr, &indices, probs, seeds.data_ptr(), ids64, hops, H, replace, rng.first,
+                                   rng.second, ws.data_ptr(), ws_bytes, w.sizes(), w.status(), stream));
+    read_sizes();
   }
   if (outgrown) {
     // The bound assumes that neighbour ids lie in indptr's node space.  On a bipartite CSC whose column ids

@@ -100,6 +100,8 @@ class BlockPipeline : public torch::CustomClassHolder {
     ws_bytes_ = dgs_sample_blocks_workspace_bytes(hops, H_);
     const int64_t esz = ids64_ ? 8 : 4;
     int64_t slot_bytes = static_cast<int64_t>(ws_bytes_) + max_seeds_ * esz;
+    // one word per id of the id space where that is the faster form; the workspace holds either form
+    const size_t dense_bytes = dgs_sample_blocks_dense_workspace_bytes(hops, H_, id_space_);
     for (int h = 0; h < H_; ++h) {
       edge_cap_[h] = hops[h].seed_bound * hops[h].fanout;
       frontier_cap_[h] = hops[h].frontier_bound;
@@ -109,6 +111,11 @@ class BlockPipeline : public torch::CustomClassHolder {
       slot_bytes += frontier_cap_[H_ - 1] * features_->elem_stride() * static_cast<int64_t>(dtype_size(features_->dtype()));
     TORCH_CHECK(slot_bytes * depth <= kBudgetBytes, "BlockPipeline: ", depth, " slots of ", slot_bytes,
                 " bytes exceed the ", kBudgetBytes, "-byte budget; lower max_seeds, the fan-outs or depth");
+    const int64_t more = dense_bytes > ws_bytes_ ? static_cast<int64_t>(dense_bytes - ws_bytes_) : 0;
+    if (dense_bytes > 0 && dgs_sample_blocks_dense_wins(hops, H_, id_space_) && (slot_bytes + more) * depth <= kBudgetBytes) {
+      dense_.store(true);
+      ws_bytes_ = std::max(ws_bytes_, dense_bytes);
+    }
 
     const auto dev = torch::Device(torch::kCUDA, static_cast<c10::DeviceIndex>(device_));
     const auto id_opt = torch::TensorOptions().dtype(indptr_->dtype()).device(dev);
@@ -215,7 +222,7 @@ class BlockPipeline : public torch::CustomClassHolder {
       for (int h = 0; h < H_; ++h) s.sizes[2 * h] = s.sizes[2 * h + 1] = kPending;
       Job job;
       job.slot = static_cast<int>(head_ % slots_.size());
-      job.rng = next_rng(static_cast<uint64_t>(H_));
+      job.rng = s.rng = next_rng(static_cast<uint64_t>(H_));
       if (worker_.joinable()) {
         s.state.store(kQueuing, std::memory_order_release);
         {
@@ -262,6 +269,7 @@ class BlockPipeline : public torch::CustomClassHolder {
         --in_flight_;
         TORCH_CHECK(false, msg);
       }
+      if (s.dense) requeue_if_beyond_id_space(s);
       for (int h = 0; h < H_; ++h) {
         const int64_t nnz = wait_size(s.sizes + 2 * h, s.stream, "BlockPipeline.next");
         const int64_t nu = wait_size(s.sizes + 2 * h + 1, s.stream, "BlockPipeline.next");
@@ -338,7 +346,31 @@ class BlockPipeline : public torch::CustomClassHolder {
     std::vector<torch::Tensor> rows, cols, frontier;  // indexed by hop of application
     int64_t edge_bound[DGS_MAX_HOPS] = {0}, frontier_bound[DGS_MAX_HOPS] = {0};
     int64_t n_seeds = 0, batch = -1;
+    std::pair<uint64_t, uint64_t> rng;  // of the batch
+    bool dense = false, recorded_dense = false;  // form the batch / the recording was queued in
   };
+
+  // A batch that met column ids at or beyond the id space (a bipartite CSC without src_nodes) is queued again in the
+  // form that takes any id, with the same random stream; the pipeline stays with that form from there on.
+  void requeue_if_beyond_id_space(Slot& s) {
+    for (int h = 0; h < 2 * H_; ++h) wait_size(s.sizes + h, s.stream, "BlockPipeline.next");
+    if (*static_cast<volatile int32_t*>(s.status) != DGS_ERR_ID_SPACE) return;
+    dense_.store(false);
+    TORCH_CHECK(cudaEventSynchronize(s.done) == cudaSuccess, "BlockPipeline.next: synchronisation failed");
+    *s.status = 0;
+    for (int h = 0; h < H_; ++h) s.sizes[2 * h] = s.sizes[2 * h + 1] = kPending;
+    Job job;
+    job.slot = static_cast<int>(&s - slots_.data());
+    job.rng = s.rng;
+    queue_batch(job);
+    if (!s.error.empty()) {
+      const std::string msg = s.error;
+      s.error.clear();
+      ++tail_;
+      --in_flight_;
+      TORCH_CHECK(false, msg);
+    }
+  }
 
   void worker_loop() {
     cudaSetDevice(device_);
@@ -373,16 +405,27 @@ class BlockPipeline : public torch::CustomClassHolder {
         s.frontier_bound[h] = hops[h].frontier_bound;
       }
       const dgs_chunk_desc* probs = probs_.defined() ? &probs_->desc() : nullptr;
+      s.dense = dense_.load();
+      if (s.recording != nullptr && s.recorded_dense != s.dense) {
+        dgs_sample_blocks_recording_free(s.recording);
+        s.recording = nullptr;
+        s.recorded_seeds = -1;
+      }
       if (record_ && s.recorded_seeds != n && (s.recording == nullptr || s.odd_seeds == n)) {
         // first batch of the slot, or a new batch size seen twice in a row: record the sequence for it
         dgs_sample_blocks_recording_free(s.recording);
         s.recording = nullptr;
         s.recorded_seeds = -1;
-        const int rc = dgs_sample_blocks_record(&indptr_->desc(), &indices_->desc(), probs, s.seeds.data_ptr(), ids64_,
-                                                hops, H_, replace_, s.rng_words, s.ws.data_ptr(), ws_bytes_, s.sizes,
-                                                s.status, s.stream, &s.recording);
+        const int rc =
+            s.dense ? dgs_sample_blocks_dense_record(&indptr_->desc(), &indices_->desc(), probs, s.seeds.data_ptr(), ids64_,
+                                                     hops, H_, replace_, id_space_, s.rng_words, s.ws.data_ptr(), ws_bytes_,
+                                                     s.sizes, s.status, s.stream, &s.recording)
+                    : dgs_sample_blocks_record(&indptr_->desc(), &indices_->desc(), probs, s.seeds.data_ptr(), ids64_, hops,
+                                               H_, replace_, s.rng_words, s.ws.data_ptr(), ws_bytes_, s.sizes, s.status,
+                                               s.stream, &s.recording);
         if (rc == DGS_OK) {
           s.recorded_seeds = n;
+          s.recorded_dense = s.dense;
         } else {
           // recording is an optimisation: say so once and go on with individual launches
           record_ = false;
@@ -395,6 +438,10 @@ class BlockPipeline : public torch::CustomClassHolder {
         s.rng_words[0] = job.rng.first;
         s.rng_words[1] = job.rng.second;
         DGS_CHECK_RC(dgs_sample_blocks_replay(s.recording, s.stream));
+      } else if (s.dense) {
+        DGS_CHECK_RC(dgs_sample_blocks_dense(&indptr_->desc(), &indices_->desc(), probs, s.seeds.data_ptr(), ids64_, hops, H_,
+                                             replace_, id_space_, job.rng.first, job.rng.second, s.ws.data_ptr(), ws_bytes_,
+                                             s.sizes, s.status, s.stream));
       } else {
         DGS_CHECK_RC(dgs_sample_blocks(&indptr_->desc(), &indices_->desc(), probs, s.seeds.data_ptr(), ids64_, hops, H_,
                                        replace_, job.rng.first, job.rng.second, s.ws.data_ptr(), ws_bytes_, s.sizes,
@@ -402,7 +449,8 @@ class BlockPipeline : public torch::CustomClassHolder {
       }
       cudaStream_t last = s.stream;
       if (features_.defined()) {
-        const int64_t* n_dev = dgs_sample_blocks_frontier_count(hops, H_, s.ws.data_ptr());
+        const int64_t* n_dev = s.dense ? dgs_sample_blocks_dense_frontier_count(hops, H_, id_space_, s.ws.data_ptr())
+                                       : dgs_sample_blocks_frontier_count(hops, H_, s.ws.data_ptr());
         TORCH_CHECK(n_dev != nullptr, "BlockPipeline: no frontier count");
         if (s.gather_stream != nullptr) {
           TORCH_CHECK(cudaEventRecord(s.sampled, s.stream) == cudaSuccess &&
@@ -432,10 +480,12 @@ class BlockPipeline : public torch::CustomClassHolder {
 
   c10::intrusive_ptr<ChunkTensor> indptr_, indices_, probs_, features_;
   std::vector<int64_t> applied_;
-  bool replace_ = false, ids64_ = true, record_ = true;
+  bool replace_ = false, ids64_ = true;
+  std::atomic<bool> record_{true};
   int H_ = 0;
   int device_ = 0;
   int64_t max_seeds_ = 0, id_space_ = 0;
+  std::atomic<bool> dense_{false};  // number nodes through one word per id (dgs_sample_blocks_dense)
   size_t ws_bytes_ = 0;
   int64_t edge_cap_[DGS_MAX_HOPS] = {0}, frontier_cap_[DGS_MAX_HOPS] = {0};
   std::vector<Slot> slots_;

@@ -14,6 +14,8 @@
 // than the graph has), and the actual sizes go to a caller-supplied (pinned)
 // array that the host reads once, after everything is queued.
 //
+// Graphs of up to 2^24 ids take the form at dgs_sample_blocks_dense (one word per id); what follows is the form with a hash
+// table per hop, which takes any id.
 // Per hop: sample -> insert -> number.  The number launch of a hop also makes the
 // plan of the next one (its unique list is the next seed list); only the first
 // hop has a plan launch.  The sample launch carries, as extra CTAs, two jobs that
@@ -23,6 +25,7 @@
 // is a relabel's unique list, so a seed's relabelled id is its position and the
 // sampler writes that directly; only the first hop (whose seeds the caller may
 // repeat) looks its rows up.
+#include <algorithm>
 #include <cstdlib>
 #include <new>
 
@@ -109,11 +112,117 @@ extern "C" const int64_t* dgs_sample_blocks_frontier_count(const dgs_hop* hops, 
 namespace dgs {
 namespace {
 
-// Queues the whole sequence on `stream`.  rng_words == nullptr: the keys come from (rng_seed, rng_offset) as
+// ---- the form with one word per id -----------------------------------------------
+// The hash tables cost an insert launch per hop (load, compare-and-swap and probes per key, 21 us for the 876 k keys of a
+// last hop) and a table cleared per hop.  A fire-and-forget atomic in the sampling launch costs nothing that shows there
+// (18.9 us with it, 18.5 without), and what numbers the nodes reads ids and words only.  Batches of 1 024 seeds [15, 10, 5]
+// over 2.4 M nodes with 100 features, one at a time 191 -> 147 us, six in flight 806 -> 674; 64 seeds [10, 5] 77 -> 63.
+// control words | plans | tickets and tile words of all hops | one word per id
+struct DenseSpace {
+  int64_t* n0;
+  uint64_t* keys;
+  int64_t* totals;            // [n_hops] length of each hop's frontier
+  void* plan[DGS_MAX_HOPS];
+  unsigned int* ticket[DGS_MAX_HOPS];
+  unsigned long long* tiles[DGS_MAX_HOPS];
+  uint32_t* first;
+  FillJob fill;               // tickets, tile words and words of the ids
+  size_t bytes;
+};
+static_assert(sizeof(int64_t) * (1 + 2 * DGS_MAX_HOPS) <= WS_ALIGN, "control words: n0, a key and a frontier length per hop");
+
+// The line: clearing a word per id (the first launch does it beside the plan) against the probes it saves.  Recorded
+// sequences, hash tables -> one word per id, us: 16 seeds [10, 5] over 0.5 M ids 39 -> 28, 2.4 M 39 -> 27, 8 M 40 -> 29,
+// 20 M 37 -> 35, 111 M 37 -> 88; 1 024 seeds [15, 10, 5] over 2.4 M ids 141 -> 92, 8 M 141 -> 90, 20 M 131 -> 111, 111 M
+// 134 -> 214.  A table of 2^24 words is 64 MB, half of the L2.
+constexpr int64_t DENSE_MAX_IDS = int64_t(1) << 24;
+constexpr unsigned FILL_CTA_UNITS = 4096;  // 64 KB a CTA of 1 024 threads
+
+DenseSpace dense_space(const dgs_hop* hops, int32_t n_hops, int64_t ids, void* workspace) {
+  DenseSpace d{};
+  char* const base = static_cast<char*>(workspace);
+  size_t at = WS_ALIGN;
+  d.n0 = reinterpret_cast<int64_t*>(base);
+  d.keys = reinterpret_cast<uint64_t*>(d.n0 + 1);
+  d.totals = d.n0 + 1 + DGS_MAX_HOPS;
+  for (int h = 0; h < n_hops; ++h) {
+    d.plan[h] = base + at;
+    at += ws_align(dgs_sample_plan_bytes(hops[h].seed_bound));
+  }
+  const size_t cleared = at;
+  for (int h = 0; h < n_hops; ++h) {
+    d.ticket[h] = reinterpret_cast<unsigned int*>(base + at);
+    d.tiles[h] = reinterpret_cast<unsigned long long*>(base + at + 16);
+    at += 16 + 16 * static_cast<size_t>(dense_tiles(hops[h].seed_bound, hops[h].seed_bound * hops[h].fanout));
+  }
+  d.first = reinterpret_cast<uint32_t*>(base + at);
+  at += (static_cast<size_t>(ids) * sizeof(uint32_t) + 15) / 16 * 16;
+  d.fill.at = reinterpret_cast<ulonglong2*>(base + cleared);
+  d.fill.units = static_cast<int64_t>((at - cleared) / 16);
+  d.fill.ctas = static_cast<unsigned>(std::min<int64_t>((d.fill.units + FILL_CTA_UNITS - 1) / FILL_CTA_UNITS, 1 << 16));
+  d.bytes = ws_align(at);
+  return d;
+}
+
+// Per hop: sample (which marks what it draws) -> number (+ the next hop's plan); one lookup for all hops at the end.  The
+// first launch, which makes the first hop's plan, also clears the words.
+int queue_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, const dgs_chunk_desc* probs, const void* seeds,
+                bool ids64, const dgs_hop* hops, int32_t n_hops, bool replace, int64_t id_space, uint64_t rng_seed,
+                uint64_t rng_offset, const uint64_t* rng_words, void* workspace, int64_t* sizes, int32_t* status,
+                cudaStream_t s) {
+  const DenseSpace d = dense_space(hops, n_hops, id_space, workspace);
+  const InitWords init{d.n0, hops[0].seed_bound, rng_words, d.keys, n_hops};
+  int rc = launch_sample_plan(*indptr, seeds, ids64, hops[0].seed_bound, hops[0].fanout, replace, d.plan[0], nullptr, init,
+                              d.fill, status, s);
+  if (rc != DGS_OK) return rc;
+  DenseLookup lookup{};
+  lookup.first = d.first;
+  lookup.ids = id_space;
+  lookup.n_hops = n_hops;
+  lookup.row0 = hops[0].coo_row;
+  SizesReport report{};
+  report.dst = sizes;
+  const void* hop_seeds = seeds;
+  const int64_t* n_dev = d.n0;
+  for (int h = 0; h < n_hops; ++h) {
+    const dgs_hop& hp = hops[h];
+    const int64_t k = hp.fanout, edge_bound = hp.seed_bound * k;
+    const Count n{hp.seed_bound, n_dev};
+    const bool later = h > 0;  // the plan came with the numbering of these seeds, which are unique and labelled
+    const RngKey key = rng_words != nullptr
+                           ? RngKey{0, d.keys + h}
+                           : host_key(sample_rng_key(rng_seed, rng_offset + static_cast<uint64_t>(h)));
+    const IdMarks marks{d.first, id_space, !later};
+    rc = probs != nullptr
+             ? launch_sample_weighted(*indices, *probs, hop_seeds, ids64, n, k, replace, d.plan[h], later, key, hp.coo_row,
+                                      hp.coo_col, edge_bound, nullptr, later, SideJobs{}, marks, status, s)
+             : launch_sample_uniform(*indices, hop_seeds, ids64, n, k, replace, d.plan[h], later, key, hp.coo_row,
+                                     hp.coo_col, edge_bound, nullptr, later, SideJobs{}, marks, status, s);
+    if (rc != DGS_OK) return rc;
+    const Count nnz{edge_bound, sample_plan_total(d.plan[h], hp.seed_bound)};
+    report.src[2 * h] = nnz.dev;
+    report.src[2 * h + 1] = d.totals + h;
+    NextPlan next{};
+    if (h + 1 < n_hops) next = make_next_plan(*indptr, hops[h + 1].seed_bound, hops[h + 1].fanout, replace, d.plan[h + 1]);
+    else report.n = 2 * n_hops;  // the last hop's numbering sends all sizes to the host at once
+    const DenseNumbering number{d.first, id_space, d.ticket[h], d.tiles[h], d.totals + h, later};
+    rc = launch_dense_number(ids64, number, hop_seeds, n, hp.coo_col, nnz, hp.frontier, hp.frontier_bound, report, next,
+                             status, s);
+    if (rc != DGS_OK) return rc;
+    lookup.col[h] = hp.coo_col;
+    lookup.n[h] = nnz;
+    lookup.end_cta[h] = (h > 0 ? lookup.end_cta[h - 1] : 0u) + static_cast<unsigned>((edge_bound + RL_TILE - 1) / RL_TILE);
+    hop_seeds = hp.frontier;
+    n_dev = d.totals + h;
+  }
+  return launch_dense_lookup(lookup, ids64, s);
+}
+
+// Queues the whole sequence on `stream`.  id_space > 0: with one word per id below it.  rng_words == nullptr: the keys come from (rng_seed, rng_offset) as
 // launch parameters; otherwise the first kernel reads (seed, offset) from rng_words when it RUNS.
 int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, const dgs_chunk_desc* probs,
                  const void* seeds, int32_t ids64, const dgs_hop* hops, int32_t n_hops, int32_t replace,
-                 uint64_t rng_seed, uint64_t rng_offset, const uint64_t* rng_words, void* workspace,
+                 int64_t id_space, uint64_t rng_seed, uint64_t rng_offset, const uint64_t* rng_words, void* workspace,
                  size_t workspace_bytes, int64_t* sizes, int32_t* status, dgs_stream_t stream) {
   int rc = validate_desc(indptr, "dgs_sample_blocks(indptr)");
   if (rc != DGS_OK) return rc;
@@ -138,7 +247,9 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
     return DGS_OK;
   }
   DGS_REQUIRE(seeds != nullptr, DGS_ERR_INVALID, "dgs_sample_blocks: null seeds");
-  DGS_REQUIRE(workspace != nullptr && workspace_bytes >= dgs_sample_blocks_workspace_bytes(hops, n_hops) &&
+  const size_t need = id_space > 0 ? dense_space(hops, n_hops, id_space, nullptr).bytes
+                                   : dgs_sample_blocks_workspace_bytes(hops, n_hops);
+  DGS_REQUIRE(workspace != nullptr && workspace_bytes >= need &&
                   (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
               DGS_ERR_INVALID, "dgs_sample_blocks: workspace too small or not 16-byte aligned");
   for (int h = 0; h < n_hops; ++h) {
@@ -148,6 +259,9 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
                 "dgs_sample_blocks: weighted fan-out %lld > 32 without replacement is not supported",
                 (long long)hops[h].fanout);
   }
+
+  if (id_space > 0) return queue_dense(indptr, indices, probs, seeds, ids64 != 0, hops, n_hops, replace != 0, id_space, rng_seed,
+                                       rng_offset, rng_words, workspace, sizes, status, s);
 
   // ---- carve the workspace ----
   char* p = static_cast<char*>(workspace);
@@ -175,7 +289,7 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
   SizesReport report{};
   report.dst = sizes;
   const InitWords init{n0_dev, n0, rng_words, keys_dev, n_hops};
-  rc = launch_sample_plan(*indptr, seeds, ids64 != 0, n0, hops[0].fanout, replace != 0, plan[0], nullptr, init, status, s);
+  rc = launch_sample_plan(*indptr, seeds, ids64 != 0, n0, hops[0].fanout, replace != 0, plan[0], nullptr, init, FillJob{}, status, s);
   if (rc != DGS_OK) return rc;
   for (int h = 0; h < n_hops; ++h) {
     const dgs_hop& hp = hops[h];
@@ -193,9 +307,9 @@ int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, co
     const bool later = h > 0;  // the plan came with the numbering of these seeds, which are unique
     rc = probs != nullptr
              ? launch_sample_weighted(*indices, *probs, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], later,
-                                      key, hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, status, s)
+                                      key, hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, IdMarks{}, status, s)
              : launch_sample_uniform(*indices, hop_seeds, ids64 != 0, n, k, replace != 0, plan[h], later, key,
-                                     hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, status, s);
+                                     hp.coo_row, hp.coo_col, edge_bound, nullptr, later, jobs, IdMarks{}, status, s);
     if (rc != DGS_OK) return rc;
     const Count nnz{edge_bound, nnz_dev};
     report.src[2 * h] = nnz_dev;
@@ -221,8 +335,39 @@ extern "C" int dgs_sample_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_d
                                  const dgs_hop* hops, int32_t n_hops, int32_t replace, uint64_t rng_seed,
                                  uint64_t rng_offset, void* workspace, size_t workspace_bytes,
                                  int64_t* sizes, int32_t* status, dgs_stream_t stream) {
-  return dgs::queue_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, rng_seed, rng_offset, nullptr,
+  return dgs::queue_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, 0, rng_seed, rng_offset, nullptr,
                            workspace, workspace_bytes, sizes, status, stream);
+}
+
+extern "C" size_t dgs_sample_blocks_dense_workspace_bytes(const dgs_hop* hops, int32_t n_hops, int64_t id_space) {
+  using namespace dgs;
+  if (hops == nullptr || n_hops < 1 || n_hops > DGS_MAX_HOPS || id_space < 1 || id_space > COMPACT_KEY_LIMIT) return 0;
+  return dense_space(hops, n_hops, id_space, nullptr).bytes;
+}
+
+extern "C" int32_t dgs_sample_blocks_dense_wins(const dgs_hop* hops, int32_t n_hops, int64_t id_space) {
+  using namespace dgs;
+  if (hops == nullptr || n_hops < 1 || n_hops > DGS_MAX_HOPS || id_space < 1 || id_space > COMPACT_KEY_LIMIT) return 0;
+  return id_space <= DENSE_MAX_IDS;
+}
+
+extern "C" const int64_t* dgs_sample_blocks_dense_frontier_count(const dgs_hop* hops, int32_t n_hops, int64_t id_space,
+                                                                 void* workspace) {
+  using namespace dgs;
+  if (hops == nullptr || workspace == nullptr || n_hops < 1 || n_hops > DGS_MAX_HOPS || id_space < 1) return nullptr;
+  return dense_space(hops, n_hops, id_space, workspace).totals + n_hops - 1;
+}
+
+extern "C" int dgs_sample_blocks_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
+                                       const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
+                                       const dgs_hop* hops, int32_t n_hops, int32_t replace, int64_t id_space,
+                                       uint64_t rng_seed, uint64_t rng_offset, void* workspace, size_t workspace_bytes,
+                                       int64_t* sizes, int32_t* status, dgs_stream_t stream) {
+  using namespace dgs;
+  DGS_REQUIRE(id_space >= 1 && id_space <= COMPACT_KEY_LIMIT && status != nullptr, DGS_ERR_INVALID,
+              "dgs_sample_blocks_dense: an id space of 1 to 2^32 - 1 ids and a status word, please (%lld)", (long long)id_space);
+  return queue_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, id_space, rng_seed, rng_offset, nullptr,
+                      workspace, workspace_bytes, sizes, status, stream);
 }
 
 // ---- the sequence recorded once and replayed ------------------------------------
@@ -234,13 +379,12 @@ struct dgs_blocks_recording {
   cudaGraphExec_t exec = nullptr;
 };
 
-extern "C" int dgs_sample_blocks_record(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
-                                        const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
-                                        const dgs_hop* hops, int32_t n_hops, int32_t replace,
-                                        const uint64_t* rng_words, void* workspace, size_t workspace_bytes,
-                                        int64_t* sizes, int32_t* status, dgs_stream_t capture_stream,
-                                        dgs_blocks_recording** out) {
-  using namespace dgs;
+namespace dgs {
+namespace {
+int record_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, const dgs_chunk_desc* probs,
+                  const void* seeds, int32_t ids64, const dgs_hop* hops, int32_t n_hops, int32_t replace, int64_t id_space,
+                  const uint64_t* rng_words, void* workspace, size_t workspace_bytes, int64_t* sizes, int32_t* status,
+                  dgs_stream_t capture_stream, dgs_blocks_recording** out) {
   DGS_REQUIRE(out != nullptr && rng_words != nullptr, DGS_ERR_INVALID, "dgs_sample_blocks_record: null argument");
   DGS_REQUIRE(capture_stream != nullptr, DGS_ERR_INVALID,
               "dgs_sample_blocks_record: the default stream cannot record; pass a stream of your own");
@@ -248,8 +392,8 @@ extern "C" int dgs_sample_blocks_record(const dgs_chunk_desc* indptr, const dgs_
   cudaStream_t s = static_cast<cudaStream_t>(capture_stream);
   // thread-local mode: other host threads keep allocating and copying while this one records
   DGS_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-  const int rc = queue_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, 0, 0, rng_words, workspace,
-                              workspace_bytes, sizes, status, capture_stream);
+  const int rc = queue_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, id_space, 0, 0, rng_words,
+                              workspace, workspace_bytes, sizes, status, capture_stream);
   cudaGraph_t graph = nullptr;
   const cudaError_t end = cudaStreamEndCapture(s, &graph);  // always closed, also after a refused argument
   if (rc != DGS_OK) {
@@ -270,6 +414,32 @@ extern "C" int dgs_sample_blocks_record(const dgs_chunk_desc* indptr, const dgs_
   rec->exec = exec;
   *out = rec;
   return DGS_OK;
+}
+}  // namespace
+}  // namespace dgs
+
+extern "C" int dgs_sample_blocks_record(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
+                                        const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
+                                        const dgs_hop* hops, int32_t n_hops, int32_t replace,
+                                        const uint64_t* rng_words, void* workspace, size_t workspace_bytes,
+                                        int64_t* sizes, int32_t* status, dgs_stream_t capture_stream,
+                                        dgs_blocks_recording** out) {
+  return dgs::record_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, 0, rng_words, workspace,
+                            workspace_bytes, sizes, status, capture_stream, out);
+}
+
+extern "C" int dgs_sample_blocks_dense_record(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
+                                              const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
+                                              const dgs_hop* hops, int32_t n_hops, int32_t replace, int64_t id_space,
+                                              const uint64_t* rng_words, void* workspace, size_t workspace_bytes,
+                                              int64_t* sizes, int32_t* status, dgs_stream_t capture_stream,
+                                              dgs_blocks_recording** out) {
+  using namespace dgs;
+  DGS_REQUIRE(id_space >= 1 && id_space <= COMPACT_KEY_LIMIT && status != nullptr, DGS_ERR_INVALID,
+              "dgs_sample_blocks_dense_record: an id space of 1 to 2^32 - 1 ids and a status word, please (%lld)",
+              (long long)id_space);
+  return record_blocks(indptr, indices, probs, seeds, ids64, hops, n_hops, replace, id_space, rng_words, workspace,
+                       workspace_bytes, sizes, status, capture_stream, out);
 }
 
 extern "C" int dgs_sample_blocks_replay(dgs_blocks_recording* rec, dgs_stream_t stream) {

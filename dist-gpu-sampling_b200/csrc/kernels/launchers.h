@@ -21,7 +21,8 @@ struct InitWords {
   int n_keys;
 };
 int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, int64_t n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, int32_t* status, cudaStream_t s);
+                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, const FillJob& fill, int32_t* status,
+                       cudaStream_t s);
 // The plan of a hop whose seeds are being numbered (launch_unique_pair writes it): offsets are those in the whole
 // output, so sampling takes whole_offsets = true.  n_edges == nullptr: no plan wanted.
 struct NextPlan {
@@ -41,17 +42,18 @@ struct SideJobs {
   unsigned main_ctas;  // set by the launcher
 };
 
+// marks: record what is emitted in the table of a sequence that numbers its nodes through one word per id.
 // row_is_position: write the seed's position in the seed list to coo_row instead
 // of the seed id (valid as a relabelled id when the seed list has no duplicates).
 int launch_sample_uniform(const dgs_chunk_desc& indices, const void* seeds, bool ids64, Count n, int64_t k,
                           bool replace, void* plan, bool whole_offsets, RngKey key, void* coo_row,
                           void* coo_col, int64_t out_capacity, int64_t* picked_pos, bool row_is_position,
-                          const SideJobs& jobs, int32_t* status, cudaStream_t s);
+                          const SideJobs& jobs, const IdMarks& marks, int32_t* status, cudaStream_t s);
 int launch_sample_weighted(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds,
                            bool ids64, Count n, int64_t k, bool replace, void* plan, bool whole_offsets,
                            RngKey key, void* coo_row, void* coo_col, int64_t out_capacity,
-                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, int32_t* status,
-                           cudaStream_t s);
+                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, const IdMarks& marks,
+                           int32_t* status, cudaStream_t s);
 uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset);
 
 // ---- relabel.cu ----------------------------------------------------------------
@@ -73,5 +75,23 @@ int launch_unique_pair(bool ids64, const void* a, Count na, const void* b, Count
                        int64_t* n_unique_out, const SizesReport& report, const NextPlan& plan, int32_t* status,
                        cudaStream_t s);
 int64_t* unique_total(void* table, int64_t key_bound);
+
+// The same numbering through a table of one word per id (IdMarks), which the sampling launch before it has marked.
+// seeds_known: the seeds carry their labels already (they are the unique list of the hop before).
+struct DenseNumbering {
+  uint32_t* first;
+  int64_t ids;
+  unsigned int* ticket;       // [4]  cleared with the table
+  unsigned long long* tiles;  // [2 * dense_tiles(bounds)], cleared with the table
+  int64_t* total;
+  bool seeds_known;
+};
+inline int64_t dense_tiles(int64_t seed_bound, int64_t edge_bound) {
+  return (seed_bound + RL_TILE - 1) / RL_TILE + (edge_bound + RL_TILE - 1) / RL_TILE;
+}
+int launch_dense_number(bool ids64, const DenseNumbering& d, const void* seeds, Count n_seeds, const void* cols, Count n_cols,
+                        void* unique_out, int64_t unique_capacity, const SizesReport& report, const NextPlan& plan,
+                        int32_t* status, cudaStream_t s);
+int launch_dense_lookup(const DenseLookup& job, bool ids64, cudaStream_t s);
 
 }  // namespace dgs

@@ -239,6 +239,157 @@ relabel_number_kernel(const __grid_constant__ Keys keys, const TableParts t, IdT
   }
 }
 
+// The numbering of a sequence that keeps one word per id (see IdMarks): input i -- the seeds, then the neighbours in the
+// order they were drawn -- is a first occurrence iff the word of its id holds i.  The sampling launch has put the smallest
+// index there, so nothing was probed, and a tile reads its ids, their words, and is where relabel_number_kernel is.
+// Seeds and neighbours have tiles of their own; seeds that are labelled already (their label is their position) need
+// no word and no look-back.  A warp owns 128 consecutive inputs, 32 at a time, so that ids are read in whole lines and ranks
+// come out of votes.
+template <typename IdT, bool PLAN>
+__global__ void __launch_bounds__(RL_BLOCK)
+dense_number_kernel(const DenseNumbering d, const IdT* __restrict__ seeds, const Count na, const IdT* __restrict__ cols,
+                    const Count nb, IdT* __restrict__ unique_out, const int64_t unique_capacity, const SizesReport report,
+                    const __grid_constant__ NextPlan plan, int32_t* __restrict__ status) {
+  __shared__ int64_t smem[RL_BLOCK / 32 + 1];
+  __shared__ TileScanShared<RL_BLOCK> s_tiles;
+  __shared__ unsigned int s_tile;
+  __shared__ int s_count[RL_BLOCK / 32];
+  pdl_enter();
+  if (threadIdx.x == 0) s_tile = atomicAdd(d.ticket, 1u) + 1u;
+  const int64_t n_seeds = count_of(na), n_cols = count_of(nb);
+  __syncthreads();
+  const int64_t tile = s_tile;
+  const int64_t seed_tiles = (n_seeds + RL_TILE - 1) / RL_TILE, tiles = seed_tiles + (n_cols + RL_TILE - 1) / RL_TILE;
+  const bool last_tile = tile == tiles - 1 || (tile == 0 && tiles == 0);
+  if (tile >= tiles && !last_tile) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool of_seeds = tile < seed_tiles;
+  const bool known = of_seeds && d.seeds_known;
+  const IdT* list = of_seeds ? seeds : cols;
+  const int64_t list_len = of_seeds ? n_seeds : n_cols, list_at = of_seeds ? 0 : n_seeds;
+  const int64_t base = (of_seeds ? tile : tile - seed_tiles) * RL_TILE + warp * 32 * RL_ITEMS + lane;  // in the list
+  int64_t id[RL_ITEMS];
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) id[u] = base + 32 * u < list_len ? static_cast<int64_t>(list[base + 32 * u]) : -1;
+  uint32_t word[RL_ITEMS];
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    const bool in = static_cast<uint64_t>(id[u]) < static_cast<uint64_t>(d.ids);
+    word[u] = !in ? NOT_MET : known ? static_cast<uint32_t>(base + 32 * u) : *reinterpret_cast<const volatile uint32_t*>(d.first + id[u]);
+  }
+  unsigned votes[RL_ITEMS];
+  int c = 0;
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    votes[u] = __ballot_sync(FULL_MASK, word[u] == static_cast<uint32_t>(list_at + base + 32 * u) && word[u] != NOT_MET);
+    c += __popc(votes[u]);
+  }
+  if (lane == 0) s_count[warp] = c;
+  __syncthreads();
+  int ex = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < RL_BLOCK / 32; ++w) {
+    if (w < warp) ex += s_count[w];
+    total += s_count[w];
+  }
+  int64_t before;
+  if (known) {
+    before = tile * RL_TILE;
+    if (threadIdx.x == 0) store_tile_word(d.tiles + tile, TILE_RUNNING | static_cast<unsigned long long>(before + total));
+  } else {
+    before = sum_of_tiles_before<RL_BLOCK>(tile, total, d.tiles, s_tiles, status);
+  }
+  if (last_tile && threadIdx.x == 0) {
+    *d.total = before + total;
+    if (report.n > 0) {  // the same thread that wrote *d.total just above
+      for (int k = 0; k < report.n; ++k) report.dst[k] = *report.src[k];
+      __threadfence_system();
+    }
+  }
+  int64_t label[RL_ITEMS];
+  int64_t next = before + ex;
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    const bool first = (votes[u] >> lane) & 1u;
+    label[u] = next + __popc(votes[u] & ((1u << lane) - 1u));
+    next += __popc(votes[u]);
+    if (first) {
+      if (!known) d.first[id[u]] = static_cast<uint32_t>(label[u]);
+      if (label[u] < unique_capacity) {
+        unique_out[label[u]] = static_cast<IdT>(id[u]);
+      } else {
+        raise_status(status, DGS_ERR_RANGE);
+        id[u] = -1;
+      }
+    } else {
+      id[u] = -1;
+    }
+  }
+  if (!PLAN) return;
+  int64_t rb[RL_ITEMS], deg[RL_ITEMS], off[RL_ITEMS], warp_edges = 0;
+  bool good[RL_ITEMS];
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    good[u] = id[u] >= 0 && id[u] + 1 < plan.indptr.total;
+    if (id[u] >= 0 && !good[u]) raise_status(status, DGS_ERR_RANGE);
+  }
+  row_bounds<IdT, RL_ITEMS>(plan.indptr, id, good, rb, deg, status);
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    const int64_t n = pick_count(deg[u], plan.k, plan.replace);
+    int64_t inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(FULL_MASK, inc, o);
+      if (lane >= o) inc += t;
+    }
+    off[u] = warp_edges + inc - n;
+    warp_edges += __shfl_sync(FULL_MASK, inc, 31);
+  }
+  if (lane == 0) smem[warp] = warp_edges;
+  __syncthreads();
+  int64_t at = 0, tile_edges = 0;
+#pragma unroll
+  for (int w = 0; w < RL_BLOCK / 32; ++w) {
+    if (w < warp) at += smem[w];
+    tile_edges += smem[w];
+  }
+  const int64_t edges_before = sum_of_tiles_before<RL_BLOCK>(tile, tile_edges, d.tiles + gridDim.x, s_tiles, status);
+  if (last_tile && threadIdx.x == 0) *plan.n_edges = edges_before + tile_edges;
+#pragma unroll
+  for (int u = 0; u < RL_ITEMS; ++u) {
+    if (id[u] < 0) continue;
+    plan.row_begin[label[u]] = rb[u];
+    plan.deg[label[u]] = deg[u];
+    plan.off[label[u]] = edges_before + at + off[u];
+  }
+}
+
+// The COO of all hops through that table, in place: an id that is not in it becomes -1.  Bound by the random reads of
+// the words; four ids per thread in flight.
+template <typename IdT>
+__global__ void __launch_bounds__(RL_BLOCK) dense_lookup_kernel(const __grid_constant__ DenseLookup job) {
+  pdl_enter();
+  int h = 0;
+  while (h + 1 < job.n_hops && blockIdx.x >= job.end_cta[h]) ++h;
+  const int64_t base = static_cast<int64_t>(blockIdx.x - (h > 0 ? job.end_cta[h - 1] : 0u)) * RL_TILE + threadIdx.x;
+  const int64_t n = count_of(job.n[h]);
+  auto relabel = [&](IdT* ids) {
+    int64_t id[RL_ITEMS];
+    uint32_t word[RL_ITEMS];
+#pragma unroll
+    for (int u = 0; u < RL_ITEMS; ++u) id[u] = base + u * RL_BLOCK < n ? static_cast<int64_t>(ids[base + u * RL_BLOCK]) : -1;
+#pragma unroll
+    for (int u = 0; u < RL_ITEMS; ++u)
+      word[u] = static_cast<uint64_t>(id[u]) < static_cast<uint64_t>(job.ids) ? job.first[id[u]] : NOT_MET;
+#pragma unroll
+    for (int u = 0; u < RL_ITEMS; ++u)
+      if (base + u * RL_BLOCK < n) ids[base + u * RL_BLOCK] = word[u] == NOT_MET ? static_cast<IdT>(-1) : static_cast<IdT>(word[u]);
+  };
+  relabel(static_cast<IdT*>(job.col[h]));
+  if (h == 0) relabel(static_cast<IdT*>(job.row0));
+}
+
 // lookup: label of each id, -1 when absent
 template <typename IdT>
 __global__ void __launch_bounds__(RL_BLOCK)
@@ -327,6 +478,36 @@ int launch_unique_pair(bool ids64, const void* a, Count na, const void* b, Count
                                                report, plan, status, s)
                : run_unique<int32_t, PairKeys>(keys, key_bound, size, t, unique_out, unique_capacity, n_unique_out,
                                                report, plan, status, s);
+}
+
+int launch_dense_number(bool ids64, const DenseNumbering& d, const void* seeds, Count n_seeds, const void* cols, Count n_cols,
+                        void* unique_out, int64_t unique_capacity, const SizesReport& report, const NextPlan& plan,
+                        int32_t* status, cudaStream_t s) {
+  const int64_t tiles = dense_tiles(n_seeds.bound, n_cols.bound);
+  DGS_REQUIRE(tiles > 0 && n_seeds.bound + n_cols.bound < (1ll << 30), DGS_ERR_UNSUPPORTED, "relabel: %lld keys",
+              (long long)(n_seeds.bound + n_cols.bound));
+  const unsigned grid = static_cast<unsigned>(tiles);
+#define DGS_LAUNCH_DENSE(IdT, PLAN)                                                                                     \
+  DGS_CUDA_TRY(launch_chained(SITE_NUMBER, (dense_number_kernel<IdT, PLAN>), grid, RL_BLOCK, s, d,                      \
+                              static_cast<const IdT*>(seeds), n_seeds, static_cast<const IdT*>(cols), n_cols,           \
+                              static_cast<IdT*>(unique_out), unique_capacity, report, plan, status))
+  if (plan.n_edges != nullptr) {
+    if (ids64) DGS_LAUNCH_DENSE(int64_t, true);
+    else DGS_LAUNCH_DENSE(int32_t, true);
+  } else {
+    if (ids64) DGS_LAUNCH_DENSE(int64_t, false);
+    else DGS_LAUNCH_DENSE(int32_t, false);
+  }
+#undef DGS_LAUNCH_DENSE
+  return DGS_OK;
+}
+
+int launch_dense_lookup(const DenseLookup& job, bool ids64, cudaStream_t s) {
+  const unsigned grid = job.end_cta[job.n_hops - 1];
+  if (grid == 0) return DGS_OK;
+  if (ids64) DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, dense_lookup_kernel<int64_t>, grid, RL_BLOCK, s, job));
+  else DGS_CUDA_TRY(launch_chained(SITE_LOOKUP, dense_lookup_kernel<int32_t>, grid, RL_BLOCK, s, job));
+  return DGS_OK;
 }
 
 int launch_lookup(const LookupJob& job, bool ids64, cudaStream_t s) {

@@ -70,7 +70,52 @@ struct SizesReport {
   const int64_t* src[2 * DGS_MAX_HOPS];
 };
 
+// The other form of the table, for a sequence whose ids lie below a known bound: one 32-bit word per id of the id space,
+// addressed by the id itself.  The word holds the smallest input index that an id was met at and, once numbered, its
+// label; all ones is "not met".  ONE table serves all hops of a batch: a hop's frontier begins with its seeds, so a label
+// given by one hop is the node's position among the next hop's inputs and stays the smallest there.
+// A label never reads as another input's index: the label of the id first met at input e is at most e, and whoever
+// meets that id again does so at an input behind e.
+constexpr uint32_t NOT_MET = 0xFFFFFFFFu;
+
+// Inputs that a sampling launch records in that table as it emits them (first == nullptr: none).
+struct IdMarks {
+  uint32_t* first;
+  int64_t ids;  // words of the table
+  bool seeds;   // the seeds are inputs too (first hop; from the second on they are labelled already)
+};
+
+// What relabels the COO of all hops of a sequence through that table, in one launch.
+struct DenseLookup {
+  const uint32_t* first;
+  int64_t ids;
+  int n_hops;
+  void* row0;  // rows of the first hop (those of the others are positions already)
+  void* col[DGS_MAX_HOPS];
+  Count n[DGS_MAX_HOPS];
+  unsigned end_cta[DGS_MAX_HOPS];  // RL_TILE ids a CTA; running
+};
+
+// Words to set to all ones, as extra CTAs of the first launch of a sequence (16-byte units; ctas == 0: none).
+struct FillJob {
+  ulonglong2* at;
+  int64_t units;
+  unsigned ctas;
+};
+
 #ifdef __CUDACC__
+
+__device__ __forceinline__ void mark_id(const IdMarks& m, int64_t id, uint32_t input, int32_t* status) {
+  if (static_cast<uint64_t>(id) < static_cast<uint64_t>(m.ids)) atomicMin(m.first + id, input);
+  else raise_status(status, id < 0 ? DGS_ERR_RANGE : DGS_ERR_ID_SPACE);
+}
+
+__device__ __forceinline__ void run_fill_cta(const FillJob& j, unsigned cta) {
+  const int64_t stride = static_cast<int64_t>(j.ctas) * blockDim.x;
+  const ulonglong2 ones = make_ulonglong2(~0ull, ~0ull);
+#pragma unroll 4
+  for (int64_t i = static_cast<int64_t>(cta) * blockDim.x + threadIdx.x; i < j.units; i += stride) j.at[i] = ones;
+}
 
 __device__ __forceinline__ uint64_t table_slots(const TableSize& t) { return slots_for(count_of(t.n) * t.mult); }
 

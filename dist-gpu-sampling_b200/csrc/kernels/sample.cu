@@ -90,8 +90,12 @@ __device__ __forceinline__ void run_init(const InitWords& w) {
     w.keys[threadIdx.x] = fold_rng_key(src[0], src[1] + static_cast<uint64_t>(threadIdx.x));
   }
 }
-__global__ void init_kernel(const InitWords w, unsigned int* ticket) {
+__global__ void init_kernel(const InitWords w, unsigned int* ticket, const FillJob fill) {
   pdl_enter();
+  if (blockIdx.x > 0) {
+    run_fill_cta(fill, blockIdx.x - 1);
+    return;
+  }
   if (threadIdx.x == 0) *ticket = 0u;
   run_init(w);
 }
@@ -149,9 +153,13 @@ template <typename IdT>
 __global__ void __launch_bounds__(SMALL_PLAN_BLOCK)
 sample_small_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __restrict__ seeds, const int n,
                          const int64_t k, const bool replace, const PlanView plan, int64_t* nnz_out,
-                         const __grid_constant__ InitWords init, int32_t* __restrict__ status) {
+                         const __grid_constant__ InitWords init, const FillJob fill, int32_t* __restrict__ status) {
   __shared__ int64_t smem[SMALL_PLAN_BLOCK / 32 + 1];
   pdl_enter();
+  if (blockIdx.x > 0) {
+    run_fill_cta(fill, blockIdx.x - 1);
+    return;
+  }
   run_init(init);
   int64_t s[SMALL_PLAN_ITEMS], rb[SMALL_PLAN_ITEMS], deg[SMALL_PLAN_ITEMS];
   bool good[SMALL_PLAN_ITEMS];
@@ -230,9 +238,9 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
                       const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                       const RngKey rng, IdT* coo_row, IdT* coo_col,
                       const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                      const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                      const bool row_is_position, const __grid_constant__ SideJobs jobs, const IdMarks marks,
                       int32_t* __restrict__ status) {
-  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
+  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status, marks, nc};
   pdl_enter();
   if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng);
@@ -247,6 +255,7 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
   const int64_t seed_raw = !in_bound ? 0 : (row_is_position ? i : static_cast<int64_t>(seeds[i]));
   const bool valid = i < count_of(nc);
   const int64_t o = valid ? sp.o : 0;
+  if (valid && marks.seeds && (threadIdx.x & (G - 1)) == 0) mark_id(marks, seed_raw, static_cast<uint32_t>(i), status);
   if (!sample_uniform_row(key, i, valid ? sp.deg : 0, k, replace, G, s_taken + group * (G * TAKEN_WORDS_PER_LANE),
                           coo_col + o, o + k <= out_capacity, status,
                           [&](int64_t t, int64_t pos) { emit(o, t, seed_raw, sp.rb, pos); }))
@@ -258,16 +267,16 @@ sample_uniform_kernel(const __grid_constant__ dgs_chunk_desc indices, const IdT*
 // Bound by issue slots: 449 warp instructions per two seeds at 32 registers (76 % of the warps), where the general kernel
 // has 544 at 40 (57 %): the address arithmetic of chunked tensors, 64-bit positions and the branches around both.
 // 60 000 seeds, fan-out 15: 26 -> 17.7 us.
-template <typename IdT, int G>
+template <typename IdT, int G, bool MARK>
 __global__ void __launch_bounds__(SAMPLE_BLOCK)
 sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edges, const IdT* __restrict__ seeds,
                            const Count nc, const uint32_t k, const int64_t* __restrict__ plan_rb,
                            const int64_t* __restrict__ plan_deg, const int64_t* __restrict__ local_off,
                            const int64_t* __restrict__ tile_off, const RngKey rng, IdT* coo_row, IdT* coo_col,
                            const uint32_t out_capacity, const bool row_is_position, const __grid_constant__ SideJobs jobs,
-                           int32_t* __restrict__ status) {
+                           const IdMarks marks, int32_t* __restrict__ status) {
   pdl_enter();
-  if (run_side_job<IdT>(jobs)) return;
+  if (!MARK && run_side_job<IdT>(jobs)) return;  // the sequence with marks has no side jobs
   const uint64_t key = key_of(rng);
   constexpr uint32_t GROUPS = SAMPLE_BLOCK / G;  // seeds per CTA
   constexpr uint32_t WORDS = G * TAKEN_WORDS_PER_LANE;
@@ -281,8 +290,10 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
   const uint32_t o = in_bound ? static_cast<uint32_t>(local_off[i] + (tile_off != nullptr ? tile_off[i / SAMPLE_TILE] : 0)) : 0u;
   const IdT seed = row_is_position ? static_cast<IdT>(i) : in_bound ? seeds[i] : IdT(0);
   const bool live = in_bound && (nc.dev == nullptr || i < *nc.dev);
+  const uint32_t n_seeds = MARK ? static_cast<uint32_t>(count_of(nc)) : 0u;
   const uint32_t deg = !live ? 0u : deg_plan > 0xFFFFFFFFll ? 0xFFFFFFFFu : static_cast<uint32_t>(deg_plan);
   if (live && deg_plan > 0xFFFFFFFFll) raise_status(status, DGS_ERR_RANGE);  // longer than `indices`: broken row bounds
+  if (MARK && marks.seeds && live && l == 0) mark_id(marks, static_cast<int64_t>(seed), i, status);
 
   const bool sampled = deg > k;
   const bool complement = sampled && deg < 2 * k;  // draw the deg - k positions to leave out
@@ -365,6 +376,7 @@ sample_uniform_lean_kernel(const IdT* __restrict__ indices, const int64_t n_edge
     else raise_status(status, DGS_ERR_RANGE);
     coo_row[at] = seed;
     coo_col[at] = col;
+    if (MARK) mark_id(marks, static_cast<int64_t>(col), n_seeds + at, status);
   };
   if (emits) emit(o + t, c);
   if (second) emit(o + t2, c2);
@@ -675,9 +687,9 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
                        const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                        const RngKey rng, IdT* coo_row, IdT* coo_col,
                        const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                       const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                       const bool row_is_position, const __grid_constant__ SideJobs jobs, const IdMarks marks,
                        int32_t* __restrict__ status) {
-  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
+  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status, marks, nc};
   pdl_enter();
   if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng) ^ (static_cast<uint64_t>(TAG_ARES) << 32);
@@ -701,6 +713,7 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
   if (i0 + warp < n) {
     sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
     seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
+    if (marks.seeds && l == 0) mark_id(marks, seed, static_cast<uint32_t>(i0 + warp), status);
     if (sp.deg <= k) {
       if (l < sp.deg) pick = l;
     } else if (sp.rb + sp.deg > probs.total || sp.deg >> 35 != 0) {  // places within a share fit 32 bits below 2^35
@@ -886,9 +899,9 @@ sample_weighted_replace_kernel(const __grid_constant__ dgs_chunk_desc indices,
                                const int64_t* __restrict__ local_off, const int64_t* __restrict__ tile_off,
                                const RngKey rng, IdT* coo_row, IdT* coo_col,
                                const int64_t out_capacity, int64_t* __restrict__ picked_pos,
-                               const bool row_is_position, const __grid_constant__ SideJobs jobs,
+                               const bool row_is_position, const __grid_constant__ SideJobs jobs, const IdMarks marks,
                                int32_t* __restrict__ status) {
-  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status};
+  const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status, marks, nc};
   pdl_enter();
   if (run_side_job<IdT>(jobs)) return;
   const uint64_t key = key_of(rng);
@@ -955,6 +968,7 @@ sample_weighted_replace_kernel(const __grid_constant__ dgs_chunk_desc indices,
   if (i0 + warp < n) {
     const SeedPlan sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
     const int64_t seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
+    if (marks.seeds && l == 0) mark_id(marks, seed, static_cast<uint32_t>(i0 + warp), status);
     if (sp.deg > 0 && sp.rb + sp.deg > probs.total) {
       if (l == 0) raise_status(status, DGS_ERR_RANGE);
     } else if (sp.deg > HUB_DEG) {
@@ -1006,13 +1020,14 @@ int check_sample_args(const char* who, const void* seeds, int64_t n, int64_t k, 
 
 template <typename IdT>
 int plan_typed(const dgs_chunk_desc& indptr, const void* seeds, Count n, int64_t k, bool replace,
-               const PlanView& pv, int64_t* nnz, const InitWords& init, int32_t* status, cudaStream_t s) {
+               const PlanView& pv, int64_t* nnz, const InitWords& init, const FillJob& fill, int32_t* status, cudaStream_t s) {
   if (n.bound <= SMALL_PLAN) {
-    DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_small_plan_kernel<IdT>, 1u, SMALL_PLAN_BLOCK, s, indptr,
-                                static_cast<const IdT*>(seeds), static_cast<int>(n.bound), k, replace, pv, nnz, init, status));
+    DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_small_plan_kernel<IdT>, 1u + fill.ctas, SMALL_PLAN_BLOCK, s, indptr,
+                                static_cast<const IdT*>(seeds), static_cast<int>(n.bound), k, replace, pv, nnz, init, fill,
+                                status));
     return DGS_OK;
   }
-  DGS_CUDA_TRY(launch_chained(SITE_INIT, init_kernel, 1u, 32u, s, init, pv.ticket));
+  DGS_CUDA_TRY(launch_chained(SITE_INIT, init_kernel, 1u + fill.ctas, fill.ctas > 0 ? 1024u : 32u, s, init, pv.ticket, fill));
   DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_plan_kernel<IdT>, static_cast<unsigned>(pv.ntiles), SAMPLE_BLOCK, s, indptr,
                               static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, pv.local_off,
                               pv.tile_off, pv.total, pv.ticket, nnz, status));
@@ -1022,7 +1037,7 @@ int plan_typed(const dgs_chunk_desc& indptr, const void* seeds, Count n, int64_t
 template <typename IdT>
 int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int64_t k, bool replace,
                   const PlanView& pv, RngKey key, void* coo_row, void* coo_col,
-                  int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, int32_t* status, cudaStream_t s) {
+                  int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, const IdMarks& marks, int32_t* status, cudaStream_t s) {
 #define DGS_LAUNCH_U(G)                                                                                       \
   do {                                                                                                        \
     jobs.main_ctas = static_cast<unsigned>((n.bound + SAMPLE_BLOCK / G - 1) / (SAMPLE_BLOCK / G));            \
@@ -1030,28 +1045,35 @@ int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int
                                 jobs.main_ctas + jobs.clear.ctas + jobs.lookup.ctas, SAMPLE_BLOCK, s,         \
                                 indices, static_cast<const IdT*>(seeds), n, k, replace, pv.row_begin, pv.deg, \
                                 pv.local_off, pv.tile_off, key, static_cast<IdT*>(coo_row),                   \
-                                static_cast<IdT*>(coo_col), cap, pos, rowpos, jobs, status));                 \
+                                static_cast<IdT*>(coo_col), cap, pos, rowpos, jobs, marks, status));          \
   } while (0)
-#define DGS_LAUNCH_LEAN(G)                                                                                    \
+#define DGS_LAUNCH_LEAN(G, MARK)                                                                              \
   do {                                                                                                        \
     jobs.main_ctas = static_cast<unsigned>((n.bound + SAMPLE_BLOCK / G - 1) / (SAMPLE_BLOCK / G));            \
-    DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, sample_uniform_lean_kernel<IdT, G>,                              \
+    DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, (sample_uniform_lean_kernel<IdT, G, MARK>),                       \
                                 jobs.main_ctas + jobs.clear.ctas + jobs.lookup.ctas, SAMPLE_BLOCK, s,         \
                                 static_cast<const IdT*>(indices.dev[0]), indices.total,                       \
                                 static_cast<const IdT*>(seeds), n, static_cast<uint32_t>(k), pv.row_begin,    \
                                 pv.deg, pv.local_off, pv.tile_off, key, static_cast<IdT*>(coo_row),           \
-                                static_cast<IdT*>(coo_col), static_cast<uint32_t>(cap), rowpos, jobs, status)); \
+                                static_cast<IdT*>(coo_col), static_cast<uint32_t>(cap), rowpos, jobs, marks, status)); \
   } while (0)
   // one storage region, and everything that is counted fits 32 bits: rows (they lie in indices), seeds, and the offsets of
   // all outputs that a plan may hold, also of those past the capacity
   const bool lean = !replace && k <= 32 && pos == nullptr && indices.num_parts == 1 && indices.threshold == indices.total &&
                     indices.total <= 0xFFFFFFFFll && cap >= 0 && cap < (1ll << 31) && n.bound < (1ll << 31) &&
                     n.bound * k < (1ll << 32) - 64;
+  if (lean && marks.first != nullptr) {
+    if (k <= 4) DGS_LAUNCH_LEAN(4, true);
+    else if (k <= 8) DGS_LAUNCH_LEAN(8, true);
+    else if (k <= 16) DGS_LAUNCH_LEAN(16, true);
+    else DGS_LAUNCH_LEAN(32, true);
+    return DGS_OK;
+  }
   if (lean) {
-    if (k <= 4) DGS_LAUNCH_LEAN(4);
-    else if (k <= 8) DGS_LAUNCH_LEAN(8);
-    else if (k <= 16) DGS_LAUNCH_LEAN(16);
-    else DGS_LAUNCH_LEAN(32);
+    if (k <= 4) DGS_LAUNCH_LEAN(4, false);
+    else if (k <= 8) DGS_LAUNCH_LEAN(8, false);
+    else if (k <= 16) DGS_LAUNCH_LEAN(16, false);
+    else DGS_LAUNCH_LEAN(32, false);
     return DGS_OK;
   }
   if (k <= 4) DGS_LAUNCH_U(4);
@@ -1066,14 +1088,14 @@ int uniform_typed(const dgs_chunk_desc& indices, const void* seeds, Count n, int
 template <typename IdT>
 int weighted_typed(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds, Count n,
                    int64_t k, bool replace, const PlanView& pv, RngKey key,
-                   void* coo_row, void* coo_col, int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, int32_t* status,
-                   cudaStream_t s) {
+                   void* coo_row, void* coo_col, int64_t cap, int64_t* pos, bool rowpos, SideJobs jobs, const IdMarks& marks,
+                   int32_t* status, cudaStream_t s) {
   jobs.main_ctas = static_cast<unsigned>((n.bound + WEIGHTED_WARPS - 1) / WEIGHTED_WARPS);
   auto kernel = replace ? sample_weighted_replace_kernel<IdT> : sample_weighted_kernel<IdT>;
   DGS_CUDA_TRY(launch_chained(SITE_SAMPLE, kernel, jobs.main_ctas + jobs.clear.ctas + jobs.lookup.ctas, SAMPLE_BLOCK, s,
                               indices, probs, static_cast<const IdT*>(seeds), n, k, pv.row_begin, pv.deg, pv.local_off,
                               pv.tile_off, key, static_cast<IdT*>(coo_row), static_cast<IdT*>(coo_col), cap,
-                              pos, rowpos, jobs, status));
+                              pos, rowpos, jobs, marks, status));
   return DGS_OK;
 }
 
@@ -1086,11 +1108,12 @@ uint64_t sample_rng_key(uint64_t rng_seed, uint64_t rng_offset) {
 }
 
 int launch_sample_plan(const dgs_chunk_desc& indptr, const void* seeds, bool ids64, int64_t n, int64_t k,
-                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, int32_t* status, cudaStream_t s) {
+                       bool replace, void* plan, int64_t* nnz_out, const InitWords& init, const FillJob& fill, int32_t* status,
+                       cudaStream_t s) {
   const PlanView pv = plan_view(plan, n);
   const Count nc = exact_count(n);
-  return ids64 ? plan_typed<int64_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, status, s)
-               : plan_typed<int32_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, status, s);
+  return ids64 ? plan_typed<int64_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, fill, status, s)
+               : plan_typed<int32_t>(indptr, seeds, nc, k, replace, pv, nnz_out, init, fill, status, s);
 }
 
 NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k, bool replace, void* plan) {
@@ -1101,27 +1124,27 @@ NextPlan make_next_plan(const dgs_chunk_desc& indptr, int64_t n_bound, int64_t k
 int launch_sample_uniform(const dgs_chunk_desc& indices, const void* seeds, bool ids64, Count n, int64_t k,
                           bool replace, void* plan, bool whole_offsets, RngKey key, void* coo_row,
                           void* coo_col, int64_t out_capacity, int64_t* picked_pos, bool row_is_position,
-                          const SideJobs& jobs, int32_t* status, cudaStream_t s) {
+                          const SideJobs& jobs, const IdMarks& marks, int32_t* status, cudaStream_t s) {
   static_assert(SAMPLE_BLOCK == RL_BLOCK, "the jobs riding on the sampling launch assume its CTA size");
   PlanView pv = plan_view(plan, n.bound);
   if (whole_offsets) pv.tile_off = nullptr;
   return ids64 ? uniform_typed<int64_t>(indices, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                        out_capacity, picked_pos, row_is_position, jobs, status, s)
+                                        out_capacity, picked_pos, row_is_position, jobs, marks, status, s)
                : uniform_typed<int32_t>(indices, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                        out_capacity, picked_pos, row_is_position, jobs, status, s);
+                                        out_capacity, picked_pos, row_is_position, jobs, marks, status, s);
 }
 
 int launch_sample_weighted(const dgs_chunk_desc& indices, const dgs_chunk_desc& probs, const void* seeds,
                            bool ids64, Count n, int64_t k, bool replace, void* plan, bool whole_offsets,
                            RngKey key, void* coo_row, void* coo_col, int64_t out_capacity,
-                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, int32_t* status,
-                           cudaStream_t s) {
+                           int64_t* picked_pos, bool row_is_position, const SideJobs& jobs, const IdMarks& marks,
+                           int32_t* status, cudaStream_t s) {
   PlanView pv = plan_view(plan, n.bound);
   if (whole_offsets) pv.tile_off = nullptr;
   return ids64 ? weighted_typed<int64_t>(indices, probs, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                         out_capacity, picked_pos, row_is_position, jobs, status, s)
+                                         out_capacity, picked_pos, row_is_position, jobs, marks, status, s)
                : weighted_typed<int32_t>(indices, probs, seeds, n, k, replace, pv, key, coo_row, coo_col,
-                                         out_capacity, picked_pos, row_is_position, jobs, status, s);
+                                         out_capacity, picked_pos, row_is_position, jobs, marks, status, s);
 }
 
 }  // namespace dgs
@@ -1150,7 +1173,7 @@ extern "C" int dgs_sample_plan(const dgs_chunk_desc* indptr, const void* seeds, 
     }
     return DGS_OK;
   }
-  return launch_sample_plan(*indptr, seeds, ids64 != 0, n, k, replace != 0, plan, nnz, InitWords{}, status, s);
+  return launch_sample_plan(*indptr, seeds, ids64 != 0, n, k, replace != 0, plan, nnz, InitWords{}, FillJob{}, status, s);
 }
 
 extern "C" int dgs_sample_uniform(const dgs_chunk_desc* indices, const void* seeds, int32_t ids64,
@@ -1177,7 +1200,7 @@ extern "C" int dgs_sample_uniform(const dgs_chunk_desc* indices, const void* see
               "dgs_sample_uniform: null output");
   rc = launch_sample_uniform(*indices, seeds, ids64 != 0, exact_count(n), k, replace != 0, const_cast<void*>(plan),
                              false, host_key(sample_rng_key(rng_seed, rng_offset)), coo_row, coo_col, out_capacity,
-                             picked_pos, false, SideJobs{}, status, s);
+                             picked_pos, false, SideJobs{}, IdMarks{}, status, s);
   if (rc != DGS_OK) return rc;
   if (nnz != nullptr) {
     copy_total_kernel<<<1, 1, 0, s>>>(sample_plan_total(const_cast<void*>(plan), n), nnz);
@@ -1217,7 +1240,7 @@ extern "C" int dgs_sample_weighted(const dgs_chunk_desc* indices, const dgs_chun
               "dgs_sample_weighted: null output");
   rc = launch_sample_weighted(*indices, *probs, seeds, ids64 != 0, exact_count(n), k, replace != 0,
                               const_cast<void*>(plan), false, host_key(sample_rng_key(rng_seed, rng_offset)), coo_row,
-                              coo_col, out_capacity, picked_pos, false, SideJobs{}, status, s);
+                              coo_col, out_capacity, picked_pos, false, SideJobs{}, IdMarks{}, status, s);
   if (rc != DGS_OK) return rc;
   if (nnz != nullptr) {
     copy_total_kernel<<<1, 1, 0, s>>>(sample_plan_total(const_cast<void*>(plan), n), nnz);

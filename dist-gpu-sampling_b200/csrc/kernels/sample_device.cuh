@@ -3,6 +3,7 @@
 #pragma once
 #include "common.cuh"
 #include "philox.cuh"
+#include "relabel_device.cuh"
 
 namespace dgs {
 
@@ -67,6 +68,8 @@ struct Emit {
   int64_t* picked_pos;
   int64_t out_capacity;
   int32_t* status;
+  const IdMarks& marks;
+  const Count& n_seeds;
 
   // t-th output of a seed whose outputs start at o; `pos` = position in its row
   __device__ __forceinline__ void operator()(int64_t o, int64_t t, int64_t seed, int64_t rb,
@@ -84,6 +87,7 @@ struct Emit {
     coo_row[at] = static_cast<IdT>(seed);
     coo_col[at] = c;
     if (picked_pos != nullptr) picked_pos[at] = pos;
+    if (marks.first != nullptr) mark_id(marks, static_cast<int64_t>(c), static_cast<uint32_t>(count_of(n_seeds) + at), status);
   }
 };
 

@@ -52,7 +52,8 @@ enum {
   DGS_ERR_UNSUPPORTED = 5, /* size / dtype outside what the kernels handle */
   DGS_ERR_RANGE = 6,       /* a kernel met an out-of-range id (status word) */
   DGS_ERR_TABLE_FULL = 7,  /* hash table probe ran out of slots (status word) */
-  DGS_ERR_MISMATCH = 8     /* ranks disagree on the ChunkTensor metadata */
+  DGS_ERR_MISMATCH = 8,    /* ranks disagree on the ChunkTensor metadata */
+  DGS_ERR_ID_SPACE = 9     /* a kernel met an id beyond the id space it was given (status word) */
 };
 
 typedef void* dgs_stream_t; /* cudaStream_t */
@@ -337,6 +338,34 @@ DGS_API int dgs_sample_blocks_record(const dgs_chunk_desc* indptr, const dgs_chu
                                      dgs_stream_t capture_stream, dgs_blocks_recording** out);
 DGS_API int dgs_sample_blocks_replay(dgs_blocks_recording* rec, dgs_stream_t stream);
 DGS_API void dgs_sample_blocks_recording_free(dgs_blocks_recording* rec);
+
+/* The same sequence for ids below a known id space: nodes are numbered through a
+ * table of one 32-bit word per id (id_space of them, cleared by the sequence's
+ * first launch and kept through all its hops) instead of a hash table per hop, so
+ * the sampling launch marks what it draws and no launch probes.  Same results, bit
+ * for bit.  An id at or beyond id_space raises DGS_ERR_ID_SPACE in *status (which
+ * must not be NULL) and the outputs are then not valid: queue the batch again with
+ * dgs_sample_blocks and the same (rng_seed, rng_offset), which takes any id.
+ * _wins: whether this form is the faster one (clearing a word per id of a very
+ * large graph costs more than the probes it saves).
+ * _workspace_bytes: 0 on bad arguments.  _record: replayed and freed like a
+ * recording of dgs_sample_blocks_record.  No counterpart in the reference. */
+DGS_API int32_t dgs_sample_blocks_dense_wins(const dgs_hop* hops, int32_t n_hops, int64_t id_space);
+DGS_API size_t dgs_sample_blocks_dense_workspace_bytes(const dgs_hop* hops, int32_t n_hops, int64_t id_space);
+DGS_API int dgs_sample_blocks_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
+                                    const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
+                                    const dgs_hop* hops, int32_t n_hops, int32_t replace,
+                                    int64_t id_space, uint64_t rng_seed, uint64_t rng_offset,
+                                    void* workspace, size_t workspace_bytes, int64_t* sizes,
+                                    int32_t* status, dgs_stream_t stream);
+DGS_API const int64_t* dgs_sample_blocks_dense_frontier_count(const dgs_hop* hops, int32_t n_hops,
+                                                              int64_t id_space, void* workspace);
+DGS_API int dgs_sample_blocks_dense_record(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices,
+                                           const dgs_chunk_desc* probs, const void* seeds, int32_t ids64,
+                                           const dgs_hop* hops, int32_t n_hops, int32_t replace,
+                                           int64_t id_space, const uint64_t* rng_words, void* workspace,
+                                           size_t workspace_bytes, int64_t* sizes, int32_t* status,
+                                           dgs_stream_t capture_stream, dgs_blocks_recording** out);
 
 /* ---- PaGraph-style feature cache ---------------------------------------- */
 /* CreateHashMapTensorCUDA, src/cuda/pagraph.cu:94-124: open-addressing table
