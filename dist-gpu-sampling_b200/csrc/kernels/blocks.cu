@@ -14,7 +14,7 @@
 // than the graph has), and the actual sizes go to a caller-supplied (pinned)
 // array that the host reads once, after everything is queued.
 //
-// Graphs of up to 2^24 ids take the form at dgs_sample_blocks_dense (one word per id); what follows is the form with a hash
+// Graphs of up to 2^23 ids take the form at dgs_sample_blocks_dense (one word per id); what follows is the form with a hash
 // table per hop, which takes any id.
 // Per hop: sample -> insert -> number.  The number launch of a hop also makes the
 // plan of the next one (its unique list is the next seed list); only the first
@@ -134,8 +134,9 @@ static_assert(sizeof(int64_t) * (1 + 2 * DGS_MAX_HOPS) <= WS_ALIGN, "control wor
 // The line: clearing a word per id (the first launch does it beside the plan) against the probes it saves.  Recorded
 // sequences, hash tables -> one word per id, us: 16 seeds [10, 5] over 0.5 M ids 39 -> 28, 2.4 M 39 -> 27, 8 M 40 -> 29,
 // 20 M 37 -> 35, 111 M 37 -> 88; 1 024 seeds [15, 10, 5] over 2.4 M ids 141 -> 92, 8 M 141 -> 90, 20 M 131 -> 111, 111 M
-// 134 -> 214.  A table of 2^24 words is 64 MB, half of the L2.
-constexpr int64_t DENSE_MAX_IDS = int64_t(1) << 24;
+// 134 -> 214.  With six batches in flight there are six tables, and past the L2 (126 MB) their words come from HBM:
+// 8 M ids 730 -> 684 us, 16 M 711 -> 744.
+constexpr int64_t DENSE_MAX_IDS = int64_t(1) << 23;
 constexpr unsigned FILL_CTA_UNITS = 4096;  // 64 KB a CTA of 1 024 threads
 
 DenseSpace dense_space(const dgs_hop* hops, int32_t n_hops, int64_t ids, void* workspace) {
