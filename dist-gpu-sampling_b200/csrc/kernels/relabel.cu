@@ -275,7 +275,7 @@ dense_number_kernel(const DenseNumbering d, const IdT* __restrict__ seeds, const
 #pragma unroll
   for (int u = 0; u < RL_ITEMS; ++u) {
     const bool in = static_cast<uint64_t>(id[u]) < static_cast<uint64_t>(d.ids);
-    word[u] = !in ? NOT_MET : known ? static_cast<uint32_t>(base + 32 * u) : *reinterpret_cast<const volatile uint32_t*>(d.first + id[u]);
+    word[u] = !in ? NOT_MET : known ? static_cast<uint32_t>(base + 32 * u) : load_kept(d.first + id[u], l2_evict_last_policy());
   }
   unsigned votes[RL_ITEMS];
   int c = 0;
@@ -314,7 +314,7 @@ dense_number_kernel(const DenseNumbering d, const IdT* __restrict__ seeds, const
     label[u] = next + __popc(votes[u] & ((1u << lane) - 1u));
     next += __popc(votes[u]);
     if (first) {
-      if (!known) d.first[id[u]] = static_cast<uint32_t>(label[u]);
+      if (!known) store_kept(d.first + id[u], static_cast<uint32_t>(label[u]), l2_evict_last_policy());
       if (label[u] < unique_capacity) {
         unique_out[label[u]] = static_cast<IdT>(id[u]);
       } else {
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(RL_BLOCK) dense_lookup_kernel(const __grid_con
     for (int u = 0; u < RL_ITEMS; ++u) id[u] = base + u * RL_BLOCK < n ? static_cast<int64_t>(ids[base + u * RL_BLOCK]) : -1;
 #pragma unroll
     for (int u = 0; u < RL_ITEMS; ++u)
-      word[u] = static_cast<uint64_t>(id[u]) < static_cast<uint64_t>(job.ids) ? job.first[id[u]] : NOT_MET;
+      word[u] = static_cast<uint64_t>(id[u]) < static_cast<uint64_t>(job.ids) ? load_kept(job.first + id[u], l2_evict_last_policy()) : NOT_MET;
 #pragma unroll
     for (int u = 0; u < RL_ITEMS; ++u)
       if (base + u * RL_BLOCK < n) ids[base + u * RL_BLOCK] = word[u] == NOT_MET ? static_cast<IdT>(-1) : static_cast<IdT>(word[u]);

