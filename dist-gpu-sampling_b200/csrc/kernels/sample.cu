@@ -37,7 +37,7 @@
 //     memory: the row is summed once into at most 128 groups, and every lane
 //     finds its own draw's group by bisection and walks the edges in it.
 //   * counts, offsets and the total come from a plan: one CTA for up to 2 048
-//     seeds; above, every CTA scans its 256 seeds and the one that finishes last
+//     seeds, a cluster of eight for up to 8 192; above, every CTA scans its 256 seeds and the one that finishes last
 //     (an atomic ticket, nobody waits) scans the per-tile sums; from the second
 //     hop of a multi-hop sequence on, the kernel that numbers the seeds.  The
 //     total goes to a caller-supplied (pinned) word, so the host learns the
@@ -50,6 +50,8 @@
 #include "philox.cuh"
 #include "sample_device.cuh"
 #include "tile_scan.cuh"
+
+#include <cooperative_groups.h>
 
 namespace dgs {
 namespace {
@@ -198,6 +200,85 @@ sample_small_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const Id
     }
   }
 }
+
+// The plan of an operator call's up to CLUSTER_PLAN seeds by one cluster of eight CTAs: each takes an eighth of the seeds, and
+// the CTAs' sums are read over distributed shared memory -- nothing to clear before it, and no round trip through L2 for
+// the offsets.  (The multi-hop sequence keeps to the forms before and behind: its batches run beside others, and a
+// cluster waits for room on eight SMs at once.)
+// Against the clearing launch and a CTA per 256 seeds, whole operator calls: 4 096 weighted draws with replacement 45.7 ->
+// 42.4 us, 3 000 of them 45.9 -> 42.6, 8 000 without replacement (fan-out 5) 45.8 -> 43.7.  With four seeds per thread, for
+// 11 000 seeds, level or slower (91.2 -> 92.2).
+constexpr int CLUSTER_PLAN_CTAS = 8;
+constexpr int CLUSTER_PLAN_BLOCK = 512;
+constexpr int CLUSTER_PLAN_ITEMS = 2;
+constexpr int CLUSTER_PLAN = CLUSTER_PLAN_CTAS * CLUSTER_PLAN_BLOCK * CLUSTER_PLAN_ITEMS;
+
+template <typename IdT>
+__global__ void __cluster_dims__(CLUSTER_PLAN_CTAS, 1, 1) __launch_bounds__(CLUSTER_PLAN_BLOCK)
+sample_cluster_plan_kernel(const __grid_constant__ dgs_chunk_desc indptr, const IdT* __restrict__ seeds, const int n,
+                           const int64_t k, const bool replace, const PlanView plan, int64_t* nnz_out,
+                           int32_t* __restrict__ status) {
+  __shared__ int64_t smem[CLUSTER_PLAN_BLOCK / 32 + 1];
+  __shared__ int64_t s_sum;
+  auto cluster = cooperative_groups::this_cluster();
+  pdl_enter();
+  const int rank = blockIdx.x;
+  const int per = (n + CLUSTER_PLAN_CTAS - 1) / CLUSTER_PLAN_CTAS, lo = rank * per, end = min(lo + per, n);
+  int64_t s[CLUSTER_PLAN_ITEMS], rb[CLUSTER_PLAN_ITEMS], deg[CLUSTER_PLAN_ITEMS], off[CLUSTER_PLAN_ITEMS];
+  bool good[CLUSTER_PLAN_ITEMS];
+#pragma unroll
+  for (int u = 0; u < CLUSTER_PLAN_ITEMS; ++u) {
+    const int i = lo + u * CLUSTER_PLAN_BLOCK + threadIdx.x;
+    s[u] = i < end ? static_cast<int64_t>(seeds[i]) : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < CLUSTER_PLAN_ITEMS; ++u) {
+    good[u] = s[u] >= 0 && s[u] + 1 < indptr.total;
+    if (lo + u * CLUSTER_PLAN_BLOCK + static_cast<int>(threadIdx.x) < end && !good[u]) raise_status(status, DGS_ERR_RANGE);
+  }
+  row_bounds<IdT, CLUSTER_PLAN_ITEMS>(indptr, s, good, rb, deg, status);
+  int64_t carry = 0;
+#pragma unroll
+  for (int u = 0; u < CLUSTER_PLAN_ITEMS; ++u) {
+    off[u] = 0;
+    if (lo + u * CLUSTER_PLAN_BLOCK >= end) continue;  // uniform
+    const int i = lo + u * CLUSTER_PLAN_BLOCK + threadIdx.x;
+    int64_t total;
+    off[u] = carry + block_exclusive_scan<int64_t, CLUSTER_PLAN_BLOCK>(i < end ? pick_count(deg[u], k, replace) : 0, smem, &total);
+    carry += total;
+  }
+  if (threadIdx.x == 0) s_sum = carry;
+  cluster.sync();
+  int64_t before = 0, all = 0;
+#pragma unroll
+  for (int r = 0; r < CLUSTER_PLAN_CTAS; ++r) {
+    const int64_t v = *cluster.map_shared_rank(&s_sum, r);
+    if (r < rank) before += v;
+    all += v;
+  }
+#pragma unroll
+  for (int u = 0; u < CLUSTER_PLAN_ITEMS; ++u) {
+    const int i = lo + u * CLUSTER_PLAN_BLOCK + threadIdx.x;
+    if (i < end) {
+      plan.row_begin[i] = rb[u];
+      plan.deg[i] = deg[u];
+      plan.local_off[i] = before + off[u];
+    }
+  }
+  if (rank == 0) {
+    // offsets are those in the whole output, whichever way the sampling launch adds them up
+    if (static_cast<int64_t>(threadIdx.x) < plan.ntiles) plan.tile_off[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+      *plan.total = all;
+      if (nnz_out != nullptr) {
+        *nnz_out = all;
+        __threadfence_system();
+      }
+    }
+  }
+  cluster.sync();  // the sums stay until all CTAs have read them
+}
+static_assert(CLUSTER_PLAN / SAMPLE_TILE <= CLUSTER_PLAN_BLOCK, "a thread per tile offset");
 
 // CTAs of a sampling launch beyond the main ones carry two jobs of the multi-hop sequence that depend on nothing the
 // launch does: clearing the table this hop will fill, relabelling the COO of the hop before.
@@ -1025,6 +1106,11 @@ int plan_typed(const dgs_chunk_desc& indptr, const void* seeds, Count n, int64_t
     DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_small_plan_kernel<IdT>, 1u + fill.ctas, SMALL_PLAN_BLOCK, s, indptr,
                                 static_cast<const IdT*>(seeds), static_cast<int>(n.bound), k, replace, pv, nnz, init, fill,
                                 status));
+    return DGS_OK;
+  }
+  if (n.bound <= CLUSTER_PLAN && init.n0 == nullptr && fill.ctas == 0) {
+    DGS_CUDA_TRY(launch_chained(SITE_PLAN, sample_cluster_plan_kernel<IdT>, CLUSTER_PLAN_CTAS, CLUSTER_PLAN_BLOCK, s, indptr,
+                                static_cast<const IdT*>(seeds), static_cast<int>(n.bound), k, replace, pv, nnz, status));
     return DGS_OK;
   }
   DGS_CUDA_TRY(launch_chained(SITE_INIT, init_kernel, 1u + fill.ctas, fill.ctas > 0 ? 1024u : 32u, s, init, pv.ticket, fill));
