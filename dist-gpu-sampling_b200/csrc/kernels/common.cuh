@@ -108,6 +108,14 @@ __device__ __forceinline__ int64_t count_of(const Count& c) {
 
 __device__ __forceinline__ uint64_t key_of(const RngKey& k) { return k.dev == nullptr ? k.value : *k.dev; }
 
+// A value that is the same in all lanes of a full warp, as one that the compiler knows to be so (the key schedule of Philox
+// then runs on the uniform datapath and leaves the loops).
+__device__ __forceinline__ uint64_t uniform_word(uint64_t v) {
+  const uint32_t lo = __reduce_or_sync(FULL_MASK, static_cast<uint32_t>(v));
+  const uint32_t hi = __reduce_or_sync(FULL_MASK, static_cast<uint32_t>(v >> 32));
+  return (static_cast<uint64_t>(hi) << 32) | lo;
+}
+
 // Sticky status word: first error wins, later ones are dropped.
 __device__ __forceinline__ void raise_status(int32_t* status, int32_t code) {
   if (status != nullptr) atomicCAS(status, 0, code);

@@ -31,8 +31,8 @@
 //     log domain, log(u)/w, which orders exactly like u^(1/w) but does not
 //     underflow for small weights.  The first 512 edges of a row give one warp
 //     a list and a bar; the 512-edge windows behind them (16 loads in flight
-//     per lane) are dealt out to the eight warps of the CTA, which spend a
-//     logarithm only on edges that may beat the bar, and the lists are joined.
+//     per lane) are dealt out to the eight warps of the CTA, which collect the
+//     edges that may beat the bar, and one warp per row joins them with its list.
 //   * weighted sampling with replacement builds no cumulative array in global
 //     memory: the row is summed once into at most 128 groups, and every lane
 //     finds its own draw's group by bisection and walks the edges in it.
@@ -485,9 +485,14 @@ struct RowWeights {
   __device__ __forceinline__ void load(float (&v)[COUNT], int64_t base, int64_t deg, int l) const {
     if (direct != nullptr) {
       const float* p = direct + base + l;
-      const int left = deg - base - l < 32 * COUNT ? static_cast<int>(deg - base - l) : 32 * COUNT;  // <= 0: none
+      if (deg - base >= 32 * COUNT) {
 #pragma unroll
-      for (int j = 0; j < COUNT; ++j) v[j] = j * 32 < left ? p[j * 32] : 0.f;
+        for (int j = 0; j < COUNT; ++j) v[j] = p[j * 32];
+      } else {
+        const int left = static_cast<int>(deg - base) - l;  // <= 0: none
+#pragma unroll
+        for (int j = 0; j < COUNT; ++j) v[j] = j * 32 < left ? p[j * 32] : 0.f;
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < COUNT; ++j) v[j] = base + j * 32 + l < deg ? straddling_weight(&probs, rb + base + j * 32 + l) : 0.f;
@@ -503,38 +508,80 @@ __device__ __forceinline__ RowWeights row_weights(const dgs_chunk_desc& probs, i
 constexpr int64_t HUB_DEG = 4096;  // with replacement: rows above this are left to the whole CTA
 constexpr int WEIGHTED_WARPS = SAMPLE_BLOCK / 32;
 
-// Sorts 32 (key, position) pairs, one per lane, by (key descending, position ascending).  Out of line: called from
-// three places, 15 exchange steps each.
-__device__ __noinline__ float2 sort32(float key, float position) {
+// One entry of a list of candidates, as an integer whose order is the list's: the key in the high half (both zeros are one
+// key), the complement of the edge's place in the low half, so that of equal keys the earlier place comes first.
+using Entry = unsigned long long;
+constexpr Entry NO_ENTRY = 0x007FFFFF00000000ull;  // key -inf, behind every edge
+__device__ __forceinline__ Entry make_entry(float key, uint32_t place) {
+  const uint32_t u = __float_as_uint(key + 0.f);
+  const uint32_t up = (u & 0x80000000u) ? ~u : u | 0x80000000u;
+  return (static_cast<Entry>(up) << 32) | static_cast<uint32_t>(~place);
+}
+__device__ __forceinline__ float entry_key(Entry e) {
+  const uint32_t up = static_cast<uint32_t>(e >> 32);
+  return __uint_as_float((up & 0x80000000u) ? up ^ 0x80000000u : ~up);
+}
+__device__ __forceinline__ uint32_t entry_place(Entry e) { return ~static_cast<uint32_t>(e); }
+
+// Sorts 32 entries, one per lane, the best to lane 0.  Out of line: 15 exchange steps, called from several places.
+__device__ __noinline__ Entry sort32(Entry e) {
   const int l = threadIdx.x & 31;
-  uint32_t pos = __float_as_uint(position);
 #pragma unroll
   for (int size = 2; size <= 32; size <<= 1) {
 #pragma unroll
     for (int d = size >> 1; d > 0; d >>= 1) {
-      const float ok = __shfl_xor_sync(FULL_MASK, key, d);
-      const uint32_t op = __shfl_xor_sync(FULL_MASK, pos, d);
-      const bool mine_first = key > ok || (key == ok && pos < op);
-      const bool want_first = ((l & d) == 0) == ((l & size) == 0);
-      if (mine_first != want_first) {
-        key = ok;
-        pos = op;
-      }
+      const Entry o = __shfl_xor_sync(FULL_MASK, e, d);
+      const bool want_larger = ((l & d) == 0) == ((l & size) == 0);
+      if ((o > e) == want_larger) e = o;
     }
   }
-  return make_float2(key, __uint_as_float(pos));
+  return e;
 }
 
-// The running top-k of one warp: lane j holds the j-th largest key and its
-// place in the warp's share of the row; `thresh` is the key held by lane k-1 (the entry bar).
-template <typename P>
-struct TopK {
-  float key;
-  P pos;
+// The k-th largest of 32 values, one per lane.
+__device__ __forceinline__ float kth_of_32(float v, int l, int k) {
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+    for (int d = size >> 1; d > 0; d >>= 1) {
+      const float o = __shfl_xor_sync(FULL_MASK, v, d);
+      v = ((l & d) == 0) == ((l & size) == 0) ? fmaxf(v, o) : fminf(v, o);
+    }
+  }
+  return __shfl_sync(FULL_MASK, v, k - 1);
+}
+
+// The best edges of a row so far: lane j holds the j-th; `thresh` is the key held by lane k-1 (the bar to beat).
+struct ShareList {
+  Entry e;
   float thresh;
-  __device__ __forceinline__ void shift_in(float nk, P np, int p, int l, int k) {
+  __device__ __forceinline__ void set(Entry sorted, int k) {
+    e = sorted;
+    thresh = entry_key(__shfl_sync(FULL_MASK, e, k - 1));
+  }
+  // 32 more entries, one per lane, in any order
+  __device__ __forceinline__ void merge(Entry more, int l, int k) {
+    const Entry c = __shfl_sync(FULL_MASK, sort32(more), 31 - l);
+    Entry m = c > e ? c : e;  // the 32 best of both, in bitonic order
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const Entry o = __shfl_xor_sync(FULL_MASK, m, d);
+      if ((o > m) == ((l & d) == 0)) m = o;
+    }
+    set(m, k);
+  }
+};
+
+// The same with positions of 64 bits, one insertion at a time.
+struct RowList {
+  float key;
+  int64_t pos;
+  float thresh;
+  __device__ __forceinline__ void insert(float nk, int64_t np, int l, int k) {
+    // warp-uniform call with nk > thresh; the keys >= nk form a prefix of the lanes
+    const int p = __popc(__ballot_sync(FULL_MASK, key >= nk));  // <= k-1
     const float up_key = __shfl_up_sync(FULL_MASK, key, 1);
-    const P up_pos = __shfl_up_sync(FULL_MASK, pos, 1);
+    const int64_t up_pos = __shfl_up_sync(FULL_MASK, pos, 1);
     if (l > p) {
       key = up_key;
       pos = up_pos;
@@ -544,21 +591,9 @@ struct TopK {
     }
     thresh = __shfl_sync(FULL_MASK, key, k - 1);
   }
-  __device__ __forceinline__ void insert(float nk, P np, int l, int k) {
-    // warp-uniform call with nk > thresh; the keys >= nk form a prefix of the lanes
-    shift_in(nk, np, __popc(__ballot_sync(FULL_MASK, key >= nk)), l, k);  // p <= k-1
-  }
-  // one key per lane: the order that 32 single insertions give
-  __device__ __forceinline__ void fill(float nk, uint32_t np, int k) {
-    const float2 sorted = sort32(nk, __uint_as_float(np));
-    key = sorted.x;
-    pos = __float_as_uint(sorted.y);
-    thresh = __shfl_sync(FULL_MASK, key, k - 1);
-  }
 };
-using ShareList = TopK<uint32_t>;  // places within a share: 512 per window
 
-// Floats in an order-preserving integer form (for atomicMax in shared memory); its own inverse.
+// Floats in an order-preserving integer form; its own inverse.
 __device__ __forceinline__ int ordered_float(float f) {
   const int i = __float_as_int(f);
   return i >= 0 ? i : i ^ 0x7fffffff;
@@ -587,40 +622,43 @@ __device__ __forceinline__ Philox4 ares_words(uint64_t key, uint32_t i_lo, uint3
   return philox4x32_10(key, i_lo, i_hi, static_cast<uint32_t>(ctr), static_cast<uint32_t>(ctr >> 32));
 }
 
-// `entry`: only keys above it are of interest (the list's own bar or a higher one the caller knows of)
-__device__ __forceinline__ void insert_above(ShareList& top, float& entry, float ck, uint32_t place, int l, int k) {
-  unsigned cand = __ballot_sync(FULL_MASK, ck > entry);
-  while (cand) {
-    const int src = __ffs(cand) - 1;
-    cand &= cand - 1;
-    const float nk = __shfl_sync(FULL_MASK, ck, src);
-    if (nk > entry) {  // the bar may have risen since the ballot
-      top.insert(nk, place + src, l, k);
-      entry = fmaxf(entry, top.thresh);
-    }
-  }
-}
-
 constexpr int ARES_EDGES = 512;  // edges per window
-constexpr int ARES_ITEMS = ARES_EDGES / 32;
+constexpr int ARES_GROUP = 128;  // edges per step: four per lane, one Philox block
+constexpr int ARES_PACK_K = 20;  // fan-outs for which the k-th largest of 32 lane maxima leaves fewer than 32 candidates
 
-// The first 512 edges of a row.  Every lane computes its 16 keys; the k-th largest of the 32 lane maxima is a bar that at
-// least k keys reach and, for k well below 32, few more than k (expected -32 ln(1 - k/32) of them: 12 at k = 10, 22
-// at k = 16), so those are packed into one per lane and sorted at once -- 15 exchange steps, where inserting one
-// after the other is a chain of ~28 insertions of ~150 cycles each for k = 10.  With more than 32 at the bar (large
-// k, ties) they are inserted one by one after all.
-__device__ __forceinline__ void ares_first_window(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key,
-                                                  uint32_t i_lo, uint32_t i_hi, int l, int k, float* pack_key,
-                                                  uint16_t* pack_at) {
+// Edges that passed the filter below and whose keys are still to be computed: of a row's windows of one round, a stretch
+// of `room` entries each, with their offsets in the window.
+struct Survivors {
+  static constexpr int ROOM = 256;
+  uint2 word_weight[ROOM];
+  uint16_t at[ROOM];
+};
+// The same of one warp that scans a row by itself.
+struct Pending {
+  static constexpr int ROOM = 31 + ARES_GROUP;
+  uint2 word_weight[ROOM];
+  uint32_t place[ROOM];
+};
+union Scratch {  // of a row: one or the other
+  Survivors survivors;
+  Pending pending;
+};
+
+// The first 512 edges of a row, for k well below 32: every lane computes its 16 keys; the k-th largest of the 32 lane
+// maxima is a bar that at least k keys reach and few more than k (expected -32 ln(1 - k/32) of them: 12 at k = 10, 22
+// at k = 16), so those are packed into one per lane and sorted once.  False: more than 32 are at the bar (ties).
+__device__ __forceinline__ bool ares_first_window(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo,
+                                                  uint32_t i_hi, int l, int k, Entry* pack) {
+  constexpr int ITEMS = ARES_EDGES / 32;
   const float NEG_INF = __int_as_float(0xff800000);
-  float ck[ARES_ITEMS];
+  float ck[ITEMS];
   W.load(ck, 0, deg, l);
   float best = NEG_INF;
   const int left = deg < ARES_EDGES ? static_cast<int>(deg) - l : ARES_EDGES;
 #pragma unroll
-  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
-    if (q * 128 < deg) {  // warp-uniform
-      const Philox4 r = ares_words(key, i_lo, i_hi, q * 128, l);
+  for (int q = 0; q < ITEMS / 4; ++q) {
+    if (q * ARES_GROUP < deg) {  // warp-uniform
+      const Philox4 r = ares_words(key, i_lo, i_hi, q * ARES_GROUP, l);
       const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
       for (int j = 4 * q; j < 4 * q + 4; ++j) {
@@ -633,82 +671,251 @@ __device__ __forceinline__ void ares_first_window(ShareList& top, const RowWeigh
     }
   }
   if (deg <= 32) {
-    top.fill(ck[0], static_cast<uint32_t>(l), k);
-    return;
+    top.set(sort32(ck[0] > NEG_INF ? make_entry(ck[0], l) : NO_ENTRY), k);
+    return true;
   }
-  ShareList maxima;
-  maxima.fill(best, static_cast<uint32_t>(l), k);
-  const float bar = maxima.thresh;
+  const float bar = kth_of_32(best, l, k);
   int have = 0;
 #pragma unroll
-  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
-    if (q * 128 >= deg) break;  // warp-uniform
+  for (int q = 0; q < ITEMS / 4; ++q) {
+    if (q * ARES_GROUP >= deg) break;  // warp-uniform
 #pragma unroll
     for (int j = 4 * q; j < 4 * q + 4; ++j) {
       const bool in = ck[j] >= bar && ck[j] > NEG_INF;
       const unsigned m = __ballot_sync(FULL_MASK, in);
       const int at = have + __popc(m & ((1u << l) - 1u));
-      if (in && at < 32) {
-        pack_key[at] = ck[j];
-        pack_at[at] = static_cast<uint16_t>(j * 32 + l);
-      }
+      if (in && at < 32) pack[at] = make_entry(ck[j], j * 32 + l);
       have += __popc(m);
     }
   }
   __syncwarp();
-  if (have <= 32) {
-    top.fill(l < have ? pack_key[l] : NEG_INF, l < have ? pack_at[l] : ARES_EDGES + l, k);
-  } else {
-    top.fill(ck[0], static_cast<uint32_t>(l), k);
-    float above = fmaxf(top.thresh, key_below(bar));
-#pragma unroll 1
-    for (int j = 1; j < ARES_ITEMS; ++j) {
-      float c = ck[0];
-#pragma unroll
-      for (int x = 1; x < ARES_ITEMS; ++x) c = x == j ? ck[x] : c;
-      insert_above(top, above, c, j * 32, l, k);
-    }
-  }
-  __syncwarp();
+  top.set(sort32(l < have ? pack[l] : NO_ENTRY), k);
+  __syncwarp();  // the room is used again
+  return have <= 32;
 }
 
-// A further window of a list.  Of a row's n edges only about k (1 + ln(n/k)) ever enter the list, so the logarithm
-// and the division are spent only on edges that a bound lets through: log(u) <= u - 1, so an edge whose
-// u - 1 <= bar * w cannot beat the bar.  The test below is that inequality with the slack that the errors of __logf
-// (2^-21.4 absolute on [0.5, 2]), __fdividef (2 ulp) and of the 23 random bits it looks at need, so every edge that
-// the exact key lets in passes, and the exact key decides.  One vote per 128 edges.  A bar above -1e-30 is taken as
-// -1e-30 (weights so large that __fdividef gives 0 then always pass); at or below the clamp of positive weights the
-// inequality says nothing about keys that were clamped, and every edge passes; so do products that are no number
-// (0 * inf: a weight <= 0 then).
-__device__ __forceinline__ void ares_next_window(ShareList& top, float& entry, const RowWeights& W, int64_t base,
-                                                 uint32_t place, int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k) {
+// The first 128 edges of a row, for larger k: keys computed for all of them (w: the lane's four weights), the four quarters
+// merged one by one.
+__device__ __forceinline__ void ares_first_group(ShareList& top, const float (&w)[4], int64_t deg, uint64_t key, uint32_t i_lo,
+                                                 uint32_t i_hi, int l, int k) {
   const float NEG_INF = __int_as_float(0xff800000);
-  constexpr float PASS = 2.0f - 0x1p-18f;
-  float wv[ARES_ITEMS];
-  W.load(wv, base, deg, l);
+  const Philox4 r = ares_words(key, i_lo, i_hi, 0, l);
+  const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll 1
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t word = j == 0 ? rw[0] : j == 1 ? rw[1] : j == 2 ? rw[2] : rw[3];
+    const float weight = j == 0 ? w[0] : j == 1 ? w[1] : j == 2 ? w[2] : w[3];
+    const float ck = j * 32 + l < deg ? ares_key(word, weight) : NEG_INF;
+    if (__any_sync(FULL_MASK, ck > top.thresh)) top.merge(ck > top.thresh ? make_entry(ck, j * 32 + l) : NO_ENTRY, l, k);
+  }
+}
+
+// The order of equal keys (zero weights, equal weights): window w of 512 edges belongs to share w % 8; equal keys are
+// ordered by share and then position, which up to eight windows is by position.  The tag of an edge holds that in 32
+// bits for rows below 2^32 edges.
+constexpr int ARES_SHARES = 8;
+__device__ __forceinline__ uint32_t window_tag(int64_t window) {
+  return (static_cast<uint32_t>(window & (ARES_SHARES - 1)) << 29) | (static_cast<uint32_t>(window / ARES_SHARES) * ARES_EDGES);
+}
+// position in the row of a place (512 per window) in share r
+__device__ __forceinline__ int64_t position_of(int r, uint32_t place) {
+  return static_cast<int64_t>(place & ~(ARES_EDGES - 1u)) * ARES_SHARES + r * ARES_EDGES + (place & (ARES_EDGES - 1u));
+}
+__device__ __forceinline__ int64_t tag_position(uint32_t tag) { return position_of(static_cast<int>(tag >> 29), tag & 0x1FFFFFFFu); }
+
+// Of a row's n edges only about k (1 + ln(n/k)) ever enter its list, so the logarithm and the division are spent only on
+// edges that a bound lets through: log(u) <= u - 1, so an edge whose u - 1 <= bar * w cannot beat the bar.  The test is
+// that inequality with the slack that the errors of __logf (2^-21.4 absolute on [0.5, 2]), __fdividef (2 ulp) and of the 23
+// random bits it looks at need, so every edge that the exact key lets in passes, and the exact key decides.  A bar above
+// -1e-30 is taken as -1e-30 (weights so large that __fdividef gives 0 then always pass); at or below the clamp of positive
+// weights the inequality says nothing about keys that were clamped, and every edge passes; so do products that are no
+// number (0 * inf: a weight <= 0 then).
+constexpr float ARES_PASS = 2.0f - 0x1p-18f;
+__device__ __forceinline__ float filter_bar(float above) {  // for keys above `above`
+  return above <= FLOOR_POS_W ? __int_as_float(0xff800000) : fminf(above * 1.00001f, -1e-30f);
+}
+__device__ __forceinline__ bool may_beat(float bar, uint32_t word, float w) {
+  return !(__uint_as_float((word >> 9) | 0x3f800000u) <= fmaf(bar, fmaxf(w, 0.f), ARES_PASS));
+}
+
+// The edges of a window (from its group FIRST on; `base`: its first edge) that may beat `bar`, into s[from, from + room);
+// their number, which may exceed the room: what has none is dropped.  (Past the row's end weights are 0; what passes
+// there is left out when the keys are computed.)
+template <int FIRST>
+__device__ __forceinline__ int ares_collect(const RowWeights& W, int64_t deg, int64_t base, uint64_t key, uint32_t i_lo,
+                                            uint32_t i_hi, int l, float bar, Survivors& s, int from, int room) {
+  float w[(4 - FIRST) * 4];
+  W.load(w, base + FIRST * ARES_GROUP, deg, l);
+  const uint64_t ctr = static_cast<uint64_t>(base >> 2);  // the low seven bits are clear
+  const uint32_t c_lo = static_cast<uint32_t>(ctr) | l, c_hi = static_cast<uint32_t>(ctr >> 32);
+  int have = 0;
 #pragma unroll
-  for (int q = 0; q < ARES_ITEMS / 4; ++q) {
-    const int64_t e0 = base + q * 128;
-    if (e0 >= deg) break;  // warp-uniform
-    const Philox4 r = ares_words(key, i_lo, i_hi, e0, l);
-    const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
-    const float bar = entry <= FLOOR_POS_W ? NEG_INF : fminf(entry * 1.00001f, -1e-30f);
+  for (int q = FIRST; q < 4; ++q) {
+    if (base + q * ARES_GROUP >= deg) break;  // warp-uniform
+    const Philox4 rnd = philox4x32_10(key, i_lo, i_hi, c_lo + q * 32, c_hi);
+    const uint32_t rw[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
     bool pass[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float v = __uint_as_float((rw[j] >> 9) | 0x3f800000u);
-      pass[j] = !(v <= fmaf(bar, fmaxf(wv[q * 4 + j], 0.f), PASS));
-    }
+    for (int j = 0; j < 4; ++j) pass[j] = may_beat(bar, rw[j], w[(q - FIRST) * 4 + j]);
     if (!__any_sync(FULL_MASK, pass[0] || pass[1] || pass[2] || pass[3])) continue;
-#pragma unroll 1
+#pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool p = j == 0 ? pass[0] : j == 1 ? pass[1] : j == 2 ? pass[2] : pass[3];
-      if (!__any_sync(FULL_MASK, p)) continue;
-      const uint32_t word = j == 0 ? rw[0] : j == 1 ? rw[1] : j == 2 ? rw[2] : rw[3];
-      const float w = j == 0 ? wv[q * 4] : j == 1 ? wv[q * 4 + 1] : j == 2 ? wv[q * 4 + 2] : wv[q * 4 + 3];
-      insert_above(top, entry, p && e0 + j * 32 + l < deg ? ares_key(word, w) : NEG_INF, place + q * 128 + j * 32, l, k);
+      const unsigned m = __ballot_sync(FULL_MASK, pass[j]);
+      const int at = have + __popc(m & ((1u << l) - 1u));
+      if (pass[j] && at < room) {
+        s.word_weight[from + at] = make_uint2(rw[j], __float_as_uint(w[(q - FIRST) * 4 + j]));
+        s.at[from + at] = static_cast<uint16_t>(q * ARES_GROUP + j * 32 + l);
+      }
+      have += __popc(m);
     }
   }
+  return have;
+}
+
+// Joins a row's list with what its windows w0, w0 + 1, ... have collected: stretch b of `room` entries holds as many
+// as lane b says.
+// With more than 32 the k-th largest of the lanes' best keys is a bar that few more than k reach (for k well below 32),
+// so that one sort and one merge do.
+__device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int count, int room, int64_t w0, int64_t deg, int l,
+                                          int k) {
+  int upto = count;  // entries of the stretches up to this lane's
+#pragma unroll
+  for (int o = 1; o < ARES_SHARES; o <<= 1) {
+    const int t = __shfl_up_sync(FULL_MASK, upto, o);
+    if (l >= o) upto += t;
+  }
+  const int total = __shfl_sync(FULL_MASK, upto, ARES_SHARES - 1);
+  if (total == 0) return;
+  // the i-th entry of all: its stretch, and its slot
+  auto slot_of = [&](int i, int* stretch) {
+    int b = 0, before = 0;
+#pragma unroll
+    for (int x = 0; x < ARES_SHARES - 1; ++x) {
+      const int end = __shfl_sync(FULL_MASK, upto, x);
+      if (i >= end) {
+        b = x + 1;
+        before = end;
+      }
+    }
+    *stretch = b;
+    return b * room + i - before;
+  };
+  Entry* out = reinterpret_cast<Entry*>(s.word_weight);
+  Entry first = NO_ENTRY, best = NO_ENTRY;
+  __syncwarp();
+#pragma unroll 1
+  for (int i0 = 0; i0 < total; i0 += 32) {
+    int b;
+    const int slot = slot_of(i0 + l, &b);
+    Entry e = NO_ENTRY;
+    if (i0 + l < total) {
+      const uint2 x = s.word_weight[slot];
+      const uint32_t off = s.at[slot];
+      if ((w0 + b) * ARES_EDGES + off < deg) e = make_entry(ares_key(x.x, __uint_as_float(x.y)), window_tag(w0 + b) + off);
+      out[slot] = e;
+      best = e > best ? e : best;
+    }
+    if (i0 == 0) first = e;
+  }
+  if (total <= 32) {
+    if (__any_sync(FULL_MASK, entry_key(first) >= top.thresh)) top.merge(first, l, k);
+    return;
+  }
+  float bar = top.thresh;
+  if (k <= ARES_PACK_K) bar = fmaxf(bar, kth_of_32(entry_key(best), l, k));
+  __syncwarp();
+  // those that reach the bar, 32 at a time.  Packed in place: what is written lies in front of what is still to be read
+  int have = 0;
+#pragma unroll 1
+  for (int i0 = 0; i0 < total; i0 += 32) {
+    int b;
+    const int slot = slot_of(i0 + l, &b);
+    const Entry e = i0 + l < total ? out[slot] : NO_ENTRY;
+    const bool in = e != NO_ENTRY && entry_key(e) >= bar;
+    const unsigned m = __ballot_sync(FULL_MASK, in);
+    __syncwarp();
+    if (in) out[have + __popc(m & ((1u << l) - 1u))] = e;  // at most 31 + 32 of them
+    have += __popc(m);
+    __syncwarp();
+    const bool last = i0 + 32 >= total;
+    if (have >= 32 || last) {
+      const Entry one = l < have ? out[l] : NO_ENTRY, two = l + 32 < have ? out[l + 32] : NO_ENTRY;
+      __syncwarp();
+      if (have > 0) top.merge(one, l, k);
+      if (have > 32) {
+        if (last) top.merge(two, l, k);
+        else if (l + 32 < have) out[l] = two;
+      }
+      have = have > 32 ? have - 32 : 0;
+      __syncwarp();
+    }
+  }
+}
+
+// Share r of a row by one warp, 128 edges at a time, for rows whose survivors found no room (more than a few equal keys at
+// the bar) or whose tags do not fit 32 bits.  What passes is put aside, and whenever 32 are waiting their keys are
+// computed, sorted and merged.  `above`: only keys above it are of interest.
+__device__ __noinline__ void ares_scan(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo,
+                                       uint32_t i_hi, int r, float above, int l, int k, Pending& pend) {
+  int have = 0;
+  top.set(NO_ENTRY, k);
+  float bar = filter_bar(above);
+  bool more = position_of(r, 0) < deg;
+#pragma unroll 1
+  for (uint32_t place = 0; more;) {
+    const int64_t e0 = position_of(r, place);
+    float w[4];
+    W.load(w, e0, deg, l);
+    const Philox4 rnd = ares_words(key, i_lo, i_hi, e0, l);
+    const uint32_t rw[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool pass = may_beat(bar, rw[j], w[j]) && e0 + j * 32 + l < deg;
+      const unsigned m = __ballot_sync(FULL_MASK, pass);
+      if (pass) {
+        const int at = have + __popc(m & ((1u << l) - 1u));
+        pend.word_weight[at] = make_uint2(rw[j], __float_as_uint(w[j]));
+        pend.place[at] = place + j * 32 + l;
+      }
+      have += __popc(m);
+    }
+    place += ARES_GROUP;
+    more = place != 0 && position_of(r, place) < deg;  // 0: past 2^32 places
+    while (have >= 32 || (!more && have > 0)) {
+      const int take = have < 32 ? have : 32;
+      have -= take;
+      __syncwarp();
+      Entry c = NO_ENTRY;
+      if (l < take) {
+        const uint2 x = pend.word_weight[have + l];
+        c = make_entry(ares_key(x.x, __uint_as_float(x.y)), pend.place[have + l]);
+      }
+      __syncwarp();
+      top.merge(c, l, k);
+      bar = filter_bar(fmaxf(above, top.thresh));
+    }
+  }
+}
+
+// A whole row that way: its shares in order; lane t's position of rank t.
+__device__ __noinline__ int64_t ares_row(const dgs_chunk_desc* probs, int64_t rb, int64_t deg, uint64_t key, uint32_t i_lo,
+                                         uint32_t i_hi, int l, int k, Pending& pend) {
+  const float NEG_INF = __int_as_float(0xff800000);
+  const RowWeights W = row_weights(*probs, rb, deg);
+  RowList row{NEG_INF, 0, NEG_INF};
+#pragma unroll 1
+  for (int r = 0; r < ARES_SHARES; ++r) {
+    ShareList top;
+    ares_scan(top, W, deg, key, i_lo, i_hi, r, row.thresh, l, k, pend);
+#pragma unroll 1
+    for (int t = 0; t < k; ++t) {
+      const Entry next = __shfl_sync(FULL_MASK, top.e, t);
+      const float nk = entry_key(next);
+      if (!(nk > row.thresh)) break;  // the list is sorted: the rest of it is behind the bar too
+      row.insert(nk, position_of(r, entry_place(next)), l, k);
+    }
+  }
+  return row.pos;
 }
 
 // (The exponential-jump form of the sampler -- keys only for the edges that enter, a
@@ -716,49 +923,13 @@ __device__ __forceinline__ void ares_next_window(ShareList& top, float& entry, c
 // 10-32 and rows of 10^3-10^4 edges an entry costs ~250 instructions at a rate of k/n
 // per edge, and the kernel ran 1.6-2.3x slower than with per-edge keys, so it is not used.)
 
-// How a row is dealt out: share r of (at most) eight takes windows r, r + 8, ...  Within a share places ascend, and
-// shares are joined in order, so equal keys (zero weights, equal weights) keep one fixed order: by position up to
-// eight windows, by share and then position above.
-__device__ __forceinline__ int row_shares(int64_t deg) {
-  const int64_t windows = (deg + ARES_EDGES - 1) / ARES_EDGES;
-  return windows < WEIGHTED_WARPS ? static_cast<int>(windows) : WEIGHTED_WARPS;
-}
-// position in the row of a place (512 per window) in share r
-__device__ __forceinline__ int64_t position_of(int r, uint32_t place) {
-  return static_cast<int64_t>(place & ~(ARES_EDGES - 1u)) * WEIGHTED_WARPS + r * ARES_EDGES + (place & (ARES_EDGES - 1u));
-}
-
-// What is left of one share of a row after the row's window 0, into shared memory.  `bar` (shared by the row's shares,
-// ordered form) is the best k-th key any of them holds: whatever is below it cannot be among the row's top k.
-__device__ __forceinline__ void ares_share(const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo, uint32_t i_hi,
-                                           int r, int l, int k, int* bar, float* list_key, uint32_t* list_place) {
-  const float NEG_INF = __int_as_float(0xff800000);
-  // share 0 goes on from the list of window 0; the others start empty, with the row's bar to beat
-  ShareList top{r == 0 ? list_key[l] : NEG_INF, r == 0 ? list_place[l] : 0u, NEG_INF};
-  top.thresh = __shfl_sync(FULL_MASK, top.key, k - 1);
-  float entry = top.thresh;
-  for (uint32_t place = r == 0 ? ARES_EDGES : 0;; place += ARES_EDGES) {
-    const int64_t base = position_of(r, place);
-    if (base >= deg) break;
-    const int mine = ordered_float(top.thresh);
-    const int best = __shfl_sync(FULL_MASK, *static_cast<volatile int*>(bar), 0);  // one value for the warp
-    if (mine > best) {
-      if (l == 0) atomicMax(bar, mine);
-    } else {
-      entry = fmaxf(entry, key_below(float_of_ordered(best)));  // a key equal to it may still win by its place
-    }
-    ares_next_window(top, entry, W, base, place, deg, key, i_lo, i_hi, l, k);
-  }
-  list_key[l] = top.key;
-  list_place[l] = top.pos;
-}
-
-// A-Res without replacement.  Bound by issue slots (164 warp instructions per 32 edges of rows of 380) and the latency of the list
-// operations, not by the bytes of the weights.  Eight seeds per CTA of eight warps: each warp takes the first 512
-// edges of its own row, which gives the row a bar to beat; what is left of the CTA's longer rows is dealt out to its
-// warps in shares, and one warp per row joins them.  11 000 rows, 9.1 M weights, fan-out 10: 89 us, against 188 us
-// when a warp kept its row up to 4096 edges and inserted every key by itself.  (Four CTAs per SM at 64 registers
-// measured the same as three at 72.)
+// A-Res without replacement.  Bound by issue slots (8 200 warp instructions a row of 4 096 edges) and the CTA's barriers,
+// not by the bytes of the weights.  Eight seeds per CTA of eight warps.  Each warp takes the first 512 edges of its own row, which gives the row a list and a bar to beat; then, in
+// rounds, the windows behind them are dealt out to the CTA's warps, which only collect the edges that may beat the bar,
+// and each row's own warp joins what was collected with the list: one sort and one merge a round, where a list per share
+// of the row, kept sorted by its warp and joined entry by entry, took 12 300 instructions for such a row.
+// 11 000 rows of a hub-heavy graph (9.1 M weights), whole calls: fan-out 10 91 -> 73.5 us, fan-out 25 149 -> 102; 2 000 rows,
+// fan-out 15 29 -> 21.4; 400 rows, fan-out 10 22.8 -> 16.4.  (Four CTAs per SM at 64 registers: level.)
 template <typename IdT>
 __global__ void __launch_bounds__(SAMPLE_BLOCK, 3)
 sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
@@ -773,77 +944,140 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
   const Emit<IdT> emit{indices, coo_row, coo_col, picked_pos, out_capacity, status, marks, nc};
   pdl_enter();
   if (run_side_job<IdT>(jobs)) return;
-  const uint64_t key = key_of(rng) ^ (static_cast<uint64_t>(TAG_ARES) << 32);
+  const uint64_t key = uniform_word(key_of(rng) ^ (static_cast<uint64_t>(TAG_ARES) << 32));
   const int64_t n = count_of(nc);
   const int l = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int kk = static_cast<int>(k);
-  const float NEG_INF = __int_as_float(0xff800000);
-  __shared__ int s_shares[WEIGHTED_WARPS];  // of each warp's seed; 0: nothing to sample
-  __shared__ int s_bar[WEIGHTED_WARPS];
-  __shared__ int64_t s_rb[WEIGHTED_WARPS], s_deg[WEIGHTED_WARPS];
-  __shared__ float s_key[WEIGHTED_WARPS][WEIGHTED_WARPS][32];       // [row][share][rank]
-  __shared__ uint32_t s_place[WEIGHTED_WARPS][WEIGHTED_WARPS][32];
-  __shared__ float s_pack_key[WEIGHTED_WARPS][32];
-  __shared__ uint16_t s_pack_at[WEIGHTED_WARPS][32];
+  // how a row's room is divided in a round: with the bar of 512 edges a window has about k survivors, give or take
+  // sqrt(2k)
+  const int room = kk <= 10 ? 32 : 64, windows_a_round = Survivors::ROOM / room;
+  enum : int { NOTHING, WHOLE, LIST, ALONE };  // how a warp's row is sampled; ALONE: by the warp, behind everything else
+  __shared__ int s_how[WEIGHTED_WARPS];
+  __shared__ float s_bar[WEIGHTED_WARPS];
+  __shared__ int64_t s_rb[WEIGHTED_WARPS], s_deg[WEIGHTED_WARPS], s_off[WEIGHTED_WARPS], s_seed[WEIGHTED_WARPS];
+  __shared__ int64_t s_left[WEIGHTED_WARPS];  // s_deg where there are windows to scan, else 0
+  __shared__ int s_count[WEIGHTED_WARPS][ARES_SHARES];
+  __shared__ __align__(16) Scratch s_scratch[WEIGHTED_WARPS];
 
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * WEIGHTED_WARPS;
-  SeedPlan sp{0, 0, 0};
-  int64_t seed = 0, pick = -1;  // lane l emits the edge at `pick` as the seed's l-th
-  int my_shares = 0;
-  if (i0 + warp < n) {
-    sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
-    seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
-    if (marks.seeds && l == 0) mark_id(marks, seed, static_cast<uint32_t>(i0 + warp), status);
-    if (sp.deg <= k) {
-      if (l < sp.deg) pick = l;
-    } else if (sp.rb + sp.deg > probs.total || sp.deg >> 35 != 0) {  // places within a share fit 32 bits below 2^35
-      if (l == 0) raise_status(status, DGS_ERR_RANGE);
-    } else {
-      my_shares = row_shares(sp.deg);
-      const uint64_t i = static_cast<uint64_t>(i0 + warp);
-      ShareList top{NEG_INF, 0, NEG_INF};
-      ares_first_window(top, row_weights(probs, sp.rb, sp.deg), sp.deg, key, static_cast<uint32_t>(i),
-                        static_cast<uint32_t>(i >> 32), l, kk, s_pack_key[warp], s_pack_at[warp]);
-      s_key[warp][0][l] = top.key;
-      s_place[warp][0][l] = top.pos;
-      if (l == 0) s_bar[warp] = ordered_float(top.thresh);
+  ShareList top{NO_ENTRY, __int_as_float(0xff800000)};
+  {
+    SeedPlan sp{0, 0, 0};
+    int64_t seed = 0;
+    int how = NOTHING;
+    if (i0 + warp < n) {
+      sp = seed_plan(plan_rb, plan_deg, local_off, tile_off, i0 + warp, true);
+      seed = row_is_position ? i0 + warp : static_cast<int64_t>(seeds[i0 + warp]);
+      if (marks.seeds && l == 0) mark_id(marks, seed, static_cast<uint32_t>(i0 + warp), status);
+      if (sp.deg <= k) {
+        how = WHOLE;
+      } else if (sp.rb + sp.deg > probs.total || sp.deg >> 35 != 0) {  // places within a share fit 32 bits below 2^35
+        if (l == 0) raise_status(status, DGS_ERR_RANGE);
+      } else if (sp.deg >> 32 != 0) {
+        how = ALONE;
+      } else {
+        how = LIST;
+        const uint32_t i_lo = static_cast<uint32_t>(i0 + warp), i_hi = static_cast<uint32_t>((i0 + warp) >> 32);
+        const RowWeights W = row_weights(probs, sp.rb, sp.deg);
+        Survivors& s = s_scratch[warp].survivors;
+        if (kk <= ARES_PACK_K) {
+          if (!ares_first_window(top, W, sp.deg, key, i_lo, i_hi, l, kk, reinterpret_cast<Entry*>(s.word_weight))) how = ALONE;
+        } else {
+          float w[4];
+          W.load(w, 0, sp.deg, l);
+          ares_first_group(top, w, sp.deg, key, i_lo, i_hi, l, kk);
+        }
+        if (kk > ARES_PACK_K && sp.deg > ARES_GROUP) {
+          // what is above the bar: of equal keys the earlier ones, which are in the list, win
+          const int have = ares_collect<1>(W, sp.deg, 0, key, i_lo, i_hi, l, filter_bar(top.thresh), s, 0, Survivors::ROOM);
+          if (have > Survivors::ROOM) how = ALONE;
+          else ares_join(top, s, l == 0 ? have : 0, Survivors::ROOM, 0, sp.deg, l, kk);
+        }
+      }
+    }
+    if (l == 0) {
+      s_how[warp] = how;
+      s_rb[warp] = sp.rb;
+      s_deg[warp] = sp.deg;
+      s_off[warp] = sp.o;
+      s_seed[warp] = seed;
+      s_left[warp] = how == LIST && sp.deg > ARES_EDGES ? sp.deg : 0;
+      s_bar[warp] = top.thresh;
     }
   }
-  if (l == 0) {
-    s_shares[warp] = my_shares;
-    s_rb[warp] = sp.rb;
-    s_deg[warp] = sp.deg;
-  }
   __syncthreads();
-  int task = 0;
+  for (int64_t w0 = 1;; w0 += windows_a_round) {
+    // lane r: the windows of row r in this round, and how many tasks the rows up to it make
+    const int64_t rest = (l < WEIGHTED_WARPS ? s_left[l] : 0) - w0 * ARES_EDGES;
+    const int windows = rest <= 0                               ? 0
+                        : rest >= windows_a_round * ARES_EDGES ? windows_a_round
+                                                                : (static_cast<int>(rest) + ARES_EDGES - 1) / ARES_EDGES;
+    if (__ballot_sync(FULL_MASK, windows > 0) == 0u) break;  // the same for all warps
+    int upto = windows;
+#pragma unroll
+    for (int o = 1; o < WEIGHTED_WARPS; o <<= 1) {
+      const int t = __shfl_up_sync(FULL_MASK, upto, o);
+      if (l >= o) upto += t;
+    }
+    const int tasks = __shfl_sync(FULL_MASK, upto, WEIGHTED_WARPS - 1);
 #pragma unroll 1
-  for (int row = 0; row < WEIGHTED_WARPS; ++row) {
-    if (s_shares[row] == 0) continue;
-    const int64_t deg = s_deg[row];
-    const int from = deg > ARES_EDGES * WEIGHTED_WARPS ? 0 : 1;  // share 0 of up to eight windows is done
-    const int shares = s_shares[row] - from;
-    const int r = from + ((warp - task) & (WEIGHTED_WARPS - 1));  // this warp's share of the row, if it has so many
-    task += shares;
-    if (r >= shares + from) continue;
-    const uint64_t i = static_cast<uint64_t>(i0 + row);
-    ares_share(row_weights(probs, s_rb[row], deg), deg, key, static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), r,
-               l, kk, &s_bar[row], s_key[row][r], s_place[row][r]);
-  }
-  __syncthreads();
-  if (my_shares > 0) {
-    TopK<int64_t> top{s_key[warp][0][l], position_of(0, s_place[warp][0][l]), NEG_INF};
-    top.thresh = __shfl_sync(FULL_MASK, top.key, kk - 1);
-#pragma unroll 1
-    for (int r = 1; r < my_shares; ++r)
-      for (int t = 0; t < kk; ++t) {
-        const float nk = s_key[warp][r][t];  // same address for all lanes: broadcast
-        if (!(nk > top.thresh)) break;       // every list is sorted: the rest of this one is behind the bar too
-        top.insert(nk, position_of(r, s_place[warp][r][t]), l, kk);
+    for (int t = warp; t < tasks; t += WEIGHTED_WARPS) {
+      const int row = __popc(__ballot_sync(FULL_MASK, l < WEIGHTED_WARPS && upto <= t));
+      const int b = t - __shfl_sync(FULL_MASK, upto - windows, row);
+      const int64_t deg = s_deg[row];
+      const uint64_t ri = static_cast<uint64_t>(i0 + row);
+      // a key equal to the bar may still win: its share may come before the one that holds the bar
+      const int have = ares_collect<0>(row_weights(probs, s_rb[row], deg), deg, (w0 + b) * ARES_EDGES, key,
+                                       static_cast<uint32_t>(ri), static_cast<uint32_t>(ri >> 32), l,
+                                       filter_bar(key_below(s_bar[row])), s_scratch[row].survivors, b * room, room);
+      if (l == 0) s_count[row][b] = have;
+    }
+    __syncthreads();
+    const int mine = __shfl_sync(FULL_MASK, windows, warp);
+    if (mine > 0) {
+      const int count = l < mine ? s_count[warp][l] : 0;
+      Survivors& s = s_scratch[warp].survivors;
+      const int64_t deg = s_deg[warp];
+      unsigned over = __ballot_sync(FULL_MASK, count > room);
+      ares_join(top, s, count > room ? 0 : count, room, w0, deg, l, kk);
+      // windows that had more survivors than room once more, with the bar that there is now and all of the room
+      bool lost = false;
+      for (; over != 0u; over &= over - 1) {
+        const int b = __ffs(over) - 1;
+        const uint64_t i = static_cast<uint64_t>(i0 + warp);
+        __syncwarp();
+        const int have = ares_collect<0>(row_weights(probs, s_rb[warp], deg), deg, (w0 + b) * ARES_EDGES, key,
+                                         static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), l,
+                                         filter_bar(key_below(top.thresh)), s, 0, Survivors::ROOM);
+        lost = lost || have > Survivors::ROOM;
+        if (!lost) ares_join(top, s, l == 0 ? have : 0, Survivors::ROOM, w0 + b, deg, l, kk);
       }
-    if (l < k) pick = top.pos;
+      __syncwarp();
+      if (l == 0) {
+        s_bar[warp] = top.thresh;
+        if (lost) {
+          s_how[warp] = ALONE;
+          s_left[warp] = 0;
+        }
+      }
+    }
+    __syncthreads();
   }
-  if (pick >= 0) emit(sp.o, l, seed, sp.rb, pick);
+  const int how = s_how[warp];
+  if (how == NOTHING) return;
+  int64_t pick = -1;  // lane l emits the edge at `pick` as the seed's l-th
+  if (how == WHOLE) {
+    if (l < s_deg[warp]) pick = l;
+  } else if (how == LIST) {
+    if (l < k) pick = tag_position(entry_place(top.e));
+  } else {
+    const uint64_t i = static_cast<uint64_t>(i0 + warp);
+    const int64_t at = ares_row(&probs, s_rb[warp], s_deg[warp], key, static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), l,
+                                kk, s_scratch[warp].pending);
+    if (l < k) pick = at;
+  }
+  if (pick >= 0) emit(s_off[warp], l, s_seed[warp], s_rb[warp], pick);
 }
 
 // ---- proportional draws with replacement --------------------------------------
