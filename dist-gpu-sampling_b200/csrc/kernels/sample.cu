@@ -891,6 +891,8 @@ __device__ __noinline__ void ares_scan(ShareList& top, const RowWeights& W, int6
         c = make_entry(ares_key(x.x, __uint_as_float(x.y)), pend.place[have + l]);
       }
       __syncwarp();
+      // (rows of mostly zero weights: all pass the filter, none of them this)
+      if (!__any_sync(FULL_MASK, c > __shfl_sync(FULL_MASK, top.e, k - 1))) continue;
       top.merge(c, l, k);
       bar = filter_bar(fmaxf(above, top.thresh));
     }
