@@ -925,7 +925,7 @@ __device__ __noinline__ int64_t ares_row(const dgs_chunk_desc* probs, int64_t rb
 // 10-32 and rows of 10^3-10^4 edges an entry costs ~250 instructions at a rate of k/n
 // per edge, and the kernel ran 1.6-2.3x slower than with per-edge keys, so it is not used.)
 
-// A-Res without replacement.  Bound by issue slots (8 200 warp instructions a row of 4 096 edges) and the CTA's barriers,
+// A-Res without replacement.  Bound by issue slots (8 400 warp instructions a row of 4 096 edges) and the CTA's barriers,
 // not by the bytes of the weights.  Eight seeds per CTA of eight warps.  Each warp takes the first 512 edges of its own row, which gives the row a list and a bar to beat; then, in
 // rounds, the windows behind them are dealt out to the CTA's warps, which only collect the edges that may beat the bar,
 // and each row's own warp joins what was collected with the list: one sort and one merge a round, where a list per share
