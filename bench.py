@@ -74,13 +74,19 @@ WORKLOADS = {
 # kernels of this library launched per operator call (memsets and copies are not kernels)
 LAUNCHES_RELABEL = 3     # insert, number (+ look-back), lookup
 LAUNCHES_GATHER = 1
-LAUNCHES_HOP_FUSED = 3   # sample (+ table clear + previous hop's lookup), insert, number (+ the next hop's plan)
 LAUNCHES_LAST_LOOKUP = 1
 
 
-def launches_plan(seeds):
-    """One CTA up to 2 048 seeds; above, a clearing launch and a CTA per 256 seeds."""
-    return 1 if seeds <= 2048 else 2
+def launches_hop_fused(nodes):
+    """A hop of the queued sequence.  Up to 2^23 nodes: sample (marks one word per id), number (+ the next hop's plan);
+    above: sample (+ table clear + previous hop's lookup), insert, number (+ the next hop's plan)."""
+    return 2 if nodes <= 1 << 23 else 3
+
+
+def launches_plan(seeds, operator=False):
+    """One CTA up to 2 048 seeds, in an operator call one cluster up to 8 192; above, a clearing launch and a CTA per 256
+    seeds."""
+    return 1 if seeds <= (8192 if operator else 2048) else 2
 
 
 PRIME_STEPS = 8          # untimed one-at-a-time steps that populate torch's caching allocator
@@ -919,10 +925,10 @@ def main_ours(args):
             return {"api": label, "value": rate(r, name), "unit": "edges/s", "ms_per_step": r[name]["ms"] / steps}
         main = args.api
         others = [entry(red, n, args.steps) for n in ("pipeline", "blocks", "per-hop") if n != main]
-        fused = launches_plan(args.batch) + H * LAUNCHES_HOP_FUSED + LAUNCHES_LAST_LOOKUP + LAUNCHES_GATHER
+        fused = launches_plan(args.batch) + H * launches_hop_fused(w["nodes"]) + LAUNCHES_LAST_LOOKUP + LAUNCHES_GATHER
         per_hop, seeds_bound = LAUNCHES_GATHER, args.batch
         for k in reversed(fanouts):  # operator by operator; the later hops' seeds by their bound
-            per_hop += launches_plan(seeds_bound) + 1 + LAUNCHES_RELABEL
+            per_hop += launches_plan(seeds_bound, operator=True) + 1 + LAUNCHES_RELABEL
             seeds_bound *= 1 + k
         launches_step = {"pipeline": fused, "blocks": fused, "per-hop": per_hop}[main]
         bl = red["blocks"]
