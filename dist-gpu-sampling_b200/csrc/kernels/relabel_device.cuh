@@ -57,7 +57,9 @@ struct TableParts {
   unsigned long long* tiles2;   // [ntiles]  the same of the edges that the distinct keys will be given
   long long* wide_keys;         // [n]       by label: keys of 2^32 and more (64-bit ids only)
   uint32_t* slot_of;            // [n]       slot of every input
+  unsigned long long* largest;  // [ntiles] where the largest key is looked at: those that the clearing CTAs have met
   int64_t* total;               // [1]
+  int64_t* dense;               // [1]       and whether the words are addressed by the key
   int64_t ntiles;
 };
 
