@@ -72,7 +72,6 @@ WORKLOADS = {
 }
 
 # kernels of this library launched per operator call (memsets and copies are not kernels)
-LAUNCHES_RELABEL = 3     # insert, number (+ look-back), lookup
 LAUNCHES_GATHER = 1
 LAUNCHES_LAST_LOOKUP = 1
 
@@ -81,6 +80,11 @@ def launches_hop_fused(nodes):
     """A hop of the queued sequence.  Up to 2^23 nodes: sample (marks one word per id), number (+ the next hop's plan);
     above: sample (+ table clear + previous hop's lookup), insert, number (+ the next hop's plan)."""
     return 2 if nodes <= 1 << 23 else 3
+
+
+def launches_relabel(keys):
+    """insert, number (+ look-back), lookup; from 2^19 to 2^21 keys a clearing launch that looks for the largest."""
+    return 4 if 1 << 19 <= keys < 1 << 21 else 3
 
 
 def launches_plan(seeds, operator=False):
@@ -928,7 +932,7 @@ def main_ours(args):
         fused = launches_plan(args.batch) + H * launches_hop_fused(w["nodes"]) + LAUNCHES_LAST_LOOKUP + LAUNCHES_GATHER
         per_hop, seeds_bound = LAUNCHES_GATHER, args.batch
         for k in reversed(fanouts):  # operator by operator; the later hops' seeds by their bound
-            per_hop += launches_plan(seeds_bound, operator=True) + 1 + LAUNCHES_RELABEL
+            per_hop += launches_plan(seeds_bound, operator=True) + 1 + launches_relabel(seeds_bound * (1 + k))
             seeds_bound *= 1 + k
         launches_step = {"pipeline": fused, "blocks": fused, "per-hop": per_hop}[main]
         bl = red["blocks"]
