@@ -31,6 +31,7 @@ ABI_SOURCES = [
 ]
 HEADERS = [
     "kernels/common.cuh",
+    "kernels/host_report.cuh",
     "kernels/philox.cuh",
     "kernels/tile_scan.cuh",
     "kernels/launchers.h",

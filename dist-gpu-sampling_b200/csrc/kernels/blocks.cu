@@ -126,6 +126,7 @@ struct DenseSpace {
   unsigned int* ticket[DGS_MAX_HOPS];
   unsigned long long* tiles[DGS_MAX_HOPS];
   uint32_t* first;
+  uint32_t* beyond;           // a word beside the first hop's ticket
   FillJob fill;               // tickets, tile words and words of the ids
   size_t bytes;
 };
@@ -156,6 +157,7 @@ DenseSpace dense_space(const dgs_hop* hops, int32_t n_hops, int64_t ids, void* w
     d.tiles[h] = reinterpret_cast<unsigned long long*>(base + at + 16);
     at += 16 + 16 * static_cast<size_t>(dense_tiles(hops[h].seed_bound, hops[h].seed_bound * hops[h].fanout));
   }
+  d.beyond = d.ticket[0] + 1;
   d.first = reinterpret_cast<uint32_t*>(base + at);
   at += (static_cast<size_t>(ids) * sizeof(uint32_t) + 15) / 16 * 16;
   d.fill.at = reinterpret_cast<ulonglong2*>(base + cleared);
@@ -193,7 +195,7 @@ int queue_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, con
     const RngKey key = rng_words != nullptr
                            ? RngKey{0, d.keys + h}
                            : host_key(sample_rng_key(rng_seed, rng_offset + static_cast<uint64_t>(h)));
-    const IdMarks marks{d.first, id_space, !later};
+    const IdMarks marks{d.first, id_space, !later, d.beyond};
     rc = probs != nullptr
              ? launch_sample_weighted(*indices, *probs, hop_seeds, ids64, n, k, replace, d.plan[h], later, key, hp.coo_row,
                                       hp.coo_col, edge_bound, nullptr, later, SideJobs{}, marks, status, s)
@@ -206,7 +208,7 @@ int queue_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, con
     NextPlan next{};
     if (h + 1 < n_hops) next = make_next_plan(*indptr, hops[h + 1].seed_bound, hops[h + 1].fanout, replace, d.plan[h + 1]);
     else report.n = 2 * n_hops;  // the last hop's numbering sends all sizes to the host at once
-    const DenseNumbering number{d.first, id_space, d.ticket[h], d.tiles[h], d.totals + h, later};
+    const DenseNumbering number{d.first, id_space, d.ticket[h], d.beyond, d.tiles[h], d.totals + h, later};
     rc = launch_dense_number(ids64, number, hop_seeds, n, hp.coo_col, nnz, hp.frontier, hp.frontier_bound, report, next,
                              status, s);
     if (rc != DGS_OK) return rc;

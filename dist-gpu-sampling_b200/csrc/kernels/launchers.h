@@ -82,6 +82,7 @@ struct DenseNumbering {
   uint32_t* first;
   int64_t ids;
   unsigned int* ticket;       // [4]  cleared with the table
+  const uint32_t* beyond;     // IdMarks::beyond
   unsigned long long* tiles;  // [2 * dense_tiles(bounds)], cleared with the table
   int64_t* total;
   bool seeds_known;

@@ -23,6 +23,7 @@
 //     bounds of the nodes it numbers and places their outputs: the next hop's plan.
 //   * the number of distinct keys goes to a caller-supplied (pinned) word.
 #include "common.cuh"
+#include "host_report.cuh"
 #include "launchers.h"
 #include "relabel_device.cuh"
 #include "sample_device.cuh"
@@ -362,10 +363,7 @@ relabel_number_kernel(const __grid_constant__ Keys keys, const TableParts t, IdT
       *n_unique_out = before + total;
       __threadfence_system();
     }
-    if (report.n > 0) {  // the same thread that wrote *t.total just above
-      for (int k = 0; k < report.n; ++k) report.dst[k] = *report.src[k];
-      __threadfence_system();
-    }
+    if (report.n > 0) report_sizes(report.dst, report.src, report.n, 0, status);  // the same thread that wrote *t.total
   }
   int64_t label = before + ex;
   int64_t id[RL_ITEMS];
@@ -436,6 +434,7 @@ dense_number_kernel(const DenseNumbering d, const IdT* __restrict__ seeds, const
   pdl_enter();
   if (threadIdx.x == 0) s_tile = atomicAdd(d.ticket, 1u) + 1u;
   const int64_t n_seeds = count_of(na), n_cols = count_of(nb);
+  const bool beyond = report.n > 0 && threadIdx.x == 0 && *static_cast<const volatile uint32_t*>(d.beyond) != NOT_MET;
   __syncthreads();
   const int64_t tile = s_tile;
   const int64_t seed_tiles = (n_seeds + RL_TILE - 1) / RL_TILE, tiles = seed_tiles + (n_cols + RL_TILE - 1) / RL_TILE;
@@ -480,10 +479,8 @@ dense_number_kernel(const DenseNumbering d, const IdT* __restrict__ seeds, const
   }
   if (last_tile && threadIdx.x == 0) {
     *d.total = before + total;
-    if (report.n > 0) {  // the same thread that wrote *d.total just above
-      for (int k = 0; k < report.n; ++k) report.dst[k] = *report.src[k];
-      __threadfence_system();
-    }
+    // the same thread that wrote *d.total just above
+    if (report.n > 0) report_sizes(report.dst, report.src, report.n, beyond ? DGS_ERR_ID_SPACE : 0, status);
   }
   int64_t label[RL_ITEMS];
   int64_t next = before + ex;

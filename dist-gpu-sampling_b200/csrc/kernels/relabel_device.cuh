@@ -85,6 +85,7 @@ struct IdMarks {
   uint32_t* first;
   int64_t ids;  // words of the table
   bool seeds;   // the seeds are inputs too (first hop; from the second on they are labelled already)
+  uint32_t* beyond;  // cleared with the table; anything but NOT_MET: an id at or beyond `ids` was met
 };
 
 // What relabels the COO of all hops of a sequence through that table, in one launch.
@@ -128,7 +129,8 @@ __device__ __forceinline__ void min_kept(uint32_t* p, uint32_t v, uint64_t polic
 }
 __device__ __forceinline__ void mark_id(const IdMarks& m, int64_t id, uint32_t input, int32_t* status) {
   if (static_cast<uint64_t>(id) < static_cast<uint64_t>(m.ids)) min_kept(m.first + id, input, l2_evict_last_policy());
-  else raise_status(status, id < 0 ? DGS_ERR_RANGE : DGS_ERR_ID_SPACE);
+  else if (id < 0) raise_status(status, DGS_ERR_RANGE);
+  else *static_cast<volatile uint32_t*>(m.beyond) = 0u;  // reported with the sizes
 }
 
 __device__ __forceinline__ void run_fill_cta(const FillJob& j, unsigned cta) {
