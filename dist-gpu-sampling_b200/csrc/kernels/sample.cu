@@ -602,6 +602,7 @@ __device__ __forceinline__ float float_of_ordered(int i) { return __int_as_float
 
 constexpr float FLOOR_ZERO_W = -3.402823466e+38f;  // key of a weight <= 0: behind every positive weight
 constexpr float FLOOR_POS_W = -3.0e+38f;           // clamp for positive weights
+constexpr float LEAST_POS_W = -3.2e+38f;           // between the two
 
 __device__ __forceinline__ float ares_key(uint32_t word, float w) {
   float ck = fmaxf(__fdividef(__logf(unit_float(word)), w), FLOOR_POS_W);
@@ -624,29 +625,22 @@ __device__ __forceinline__ Philox4 ares_words(uint64_t key, uint32_t i_lo, uint3
 
 constexpr int ARES_EDGES = 512;  // edges per window
 constexpr int ARES_GROUP = 128;  // edges per step: four per lane, one Philox block
-constexpr int ARES_PACK_K = 20;  // fan-outs for which the k-th largest of 32 lane maxima leaves fewer than 32 candidates
 
 // Edges that passed the filter below and whose keys are still to be computed: of a row's windows of one round, a stretch
-// of `room` entries each, with their offsets in the window.
+// of `room` entries each, with their offsets in the stretch.
 struct Survivors {
   static constexpr int ROOM = 256;
   uint2 word_weight[ROOM];
   uint16_t at[ROOM];
-};
-// The same of one warp that scans a row by itself.
-struct Pending {
-  static constexpr int ROOM = 31 + ARES_GROUP;
-  uint2 word_weight[ROOM];
-  uint32_t place[ROOM];
-};
-union Scratch {  // of a row: one or the other
-  Survivors survivors;
-  Pending pending;
+  __device__ __forceinline__ Entry* entries() { return reinterpret_cast<Entry*>(word_weight); }
 };
 
-// The first 512 edges of a row, for k well below 32: every lane computes its 16 keys; the k-th largest of the 32 lane
-// maxima is a bar that at least k keys reach and few more than k (expected -32 ln(1 - k/32) of them: 12 at k = 10, 22
-// at k = 16), so those are packed into one per lane and sorted once.  False: more than 32 are at the bar (ties).
+// The first 512 edges of a row: every lane computes its 16 keys; the k-th largest of the 32 lane maxima is a bar that at
+// least k keys reach and not many more (expected -32 ln(1 - k/32) of them: 12 at k = 10, 22 at k = 16, 31 at k = 20, 49 at
+// k = 25, 130 at k = 32), so those are packed and sorted 32 at a time.
+// With fewer than k lanes that have a positive weight the bar is the key of zero weights.  Of those only the ones among the
+// first 32 edges count, which with the positive ones are k already.  False: more reach the bar than there is room for
+// (keys that are equal).
 __device__ __forceinline__ bool ares_first_window(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo,
                                                   uint32_t i_hi, int l, int k, Entry* pack) {
   constexpr int ITEMS = ARES_EDGES / 32;
@@ -675,39 +669,32 @@ __device__ __forceinline__ bool ares_first_window(ShareList& top, const RowWeigh
     return true;
   }
   const float bar = kth_of_32(best, l, k);
+  const float rest = fmaxf(bar, LEAST_POS_W);  // what the edges behind the first 32 have to reach
   int have = 0;
 #pragma unroll
   for (int q = 0; q < ITEMS / 4; ++q) {
     if (q * ARES_GROUP >= deg) break;  // warp-uniform
 #pragma unroll
     for (int j = 4 * q; j < 4 * q + 4; ++j) {
-      const bool in = ck[j] >= bar && ck[j] > NEG_INF;
+      const bool in = ck[j] >= (j == 0 ? bar : rest);
       const unsigned m = __ballot_sync(FULL_MASK, in);
       const int at = have + __popc(m & ((1u << l) - 1u));
-      if (in && at < 32) pack[at] = make_entry(ck[j], j * 32 + l);
+      if (in && at < Survivors::ROOM) pack[at] = make_entry(ck[j], j * 32 + l);
       have += __popc(m);
     }
   }
   __syncwarp();
-  top.set(sort32(l < have ? pack[l] : NO_ENTRY), k);
-  __syncwarp();  // the room is used again
-  return have <= 32;
-}
-
-// The first 128 edges of a row, for larger k: keys computed for all of them (w: the lane's four weights), the four quarters
-// merged one by one.
-__device__ __forceinline__ void ares_first_group(ShareList& top, const float (&w)[4], int64_t deg, uint64_t key, uint32_t i_lo,
-                                                 uint32_t i_hi, int l, int k) {
-  const float NEG_INF = __int_as_float(0xff800000);
-  const Philox4 r = ares_words(key, i_lo, i_hi, 0, l);
-  const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+  const bool fits = have <= Survivors::ROOM;
+  if (fits) {
+    top.set(sort32(l < have ? pack[l] : NO_ENTRY), k);
 #pragma unroll 1
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t word = j == 0 ? rw[0] : j == 1 ? rw[1] : j == 2 ? rw[2] : rw[3];
-    const float weight = j == 0 ? w[0] : j == 1 ? w[1] : j == 2 ? w[2] : w[3];
-    const float ck = j * 32 + l < deg ? ares_key(word, weight) : NEG_INF;
-    if (__any_sync(FULL_MASK, ck > top.thresh)) top.merge(ck > top.thresh ? make_entry(ck, j * 32 + l) : NO_ENTRY, l, k);
+    for (int i0 = 32; i0 < have; i0 += 32) {
+      const Entry e = i0 + l < have ? pack[i0 + l] : NO_ENTRY;
+      if (__any_sync(FULL_MASK, entry_key(e) > top.thresh)) top.merge(e, l, k);  // of equal keys the earlier win
+    }
   }
+  __syncwarp();  // the room is used again
+  return fits;
 }
 
 // The order of equal keys (zero weights, equal weights): window w of 512 edges belongs to share w % 8; equal keys are
@@ -727,44 +714,45 @@ __device__ __forceinline__ int64_t tag_position(uint32_t tag) { return position_
 // edges that a bound lets through: log(u) <= u - 1, so an edge whose u - 1 <= bar * w cannot beat the bar.  The test is
 // that inequality with the slack that the errors of __logf (2^-21.4 absolute on [0.5, 2]), __fdividef (2 ulp) and of the 23
 // random bits it looks at need, so every edge that the exact key lets in passes, and the exact key decides.  A bar above
-// -1e-30 is taken as -1e-30 (weights so large that __fdividef gives 0 then always pass); at or below the clamp of positive
-// weights the inequality says nothing about keys that were clamped, and every edge passes; so do products that are no
-// number (0 * inf: a weight <= 0 then).
+// -2.5e-38 is taken as that: keys nearer to zero than 2^-126 may come out as zero, those of weights from 2^126 on do.  (With
+// -1e-30 in its place a row of weights around 1e32 passed as a whole.)  At or below the clamp of positive weights the
+// inequality says nothing about keys that were clamped, and every positive weight passes.  Weights <= 0 (or no number) do
+// not: a list that is full has had them from the row's first edges, which come before all others of that key.  (For a
+// list that is not full yet: `zeros`.)
 constexpr float ARES_PASS = 2.0f - 0x1p-18f;
 __device__ __forceinline__ float filter_bar(float above) {  // for keys above `above`
-  return above <= FLOOR_POS_W ? __int_as_float(0xff800000) : fminf(above * 1.00001f, -1e-30f);
+  return above <= FLOOR_POS_W ? __int_as_float(0xff800000) : fminf(above * 1.00001f, -2.5e-38f);
 }
 __device__ __forceinline__ bool may_beat(float bar, uint32_t word, float w) {
-  return !(__uint_as_float((word >> 9) | 0x3f800000u) <= fmaf(bar, fmaxf(w, 0.f), ARES_PASS));
+  return __uint_as_float((word >> 9) | 0x3f800000u) > fmaf(bar, fmaxf(w, 0.f), ARES_PASS);  // not above NaN: -inf * 0
 }
 
-// The edges of a window (from its group FIRST on; `base`: its first edge) that may beat `bar`, into s[from, from + room);
-// their number, which may exceed the room: what has none is dropped.  (Past the row's end weights are 0; what passes
-// there is left out when the keys are computed.)
-template <int FIRST>
+// The edges of a window (`base`: its first edge) that may beat `bar`, behind the `have` that are in s[from, from + room)
+// already, their offsets counted from `off`; their number, which may exceed the room: what has none is dropped.  (Past the
+// row's end weights are 0; what passes there is left out when the keys are computed.)
 __device__ __forceinline__ int ares_collect(const RowWeights& W, int64_t deg, int64_t base, uint64_t key, uint32_t i_lo,
-                                            uint32_t i_hi, int l, float bar, Survivors& s, int from, int room) {
-  float w[(4 - FIRST) * 4];
-  W.load(w, base + FIRST * ARES_GROUP, deg, l);
+                                            uint32_t i_hi, int l, float bar, Survivors& s, int from, int room, int have,
+                                            int off) {
+  float w[16];
+  W.load(w, base, deg, l);
   const uint64_t ctr = static_cast<uint64_t>(base >> 2);  // the low seven bits are clear
   const uint32_t c_lo = static_cast<uint32_t>(ctr) | l, c_hi = static_cast<uint32_t>(ctr >> 32);
-  int have = 0;
 #pragma unroll
-  for (int q = FIRST; q < 4; ++q) {
+  for (int q = 0; q < 4; ++q) {
     if (base + q * ARES_GROUP >= deg) break;  // warp-uniform
     const Philox4 rnd = philox4x32_10(key, i_lo, i_hi, c_lo + q * 32, c_hi);
     const uint32_t rw[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
     bool pass[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) pass[j] = may_beat(bar, rw[j], w[(q - FIRST) * 4 + j]);
+    for (int j = 0; j < 4; ++j) pass[j] = may_beat(bar, rw[j], w[q * 4 + j]);
     if (!__any_sync(FULL_MASK, pass[0] || pass[1] || pass[2] || pass[3])) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const unsigned m = __ballot_sync(FULL_MASK, pass[j]);
       const int at = have + __popc(m & ((1u << l) - 1u));
       if (pass[j] && at < room) {
-        s.word_weight[from + at] = make_uint2(rw[j], __float_as_uint(w[(q - FIRST) * 4 + j]));
-        s.at[from + at] = static_cast<uint16_t>(q * ARES_GROUP + j * 32 + l);
+        s.word_weight[from + at] = make_uint2(rw[j], __float_as_uint(w[q * 4 + j]));
+        s.at[from + at] = static_cast<uint16_t>(off + q * ARES_GROUP + j * 32 + l);
       }
       have += __popc(m);
     }
@@ -772,12 +760,57 @@ __device__ __forceinline__ int ares_collect(const RowWeights& W, int64_t deg, in
   return have;
 }
 
-// Joins a row's list with what its windows w0, w0 + 1, ... have collected: stretch b of `room` entries holds as many
-// as lane b says.
+// A list, and the edges [lo, hi) of one window: the best of both, whatever the weights are.  For what ares_collect has no room
+// for.  Keys above `above` that may enter are put aside (waiting[63]), and whenever 32 are waiting they are sorted and merged.
+// place0: of edge lo.
+__device__ __noinline__ Entry ares_window(Entry list, const dgs_chunk_desc* probs, int64_t rb, int64_t deg, int64_t lo, int64_t hi,
+                                          uint64_t key, uint32_t i_lo, uint32_t i_hi, uint32_t place0, float above, bool zeros,
+                                          int l, int k, Entry* waiting) {
+  const RowWeights W = row_weights(*probs, rb, deg);
+  ShareList top;
+  top.set(list, k);
+  float bar = filter_bar(fmaxf(above, key_below(top.thresh)));
+  int have = 0;
+#pragma unroll 1
+  for (int64_t e0 = lo; e0 < hi && e0 < deg; e0 += ARES_GROUP) {
+    float w[4];
+    W.load(w, e0, deg, l);
+    const Philox4 r = ares_words(key, i_lo, i_hi, e0, l);
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t word = j == 0 ? r.x : j == 1 ? r.y : j == 2 ? r.z : r.w;
+      const float weight = j == 0 ? w[0] : j == 1 ? w[1] : j == 2 ? w[2] : w[3];
+      const bool pass = e0 + j * 32 + l < deg && (may_beat(bar, word, weight) || (zeros && bar == __int_as_float(0xff800000)));
+      if (!__any_sync(FULL_MASK, pass)) continue;
+      const float ck = ares_key(word, weight);
+      const Entry e = make_entry(ck, place0 + static_cast<uint32_t>(e0 - lo) + j * 32 + l);
+      const Entry last = __shfl_sync(FULL_MASK, top.e, k - 1);
+      const bool in = pass && ck > above && e > last;
+      const unsigned m = __ballot_sync(FULL_MASK, in);
+      if (in) waiting[have + __popc(m & ((1u << l) - 1u))] = e;
+      have += __popc(m);
+      if (have < 32) continue;
+      __syncwarp();
+      const Entry one = waiting[l], two = l + 32 < have ? waiting[l + 32] : NO_ENTRY;
+      __syncwarp();
+      if (l + 32 < have) waiting[l] = two;
+      have -= 32;
+      top.merge(one, l, k);
+      bar = filter_bar(fmaxf(above, key_below(top.thresh)));
+    }
+  }
+  __syncwarp();
+  if (have > 0) top.merge(l < have ? waiting[l] : NO_ENTRY, l, k);
+  __syncwarp();
+  return top.e;
+}
+
+// Joins a row's list with what its windows from w0 on have collected: stretch b, of `room` entries and `windows` windows, holds
+// as many as lane b says.
 // With more than 32 the k-th largest of the lanes' best keys is a bar that few more than k reach (for k well below 32),
 // so that one sort and one merge do.
-__device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int count, int room, int64_t w0, int64_t deg, int l,
-                                          int k) {
+__device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int count, int room, int64_t w0, int windows, int64_t deg,
+                                          int l, int k) {
   int upto = count;  // entries of the stretches up to this lane's
 #pragma unroll
   for (int o = 1; o < ARES_SHARES; o <<= 1) {
@@ -800,7 +833,7 @@ __device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int coun
     *stretch = b;
     return b * room + i - before;
   };
-  Entry* out = reinterpret_cast<Entry*>(s.word_weight);
+  Entry* out = s.entries();
   Entry first = NO_ENTRY, best = NO_ENTRY;
   __syncwarp();
 #pragma unroll 1
@@ -811,7 +844,9 @@ __device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int coun
     if (i0 + l < total) {
       const uint2 x = s.word_weight[slot];
       const uint32_t off = s.at[slot];
-      if ((w0 + b) * ARES_EDGES + off < deg) e = make_entry(ares_key(x.x, __uint_as_float(x.y)), window_tag(w0 + b) + off);
+      const int64_t w = w0 + b * windows + off / ARES_EDGES;
+      if (w * ARES_EDGES + off % ARES_EDGES < deg)
+        e = make_entry(ares_key(x.x, __uint_as_float(x.y)), window_tag(w) + off % ARES_EDGES);
       out[slot] = e;
       best = e > best ? e : best;
     }
@@ -822,7 +857,7 @@ __device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int coun
     return;
   }
   float bar = top.thresh;
-  if (k <= ARES_PACK_K) bar = fmaxf(bar, kth_of_32(entry_key(best), l, k));
+  bar = fmaxf(bar, kth_of_32(entry_key(best), l, k));
   __syncwarp();
   // those that reach the bar, 32 at a time.  Packed in place: what is written lies in front of what is still to be read
   int have = 0;
@@ -852,72 +887,138 @@ __device__ __forceinline__ void ares_join(ShareList& top, Survivors& s, int coun
   }
 }
 
-// Share r of a row by one warp, 128 edges at a time, for rows whose survivors found no room (more than a few equal keys at
-// the bar) or whose tags do not fit 32 bits.  What passes is put aside, and whenever 32 are waiting their keys are
-// computed, sorted and merged.  `above`: only keys above it are of interest.
-__device__ __noinline__ void ares_scan(ShareList& top, const RowWeights& W, int64_t deg, uint64_t key, uint32_t i_lo,
-                                       uint32_t i_hi, int r, float above, int l, int k, Pending& pend) {
-  int have = 0;
-  top.set(NO_ENTRY, k);
-  float bar = filter_bar(above);
-  bool more = position_of(r, 0) < deg;
+// A row's list with its windows [first, last), which had more survivors than room: once more, window by window, with the bar that
+// there is now and all of the row's room.
+__device__ __forceinline__ Entry ares_again(Entry list, const dgs_chunk_desc* probs, int64_t rb, int64_t deg, int64_t first, int64_t last,
+                                         uint64_t key, uint32_t i_lo, uint32_t i_hi, int l, int k, Survivors* s) {
+  ShareList top;
+  top.set(list, k);
 #pragma unroll 1
-  for (uint32_t place = 0; more;) {
-    const int64_t e0 = position_of(r, place);
-    float w[4];
-    W.load(w, e0, deg, l);
-    const Philox4 rnd = ares_words(key, i_lo, i_hi, e0, l);
-    const uint32_t rw[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const bool pass = may_beat(bar, rw[j], w[j]) && e0 + j * 32 + l < deg;
-      const unsigned m = __ballot_sync(FULL_MASK, pass);
-      if (pass) {
-        const int at = have + __popc(m & ((1u << l) - 1u));
-        pend.word_weight[at] = make_uint2(rw[j], __float_as_uint(w[j]));
-        pend.place[at] = place + j * 32 + l;
-      }
-      have += __popc(m);
-    }
-    place += ARES_GROUP;
-    more = place != 0 && position_of(r, place) < deg;  // 0: past 2^32 places
-    while (have >= 32 || (!more && have > 0)) {
-      const int take = have < 32 ? have : 32;
-      have -= take;
+  for (int64_t w = first; w < last && w * ARES_EDGES < deg; ++w) {
+    const float above = key_below(top.thresh);
+    __syncwarp();
+    const int have = ares_collect(row_weights(*probs, rb, deg), deg, w * ARES_EDGES, key, i_lo, i_hi, l, filter_bar(above), *s, 0,
+                                  Survivors::ROOM, 0, 0);
+    if (have <= Survivors::ROOM) {
+      ares_join(top, *s, l == 0 ? have : 0, Survivors::ROOM, w, 1, deg, l, k);
+    } else {
       __syncwarp();
-      Entry c = NO_ENTRY;
-      if (l < take) {
-        const uint2 x = pend.word_weight[have + l];
-        c = make_entry(ares_key(x.x, __uint_as_float(x.y)), pend.place[have + l]);
-      }
-      __syncwarp();
-      // (rows of mostly zero weights: all pass the filter, none of them this)
-      if (!__any_sync(FULL_MASK, c > __shfl_sync(FULL_MASK, top.e, k - 1))) continue;
-      top.merge(c, l, k);
-      bar = filter_bar(fmaxf(above, top.thresh));
+      top.set(ares_window(top.e, probs, rb, deg, w * ARES_EDGES, (w + 1) * ARES_EDGES, key, i_lo, i_hi, window_tag(w), above, false, l,
+                          k, s->entries()), k);
     }
   }
+  return top.e;
 }
 
-// A whole row that way: its shares in order; lane t's position of rank t.
+// A whole row by one warp, share after share, for rows whose tags do not fit 32 bits; lane t's position of rank t.
 __device__ __noinline__ int64_t ares_row(const dgs_chunk_desc* probs, int64_t rb, int64_t deg, uint64_t key, uint32_t i_lo,
-                                         uint32_t i_hi, int l, int k, Pending& pend) {
-  const float NEG_INF = __int_as_float(0xff800000);
-  const RowWeights W = row_weights(*probs, rb, deg);
-  RowList row{NEG_INF, 0, NEG_INF};
+                                         uint32_t i_hi, int l, int k, Entry* waiting) {
+  RowList row{__int_as_float(0xff800000), 0, __int_as_float(0xff800000)};
 #pragma unroll 1
   for (int r = 0; r < ARES_SHARES; ++r) {
-    ShareList top;
-    ares_scan(top, W, deg, key, i_lo, i_hi, r, row.thresh, l, k, pend);
+    uint32_t place = 0;
 #pragma unroll 1
-    for (int t = 0; t < k; ++t) {
-      const Entry next = __shfl_sync(FULL_MASK, top.e, t);
-      const float nk = entry_key(next);
-      if (!(nk > row.thresh)) break;  // the list is sorted: the rest of it is behind the bar too
-      row.insert(nk, position_of(r, entry_place(next)), l, k);
-    }
+    do {
+      const int64_t lo = position_of(r, place);
+      if (lo >= deg) break;
+      const Entry list = ares_window(NO_ENTRY, probs, rb, deg, lo, lo + ARES_EDGES, key, i_lo, i_hi, 0u, row.thresh, lo == 0, l, k,
+                                     waiting);
+#pragma unroll 1
+      for (int t = 0; t < k; ++t) {
+        const Entry next = __shfl_sync(FULL_MASK, list, t);
+        if (!(entry_key(next) > row.thresh)) break;  // the list is sorted: the rest of it is behind the bar too
+        row.insert(entry_key(next), lo + entry_place(next), l, k);
+      }
+      place += ARES_EDGES;
+    } while (place != 0);  // 0: past 2^32 places
   }
   return row.pos;
+}
+
+// What the warps of a CTA share of its eight rows.
+struct AresRows {
+  int how[WEIGHTED_WARPS];
+  float bar[WEIGHTED_WARPS];
+  int64_t rb[WEIGHTED_WARPS], deg[WEIGHTED_WARPS], off[WEIGHTED_WARPS], seed[WEIGHTED_WARPS];
+  int64_t left[WEIGHTED_WARPS];  // deg where there are windows to scan, else 0
+  int count[WEIGHTED_WARPS][ARES_SHARES];
+  __align__(16) Survivors scratch[WEIGHTED_WARPS];
+};
+
+// One round: the windows from w0 on of all rows, in stretches of up to `most` (1 unless LONG), of which a row has room for so
+// many, are dealt out to the warps, which only collect the edges that may beat the row's bar; each row's own warp joins what was
+// collected with its list.  False: no row has windows left.  *crowded: some stretch took more than half of its room (LONG).
+template <bool LONG>
+__device__ __forceinline__ bool ares_round(AresRows& c, ShareList& top, const dgs_chunk_desc& probs, uint64_t key, int64_t i0, int l,
+                                           int warp, int k, int64_t w0, int room, int most, bool* crowded) {
+  const int stretches = Survivors::ROOM / room;
+  // lane r: the stretches of row r in this round, their windows, and how many tasks the rows up to it make
+  const int64_t rest = (l < WEIGHTED_WARPS ? c.left[l] : 0) - w0 * ARES_EDGES;
+  const int left = rest <= 0 ? 0 : static_cast<int>((rest + ARES_EDGES - 1) / ARES_EDGES);
+  if (__ballot_sync(FULL_MASK, left > 0) == 0u) return false;  // the same for all warps
+  const int even = (left + stretches - 1) / stretches, windows = !LONG || even < 1 ? 1 : even < most ? even : most;
+  const int parts = LONG ? (left + windows - 1) / windows : left;
+  int upto = parts < stretches ? parts : stretches;
+#pragma unroll
+  for (int o = 1; o < WEIGHTED_WARPS; o <<= 1) {
+    const int t = __shfl_up_sync(FULL_MASK, upto, o);
+    if (l >= o) upto += t;
+  }
+  const int tasks = __shfl_sync(FULL_MASK, upto, WEIGHTED_WARPS - 1);
+  bool dense = false;
+#pragma unroll 1
+  for (int t = warp; t < tasks; t += WEIGHTED_WARPS) {
+    const int row = __popc(__ballot_sync(FULL_MASK, l < WEIGHTED_WARPS && upto <= t));
+    const int b = t - (row > 0 ? __shfl_sync(FULL_MASK, upto, row - 1) : 0);  // row: the same in all lanes
+    const int count = LONG ? __shfl_sync(FULL_MASK, windows, row) : 1;
+    const int64_t deg = c.deg[row], first = w0 + static_cast<int64_t>(b) * count;
+    // a key equal to the bar may still win: its share may come before the one that holds the bar
+    const float bar = filter_bar(key_below(c.bar[row]));
+    int have = 0;
+#pragma unroll 1
+    for (int w = 0; w < count && (!LONG || (first + w) * ARES_EDGES < deg); ++w)
+      have = ares_collect(row_weights(probs, c.rb[row], deg), deg, (first + w) * ARES_EDGES, key, static_cast<uint32_t>(i0 + row),
+                          static_cast<uint32_t>((i0 + row) >> 32), l, bar, c.scratch[row], b * room, room, have, w * ARES_EDGES);
+    dense = dense || have > room / 2;
+    if (l == 0) c.count[row][b] = have;
+  }
+  if (LONG) *crowded = __syncthreads_or(dense);
+  else __syncthreads();
+  const int own = __shfl_sync(FULL_MASK, upto, warp) - (warp > 0 ? __shfl_sync(FULL_MASK, upto, warp - 1) : 0);
+  const int own_windows = LONG ? __shfl_sync(FULL_MASK, windows, warp) : 1;
+  if (own > 0) {
+    const int count = l < own ? c.count[warp][l] : 0;
+    ares_join(top, c.scratch[warp], count > room ? 0 : count, room, w0, own_windows, c.deg[warp], l, k);
+    for (unsigned again = __ballot_sync(FULL_MASK, count > room); again != 0u; again &= again - 1) {
+      const int64_t first = w0 + static_cast<int64_t>(__ffs(again) - 1) * own_windows;
+      top.set(ares_again(top.e, &probs, c.rb[warp], c.deg[warp], first, first + own_windows, key, static_cast<uint32_t>(i0 + warp),
+                         static_cast<uint32_t>((i0 + warp) >> 32), l, k, &c.scratch[warp]), k);
+    }
+    if (l == 0) c.bar[warp] = top.thresh;
+  }
+  __syncthreads();
+  return true;
+}
+
+// The rounds from window ARES_SHORT on.  A window has about k / w survivors of the bar of w windows, so that those of eight
+// stretches of w / 8 windows are few beside the room; the rounds double, and a row of 10^5 edges takes 8 of them instead of 24.
+// Where a stretch takes more than half of its room -- weights that rise along the row -- they stay half as long from there on.
+// One such row alone in its CTA, whole calls, fan-out 10 and 25: 73.9 and 127 us with eight (four) windows a round throughout,
+// 56 and 61 now; 64 of them 297 and 352 -> 273 and 280.  Out of line, and not before window 33: rows of a hub-heavy graph are
+// shorter and paid for it (11 000 rows, fan-out 10: 60.8 without, 62.6 from window 17 on, 60.5 from 33 on, 61.0 from 65 on).
+constexpr int ARES_SHORT = 33;
+__device__ __noinline__ Entry ares_long_rounds(Entry list, AresRows* c, const dgs_chunk_desc* probs, uint64_t key, int64_t i0, int l,
+                                               int warp, int k, int64_t w0) {
+  ShareList top;
+  top.set(list, k);
+  constexpr int room = 32;
+  bool crowded = false;
+  for (int most = 2, cap = 64; ares_round<true>(*c, top, *probs, key, i0, l, warp, k, w0, room, most, &crowded);) {
+    w0 += Survivors::ROOM / room * most;
+    if (!crowded) most = min(min(2 * most, static_cast<int>(w0 >> 3)), cap);
+    else if (most > 1) cap = most >>= 1;
+  }
+  return top.e;
 }
 
 // (The exponential-jump form of the sampler -- keys only for the edges that enter, a
@@ -925,13 +1026,14 @@ __device__ __noinline__ int64_t ares_row(const dgs_chunk_desc* probs, int64_t rb
 // 10-32 and rows of 10^3-10^4 edges an entry costs ~250 instructions at a rate of k/n
 // per edge, and the kernel ran 1.6-2.3x slower than with per-edge keys, so it is not used.)
 
-// A-Res without replacement.  Bound by issue slots (8 400 warp instructions a row of 4 096 edges) and the CTA's barriers,
-// not by the bytes of the weights.  Eight seeds per CTA of eight warps.  Each warp takes the first 512 edges of its own row, which gives the row a list and a bar to beat; then, in
-// rounds, the windows behind them are dealt out to the CTA's warps, which only collect the edges that may beat the bar,
-// and each row's own warp joins what was collected with the list: one sort and one merge a round, where a list per share
-// of the row, kept sorted by its warp and joined entry by entry, took 12 300 instructions for such a row.
-// 11 000 rows of a hub-heavy graph (9.1 M weights), whole calls: fan-out 10 91 -> 73.5 us, fan-out 25 149 -> 102; 2 000 rows,
-// fan-out 15 29 -> 21.4; 400 rows, fan-out 10 22.8 -> 16.4.  (Four CTAs per SM at 64 registers: level.)
+// A-Res without replacement.  Bound by issue slots and the CTA's barriers, not by the bytes of the weights.  Eight seeds per CTA
+// of eight warps.  Each warp takes the first 512 edges of its own row, which gives the row a list and a bar to beat; then, in
+// rounds, the windows behind them are dealt out to the CTA's warps, which only collect the edges that may beat the bar, and each
+// row's own warp joins what was collected with the list: one sort and one merge a round.
+// 11 000 rows of a hub-heavy graph (9.1 M weights), whole calls, a list per share of the row kept by its warp -> this:
+// fan-out 10 69.6 -> 60.6, 20 90.9 -> 69, 25 109 -> 70.6; 2 000 rows, fan-out 15 57.5 -> 33.9; 2 000 rows of 4 096 edges, fan-out 10
+// 61.4 -> 37.5.  Rows of which few weights are positive are as fast: one in a hundred, fan-out 10, 94.7 -> 61.  (Four CTAs per
+// SM at 64 registers: level; two at 128: 66.7 for 60.6.)
 template <typename IdT>
 __global__ void __launch_bounds__(SAMPLE_BLOCK, 3)
 sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
@@ -951,16 +1053,8 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
   const int l = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int kk = static_cast<int>(k);
-  // how a row's room is divided in a round: with the bar of 512 edges a window has about k survivors, give or take
-  // sqrt(2k)
-  const int room = kk <= 10 ? 32 : 64, windows_a_round = Survivors::ROOM / room;
   enum : int { NOTHING, WHOLE, LIST, ALONE };  // how a warp's row is sampled; ALONE: by the warp, behind everything else
-  __shared__ int s_how[WEIGHTED_WARPS];
-  __shared__ float s_bar[WEIGHTED_WARPS];
-  __shared__ int64_t s_rb[WEIGHTED_WARPS], s_deg[WEIGHTED_WARPS], s_off[WEIGHTED_WARPS], s_seed[WEIGHTED_WARPS];
-  __shared__ int64_t s_left[WEIGHTED_WARPS];  // s_deg where there are windows to scan, else 0
-  __shared__ int s_count[WEIGHTED_WARPS][ARES_SHARES];
-  __shared__ __align__(16) Scratch s_scratch[WEIGHTED_WARPS];
+  __shared__ AresRows c;
 
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * WEIGHTED_WARPS;
   ShareList top{NO_ENTRY, __int_as_float(0xff800000)};
@@ -982,104 +1076,46 @@ sample_weighted_kernel(const __grid_constant__ dgs_chunk_desc indices,
         how = LIST;
         const uint32_t i_lo = static_cast<uint32_t>(i0 + warp), i_hi = static_cast<uint32_t>((i0 + warp) >> 32);
         const RowWeights W = row_weights(probs, sp.rb, sp.deg);
-        Survivors& s = s_scratch[warp].survivors;
-        if (kk <= ARES_PACK_K) {
-          if (!ares_first_window(top, W, sp.deg, key, i_lo, i_hi, l, kk, reinterpret_cast<Entry*>(s.word_weight))) how = ALONE;
-        } else {
-          float w[4];
-          W.load(w, 0, sp.deg, l);
-          ares_first_group(top, w, sp.deg, key, i_lo, i_hi, l, kk);
-        }
-        if (kk > ARES_PACK_K && sp.deg > ARES_GROUP) {
-          // what is above the bar: of equal keys the earlier ones, which are in the list, win
-          const int have = ares_collect<1>(W, sp.deg, 0, key, i_lo, i_hi, l, filter_bar(top.thresh), s, 0, Survivors::ROOM);
-          if (have > Survivors::ROOM) how = ALONE;
-          else ares_join(top, s, l == 0 ? have : 0, Survivors::ROOM, 0, sp.deg, l, kk);
-        }
+        Survivors& s = c.scratch[warp];
+        if (!ares_first_window(top, W, sp.deg, key, i_lo, i_hi, l, kk, s.entries()))
+          top.set(ares_window(NO_ENTRY, &probs, sp.rb, sp.deg, 0, ARES_EDGES, key, i_lo, i_hi, 0u, __int_as_float(0xff800000), true,
+                              l, kk, s.entries()), kk);
       }
     }
     if (l == 0) {
-      s_how[warp] = how;
-      s_rb[warp] = sp.rb;
-      s_deg[warp] = sp.deg;
-      s_off[warp] = sp.o;
-      s_seed[warp] = seed;
-      s_left[warp] = how == LIST && sp.deg > ARES_EDGES ? sp.deg : 0;
-      s_bar[warp] = top.thresh;
+      c.how[warp] = how;
+      c.rb[warp] = sp.rb;
+      c.deg[warp] = sp.deg;
+      c.off[warp] = sp.o;
+      c.seed[warp] = seed;
+      c.left[warp] = how == LIST && sp.deg > ARES_EDGES ? sp.deg : 0;
+      c.bar[warp] = top.thresh;
     }
   }
   __syncthreads();
-  for (int64_t w0 = 1;; w0 += windows_a_round) {
-    // lane r: the windows of row r in this round, and how many tasks the rows up to it make
-    const int64_t rest = (l < WEIGHTED_WARPS ? s_left[l] : 0) - w0 * ARES_EDGES;
-    const int windows = rest <= 0                               ? 0
-                        : rest >= windows_a_round * ARES_EDGES ? windows_a_round
-                                                                : (static_cast<int>(rest) + ARES_EDGES - 1) / ARES_EDGES;
-    if (__ballot_sync(FULL_MASK, windows > 0) == 0u) break;  // the same for all warps
-    int upto = windows;
-#pragma unroll
-    for (int o = 1; o < WEIGHTED_WARPS; o <<= 1) {
-      const int t = __shfl_up_sync(FULL_MASK, upto, o);
-      if (l >= o) upto += t;
-    }
-    const int tasks = __shfl_sync(FULL_MASK, upto, WEIGHTED_WARPS - 1);
-#pragma unroll 1
-    for (int t = warp; t < tasks; t += WEIGHTED_WARPS) {
-      const int row = __popc(__ballot_sync(FULL_MASK, l < WEIGHTED_WARPS && upto <= t));
-      const int b = t - __shfl_sync(FULL_MASK, upto - windows, row);
-      const int64_t deg = s_deg[row];
-      const uint64_t ri = static_cast<uint64_t>(i0 + row);
-      // a key equal to the bar may still win: its share may come before the one that holds the bar
-      const int have = ares_collect<0>(row_weights(probs, s_rb[row], deg), deg, (w0 + b) * ARES_EDGES, key,
-                                       static_cast<uint32_t>(ri), static_cast<uint32_t>(ri >> 32), l,
-                                       filter_bar(key_below(s_bar[row])), s_scratch[row].survivors, b * room, room);
-      if (l == 0) s_count[row][b] = have;
-    }
-    __syncthreads();
-    const int mine = __shfl_sync(FULL_MASK, windows, warp);
-    if (mine > 0) {
-      const int count = l < mine ? s_count[warp][l] : 0;
-      Survivors& s = s_scratch[warp].survivors;
-      const int64_t deg = s_deg[warp];
-      unsigned over = __ballot_sync(FULL_MASK, count > room);
-      ares_join(top, s, count > room ? 0 : count, room, w0, deg, l, kk);
-      // windows that had more survivors than room once more, with the bar that there is now and all of the room
-      bool lost = false;
-      for (; over != 0u; over &= over - 1) {
-        const int b = __ffs(over) - 1;
-        const uint64_t i = static_cast<uint64_t>(i0 + warp);
-        __syncwarp();
-        const int have = ares_collect<0>(row_weights(probs, s_rb[warp], deg), deg, (w0 + b) * ARES_EDGES, key,
-                                         static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), l,
-                                         filter_bar(key_below(top.thresh)), s, 0, Survivors::ROOM);
-        lost = lost || have > Survivors::ROOM;
-        if (!lost) ares_join(top, s, l == 0 ? have : 0, Survivors::ROOM, w0 + b, deg, l, kk);
-      }
-      __syncwarp();
-      if (l == 0) {
-        s_bar[warp] = top.thresh;
-        if (lost) {
-          s_how[warp] = ALONE;
-          s_left[warp] = 0;
-        }
-      }
-    }
-    __syncthreads();
+  // with the bar of one window a window has about k survivors, give or take sqrt(2k)
+  int64_t w0 = 1;
+  bool more = true;
+  while (more && w0 < ARES_SHORT) {
+    const int room = w0 == 1 && kk > 10 ? 64 : 32;
+    more = ares_round<false>(c, top, probs, key, i0, l, warp, kk, w0, room, 1, nullptr);
+    w0 += Survivors::ROOM / room;
   }
-  const int how = s_how[warp];
+  if (more) top.set(ares_long_rounds(top.e, &c, &probs, key, i0, l, warp, kk, w0), kk);
+  const int how = c.how[warp];
   if (how == NOTHING) return;
   int64_t pick = -1;  // lane l emits the edge at `pick` as the seed's l-th
   if (how == WHOLE) {
-    if (l < s_deg[warp]) pick = l;
+    if (l < c.deg[warp]) pick = l;
   } else if (how == LIST) {
     if (l < k) pick = tag_position(entry_place(top.e));
   } else {
     const uint64_t i = static_cast<uint64_t>(i0 + warp);
-    const int64_t at = ares_row(&probs, s_rb[warp], s_deg[warp], key, static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), l,
-                                kk, s_scratch[warp].pending);
+    const int64_t at = ares_row(&probs, c.rb[warp], c.deg[warp], key, static_cast<uint32_t>(i), static_cast<uint32_t>(i >> 32), l,
+                                kk, c.scratch[warp].entries());
     if (l < k) pick = at;
   }
-  if (pick >= 0) emit(s_off[warp], l, s_seed[warp], s_rb[warp], pick);
+  if (pick >= 0) emit(c.off[warp], l, c.seed[warp], c.rb[warp], pick);
 }
 
 // ---- proportional draws with replacement --------------------------------------
