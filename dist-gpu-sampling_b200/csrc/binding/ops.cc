@@ -307,10 +307,13 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
   cudaStream_t stream = current_stream();
   const Lease w("_CAPI_sample_blocks*", seeds.device().index(), stream);
   const auto rng = next_rng(static_cast<uint64_t>(H));
-  // one word per id of indptr's node space where that is the faster form (bytes bounded like the hash tables above)
+  // One word per id of indptr's node space where that is the faster form: at most 2^23 words, so that what a small batch
+  // allocates is up to 34 MB and a large one less than with the hash tables that the budget above counts.  Not for one hop:
+  // its column ids may well lie beyond indptr's nodes (a bipartite CSC), which would cost the batch twice on every call
+  // (1 024 seeds 50 -> 80 us); a hop with another one behind it cannot draw such ids.
   const int64_t id_space = indptr.total - 1;
   size_t dense_bytes = 0;
-  if (dgs_sample_blocks_dense_wins(hops, H, id_space)) dense_bytes = dgs_sample_blocks_dense_workspace_bytes(hops, H, id_space);
+  if (H > 1 && dgs_sample_blocks_dense_wins(hops, H, id_space)) dense_bytes = dgs_sample_blocks_dense_workspace_bytes(hops, H, id_space);
   torch::Tensor ws = byte_scratch(dense_bytes > 0 ? dense_bytes : ws_bytes, seeds.device());
   std::vector<torch::Tensor> fr(H);
   for (int h = 0; h < H; ++h) {
@@ -340,7 +343,7 @@ BlocksResult blocks_impl(torch::Tensor seeds, const dgs_chunk_desc& indptr, torc
                                          rng.first, rng.second, ws.data_ptr(), dense_bytes, w.sizes(), w.status(), stream));
     read_sizes();
     if (*static_cast<volatile int32_t*>(w.status()) == DGS_ERR_ID_SPACE) {
-      // column ids beyond indptr's nodes (a bipartite CSC): the same batch again through the form that takes any id
+      // the last hop met column ids beyond indptr's nodes: the same batch again through the form that takes any id
       sync_stream();
       *w.status() = 0;
       for (int h = 0; h < 2 * H; ++h) w.sizes()[h] = kPending;
