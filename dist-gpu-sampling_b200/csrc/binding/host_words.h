@@ -38,7 +38,10 @@ constexpr int kWordsPerLease = 24;       // int64 sizes per lease (>= 2 * DGS_MA
 static_assert(2 * DGS_MAX_HOPS + 4 <= kWordsPerLease, "a lease must hold the sizes of a sample_blocks call");
 
 inline const char* status_text(int32_t st) {
-  return st == DGS_ERR_RANGE ? "an out-of-range id" : (st == DGS_ERR_TABLE_FULL ? "a full hash table" : "an error");
+  return st == DGS_ERR_RANGE        ? "an out-of-range id"
+         : st == DGS_ERR_TABLE_FULL ? "a full hash table"
+         : st == DGS_ERR_ID_SPACE   ? "an id beyond the id space"
+                                    : "an error";
 }
 
 inline bool strict_status() {

@@ -31,6 +31,15 @@ int main() {
 """
 
 
+TEXTS = r"""
+#include <cstdio>
+#include "binding/host_words.h"
+int main() {
+  for (int code : {DGS_ERR_INVALID, DGS_ERR_RANGE, DGS_ERR_TABLE_FULL, DGS_ERR_ID_SPACE}) std::puts(dgs::status_text(code));
+}
+"""
+
+
 def compiled(tmp_path, text, *flags):
     src, exe = tmp_path / "t.cc", tmp_path / "t"
     src.write_text(text)
@@ -43,3 +52,9 @@ def test_an_error_that_decides_is_at_the_host_before_the_sizes_are(tmp_path, cod
     seen = compiled(tmp_path, ORDER.replace("CODE", str(code)))
     assert seen[-1] == f"end {code} 5 6"
     assert seen[0] == ("fence 9 -1 -1" if code else "fence 0 5 6")
+
+
+def test_every_status_that_kernels_raise_has_words(tmp_path):
+    from torch.utils import cpp_extension
+    flags = [f for p in cpp_extension.include_paths() + ["/usr/local/cuda/include"] for f in ("-isystem", p)]
+    assert compiled(tmp_path, TEXTS, *flags) == ["an error", "an out-of-range id", "a full hash table", "an id beyond the id space"]
