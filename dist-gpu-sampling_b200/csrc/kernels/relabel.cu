@@ -141,12 +141,18 @@ relabel_insert_kernel(const __grid_constant__ Keys keys, const TableSize size, u
 // number of 32-bit words that the slots have, the words serve as one per id, addressed by the key (see IdMarks), and
 // nothing is hashed, probed or remembered per input.  Which it is shows on the device: the pass that clears the table
 // reads the keys too.  One hop of 60 000 seeds and fan-out 15, sampled and relabelled: 105.8 -> 94.7 us.
-// Unique and lookup, us, without -> with the look; keys that the words can address, then larger ones: 180 k 26.5 -> 19.6 and
-// 28 -> 31, 360 k 39 -> 27 and 41 -> 45, 880 k 63.8 -> 43.1 and 74 -> 75.5, 3 M 180 -> 141 and 218 -> 233.  Hence the range: below,
-// a graph is seldom small enough to make up for the others, above it the look costs them too much.
+// Relabel calls, us, without -> with the look; keys that the words can address / too large and half of them distinct / too
+// large and all distinct: 524 k 55 -> 42.5 / 49 -> 49 / 62 -> 61, 600 k 50 -> 37 / 42.7 -> 45.2 / 56 -> 55, 880 k 63 -> 43 / 54.7 -> 54.3 /
+// 74 -> 72, 1.2 M 84 -> 62 / 75.6 -> 76.2 / 95 -> 93, 1.6 M 110 -> 76 / 90.9 -> 91.3 / 118 -> 117, 2.09 M 139 -> 97 / 114 -> 117.5 / 157 -> 158.
+// Unique and lookup by themselves outside the range, with the look as it was at first: 180 k 26.5 -> 19.6 and 28 -> 31, 360 k
+// 39 -> 27 and 41 -> 45, 3 M 180 -> 141 and 218 -> 233.  Hence the range: below, a graph is seldom small enough to make up for
+// the others, above it the look costs them too much.
 constexpr int64_t LOOK_MIN_KEYS = 1ll << 19, LOOK_MAX_KEYS = 1ll << 21;
 inline bool looks_at_largest(int64_t n) { return n >= LOOK_MIN_KEYS && n < LOOK_MAX_KEYS; }
-constexpr int LARGEST = RL_BLOCK;  // CTAs that read the keys; fewer than the range has tiles
+// CTAs that read the keys; no more than the range has tiles.  (With half as many, and the stores behind the reads, keys that are
+// too large paid 2 us more from 1.6 M on.)
+constexpr int LARGEST = 2 * RL_BLOCK;
+static_assert(LARGEST <= LOOK_MIN_KEYS / RL_TILE, "a word per tile is their room");
 
 template <typename IdT>
 __global__ void __launch_bounds__(RL_BLOCK)
@@ -154,25 +160,22 @@ relabel_clear_kernel(const __grid_constant__ SegKeys keys, ulonglong2* __restric
                      unsigned long long* __restrict__ largest) {
   __shared__ unsigned long long s_max[RL_BLOCK / 32];
   pdl_enter();
-  const bool reads = blockIdx.x < LARGEST;
-  unsigned long long most = 0;
-  if (reads) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * RL_TILE + threadIdx.x; i < keys.n; i += static_cast<int64_t>(LARGEST) * RL_TILE) {
-      unsigned long long k[RL_ITEMS];
-#pragma unroll
-      for (int u = 0; u < RL_ITEMS; ++u)
-        k[u] = i + u * RL_BLOCK < keys.n
-                   ? static_cast<unsigned long long>(static_cast<long long>(keys.template load<IdT>(i + u * RL_BLOCK)))
-                   : 0ull;
-#pragma unroll
-      for (int u = 0; u < RL_ITEMS; ++u) most = k[u] > most ? k[u] : most;  // a negative key is larger than any id
-    }
-  }
   const ulonglong2 ones = make_ulonglong2(~0ull, ~0ull);
 #pragma unroll 4
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * RL_BLOCK + threadIdx.x; i < n_units; i += static_cast<int64_t>(gridDim.x) * RL_BLOCK)
     units[i] = ones;
-  if (!reads) return;
+  if (blockIdx.x >= LARGEST) return;
+  unsigned long long most = 0;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * RL_TILE + threadIdx.x; i < keys.n; i += static_cast<int64_t>(LARGEST) * RL_TILE) {
+    unsigned long long k[RL_ITEMS];
+#pragma unroll
+    for (int u = 0; u < RL_ITEMS; ++u)
+      k[u] = i + u * RL_BLOCK < keys.n
+                 ? static_cast<unsigned long long>(static_cast<long long>(keys.template load<IdT>(i + u * RL_BLOCK)))
+                 : 0ull;
+#pragma unroll
+    for (int u = 0; u < RL_ITEMS; ++u) most = k[u] > most ? k[u] : most;  // a negative key is larger than any id
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long other = __shfl_xor_sync(FULL_MASK, most, o);
@@ -194,7 +197,9 @@ relabel_mark_kernel(const __grid_constant__ SegKeys keys, const TableSize size, 
   pdl_enter();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * RL_BLOCK + threadIdx.x;
   const long long key = i < keys.n ? static_cast<long long>(keys.template load<IdT>(i)) : 0;
-  const bool dense = !__syncthreads_or(t.largest[threadIdx.x] >= 2 * table_slots(size));
+  const uint64_t words = 2 * table_slots(size);
+  static_assert(LARGEST == 2 * RL_BLOCK, "two words a thread");
+  const bool dense = !__syncthreads_or(t.largest[threadIdx.x] >= words || t.largest[threadIdx.x + RL_BLOCK] >= words);
   if (i == 0) *t.dense = dense;
   if (i >= keys.n) return;
   if (dense) atomicMin(reinterpret_cast<uint32_t*>(t.words) + key, static_cast<uint32_t>(i));
@@ -299,7 +304,7 @@ int run_unique_any(const SegKeys& keys, const TableParts& t, void* unique_out, i
   const TableSize size{exact_count(keys.n), 1, INT64_MAX};
   // slots, ticket and tile words lie one behind the other
   const int64_t units = static_cast<int64_t>(slots_for(keys.n) / 2) + ticket_units(t);
-  DGS_CUDA_TRY(launch_chained(SITE_INIT, relabel_clear_kernel<IdT>, 4u * LARGEST, RL_BLOCK, s, keys,
+  DGS_CUDA_TRY(launch_chained(SITE_INIT, relabel_clear_kernel<IdT>, 2u * LARGEST, RL_BLOCK, s, keys,
                               reinterpret_cast<ulonglong2*>(t.words), units, t.largest));
   DGS_CUDA_TRY(launch_chained(SITE_INSERT, relabel_mark_kernel<IdT>, static_cast<unsigned>((keys.n + RL_BLOCK - 1) / RL_BLOCK),
                               RL_BLOCK, s, keys, size, t, status));
