@@ -136,7 +136,11 @@ static_assert(sizeof(int64_t) * (1 + 2 * DGS_MAX_HOPS) <= WS_ALIGN, "control wor
 // sequences, hash tables -> one word per id, us: 16 seeds [10, 5] over 0.5 M ids 39 -> 28, 2.4 M 39 -> 27, 8 M 40 -> 29,
 // 20 M 37 -> 35, 111 M 37 -> 88; 1 024 seeds [15, 10, 5] over 2.4 M ids 141 -> 92, 8 M 141 -> 90, 20 M 131 -> 111, 111 M
 // 134 -> 214.  With six batches in flight there are six tables, and past the L2 (126 MB) their words come from HBM:
-// 8 M ids 730 -> 684 us, 16 M 711 -> 744.
+// 8 M ids 730 -> 684 us, 16 M 711 -> 744.  (Before their words were kept in the L2 with a hint; with it 8.3 M ids 80 -> 77 a batch.)
+// The hops do not move the line.  A batch through BlockPipeline, hash tables -> one word per id, us, one slot / six: 16 seeds
+// [10, 5] over 0.5 M ids 59 -> 49 / 28 -> 29, 2.4 M 61 -> 49 / 30 -> 29, 8.3 M 59 -> 51 / 28 -> 28; 64 seeds 63 -> 52 / 29 -> 29,
+// 63 -> 52 / 27 -> 28, 62 -> 53 / 28 -> 28; 256 seeds [15, 10, 5] 102 -> 79 / 39 -> 37, 112 -> 86 / 45 -> 38, 100 -> 80 / 39 -> 37 (with
+// six slots about 24 us is the host's share of a batch).
 constexpr int64_t DENSE_MAX_IDS = int64_t(1) << 23;
 constexpr unsigned FILL_CTA_UNITS = 4096;  // 64 KB a CTA of 1 024 threads
 
@@ -221,8 +225,8 @@ int queue_dense(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, con
   return launch_dense_lookup(lookup, ids64, s);
 }
 
-// Queues the whole sequence on `stream`.  id_space > 0: with one word per id below it.  rng_words == nullptr: the keys come from (rng_seed, rng_offset) as
-// launch parameters; otherwise the first kernel reads (seed, offset) from rng_words when it RUNS.
+// Queues the whole sequence on `stream`.  id_space > 0: with one word per id below it.  rng_words == nullptr: the keys come
+// from (rng_seed, rng_offset) as launch parameters; otherwise the first kernel reads (seed, offset) from rng_words when it RUNS.
 int queue_blocks(const dgs_chunk_desc* indptr, const dgs_chunk_desc* indices, const dgs_chunk_desc* probs,
                  const void* seeds, int32_t ids64, const dgs_hop* hops, int32_t n_hops, int32_t replace,
                  int64_t id_space, uint64_t rng_seed, uint64_t rng_offset, const uint64_t* rng_words, void* workspace,
@@ -351,7 +355,7 @@ extern "C" size_t dgs_sample_blocks_dense_workspace_bytes(const dgs_hop* hops, i
 extern "C" int32_t dgs_sample_blocks_dense_wins(const dgs_hop* hops, int32_t n_hops, int64_t id_space) {
   using namespace dgs;
   if (hops == nullptr || n_hops < 1 || n_hops > DGS_MAX_HOPS || id_space < 1 || id_space > COMPACT_KEY_LIMIT) return 0;
-  return id_space <= DENSE_MAX_IDS;
+  return id_space <= DENSE_MAX_IDS;  // whatever the hops: see there
 }
 
 extern "C" const int64_t* dgs_sample_blocks_dense_frontier_count(const dgs_hop* hops, int32_t n_hops, int64_t id_space,

@@ -110,7 +110,9 @@ struct FillJob {
 
 // The words are read and written at random by every launch of a batch while gathered rows stream through the L2: they are
 // marked to be evicted last.  Six batches in flight, 2.4 M words each: 674 -> 662 us a pass, one at a time 146 -> 145;
-// steadily one in, one out 102.5 -> 99.8 us a batch.
+// steadily one in, one out 102.5 -> 99.8 us a batch.  What runs beside them does not lose by it: ten passes over a buffer of
+// 64 MB after each batch, 2.4 M ids, 283 us a batch with hash tables and 261 with these words (8.3 M: 261 and 251); behind the
+// pipeline the same ten passes take 144 us in either case.
 __device__ __forceinline__ uint64_t l2_evict_last_policy() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));

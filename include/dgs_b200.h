@@ -344,7 +344,8 @@ DGS_API void dgs_sample_blocks_recording_free(dgs_blocks_recording* rec);
  * first launch and kept through all its hops) instead of a hash table per hop, so
  * the sampling launch marks what it draws and no launch probes.  Same results, bit
  * for bit.  An id at or beyond id_space raises DGS_ERR_ID_SPACE in *status (which
- * must not be NULL) and the outputs are then not valid: queue the batch again with
+ * must not be NULL; it is there by the time the host sees the last size) and the
+ * outputs are then not valid: queue the batch again with
  * dgs_sample_blocks and the same (rng_seed, rng_offset), which takes any id.
  * _wins: whether this form is the faster one (clearing a word per id of a very
  * large graph costs more than the probes it saves).
